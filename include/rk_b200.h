@@ -184,6 +184,18 @@ int rk_gemm_int_residual(const void* a, const float* sa, const void* b, const fl
                          const void* residual, const void* gate, int64_t tokens, void* out, int64_t m, int64_t n,
                          int64_t kpad, int bits, int tactic, void* workspace, size_t workspace_bytes, void* stream);
 
+/* W4A4 GEMM (the bits = 4 case of rk_gemm_int, or of rk_gemm_int_residual when `residual` is given) that
+ * first widens both packed operands to int8 in caller scratch and then runs the int8 kernels on the
+ * copies.  The result is the same bit for bit; it is the faster form for large products, where
+ * widening every tile again inside the GEMM costs more than writing the copies once.
+ *   scratch: 16-byte aligned, at least (m + n) * kpad bytes, need not be cleared, free again once the work
+ *   queued by the call has run; other arguments as in rk_gemm_int / rk_gemm_int_residual
+ *   (residual and gate may be NULL; tokens is read only with a residual). */
+int rk_gemm_int4_widened(const void* a, const float* sa, const void* b, const float* sb, const void* bias,
+                         const void* residual, const void* gate, int64_t tokens, void* out, int64_t m, int64_t n,
+                         int64_t kpad, int tactic, void* scratch, size_t scratch_bytes, void* workspace,
+                         size_t workspace_bytes, void* stream);
+
 /* Same product, but writes the raw int32 accumulators [m, n] (parity aid; no reference counterpart). */
 int rk_gemm_int_acc(const void* a, const void* b, int32_t* acc, int64_t m, int64_t n, int64_t kpad, int bits,
                     int tactic, void* workspace, size_t workspace_bytes, void* stream);

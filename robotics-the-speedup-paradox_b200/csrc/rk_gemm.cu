@@ -710,31 +710,43 @@ int run_tc(const TcArgs& a) {
   }
 }
 
-// Two's-complement nibbles (low nibble = even k) -> int8, 16 packed bytes per thread.
-__global__ void __launch_bounds__(256) unpack_int4_kernel(const uint4* __restrict__ in, uint4* __restrict__ out,
-                                                          long long vectors) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= vectors) return;
-  const uint4 v = in[i];
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  uint32_t o[8];
+// Two's-complement nibbles (low nibble = even k) -> int8 for both operands of a W4A4 GEMM: 8 packed bytes in,
+// 16 bytes out per thread and step, so that a warp's loads (256 bytes) and stores (512 bytes) are both dense.
+// Bound by L2: the packed weights come from HBM once, the copies stay in L2 for the GEMM that follows
+// (8192 x 2048 weights + 1764 rows: 4.2 us as a dependent launch).
+__global__ void __launch_bounds__(256) widen_int4_kernel(const uint2* __restrict__ a, uint4* __restrict__ a8, long long va,
+                                                         const uint2* __restrict__ b, uint4* __restrict__ b8, long long vb) {
+  pdl_launch_dependents();  // every thread, before any return: see launch_pdl
+  pdl_wait();
+  const long long total = va + vb;
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += 4 * step) {
+    uint2 v[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    // per-byte sign extension of the even and odd nibbles: (u ^ 8) - 8
-    const uint32_t even = __vsub4((w[j] & 0x0F0F0F0Fu) ^ 0x08080808u, 0x08080808u);
-    const uint32_t odd = __vsub4(((w[j] >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u, 0x08080808u);
-    o[2 * j] = __byte_perm(even, odd, 0x5140);      // e0 o0 e1 o1
-    o[2 * j + 1] = __byte_perm(even, odd, 0x7362);  // e2 o2 e3 o3
+    for (int u = 0; u < 4; ++u) {
+      const long long j = i + u * step;
+      v[u] = make_uint2(0u, 0u);
+      if (j < total) v[u] = j < va ? a[j] : b[j - va];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long j = i + u * step;
+      if (j >= total) continue;
+      uint4 o;
+      widen_int4(v[u].x, o.x, o.y);
+      widen_int4(v[u].y, o.z, o.w);
+      if (j < va) a8[j] = o;
+      else b8[j - va] = o;
+    }
   }
-  out[2 * i] = make_uint4(o[0], o[1], o[2], o[3]);
-  out[2 * i + 1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
-int unpack_int4(const void* in, void* out, long long packed_bytes, cudaStream_t st) {
-  const long long vectors = packed_bytes / 16;
-  unpack_int4_kernel<<<static_cast<unsigned>((vectors + 255) / 256), 256, 0, st>>>(
-      static_cast<const uint4*>(in), static_cast<uint4*>(out), vectors);
-  return check_launch("unpack_int4_kernel");
+int widen_int4_operands(const void* a, void* a8, long long a_bytes, const void* b, void* b8, long long b_bytes, cudaStream_t st) {
+  const long long va = a_bytes / 8, vb = b_bytes / 8;
+  const long long blocks = (va + vb + 1023) / 1024;  // four vectors per thread
+  launch_pdl(widen_int4_kernel, dim3(static_cast<unsigned>(blocks < 8 * kNumSms ? blocks : 8 * kNumSms)), dim3(256), st,
+             static_cast<const uint2*>(a), static_cast<uint4*>(a8), va, static_cast<const uint2*>(b), static_cast<uint4*>(b8), vb);
+  return check_launch("widen_int4_kernel");
 }
 
 template <int BN, int UW>
@@ -859,9 +871,7 @@ static int gemm_int_common(const void* a, const float* sa, const void* b, const 
     if (!workspace || workspace_bytes < need) return fail(RK_EWORKSPACE, "%s: workspace too small for the int8 copies", who);
     uint8_t* a8 = static_cast<uint8_t*>(workspace) + need - static_cast<size_t>(round_up(m + n, 16)) * kpad;
     uint8_t* b8 = a8 + static_cast<size_t>(m) * kpad;
-    int rc = unpack_int4(a, a8, m * kpad / 2, as_stream(stream));
-    if (rc != RK_OK) return rc;
-    rc = unpack_int4(b, b8, n * kpad / 2, as_stream(stream));
+    const int rc = widen_int4_operands(a, a8, m * kpad / 2, b, b8, n * kpad / 2, as_stream(stream));
     if (rc != RK_OK) return rc;
     a = a8;
     b = b8;
@@ -919,6 +929,33 @@ extern "C" int rk_gemm_int_residual(const void* a, const float* sa, const void* 
     return fail(RK_EINVAL, "%s: n must be a multiple of 8 and the bf16 pointers 2-byte aligned", who);
   return gemm_int_common(a, sa, b, sb, bias, out, nullptr, m, n, kpad, bits, tactic, workspace, workspace_bytes, stream, who,
                          false, residual, gate, tokens);
+}
+
+extern "C" int rk_gemm_int4_widened(const void* a, const float* sa, const void* b, const float* sb, const void* bias,
+                                    const void* residual, const void* gate, int64_t tokens, void* out, int64_t m, int64_t n,
+                                    int64_t kpad, int tactic, void* scratch, size_t scratch_bytes, void* workspace,
+                                    size_t workspace_bytes, void* stream) {
+  const char* who = "rk_gemm_int4_widened";
+  if (!a || !sa || !b || !sb || !out || !scratch) return fail(RK_EINVAL, "%s: null pointer", who);
+  if (kpad < 128 || kpad % 128 != 0) return fail(RK_EINVAL, "%s: kpad must be a positive multiple of 128", who);
+  if (m < 1 || n < 1 || m > (1 << 24) || n > (1 << 24) || kpad > (1 << 24)) return fail(RK_EINVAL, "%s: bad dimensions", who);
+  if (n % 8 != 0) return fail(RK_EINVAL, "%s: n must be a multiple of 8", who);
+  if (tactic < 0 || tactic > 7) return fail(RK_EINVAL, "%s: tactic must be 0..7", who);
+  if (!aligned16(a) || !aligned16(b) || !aligned16(scratch))
+    return fail(RK_EINVAL, "%s: operands and scratch must be 16-byte aligned", who);
+  if (scratch_bytes < static_cast<size_t>(m + n) * static_cast<size_t>(kpad))
+    return fail(RK_EWORKSPACE, "%s: scratch must hold (m + n) * kpad bytes", who);
+  Workspace ws;
+  int rc = carve_workspace(workspace, workspace_bytes, &ws, who);
+  if (rc != RK_OK) return rc;
+  uint8_t* const a8 = static_cast<uint8_t*>(scratch);
+  uint8_t* const b8 = a8 + static_cast<size_t>(m) * kpad;
+  rc = widen_int4_operands(a, a8, m * kpad / 2, b, b8, n * kpad / 2, as_stream(stream));
+  if (rc != RK_OK) return rc;
+  if (residual != nullptr)
+    return rk_gemm_int_residual(a8, sa, b8, sb, bias, residual, gate, tokens, out, m, n, kpad, 8, tactic, workspace,
+                                workspace_bytes, stream);
+  return gemm_int_common(a8, sa, b8, sb, bias, out, nullptr, m, n, kpad, 8, tactic, workspace, workspace_bytes, stream, who);
 }
 
 extern "C" int rk_gemm_int_acc(const void* a, const void* b, int32_t* acc, int64_t m, int64_t n, int64_t kpad, int bits,

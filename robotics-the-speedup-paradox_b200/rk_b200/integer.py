@@ -108,6 +108,18 @@ def quantize_weight(weight, bits):
     return packed, scales
 
 
+def _widen_first(m, n, kpad):
+    """W4A4: widen both operands to int8 copies once and run the int8 kernels on them, or widen every tile inside the
+    GEMM?  Inside, a 128 x 128 x 128 stage costs about 0.8 us of rewriting and each tile is rewritten for every tile it
+    meets; the copies cost one pass of (m + n) * kpad bytes through L2.  Measured, copies against inside:
+    1764 x 8192 x 2048 28.3 / 90.9 us, 1764 x 2048 x 8192 29.6 / 100.6, 256 x 2048 x 2048 8.3 / 15.7, 50 x 8192 x 2048
+    10.4 / 16.7, 1 x 1024 x 1024 5.8 / 11.5.  Inside stays for few rows with a long K (50 x 1000 x 4096: 12.5 / 11.1), for
+    many rows of a tiny weight (1764 x 256 x 256: 7.6 / 6.3) and where the copies would take over 256 MiB."""
+    if (m + n) * kpad > 1 << 28 or (m > 1024 and n * kpad < 1 << 18):
+        return False
+    return m >= 192 or kpad < 4096
+
+
 def integer_gemm(a, sa, b, sb, bias, bits, tactic, residual=None, gate=None):
     """``robotics_integer::gemm`` call shape (reference: csrc/integer_gemm.cu:130-176).
 
@@ -137,8 +149,16 @@ def integer_gemm(a, sa, b, sb, bias, bits, tactic, residual=None, gate=None):
     elif gate is not None:
         raise RuntimeError("integer GEMM: a gate needs a residual")
     with torch.cuda.device(a.device):
-        ws = _lib.gemm_workspace(_lib.OP_W8A8 if bits == 8 else _lib.OP_W4A4, a.device, m, n, kpad)
-        if residual is None:
+        ws = _lib.workspace(a.device, _lib.WORKSPACE_HEADER)
+        if bits == 4 and _widen_first(m, n, kpad):
+            # per call, from the caching allocator: concurrent streams and captured graphs each have their own
+            scratch = torch.empty((m + n) * kpad, device=a.device, dtype=torch.int8)
+            code = _lib.load().rk_gemm_int4_widened(
+                _lib.ptr(a), _lib.ptr(sa), _lib.ptr(b), _lib.ptr(sb), _lib.ptr(bias), _lib.ptr(residual), _lib.ptr(gate),
+                tokens, _lib.ptr(out), m, n, kpad, tactic, _lib.ptr(scratch), scratch.numel(), _lib.ptr(ws), ws.numel(),
+                _lib.stream_ptr(a.device),
+            )
+        elif residual is None:
             code = _lib.load().rk_gemm_int(
                 _lib.ptr(a), _lib.ptr(sa), _lib.ptr(b), _lib.ptr(sb), _lib.ptr(bias), _lib.ptr(out),
                 m, n, kpad, bits, tactic, _lib.ptr(ws), ws.numel(), _lib.stream_ptr(a.device),

@@ -145,3 +145,35 @@ def test_nvfp4_swiglu_pack_reads_the_interleaved_layout(H):
     assert torch.equal(q0, q1) and torch.equal(sf0, sf1)  # same values, different source layout
     with pytest.raises(ValueError):
         P4.pack_swiglu_nvfp4(H.randn_bf16((4, 2 * 96), 1.0, 72).to(H.DEVICE), 96, interleaved=True)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 128), (3, 24, 384), (64, 1000, 256), (127, 136, 640), (129, 264, 1152),
+                                   (257, 520, 2048), (1025, 264, 384)])
+@pytest.mark.parametrize("form", ["plain", "bias", "residual", "gated"])
+def test_w4a4_widened_copies_match_the_in_kernel_form(m, n, k, form):
+    """Both forms compute the same integers, so the results agree bit for bit; ragged widths of the copies included."""
+    from rk_b200 import _lib
+
+    lib, dev = _lib.load(), torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(m * 7 + n)
+    a = torch.randint(0, 256, (m, k // 2), generator=gen, device=dev, dtype=torch.uint8)
+    b = torch.randint(0, 256, (n, k // 2), generator=gen, device=dev, dtype=torch.uint8)
+    sa, sb = (torch.rand(c, generator=gen, device=dev) * 0.01 + 1e-3 for c in (m, n))
+    bias = torch.randn(n, generator=gen, device=dev).bfloat16() if form == "bias" else None
+    residual = torch.randn(m, n, generator=gen, device=dev).bfloat16() if form in ("residual", "gated") else None
+    gate = torch.randn(m, n, generator=gen, device=dev).bfloat16() if form == "gated" else None
+    want, got = (torch.full((m, n), 7.0, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    ws = _lib.workspace(dev, _lib.WORKSPACE_HEADER)
+    scratch = torch.full(((m + n) * k,), 77, device=dev, dtype=torch.int8)
+    operands = (_lib.ptr(a), _lib.ptr(sa), _lib.ptr(b), _lib.ptr(sb), _lib.ptr(bias))
+    tail = (_lib.ptr(ws), ws.numel(), _lib.stream_ptr(dev))
+    if residual is None:
+        _lib.check(lib.rk_gemm_int(*operands, _lib.ptr(want), m, n, k, 4, 0, *tail), "in-kernel")
+    else:
+        _lib.check(lib.rk_gemm_int_residual(*operands, _lib.ptr(residual), _lib.ptr(gate), 1, _lib.ptr(want), m, n, k, 4, 0,
+                                            *tail), "in-kernel")
+    call = (*operands, _lib.ptr(residual), _lib.ptr(gate), 1, _lib.ptr(got), m, n, k, 0, _lib.ptr(scratch))
+    _lib.check(lib.rk_gemm_int4_widened(*call, scratch.numel(), *tail), "widened")
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert _lib.read_status(ws) == 0
+    assert lib.rk_gemm_int4_widened(*call, scratch.numel() - 1, *tail) == _lib.RK_EWORKSPACE
