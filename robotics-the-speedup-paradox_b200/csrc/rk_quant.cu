@@ -1,6 +1,6 @@
 // Activation / weight quantizers and block-scale packers (HBM-bound, SIMT).
 //
-// Row quantizers: one CTA of 256 threads per row, 128-bit loads, the row cached in registers
+// Row quantizers: one CTA of 64 to 256 threads per row, 128-bit loads, the row cached in registers
 // (8192 elements at most on the cached path), warp-shuffle + shared-memory reductions, and the
 // producer op (GELU table, AdaLN modulation, LayerNorm, RMSNorm, gated residual) fused in front
 // of the absmax so the bf16 intermediate never round-trips through HBM.
@@ -11,6 +11,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp4.h>
 #include <cuda_fp8.h>
+
+#include <type_traits>
 
 #include "rk_blockscale.cuh"
 #include "rk_common.cuh"
@@ -90,24 +92,25 @@ __device__ __forceinline__ void store_codes8(uint8_t* qrow, int idx, const int (
 // round instruction and a float -> int conversion per element (those made the row quantizers
 // instruction-bound: ~31 instructions per element at 17% of DRAM bandwidth).
 //   u = v * rcp, rcp = fl(1 / scale), lies within 3 * 2^-24 * |q| <= 2.3e-5 of the correctly rounded
-//   quotient wherever the result is not clamped anyway (|q| <= 127.5); t = u + 1.5 * 2^23 rounds u to
-//   the nearest integer (ties to even) and leaves that integer in the low mantissa bits, so the low
-//   byte of the clamped t IS the two's-complement code.  Only if some u lies within 4e-5 of a tie (or
-//   is not a number) could the exact quotient round the other way; then all eight take the exact
-//   sequence (about one group of eight in a thousand).
+//   quotient; t = u + 1.5 * 2^23 rounds u to the nearest integer (ties to even) and leaves that
+//   integer in the low mantissa bits, so the low byte (nibble) of t IS the two's-complement code.  No
+//   clamp: `scale` comes from this row's own maximum, so |q| <= limit * (1 + 2^-22).  Only if some u
+//   lies within 4e-5 of a tie (or is not a number, or infinite) could the exact quotient give another
+//   code; then all eight take the exact sequence (about one group of eight in a thousand).
 // Elements at and beyond `k` must already be zero in v.
 template <int BITS>
 __device__ __forceinline__ void quantize_store8(uint8_t* qrow, int idx, const float (&v)[8], float scale, float rcp,
                                                 float limit) {
   const float magic = 12582912.0f;  // 1.5 * 2^23, bits 0x4B400000
-  float t[8];
+  uint32_t t[8];
   bool near_tie = false;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float u = __fmul_rn(v[i], rcp);
-    t[i] = __fadd_rn(u, magic);
-    const float e = __fsub_rn(u, __fsub_rn(t[i], magic));  // exact: distance of u from the integer it rounded to
+    const float r = __fadd_rn(u, magic);
+    const float e = __fsub_rn(u, __fsub_rn(r, magic));  // exact: distance of u from the integer it rounded to
     near_tie |= !(fabsf(e) < 0.49996f);
+    t[i] = __float_as_uint(r);
   }
   if (near_tie) {
     int c[8];
@@ -116,21 +119,16 @@ __device__ __forceinline__ void quantize_store8(uint8_t* qrow, int idx, const fl
     store_codes8<BITS>(qrow, idx, c);
     return;
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) t[i] = fminf(fmaxf(t[i], magic - limit), magic + limit);
+  // low bytes of t gathered four to a word
+  const uint32_t lo = __byte_perm(__byte_perm(t[0], t[1], 0x0040u), __byte_perm(t[2], t[3], 0x0040u), 0x5410u);
+  const uint32_t hi = __byte_perm(__byte_perm(t[4], t[5], 0x0040u), __byte_perm(t[6], t[7], 0x0040u), 0x5410u);
   if constexpr (BITS == 8) {
-    uint32_t b[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) b[i] = __float_as_uint(t[i]);
-    uint2 o;
-    o.x = __byte_perm(__byte_perm(b[0], b[1], 0x0040u), __byte_perm(b[2], b[3], 0x0040u), 0x5410u);
-    o.y = __byte_perm(__byte_perm(b[4], b[5], 0x0040u), __byte_perm(b[6], b[7], 0x0040u), 0x5410u);
-    *reinterpret_cast<uint2*>(qrow + idx) = o;
+    *reinterpret_cast<uint2*>(qrow + idx) = make_uint2(lo, hi);
   } else {
-    int c[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) c[i] = __float_as_int(t[i]) - 0x4B400000;
-    store_codes8<BITS>(qrow, idx, c);
+    // bytes b0 b1 b2 b3 -> (b0 & 15) | (b1 & 15) << 4 | ...: fold the odd byte of each pair onto the even one
+    const uint32_t l = lo & 0x0F0F0F0Fu, h = hi & 0x0F0F0F0Fu;
+    const uint32_t lf = l | (l >> 4), hf = h | (h >> 4);
+    *reinterpret_cast<uint32_t*>(qrow + idx / 2) = __byte_perm(lf, hf, 0x6420u);
   }
 }
 
@@ -140,36 +138,128 @@ __device__ __forceinline__ float row_scale_from_max(float maximum, float limit, 
   return true_division ? __fdiv_rn(maximum, limit) : __fmul_rn(maximum, static_cast<float>(1.0 / limit));
 }
 
-// Common tail: absmax over cached values, scale, quantize, store (zero padding to kpad).
-template <int BITS>
-__device__ __forceinline__ void finish_row(float (&vals)[kMaxVec][8], int k, int kpad, uint8_t* qrow, float* scale_out,
+// ---- rows held as packed bf16 pairs -----------------------------------------------------------------
+// A thread keeps VEC vectors of eight bf16 values as four 32-bit words each.  Products and sums of two
+// bf16 values are taken two at a time in bf16 arithmetic: one rounding of the exact result.  That is
+// what rounding the fp32 result to bf16 gives too - 24 >= 2 * 8 + 2 bits make the second rounding
+// innocuous - except for products below the normal range, where one rounding is the closer one.
+// The row kernels are bound by instructions per element (36 -> about 17 for the modulated norm), not by
+// bytes: see the launch rule below for the figures.
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// running maximum of magnitudes; like fmaxf, a NaN loses against a number
+__device__ __forceinline__ uint32_t absmax_bf16x2(uint32_t m, uint32_t v) {
+  v &= 0x7FFF7FFFu;
+  const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&m), *reinterpret_cast<const __nv_bfloat162*>(&v));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+
+struct Packed8 {
+  uint32_t w[4];
+};
+// The narrow shapes are picked for many rows: 768 resident threads per SM (1764 rows of 64 threads in one wave).
+constexpr int row_min_blocks(int threads, int vecs) { return threads < kRowThreads && threads * vecs >= 256 ? 768 / threads : 1; }
+// eight bf16 values; those at and beyond `valid` read as zero
+__device__ __forceinline__ Packed8 load8p(const __nv_bfloat16* p, bool vec, int valid) {
+  Packed8 r;
+  if (vec && valid >= 8) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    r.w[0] = u.x, r.w[1] = u.y, r.w[2] = u.z, r.w[3] = u.w;
+  } else {
+    const unsigned short* s = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t lo = 2 * i < valid ? s[2 * i] : 0u, hi = 2 * i + 1 < valid ? s[2 * i + 1] : 0u;
+      r.w[i] = lo | (hi << 16);
+    }
+  }
+  return r;
+}
+__device__ __forceinline__ void store8p(__nv_bfloat16* p, bool vec, int valid, const Packed8& v) {
+  if (vec && valid >= 8) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]);
+  } else {
+    unsigned short* s = reinterpret_cast<unsigned short*>(p);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < valid) s[i] = static_cast<unsigned short>(v.w[i >> 1] >> (16 * (i & 1)));
+  }
+}
+__device__ __forceinline__ void unpack8(const Packed8& p, float (&v)[8]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[2 * i] = bf16_lo(p.w[i]), v[2 * i + 1] = bf16_hi(p.w[i]);
+}
+// zeroes the elements at and beyond `valid`
+__device__ __forceinline__ void mask8(Packed8& p, int valid) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (2 * i >= valid) p.w[i] = 0u;
+    else if (2 * i + 1 >= valid) p.w[i] &= 0xFFFFu;
+  }
+}
+
+// Row sum over a CTA of THREADS threads in the summation order of a 256-thread CTA (thread t of that CTA
+// adds its elements, a warp's lanes are added by shuffles, the eight warps in order), so that the number
+// of threads a launch picks never changes a result.  Vector j of thread t is vector j * THREADS + t of the
+// row, i.e. it belongs to accumulator j % (256 / THREADS).  `scratch`: eight words, not reused.
+template <int THREADS>
+__device__ __forceinline__ float row_sum256(float (&acc)[kRowThreads / THREADS], float* scratch) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int r = 0; r < kRowThreads / THREADS; ++r) {
+    const float s = warp_sum(acc[r]);
+    if (lane == 0) scratch[r * (THREADS / 32) + warp] = s;
+  }
+  __syncthreads();
+  float total = scratch[0];
+#pragma unroll
+  for (int w = 1; w < kRowThreads / 32; ++w) total += scratch[w];
+  return total;
+}
+
+// Common tail: absmax over the cached values, scale, quantize, store (zero padding to kpad).  `threads`: the CTA size.
+template <int BITS, int VEC>
+__device__ __forceinline__ void finish_row(Packed8 (&vals)[VEC], int threads, int k, int kpad, uint8_t* qrow, float* scale_out,
                                            bool true_division, float* scratch) {
   const float limit = static_cast<float>((1 << (BITS - 1)) - 1);
-  float local = 0.0f;
+  uint32_t m = 0u;
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it)
+  for (int it = 0; it < VEC; ++it) {
+    const int idx = (it * threads + static_cast<int>(threadIdx.x)) * 8;
+    if (idx + 8 > k) mask8(vals[it], k - idx);  // ragged end of the row: codes beyond k are zero
 #pragma unroll
-    for (int i = 0; i < 8; ++i) local = fmaxf(local, fabsf(vals[it][i]));
-  const float maximum = block_reduce(local, true, scratch);
+    for (int i = 0; i < 4; ++i) m = absmax_bf16x2(m, vals[it].w[i]);
+  }
+  const float local = warp_max(fmaxf(bf16_lo(m), bf16_hi(m)));
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = local;
+  __syncthreads();
+  float maximum = scratch[0];
+  for (int w = 1; w < (threads >> 5); ++w) maximum = fmaxf(maximum, scratch[w]);
   const float scale = row_scale_from_max(maximum, limit, true_division);
   if (threadIdx.x == 0) *scale_out = scale;
   const float rcp = __frcp_rn(scale);
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
-    const int idx = (it * static_cast<int>(blockDim.x) + threadIdx.x) * 8;
+  for (int it = 0; it < VEC; ++it) {
+    const int idx = (it * threads + static_cast<int>(threadIdx.x)) * 8;
     if (idx < kpad) {
-      if (idx + 8 > k) {  // ragged end of the row: codes beyond k are zero
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (idx + i >= k) vals[it][i] = 0.0f;
-      }
-      quantize_store8<BITS>(qrow, idx, vals[it], scale, rcp, limit);
+      float v[8];
+      unpack8(vals[it], v);
+      quantize_store8<BITS>(qrow, idx, v, scale, rcp, limit);
     }
   }
 }
 
 // ------------------------------------------------------------------ plain / GELU-table rows
-template <int BITS, int MODE>
+// VEC vectors of eight elements per thread; rows longer than blockDim.x * VEC vectors (VEC == 4 only) take two passes
+template <int BITS, int MODE, int VEC>
 __global__ void __launch_bounds__(kRowThreads)
 quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const __nv_bfloat16* __restrict__ up,
                   long long up_stride, const __nv_bfloat16* __restrict__ lut, int k, int kpad, int n_rows,
@@ -187,60 +277,57 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const
   }
   const __nv_bfloat16* xr = x + row * x_stride;
   const __nv_bfloat16* ur = MODE == RK_ACT_LUT_MUL ? up + row * up_stride : nullptr;
-  auto values_at = [&](int idx, float (&v)[8]) {
-    const int valid = k - idx;
-    load8(xr + idx, vec_ok, valid, v);
+  const unsigned short* table = reinterpret_cast<const unsigned short*>(lut);
+  auto activate = [&](Packed8& v, const Packed8& u) {
     if constexpr (MODE != RK_ACT_PLAIN) {
-      float u[8];
-      if constexpr (MODE == RK_ACT_LUT_MUL) load8(ur + idx, vec_ok, valid, u);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (i < valid) {
-          const uint32_t bits = __float_as_uint(v[i]) >> 16;
-          float t = __bfloat162float(lut[bits]);
-          if constexpr (MODE == RK_ACT_LUT_MUL) t = round_bf16(__fmul_rn(t, u[i]));
-          v[i] = t;
-        }
+      for (int i = 0; i < 4; ++i) {
+        v.w[i] = static_cast<uint32_t>(table[v.w[i] & 0xFFFFu]) | (static_cast<uint32_t>(table[v.w[i] >> 16]) << 16);
+        if constexpr (MODE == RK_ACT_LUT_MUL) v.w[i] = mul_bf16x2(v.w[i], u.w[i]);
       }
     }
   };
-  const int threads = static_cast<int>(blockDim.x);  // 64, 128 or 256: see launch_quant_rows
-  if (k <= threads * kMaxVec * 8) {
-    float vals[kMaxVec][8];
+  const int threads = static_cast<int>(blockDim.x);  // 64, 128 or 256: see row_threads
+  if (VEC < kMaxVec || k <= threads * VEC * 8) {
+    Packed8 vals[VEC], ups[MODE == RK_ACT_LUT_MUL ? VEC : 1];
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it) {
+    for (int it = 0; it < VEC; ++it) {  // all loads first: they overlap
       const int idx = (it * threads + threadIdx.x) * 8;
-      if (idx < k) {
-        values_at(idx, vals[it]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) vals[it][i] = 0.0f;
-      }
+      vals[it] = load8p(xr + idx, vec_ok, k - idx);
+      if constexpr (MODE == RK_ACT_LUT_MUL) ups[it] = load8p(ur + idx, vec_ok, k - idx);
     }
-    finish_row<BITS>(vals, k, kpad, qrow, scales + row, true_division != 0, scratch);
+#pragma unroll
+    for (int it = 0; it < VEC; ++it) {
+      const int idx = (it * threads + threadIdx.x) * 8;
+      if (MODE != RK_ACT_PLAIN && idx < k) activate(vals[it], ups[MODE == RK_ACT_LUT_MUL ? it : 0]);
+    }
+    finish_row<BITS, VEC>(vals, threads, k, kpad, qrow, scales + row, true_division != 0, scratch);
   } else {
     // long rows: two passes over global memory (the second one hits L2)
+    auto values_at = [&](int idx) {
+      Packed8 v = load8p(xr + idx, vec_ok, k - idx), u{};
+      if constexpr (MODE == RK_ACT_LUT_MUL) u = load8p(ur + idx, vec_ok, k - idx);
+      activate(v, u);
+      if (idx + 8 > k) mask8(v, k - idx);
+      return v;
+    };
     const float limit = static_cast<float>((1 << (BITS - 1)) - 1);
-    float local = 0.0f;
+    uint32_t m = 0u;
     for (int idx = threadIdx.x * 8; idx < k; idx += threads * 8) {
-      float v[8];
-      values_at(idx, v);
+      const Packed8 v = values_at(idx);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) local = fmaxf(local, fabsf(v[i]));
+      for (int i = 0; i < 4; ++i) m = absmax_bf16x2(m, v.w[i]);
     }
-    const float maximum = block_reduce(local, true, scratch);
+    const float maximum = block_reduce(fmaxf(bf16_lo(m), bf16_hi(m)), true, scratch);
     const float scale = row_scale_from_max(maximum, limit, true_division != 0);
     if (threadIdx.x == 0) scales[row] = scale;
     const float rcp = __frcp_rn(scale);
     for (int idx = threadIdx.x * 8; idx < kpad; idx += threads * 8) {
-      float v[8];
-      if (idx < k) {
-        values_at(idx, v);
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (idx + i >= k) v[i] = 0.0f;
-      quantize_store8<BITS>(qrow, idx, v, scale, rcp, limit);
+      Packed8 v{};
+      if (idx < k) v = values_at(idx);
+      float f[8];
+      unpack8(v, f);
+      quantize_store8<BITS>(qrow, idx, f, scale, rcp, limit);
     }
   }
 }
@@ -288,8 +375,9 @@ lut_mul_amax_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, con
 }
 
 // ------------------------------------------------------------------ AdaLN modulation (+LayerNorm, +gated residual)
-template <int BITS>
-__global__ void __launch_bounds__(kRowThreads)
+// The modulation vectors are requested before the statistics are reduced, so that their latency hides behind it.
+template <int BITS, int THREADS, int VEC>
+__global__ void __launch_bounds__(THREADS, row_min_blocks(THREADS, VEC))
 quant_rows_modulated_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ mod_scale,
                             const __nv_bfloat16* __restrict__ mod_shift, int k, int kpad, int tokens, int layer_norm,
                             float eps, const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ gate,
@@ -297,82 +385,92 @@ quant_rows_modulated_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bflo
                             float* __restrict__ scales) {
   pdl_launch_dependents();  // every thread, before any return: see launch_pdl
   pdl_wait();
-  __shared__ float scratch[kRowThreads / 32];
+  constexpr int R = kRowThreads / THREADS;
+  __shared__ float scratch[3][kRowThreads / 32];
   const int row = blockIdx.x;
   const long long xoff = static_cast<long long>(row) * k;
   const long long moff = static_cast<long long>(row / tokens) * k;
   uint8_t* qrow = q + static_cast<long long>(row) * (BITS == 8 ? kpad : kpad / 2);
   const bool vec = (k % 8) == 0;
-  float vals[kMaxVec][8];
-  float sum = 0.0f;
+  Packed8 vals[VEC];
+  if (y != nullptr) {
+    Packed8 yv[VEC], gv[VEC];
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
-    const int idx = (it * kRowThreads + threadIdx.x) * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) vals[it][i] = 0.0f;
-    if (idx < k) {
-      const int valid = k - idx;
-      load8(x + xoff + idx, vec, valid, vals[it]);
-      if (y != nullptr) {
-        float yv[8], gv[8];
-        load8(y + xoff + idx, vec, valid, yv);
-        load8(gate + moff + idx, vec, valid, gv);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          // residual = bf16(x + bf16(y * gate))
-          vals[it][i] = round_bf16(__fadd_rn(vals[it][i], round_bf16(__fmul_rn(yv[i], gv[i]))));
-        }
-        store8(residual_out + xoff + idx, vec, valid, vals[it]);
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) sum += (i < valid) ? vals[it][i] : 0.0f;
+    for (int it = 0; it < VEC; ++it) {
+      const int idx = (it * THREADS + threadIdx.x) * 8;
+      vals[it] = load8p(x + xoff + idx, vec, k - idx);
+      yv[it] = load8p(y + xoff + idx, vec, k - idx);
+      gv[it] = load8p(gate + moff + idx, vec, k - idx);
     }
+#pragma unroll
+    for (int it = 0; it < VEC; ++it) {
+      const int idx = (it * THREADS + threadIdx.x) * 8;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)  // residual = bf16(x + bf16(y * gate))
+        vals[it].w[i] = add_bf16x2(vals[it].w[i], mul_bf16x2(yv[it].w[i], gv[it].w[i]));
+      if (idx < k) store8p(residual_out + xoff + idx, vec, k - idx, vals[it]);
+    }
+  } else {
+#pragma unroll
+    for (int it = 0; it < VEC; ++it) {
+      const int idx = (it * THREADS + threadIdx.x) * 8;
+      vals[it] = load8p(x + xoff + idx, vec, k - idx);
+    }
+  }
+  Packed8 sc[VEC], sh[VEC];
+#pragma unroll
+  for (int it = 0; it < VEC; ++it) {
+    const int idx = (it * THREADS + threadIdx.x) * 8;
+    sc[it] = load8p(mod_scale + moff + idx, vec, k - idx);
+    sh[it] = load8p(mod_shift + moff + idx, vec, k - idx);
   }
   if (layer_norm) {
-    const float mean = __fdiv_rn(block_reduce(sum, false, scratch), static_cast<float>(k));
-    float sq = 0.0f;
+    float acc[R];
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it) {
-      const int idx = (it * kRowThreads + threadIdx.x) * 8;
+    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+#pragma unroll
+    for (int it = 0; it < VEC; ++it) {
+      float v[8];
+      unpack8(vals[it], v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[it % R] += v[i];  // elements beyond k are zero
+    }
+    const float mean = __fdiv_rn(row_sum256<THREADS>(acc, scratch[0]), static_cast<float>(k));
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+#pragma unroll
+    for (int it = 0; it < VEC; ++it) {
+      const int idx = (it * THREADS + threadIdx.x) * 8;
+      float v[8];
+      unpack8(vals[it], v);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float c = (idx + i < k) ? __fsub_rn(vals[it][i], mean) : 0.0f;
-        vals[it][i] = c;
-        sq += c * c;
+        const float c = __fsub_rn(v[i], mean);
+        if (idx + i < k) acc[it % R] = __fmaf_rn(c, c, acc[it % R]);
       }
     }
-    const float var = __fdiv_rn(block_reduce(sq, false, scratch), static_cast<float>(k));
+    const float var = __fdiv_rn(row_sum256<THREADS>(acc, scratch[1]), static_cast<float>(k));
     const float inv = rsqrtf(var + eps);
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it)
+    for (int it = 0; it < VEC; ++it)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) vals[it][i] = round_bf16(__fmul_rn(vals[it][i], inv));
+      for (int i = 0; i < 4; ++i)
+        vals[it].w[i] = pack_bf16x2(__fmul_rn(__fsub_rn(bf16_lo(vals[it].w[i]), mean), inv),
+                                    __fmul_rn(__fsub_rn(bf16_hi(vals[it].w[i]), mean), inv));
   }
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
-    const int idx = (it * kRowThreads + threadIdx.x) * 8;
-    if (idx < k) {
-      const int valid = k - idx;
-      float sc[8], sh[8];
-      load8(mod_scale + moff + idx, vec, valid, sc);
-      load8(mod_shift + moff + idx, vec, valid, sh);
+  for (int it = 0; it < VEC; ++it)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        // bf16(bf16(x * bf16(1 + scale)) + shift)
-        const float factor = round_bf16(__fadd_rn(1.0f, sc[i]));
-        const float product = round_bf16(__fmul_rn(vals[it][i], factor));
-        vals[it][i] = (i < valid) ? round_bf16(__fadd_rn(product, sh[i])) : 0.0f;
-      }
-    }
-  }
-  finish_row<BITS>(vals, k, kpad, qrow, scales + row, false, scratch);
+    for (int i = 0; i < 4; ++i)  // bf16(bf16(x * bf16(1 + scale)) + shift)
+      vals[it].w[i] = add_bf16x2(mul_bf16x2(vals[it].w[i], add_bf16x2(0x3F803F80u, sc[it].w[i])), sh[it].w[i]);
+  finish_row<BITS, VEC>(vals, THREADS, k, kpad, qrow, scales + row, false, scratch[2]);
 }
 
 // ------------------------------------------------------------------ RMSNorm (Gemma) -> quantize
 // n = bf16( fl(fl(s * inv) * fl(1 + a)) + b ), inv = rsqrt(mean(s^2) + eps);
 //   plain:    a = weight[k], b absent;  adaptive: a = scale[row / tokens, k], b = shift[row / tokens, k].
-template <int BITS>
-__global__ void __launch_bounds__(kRowThreads)
+template <int BITS, int THREADS, int VEC>
+__global__ void __launch_bounds__(THREADS, row_min_blocks(THREADS, VEC))
 rmsnorm_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                           const __nv_bfloat16* __restrict__ gate,
                           const __nv_bfloat16* __restrict__ a_ptr, const __nv_bfloat16* __restrict__ b_ptr,
@@ -380,77 +478,102 @@ rmsnorm_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
                           __nv_bfloat16* __restrict__ norm_out, uint8_t* __restrict__ q, float* __restrict__ scales) {
   pdl_launch_dependents();  // every thread, before any return: see launch_pdl
   pdl_wait();
-  __shared__ float scratch[kRowThreads / 32];
+  constexpr int R = kRowThreads / THREADS;
+  __shared__ float scratch[2][kRowThreads / 32];
   const int row = blockIdx.x;
   const long long xoff = static_cast<long long>(row) * k;
   const long long aoff = tokens > 0 ? static_cast<long long>(row / tokens) * k : 0;
   uint8_t* qrow = BITS == 16 ? q : q + static_cast<long long>(row) * (BITS == 8 ? kpad : kpad / 2);
   const bool vec = (k % 8) == 0;
-  float vals[kMaxVec][8];
-  float sq = 0.0f;
+  Packed8 vals[VEC];
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
-    const int idx = (it * kRowThreads + threadIdx.x) * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) vals[it][i] = 0.0f;
-    if (idx < k) {
-      const int valid = k - idx;
-      load8(x + xoff + idx, vec, valid, vals[it]);
-      if (residual != nullptr) {
-        float rv[8];
-        load8(residual + xoff + idx, vec, valid, rv);
-        if (gate != nullptr) {  // gated residual: the branch is scaled per (batch entry, channel) first
-          float gv[8];
-          load8(gate + aoff + idx, vec, valid, gv);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) rv[i] = round_bf16(__fmul_rn(rv[i], gv[i]));
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) vals[it][i] = round_bf16(__fadd_rn(vals[it][i], rv[i]));
-      }
-      if (sum_out != nullptr) store8(sum_out + xoff + idx, vec, valid, vals[it]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (i < valid) sq += vals[it][i] * vals[it][i];
-    }
+  for (int it = 0; it < VEC; ++it) {
+    const int idx = (it * THREADS + threadIdx.x) * 8;
+    vals[it] = load8p(x + xoff + idx, vec, k - idx);
   }
-  const float var = __fdiv_rn(block_reduce(sq, false, scratch), static_cast<float>(k));
-  const float inv = rsqrtf(var + eps);
+  if (residual != nullptr) {
+    Packed8 rv[VEC];
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
-    const int idx = (it * kRowThreads + threadIdx.x) * 8;
-    if (idx < k) {
-      const int valid = k - idx;
-      float av[8], bv[8];
-      load8(a_ptr + aoff + idx, vec, valid, av);
-      if (b_ptr != nullptr) load8(b_ptr + aoff + idx, vec, valid, bv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float t = __fmul_rn(__fmul_rn(vals[it][i], inv), __fadd_rn(1.0f, av[i]));
-        if (b_ptr != nullptr) t = __fadd_rn(t, bv[i]);
-        t = (i < valid) ? round_bf16(t) : 0.0f;
-        vals[it][i] = t;
-      }
-      if (norm_out != nullptr) store8(norm_out + xoff + idx, vec, valid, vals[it]);
+    for (int it = 0; it < VEC; ++it) {
+      const int idx = (it * THREADS + threadIdx.x) * 8;
+      rv[it] = load8p(residual + xoff + idx, vec, k - idx);
     }
+    if (gate != nullptr) {  // gated residual: the branch is scaled per (batch entry, channel) first
+#pragma unroll
+      for (int it = 0; it < VEC; ++it) {
+        const int idx = (it * THREADS + threadIdx.x) * 8;
+        const Packed8 gv = load8p(gate + aoff + idx, vec, k - idx);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rv[it].w[i] = mul_bf16x2(rv[it].w[i], gv.w[i]);
+      }
+    }
+#pragma unroll
+    for (int it = 0; it < VEC; ++it)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) vals[it].w[i] = add_bf16x2(vals[it].w[i], rv[it].w[i]);
+  }
+  Packed8 av[VEC], bv[VEC];
+#pragma unroll
+  for (int it = 0; it < VEC; ++it) {
+    const int idx = (it * THREADS + threadIdx.x) * 8;
+    av[it] = load8p(a_ptr + aoff + idx, vec, k - idx);
+    if (b_ptr != nullptr) bv[it] = load8p(b_ptr + aoff + idx, vec, k - idx);
+  }
+  float acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+#pragma unroll
+  for (int it = 0; it < VEC; ++it) {
+    const int idx = (it * THREADS + threadIdx.x) * 8;
+    if (sum_out != nullptr && idx < k) store8p(sum_out + xoff + idx, vec, k - idx, vals[it]);
+    float v[8];
+    unpack8(vals[it], v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[it % R] = __fmaf_rn(v[i], v[i], acc[it % R]);  // elements beyond k are zero
+  }
+  const float var = __fdiv_rn(row_sum256<THREADS>(acc, scratch[0]), static_cast<float>(k));
+  const float inv = rsqrtf(var + eps);
+  uint32_t m = 0u;
+#pragma unroll
+  for (int it = 0; it < VEC; ++it) {
+    const int idx = (it * THREADS + threadIdx.x) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float t0 = __fmul_rn(__fmul_rn(bf16_lo(vals[it].w[i]), inv), __fadd_rn(1.0f, bf16_lo(av[it].w[i])));
+      float t1 = __fmul_rn(__fmul_rn(bf16_hi(vals[it].w[i]), inv), __fadd_rn(1.0f, bf16_hi(av[it].w[i])));
+      if (b_ptr != nullptr) {
+        t0 = __fadd_rn(t0, bf16_lo(bv[it].w[i]));
+        t1 = __fadd_rn(t1, bf16_hi(bv[it].w[i]));
+      }
+      vals[it].w[i] = pack_bf16x2(t0, t1);
+    }
+    if (idx + 8 > k) mask8(vals[it], k - idx);
+    if (norm_out != nullptr && idx < k) store8p(norm_out + xoff + idx, vec, k - idx, vals[it]);
   }
   if constexpr (BITS == 16) {
     // no row quantizer: the bf16 result is the output (norm_out) and the tensor's absolute maximum
     // (finite values only) is collected for a per-tensor scale; `q` is that staging word, or null
     if (q != nullptr) {
-      float local = 0.0f;
 #pragma unroll
-      for (int it = 0; it < kMaxVec; ++it)
+      for (int it = 0; it < VEC; ++it)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float a = fabsf(vals[it][i]);
-          if (a <= 3.4028234664e38f) local = fmaxf(local, a);
+        for (int i = 0; i < 4; ++i) {
+          // magnitudes order like their bit patterns; infinities and NaN count as zero
+          const uint32_t lo = vals[it].w[i] & 0x7FFFu, hi = (vals[it].w[i] >> 16) & 0x7FFFu;
+          m = max(m, lo < 0x7F80u ? lo : 0u);
+          m = max(m, hi < 0x7F80u ? hi : 0u);
         }
-      const float row_max = block_reduce(local, true, scratch);
-      if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned*>(q), __float_as_uint(row_max));
+      m = __reduce_max_sync(0xffffffffu, m);
+      if ((threadIdx.x & 31) == 0) scratch[1][threadIdx.x >> 5] = __uint_as_float(m << 16);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        float row_max = scratch[1][0];
+        for (int w = 1; w < THREADS / 32; ++w) row_max = fmaxf(row_max, scratch[1][w]);
+        atomicMax(reinterpret_cast<unsigned*>(q), __float_as_uint(row_max));
+      }
     }
   } else {
-    finish_row<BITS>(vals, k, kpad, qrow, scales + row, false, scratch);
+    finish_row<BITS, VEC>(vals, THREADS, k, kpad, qrow, scales + row, false, scratch[1]);
   }
 }
 
@@ -1013,6 +1136,40 @@ rmsnorm_producer_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 
 __global__ void probe_rcp_kernel(uint32_t* out) { *out = __float_as_uint(rcp_approx_ftz(448.0f)); }
 
+// Threads per row of the row kernels: as many as the row has vectors of eight (64 to 256), halved further (at most four
+// vectors per thread) while the rows would need more than one wave of resident threads (1536 per SM with one vector
+// each, about 1024 with more).  With few rows the latency of a thread decides; with many, fewer warps per row mean
+// fewer barriers and more rows in flight.  Against 256 threads for every row, four vectors each (most of them masked)
+// and fp32 arithmetic per element - LayerNorm + modulation + gated residual to int8: 50 x 1024 4.3 -> 2.4 us, 816 x 2048
+// 11.7 -> 5.0, 1764 x 2048 21.9 -> 9.0 (2.8 TB/s), 16384 x 2048 234 -> 74; adaptive RMSNorm: 50 x 1024 3.6 -> 2.3,
+// 400 x 1024 4.4 -> 3.4, 1764 x 2048 13.9 -> 8.6; add + RMSNorm + tensor maximum: 816 x 2048 6.4 -> 3.9; plain rows:
+// 50 x 4096 2.9 -> 2.5, 1764 x 8192 15.2 -> 12.5.  One wave against two: 816 x 2048 5.0 us with 256 threads, 5.7 with 128;
+// threads without a vector: 400 x 1024 3.9 us with 256 threads, 3.5 with 128.
+int row_threads(int64_t rows, int64_t kpad) {
+  int threads = kRowThreads;
+  while (threads > 64 && threads * 4 >= kpad) threads /= 2;
+  while (threads > 64 && rows * threads > 148 * (kpad <= threads * 8 ? 1536 : 1024) && (threads / 2) * kMaxVec * 8 >= kpad)
+    threads /= 2;
+  return threads;
+}
+// vectors of eight per thread: 1, 2 or 4 (longer rows loop in the kernels that take them)
+int row_vectors(int threads, int64_t kpad) { return kpad <= threads * 8 ? 1 : (kpad <= threads * 16 ? 2 : 4); }
+
+// Calls `f` with the (threads, vectors) pair of the rule above as compile-time constants; kpad <= kCachedK.
+template <typename F>
+void with_row_shape(int64_t rows, int64_t kpad, F&& f) {
+  const int threads = row_threads(rows, kpad), vecs = row_vectors(threads, kpad);
+  using std::integral_constant;
+  auto pick = [&](auto t) {
+    if (vecs == 1) f(t, integral_constant<int, 1>{});
+    else if (vecs == 2) f(t, integral_constant<int, 2>{});
+    else f(t, integral_constant<int, 4>{});
+  };
+  if (threads == 64) pick(integral_constant<int, 64>{});
+  else if (threads == 128) pick(integral_constant<int, 128>{});
+  else pick(integral_constant<int, 256>{});
+}
+
 template <int BITS>
 int launch_quant_rows(const void* x, int64_t rows, int64_t total_rows, int64_t k, int64_t xs, const void* up,
                       int64_t us, const void* lut, int mode, void* q, float* scales, int true_division,
@@ -1024,28 +1181,22 @@ int launch_quant_rows(const void* x, int64_t rows, int64_t total_rows, int64_t k
   auto lb = static_cast<const __nv_bfloat16*>(lut);
   auto qb = static_cast<uint8_t*>(q);
   const dim3 grid(static_cast<unsigned>(total_rows));
-  // One CTA per row.  With 256 threads a short row is one 16-byte load per thread and eight warps
-  // to reduce over; once there are enough rows to give every SM several CTAs, 64 or 128 threads per
-  // row (four vectors per thread, two or four warps to reduce, up to 32 resident CTAs per SM) are
-  // faster (1764 x 2048: 8.3 -> 6.8 us; 16384 x 2048: 64.5 -> 37.8 us).  With few rows the machine
-  // is not full and the per-thread latency decides, so those keep the full 256 threads
-  // (400 x 4096: 4.5 us with 256 threads, 9.5 us with 64).
-  int threads = kRowThreads;
-  if (total_rows >= 1024) threads = kpad <= 2048 ? 64 : (kpad <= 4096 ? 128 : kRowThreads);
+  const int threads = row_threads(total_rows, kpad);
+  const int vecs = row_vectors(threads, kpad);
+  auto launch = [&](auto kernel) {
+    launch_pdl(kernel, grid, threads, st, xb, xs, ub, us, lb, static_cast<int>(k), kpad, static_cast<int>(rows), qb, scales,
+               true_division, vec_ok);
+  };
+  auto by_vectors = [&](auto mode_c) {
+    constexpr int kMode = decltype(mode_c)::value;
+    if (vecs == 1) launch(quant_rows_kernel<BITS, kMode, 1>);
+    else if (vecs == 2) launch(quant_rows_kernel<BITS, kMode, 2>);
+    else launch(quant_rows_kernel<BITS, kMode, 4>);
+  };
   switch (mode) {
-    case RK_ACT_PLAIN:
-      launch_pdl(quant_rows_kernel<BITS, RK_ACT_PLAIN>, grid, threads, st, xb, xs, ub, us, lb, static_cast<int>(k), kpad,
-                                                                          static_cast<int>(rows), qb, scales,
-                                                                          true_division, vec_ok);
-      break;
-    case RK_ACT_LUT_MUL:
-      launch_pdl(quant_rows_kernel<BITS, RK_ACT_LUT_MUL>, grid, threads, st, 
-          xb, xs, ub, us, lb, static_cast<int>(k), kpad, static_cast<int>(rows), qb, scales, true_division, vec_ok);
-      break;
-    default:
-      launch_pdl(quant_rows_kernel<BITS, RK_ACT_LUT>, grid, threads, st, xb, xs, ub, us, lb, static_cast<int>(k), kpad,
-                                                                        static_cast<int>(rows), qb, scales,
-                                                                        true_division, vec_ok);
+    case RK_ACT_PLAIN: by_vectors(std::integral_constant<int, RK_ACT_PLAIN>{}); break;
+    case RK_ACT_LUT_MUL: by_vectors(std::integral_constant<int, RK_ACT_LUT_MUL>{}); break;
+    default: by_vectors(std::integral_constant<int, RK_ACT_LUT>{});
   }
   return check_launch("quant_rows");
 }
@@ -1105,14 +1256,16 @@ extern "C" int rk_quant_rows_modulated(const void* x, const void* scale, const v
     return fail(RK_EINVAL, "rk_quant_rows_modulated: pointers must be 16-byte aligned");
   const int kpad = static_cast<int>(round_up(k, 128));
   auto b = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
-  if (bits == 8)
-    launch_pdl(quant_rows_modulated_kernel<8>, static_cast<unsigned>(rows), kRowThreads, as_stream(stream), 
-        b(x), b(scale), b(shift), static_cast<int>(k), kpad, static_cast<int>(tokens), layer_norm, eps, b(y), b(gate),
-        static_cast<__nv_bfloat16*>(residual_out), static_cast<uint8_t*>(q), scales);
-  else
-    launch_pdl(quant_rows_modulated_kernel<4>, static_cast<unsigned>(rows), kRowThreads, as_stream(stream), 
-        b(x), b(scale), b(shift), static_cast<int>(k), kpad, static_cast<int>(tokens), layer_norm, eps, b(y), b(gate),
-        static_cast<__nv_bfloat16*>(residual_out), static_cast<uint8_t*>(q), scales);
+  auto launch = [&](auto kernel, int threads) {
+    launch_pdl(kernel, static_cast<unsigned>(rows), threads, as_stream(stream), b(x), b(scale), b(shift), static_cast<int>(k),
+               kpad, static_cast<int>(tokens), layer_norm, eps, b(y), b(gate), static_cast<__nv_bfloat16*>(residual_out),
+               static_cast<uint8_t*>(q), scales);
+  };
+  with_row_shape(rows, kpad, [&](auto t, auto v) {
+    constexpr int kT = decltype(t)::value, kV = decltype(v)::value;
+    if (bits == 8) launch(quant_rows_modulated_kernel<8, kT, kV>, kT);
+    else launch(quant_rows_modulated_kernel<4, kT, kV>, kT);
+  });
   return check_launch("quant_rows_modulated");
 }
 
@@ -1131,14 +1284,16 @@ int launch_rmsnorm_quant_rows(const char* who, const void* x, const void* residu
     return fail(RK_EINVAL, "%s: pointers must be 16-byte aligned", who);
   const int kpad = static_cast<int>(round_up(k, 128));
   auto b = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
-  if (bits == 8)
-    launch_pdl(rmsnorm_quant_rows_kernel<8>, static_cast<unsigned>(rows), kRowThreads, as_stream(stream), 
-        b(x), b(residual), b(gate), b(scale), b(shift), static_cast<int>(tokens), static_cast<int>(k), kpad, eps,
-        static_cast<__nv_bfloat16*>(sum_out), static_cast<__nv_bfloat16*>(norm_out), static_cast<uint8_t*>(q), scales);
-  else
-    launch_pdl(rmsnorm_quant_rows_kernel<4>, static_cast<unsigned>(rows), kRowThreads, as_stream(stream), 
-        b(x), b(residual), b(gate), b(scale), b(shift), static_cast<int>(tokens), static_cast<int>(k), kpad, eps,
-        static_cast<__nv_bfloat16*>(sum_out), static_cast<__nv_bfloat16*>(norm_out), static_cast<uint8_t*>(q), scales);
+  auto launch = [&](auto kernel, int threads) {
+    launch_pdl(kernel, static_cast<unsigned>(rows), threads, as_stream(stream), b(x), b(residual), b(gate), b(scale), b(shift),
+               static_cast<int>(tokens), static_cast<int>(k), kpad, eps, static_cast<__nv_bfloat16*>(sum_out),
+               static_cast<__nv_bfloat16*>(norm_out), static_cast<uint8_t*>(q), scales);
+  };
+  with_row_shape(rows, kpad, [&](auto t, auto v) {
+    constexpr int kT = decltype(t)::value, kV = decltype(v)::value;
+    if (bits == 8) launch(rmsnorm_quant_rows_kernel<8, kT, kV>, kT);
+    else launch(rmsnorm_quant_rows_kernel<4, kT, kV>, kT);
+  });
   return check_launch(who);
 }
 }  // namespace
@@ -1178,9 +1333,13 @@ extern "C" int rk_rmsnorm_tensor_scale(const void* x, const void* residual, cons
     staging = reinterpret_cast<unsigned*>(static_cast<uint8_t*>(workspace) + 64);  // zero between calls
   }
   auto b = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
-  launch_pdl(rmsnorm_quant_rows_kernel<16>, static_cast<unsigned>(rows), kRowThreads, as_stream(stream), 
-      b(x), b(residual), nullptr, b(scale), b(shift), static_cast<int>(tokens), static_cast<int>(k), 0, eps,
-      static_cast<__nv_bfloat16*>(sum_out), static_cast<__nv_bfloat16*>(norm_out), reinterpret_cast<uint8_t*>(staging), nullptr);
+  with_row_shape(rows, k, [&](auto t, auto v) {
+    constexpr int kT = decltype(t)::value, kV = decltype(v)::value;
+    launch_pdl(rmsnorm_quant_rows_kernel<16, kT, kV>, static_cast<unsigned>(rows), kT, as_stream(stream), b(x), b(residual),
+               nullptr, b(scale), b(shift), static_cast<int>(tokens), static_cast<int>(k), 0, eps,
+               static_cast<__nv_bfloat16*>(sum_out), static_cast<__nv_bfloat16*>(norm_out), reinterpret_cast<uint8_t*>(staging),
+               nullptr);
+  });
   if (staging != nullptr) launch_pdl(finalize_scale_kernel, 1, 1, as_stream(stream), staging, divisor, scale_out);
   return check_launch(who);
 }

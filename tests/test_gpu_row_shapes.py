@@ -1,0 +1,61 @@
+"""The row kernels pick threads and vectors per row by the number of rows and their length.  The choice must never show in
+a result: rows of a tall matrix (64 threads each) equal the same rows quantized alone (256 threads), bit for bit.  The small
+launches are held to the oracle by the other tests."""
+
+import numpy as np
+import pytest
+import torch
+
+from rk_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+TALL, FEW = 2400, 48  # multiples of the 48 rows that share one modulation vector
+
+
+def _randn(gen, *shape, std=1.0):
+    return (torch.randn(*shape, generator=gen, device="cuda") * std).bfloat16()
+
+
+def _bits(tensors):
+    return [t[:FEW].contiguous().view(torch.uint8) for t in tensors]
+
+
+@pytest.mark.parametrize("k", [8, 250, 333, 512, 1000, 1032, 2048, 2056, 4096, 4100, 8192])
+@pytest.mark.parametrize("bits", [8, 4])
+def test_the_shape_of_a_launch_never_changes_a_row(k, bits):
+    lib, dev, ptr = _lib.load(), torch.device("cuda:0"), _lib.ptr
+    gen = torch.Generator(device=dev).manual_seed(k)
+    x, y = _randn(gen, TALL, k), _randn(gen, TALL, k)
+    scale, shift, gate = (_randn(gen, TALL // 48, k, std=0.1) for _ in range(3))
+    x[1] = 0.0
+    x[2, 0], x[3, 0], x[4, 0] = float("inf"), float("nan"), 3e38
+    table = torch.nn.functional.gelu(torch.arange(65536, device=dev, dtype=torch.int32).to(torch.int16).view(torch.bfloat16))
+    ws = torch.zeros(_lib.WORKSPACE_HEADER, device=dev, dtype=torch.uint8)
+    width = (k + 127) // 128 * 128 * bits // 8
+
+    def run(rows):
+        q, s = torch.zeros(rows, width, device=dev, dtype=torch.uint8), torch.zeros(rows, device=dev)
+        stream, results = _lib.stream_ptr(dev), []
+        for mode in (_lib.ACT_PLAIN, _lib.ACT_LUT_MUL, _lib.ACT_LUT):
+            _lib.check(lib.rk_quant_rows(ptr(x), rows, k, k, ptr(y), k, ptr(table), mode, bits, ptr(q), ptr(s), stream), "rows")
+            results += [q.clone(), s.clone()]
+        for norm in (0, 1):
+            res = torch.zeros(rows, k, device=dev, dtype=torch.bfloat16)
+            _lib.check(lib.rk_quant_rows_modulated(ptr(x), ptr(scale), ptr(shift), rows, k, 48, norm, 1e-6, ptr(y), ptr(gate),
+                                                   ptr(res), bits, ptr(q), ptr(s), stream), "modulated")
+            results += [q.clone(), s.clone(), res]
+        res, normed = (torch.zeros(rows, k, device=dev, dtype=torch.bfloat16) for _ in range(2))
+        _lib.check(lib.rk_gated_rmsnorm_quant_rows(ptr(x), ptr(y), ptr(gate), ptr(scale), ptr(shift), 48, rows, k, 1e-6, bits,
+                                                   ptr(res), ptr(normed), ptr(q), ptr(s), stream), "rmsnorm")
+        results += [q.clone(), s.clone(), res, normed]
+        if bits == 8:
+            res, normed, one = torch.zeros_like(res), torch.zeros_like(normed), torch.zeros(1, device=dev)
+            _lib.check(lib.rk_rmsnorm_tensor_scale(ptr(x), ptr(y), ptr(scale), None, 0, rows, k, 1e-6, 2688.0, ptr(res),
+                                                   ptr(normed), ptr(one), ptr(ws), ws.numel(), stream), "tensor scale")
+            finite = normed.float()[torch.isfinite(normed)].abs().max().item()
+            assert one.item() == max(np.float32(finite) / np.float32(2688.0), np.float32(1e-12))  # the IEEE quotient
+            results += [res, normed]
+        return results
+
+    for tall, few in zip(_bits(run(TALL)), _bits(run(FEW))):
+        assert torch.equal(tall, few)
