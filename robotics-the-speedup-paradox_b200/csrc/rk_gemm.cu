@@ -749,7 +749,7 @@ int widen_int4_operands(const void* a, void* a8, long long a_bytes, const void* 
   return check_launch("widen_int4_kernel");
 }
 
-template <int BN, int UW>
+template <int BN, int UW, bool SPLIT>
 int launch_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_s, const CUtensorMap& tm_o,
               const W4Params& p, int tiles_n, int tiles_m, int smem, cudaStream_t st) {
   static bool configured_dev[64] = {};
@@ -757,22 +757,26 @@ int launch_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMa
   cudaGetDevice(&dev);
   bool& configured = configured_dev[dev & 63];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(rk_gemm_w4a16_kernel<BN, UW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rk_gemm_w4a16_kernel<BN, UW, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBudget + 1024);
     if (e != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(tiles_n, tiles_m, 1);
+  cfg.gridDim = dim3(tiles_n, tiles_m, p.splits);
   cfg.blockDim = dim3(w4_threads(UW));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = p.splits;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_w4a16_kernel<BN, UW>, tm_w, tm_x, tm_s, tm_o, p);
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_w4a16_kernel<BN, UW, SPLIT>, tm_w, tm_x, tm_s, tm_o, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(RK_ECUDA, "rk_gemm_w4a16_kernel launch: %s", cudaGetErrorString(e));
@@ -1208,7 +1212,7 @@ extern "C" int rk_gemm_mxfp8_swiglu(const void* a, const void* sfa, const void* 
   return run_tc(t);
 }
 
-template <int BN>
+template <int BN, bool SPLIT>
 int launch_w4_fold(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_s, const CUtensorMap& tm_o,
                    const W4Params& p, int tiles_n, int tiles_m, int smem, cudaStream_t st) {
   static bool configured_dev[64] = {};
@@ -1216,22 +1220,26 @@ int launch_w4_fold(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUten
   cudaGetDevice(&dev);
   bool& configured = configured_dev[dev & 63];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(rk_gemm_w4a16_fold_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rk_gemm_w4a16_fold_kernel<BN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBudget + 1024);
     if (e != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(tiles_n, tiles_m, 1);
+  cfg.gridDim = dim3(tiles_n, tiles_m, p.splits);
   cfg.blockDim = dim3(kW4fThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = p.splits;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_w4a16_fold_kernel<BN>, tm_w, tm_x, tm_s, tm_o, p);
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_w4a16_fold_kernel<BN, SPLIT>, tm_w, tm_x, tm_s, tm_o, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(RK_ECUDA, "rk_gemm_w4a16_fold_kernel launch: %s", cudaGetErrorString(e));
@@ -1274,9 +1282,56 @@ int launch_w4_fold2(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUte
   return RK_OK;
 }
 
+// How many clusters of `size` CTAs with a whole SM each the current device runs at once.  A cluster lives inside one
+// GPC, so this is less than SMs / size; one cluster too many doubles the time of a launch.
+int max_clusters(int size) {
+  static std::mutex mu;
+  static int known[64][9] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  int& entry = known[dev & 63][size];
+  if (entry == 0) {
+    auto kernel = rk_gemm_w4a16_fold_kernel<256, true>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 1024);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1, 1, size);
+    cfg.blockDim = dim3(kW4fThreads);
+    cfg.dynamicSmemBytes = kSmemBudget;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = size;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = kNumSms / (2 * size);
+    }
+    entry = n;
+  }
+  return entry;
+}
+
+// K slices per output tile.  A launch of few tiles leaves most SMs idle for a K loop of up to 128 groups, so a cluster
+// of CTAs takes a tile: the largest one (at most eight) that all run at once, with at least two group pairs each.
+// The partial sums meet in distributed shared memory (+1 us); short loops stay whole.  Measured, whole against the rule's
+// choice: 50 x 2048 x 16384 58.2 -> 15.4 us (six slices), 50 x 2048 x 2048 10.5 -> 6.7 (four), 128 x 1536 x 8192 45.8 -> 12.0
+// (eight), 256 x 2048 x 16384 90.7 -> 25.3, 50 x 4096 x 4096 17.7 -> 9.3; 50 x 2048 x 640 5.5 whole, 5.9 in two.
+int w4_splits(int tiles, int pairs) {
+  if (pairs < 6) return 1;
+  for (int s = pairs / 2 < 8 ? pairs / 2 : 8; s > 1; --s)
+    if (tiles * s <= kNumSms && tiles <= max_clusters(s)) return s;
+  return 1;
+}
+// the scale rows of the largest slice: what one scale copy brings
+int w4_scale_rows(int pairs, int splits) { return 2 * ((pairs + splits - 1) / splits); }
+
 // Activation batches above 64 rows: scale folded into the expanded weights, one accumulator for all of K.
 int run_w4_fold(const void* x, const void* q, const void* scales, W4Params p, int64_t m, int64_t n, int64_t k,
-                int scales_bytes, int tactic, cudaStream_t st, const char* who) {
+                int tactic, cudaStream_t st, const char* who) {
   const int bn = m > 128 ? 256 : 128;
   const int tiles_n = static_cast<int>((n + 127) / 128);
   const int tiles_m = static_cast<int>((m + bn - 1) / bn);
@@ -1285,16 +1340,21 @@ int run_w4_fold(const void* x, const void* q, const void* scales, W4Params p, in
   const bool pair = bn == 256 && tiles_n % 2 == 0 && (tactic & 8);
   const int x_bytes = pair ? kW4f2XBytes : bn * 128;
   const int slots = pair ? kW4f2Slots : w4f_slots(bn);
-  const int copies = (p.groups + 1) / 2;
+  const int pairs = (p.groups + 1) / 2;
+  p.splits = pair ? 1 : w4_splits(tiles_n * tiles_m, pairs);
+  p.scale_rows = pair ? p.groups : w4_scale_rows(pairs, p.splits);
+  const int copies = (pairs + p.splits - 1) / p.splits;
+  const int scales_bytes = static_cast<int>(round_up(p.scale_rows * 256, 1024));  // [scale_rows][128] bf16 in shared memory
   int w_stages = (kSmemBudget - scales_bytes - slots * x_bytes) / kW4PairBytes;
   if (w_stages > kW4MaxW) w_stages = kW4MaxW;
   if (w_stages > copies) w_stages = copies;
-  if (w_stages < 1) return fail(RK_EUNSUPPORTED, "%s: shared memory budget exceeded", who);
+  // the longest K is the one whose scales fit unsplit, however the slices fall
+  if (kSmemBudget - static_cast<int>(round_up(p.groups * 256, 1024)) - slots * x_bytes < kW4PairBytes)
+    return fail(RK_EUNSUPPORTED, "%s: shared memory budget exceeded", who);
   p.w_stages = w_stages;
   const int smem = slots * x_bytes + w_stages * kW4PairBytes + scales_bytes + 1024;
   CUtensorMap tm_w, tm_x, tm_s, tm_o;
-  const uint32_t group_box = static_cast<uint32_t>(p.groups < 256 ? p.groups : 256);
-  int rc = make_map_2d(&tm_s, scales, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, n, k / 128, n * 2, 128, group_box,
+  int rc = make_map_2d(&tm_s, scales, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, n, k / 128, n * 2, 128, p.scale_rows,
                        CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc != RK_OK) return rc;
   rc = make_map_2d(&tm_w, q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k / 2, n, k / 2, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -1306,8 +1366,11 @@ int run_w4_fold(const void* x, const void* q, const void* scales, W4Params p, in
   rc = make_map_2d(&tm_o, p.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, n, m, n * 2, 128, 32, CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc != RK_OK) return rc;
   if (pair) return launch_w4_fold2(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
-  return bn == 256 ? launch_w4_fold<256>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st)
-                   : launch_w4_fold<128>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+  if (p.splits > 1)
+    return bn == 256 ? launch_w4_fold<256, true>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st)
+                     : launch_w4_fold<128, true>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+  return bn == 256 ? launch_w4_fold<256, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st)
+                   : launch_w4_fold<128, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
 }
 
 extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scales, const void* bias, void* out,
@@ -1334,8 +1397,7 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
   p.m = static_cast<int>(m);
   p.n = static_cast<int>(n);
   p.groups = static_cast<int>(k / 128);
-  const int scales_bytes = static_cast<int>(round_up((k / 128) * 256, 1024));  // [groups][128] bf16 in shared memory
-  if (scales_bytes > 64 * 1024) return fail(RK_EUNSUPPORTED, "%s: k > 32768", who);
+  if (k > 32768) return fail(RK_EUNSUPPORTED, "%s: k > 32768", who);
   if (!aligned16(scales)) return fail(RK_EINVAL, "%s: scales must be 16-byte aligned", who);
   const int64_t gemv_slabs = k / kGemvSlab;
   const bool gemv_shape = k % kGemvSlab == 0 && (gemv_slabs == 1 || gemv_slabs == 2 || gemv_slabs == 4 || gemv_slabs % 8 == 0);
@@ -1374,17 +1436,23 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
     p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.out = static_cast<__nv_bfloat16*>(out);
     p.status = ws.status;
-    return run_w4_fold(x, q, scales, p, m, n, k, scales_bytes, tactic, as_stream(stream), who);
+    return run_w4_fold(x, q, scales, p, m, n, k, tactic, as_stream(stream), who);
   }
   // shared memory: the activation tiles of the slot ring first, the rest goes to the raw-weight
   // ring (group pairs of 16 KB), whose depth is what keeps enough HBM requests in flight
   const int x_bytes = 2 * bn * 128;
   const int slots = w4_slots(bn);
   const int pairs = (p.groups + 1) / 2;
+  p.splits = (tactic & 1) || bn == 128 ? 1 : w4_splits(tiles_n * tiles_m, pairs);
+  p.scale_rows = w4_scale_rows(pairs, p.splits);
+  const int copies = (pairs + p.splits - 1) / p.splits;
+  const int scales_bytes = static_cast<int>(round_up(p.scale_rows * 256, 1024));  // [scale_rows][128] bf16 in shared memory
   int w_stages = (kSmemBudget - scales_bytes - slots * x_bytes) / kW4PairBytes;
   if (w_stages > kW4MaxW) w_stages = kW4MaxW;
-  if (w_stages > pairs) w_stages = pairs;
-  if (w_stages < 1) return fail(RK_EUNSUPPORTED, "%s: shared memory budget exceeded", who);
+  if (w_stages > copies) w_stages = copies;
+  // the longest K is the one whose scales fit unsplit, however the slices fall
+  if (kSmemBudget - static_cast<int>(round_up(p.groups * 256, 1024)) - slots * x_bytes < kW4PairBytes)
+    return fail(RK_EUNSUPPORTED, "%s: shared memory budget exceeded", who);
   p.w_stages = w_stages;
   p.ldo = n;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
@@ -1393,8 +1461,7 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
   const int smem = slots * x_bytes + w_stages * kW4PairBytes + scales_bytes + 1024;
   if (!aligned16(scales)) return fail(RK_EINVAL, "%s: scales must be 16-byte aligned", who);
   CUtensorMap tm_w, tm_x, tm_s;
-  const uint32_t group_box = static_cast<uint32_t>(p.groups < 256 ? p.groups : 256);
-  rc = make_map_2d(&tm_s, scales, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, n, k / 128, n * 2, 128, group_box,
+  rc = make_map_2d(&tm_s, scales, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, n, k / 128, n * 2, 128, p.scale_rows,
                    CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc != RK_OK) return rc;
   // raw weights: 128 bytes (two K groups) of 128 rows per copy
@@ -1412,9 +1479,9 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
   cudaStream_t st = as_stream(stream);
   if (tactic & 1) {  // four unpack warps instead of eight
     switch (bn) {
-      case 16: return launch_w4<16, 4>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
-      case 32: return launch_w4<32, 4>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
-      case 64: return launch_w4<64, 4>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+      case 16: return launch_w4<16, 4, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+      case 32: return launch_w4<32, 4, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+      case 64: return launch_w4<64, 4, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
       default: break;
     }
   }
@@ -1422,19 +1489,28 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
   // the K loop; the register file allows them for activation tiles of up to 32 rows.  Chosen by
   // default for K <= 4096 (the ramp is a smaller share of longer loops, which run a little faster
   // with eight); tactic bit 4 forces sixteen, bit 5 forces eight.
-  const bool sixteen = (tactic & 16) || (!(tactic & 32) && p.groups <= 32);
+  const bool sixteen = (tactic & 16) || (!(tactic & 32) && 2 * copies <= 32);
+  if (p.splits > 1) {
+    if (sixteen && bn == 16) return launch_w4<16, 16, true>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+    if (sixteen && bn == 32) return launch_w4<32, 16, true>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+    switch (bn) {
+      case 16: return launch_w4<16, 8, true>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+      case 32: return launch_w4<32, 8, true>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+      default: return launch_w4<64, 8, true>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+    }
+  }
   if (sixteen) {
     switch (bn) {
-      case 16: return launch_w4<16, 16>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
-      case 32: return launch_w4<32, 16>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+      case 16: return launch_w4<16, 16, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+      case 32: return launch_w4<32, 16, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
       default: break;
     }
   }
   switch (bn) {
-    case 16: return launch_w4<16, 8>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
-    case 32: return launch_w4<32, 8>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
-    case 64: return launch_w4<64, 8>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
-    default: return launch_w4<128, 4>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+    case 16: return launch_w4<16, 8, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+    case 32: return launch_w4<32, 8, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+    case 64: return launch_w4<64, 8, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
+    default: return launch_w4<128, 4, false>(tm_w, tm_x, tm_s, tm_o, p, tiles_n, tiles_m, smem, st);
   }
 }
 

@@ -40,11 +40,70 @@ constexpr int kW4MaxSlots = 6;               // slot ring depth limit
 struct W4Params {
   int m, n, groups;  // activation rows, weight rows, K / 128
   int w_stages;      // raw-weight ring depth, in group pairs
+  int splits;        // CTAs of a cluster (along z) that share an output tile, each with a slice of K's group pairs
+  int scale_rows;    // group rows of one scale copy: the largest slice
   long long ldo;
   const __nv_bfloat16* bias;    // [n] or null
   __nv_bfloat16* out;           // [m, ldo]
   int* status;
 };
+
+// The group pairs [first, last) of this CTA's K slice, and the groups in it.
+struct W4Slice {
+  int pair0, groups;
+};
+template <bool SPLIT>
+__device__ __forceinline__ W4Slice w4_slice(const W4Params& p) {
+  if constexpr (!SPLIT) return {0, p.groups};
+  const int pairs = (p.groups + 1) >> 1, z = static_cast<int>(blockIdx.z);
+  const int first = pairs * z / p.splits, last = pairs * (z + 1) / p.splits;
+  return {first, min(p.groups, 2 * last) - 2 * first};
+}
+
+// Split K: every CTA of the cluster has parked its fp32 partial tile [cols][128 channels] at `part` (the same
+// place in each); after the cluster barrier each CTA adds a share of the columns in rank order - a fixed order -
+// and stores it.  All threads of the CTA call this.
+__device__ __forceinline__ void w4_reduce_splits(const W4Params& p, uint32_t part, int cols, int n0, int m0, const volatile int* abort_flag) {
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (*abort_flag == 0) {  // uniform: every role has finished
+    uint32_t peer[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      peer[r] = 0;
+      if (r < p.splits) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer[r]) : "r"(part), "r"(r));
+    }
+    const int per = (cols + p.splits - 1) / p.splits;
+    const int lo = static_cast<int>(blockIdx.z) * per;
+    const int items = (min(cols, lo + per) - lo) * 32;  // four channels each
+    for (int i = threadIdx.x; i < items; i += static_cast<int>(blockDim.x)) {
+      const int c = lo + (i >> 5), n = n0 + (i & 31) * 4;
+      const uint32_t at = static_cast<uint32_t>(c * 128 + (i & 31) * 4) * 4u;
+      float4 v[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        v[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < p.splits)
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[r].x), "=f"(v[r].y), "=f"(v[r].z), "=f"(v[r].w) : "r"(peer[r] + at) : "memory");
+      }
+#pragma unroll
+      for (int r = 1; r < 8; ++r) v[0].x += v[r].x, v[0].y += v[r].y, v[0].z += v[r].z, v[0].w += v[r].w;
+      if (n < p.n) {  // n is a multiple of 8: four channels exist whole or not at all
+        float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (p.bias != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) b[j] = __bfloat162float(p.bias[n + j]);
+        }
+        __nv_bfloat16* const dst = p.out + static_cast<long long>(m0 + c) * p.ldo + n;
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0].x + b[0], v[0].y + b[1]), pack_bf16x2(v[0].z + b[2], v[0].w + b[3]));
+      }
+    }
+  }
+  __syncwarp();
+  // nobody leaves while a peer may still read its shared memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 __host__ __device__ constexpr int w4_threads(int unpack_warps) { return 32 * (2 + unpack_warps + 4 + 1); }
 // TMEM budget (512 columns): every slot takes 64 columns of unpacked weights and `bn` accumulator columns.
@@ -74,7 +133,8 @@ __device__ __forceinline__ uint4 w4_unpack8(uint32_t w) {
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-template <int BN, int UW>
+// SPLIT: the kernel of a cluster that shares an output tile (W4Params::splits > 1); see w4_splits for when.
+template <int BN, int UW, bool SPLIT>
 __global__ void __launch_bounds__(w4_threads(UW), 1)
 rk_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                      const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_o,
@@ -111,15 +171,17 @@ rk_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
   const uint32_t scales_off = w_off + p.w_stages * kW4PairBytes;
   const int n0 = blockIdx.x * 128;
   const int m0 = blockIdx.y * BN;
-  const int G = p.groups;
+  const W4Slice slice = w4_slice<SPLIT>(p);
+  const int G = slice.groups;
+  const int pair0 = slice.pair0;
 
   pdl_launch_dependents();
   if (threadIdx.x == 64) {
     // first thing, by a thread that has no part in the set-up: the first raw copies and the scales
     // start their way from DRAM to L2 while the CTA sets up and the preceding kernel drains
-    tma_prefetch_l2_2d(&tm_s, n0, 0);
+    tma_prefetch_l2_2d(&tm_s, n0, 2 * pair0);
     const int ahead = min((G + 1) >> 1, kW4MaxW);
-    for (int i = 0; i < ahead; ++i) tma_prefetch_l2_2d(&tm_w, i * 128, n0);
+    for (int i = 0; i < ahead; ++i) tma_prefetch_l2_2d(&tm_w, (pair0 + i) * 128, n0);
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.w_stages; ++s) {
@@ -157,8 +219,9 @@ rk_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     if (lane == 0) {
       const uint64_t pol_w = l2_policy_evict_first();
       const uint64_t pol_x = l2_policy_evict_last();
-      mbar_arrive_expect_tx(smem_u32(&bar_scales), static_cast<uint32_t>(G) * 256u);
-      tma_load_2d_hint(smem_base + scales_off, &tm_s, n0, 0, smem_u32(&bar_scales), pol_w);
+      // a copy counts its whole box, rows beyond the matrix included
+      mbar_arrive_expect_tx(smem_u32(&bar_scales), static_cast<uint32_t>(p.scale_rows) * 256u);
+      tma_load_2d_hint(smem_base + scales_off, &tm_s, n0, 2 * pair0, smem_u32(&bar_scales), pol_w);
       const int P = (G + 1) >> 1;  // group pairs; an odd last pair reads zeros beyond K
       int gw = 0, gx = 0;
       Ring rw{0, 0}, rx{0, 0};
@@ -170,7 +233,7 @@ rk_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
           if (mbar_test_wait(smem_u32(&bar_w_empty[s]), rw.phase ^ 1)) {
             const uint32_t full = smem_u32(&bar_w_full[s]);
             mbar_arrive_expect_tx(full, kW4PairBytes);
-            tma_load_2d_hint(smem_base + w_off + s * kW4PairBytes, &tm_w, gw * 128, n0, full, pol_w);
+            tma_load_2d_hint(smem_base + w_off + s * kW4PairBytes, &tm_w, (pair0 + gw) * 128, n0, full, pol_w);
             ++gw;
             rw.advance(p.w_stages);
             progressed = true;
@@ -183,7 +246,7 @@ rk_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
             const uint32_t full = smem_u32(&bar_slot_full[t]);
             mbar_arrive_expect_tx(full, kXBytes);
             // one copy brings both 64-element column blocks of the group: box {64, BN, 2}
-            tma_load_3d_hint(smem_base + x_off + t * kXBytes, &tm_x, 0, m0, gx * 2, full, pol_x);
+            tma_load_3d_hint(smem_base + x_off + t * kXBytes, &tm_x, 0, m0, (2 * pair0 + gx) * 2, full, pol_x);
             ++gx;
             rx.advance(kSlots);
             progressed = true;
@@ -374,7 +437,13 @@ rk_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     // every epilogue warp reaches this rendezvous, whether it completed or gave up
     if (!alive) *reinterpret_cast<volatile int*>(&epi_dead) = 1;
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (*reinterpret_cast<volatile int*>(&epi_dead) == 0) {
+    if constexpr (SPLIT) {
+      // this slice's totals, for the cluster's sum below
+      float* const part = reinterpret_cast<float*>(smem_gen + x_off);
+#pragma unroll
+      for (int j = 0; j < BN; ++j) part[j * 128 + quad * 32 + lane] = acc[j];
+    }
+    if (!SPLIT && *reinterpret_cast<volatile int*>(&epi_dead) == 0) {
       // The running totals hold one output channel per lane while the output is [m][n] with n
       // contiguous: transpose through shared memory (the activation tiles are free once the last
       // group's MMAs have completed) and let TMA stores write the rows, clipping ragged edges.
@@ -395,6 +464,10 @@ rk_gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_cons
     }
   }
 
+  if constexpr (SPLIT) {
+    __syncwarp();  // the single-lane roles rejoin their warps
+    w4_reduce_splits(p, smem_base + x_off, min(BN, p.m - m0), n0, m0, &abort_flag);
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

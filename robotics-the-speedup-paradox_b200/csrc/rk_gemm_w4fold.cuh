@@ -34,7 +34,7 @@ constexpr int kW4fMaxSlots = 8;
 
 __host__ __device__ constexpr int w4f_slots(int bn) { return bn > 128 ? 5 : 8; }
 
-template <int BN>
+template <int BN, bool SPLIT>
 __global__ void __launch_bounds__(kW4fThreads, 1)
 rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                           const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_o,
@@ -68,7 +68,9 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   const uint32_t scales_off = w_off + p.w_stages * kW4PairBytes;
   const int n0 = blockIdx.x * 128;
   const int m0 = blockIdx.y * BN;
-  const int G = p.groups;
+  const W4Slice slice = w4_slice<SPLIT>(p);
+  const int G = slice.groups;
+  const int pair0 = slice.pair0;
   const int S = 2 * G;  // steps of 64 K elements
   // Every CTA of a launch reads the SAME activation tiles.  Walking K from a different start in
   // each CTA (a rotation by whole raw copies) spreads those reads over different L2 lines at any
@@ -82,10 +84,10 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   if (threadIdx.x == 64) {
     // first thing, by a thread that has no part in the set-up: the first raw copies and the scales
     // start their way from DRAM to L2 while the CTA sets up and the preceding kernel drains
-    tma_prefetch_l2_2d(&tm_s, n0, 0);
+    tma_prefetch_l2_2d(&tm_s, n0, 2 * pair0);
     const int ahead = min(P, kW4MaxW);
     for (int i = 0, kw = rot_copies; i < ahead; ++i) {
-      tma_prefetch_l2_2d(&tm_w, kw * 128, n0);
+      tma_prefetch_l2_2d(&tm_w, (pair0 + kw) * 128, n0);
       if (++kw == P) kw = 0;
     }
   }
@@ -125,8 +127,8 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     if (lane == 0) {
       const uint64_t pol_w = l2_policy_evict_first();
       const uint64_t pol_x = l2_policy_evict_last();
-      mbar_arrive_expect_tx(smem_u32(&bar_scales), static_cast<uint32_t>(G) * 256u);
-      tma_load_2d_hint(smem_base + scales_off, &tm_s, n0, 0, smem_u32(&bar_scales), pol_w);
+      mbar_arrive_expect_tx(smem_u32(&bar_scales), static_cast<uint32_t>(p.scale_rows) * 256u);
+      tma_load_2d_hint(smem_base + scales_off, &tm_s, n0, 2 * pair0, smem_u32(&bar_scales), pol_w);
       int gw = 0, sx = 0;
       int kw = rot_copies, kx = rot_steps;  // rotated positions along K
       Ring rw{0, 0}, rx{0, 0};
@@ -138,7 +140,7 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
           if (mbar_test_wait(smem_u32(&bar_w_empty[s]), rw.phase ^ 1)) {
             const uint32_t full = smem_u32(&bar_w_full[s]);
             mbar_arrive_expect_tx(full, kW4PairBytes);
-            tma_load_2d_hint(smem_base + w_off + s * kW4PairBytes, &tm_w, kw * 128, n0, full, pol_w);
+            tma_load_2d_hint(smem_base + w_off + s * kW4PairBytes, &tm_w, (pair0 + kw) * 128, n0, full, pol_w);
             if (++kw == P) kw = 0;
             ++gw;
             rw.advance(p.w_stages);
@@ -150,7 +152,7 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
           if (mbar_test_wait(smem_u32(&bar_slot_empty[t]), rx.phase ^ 1)) {
             const uint32_t full = smem_u32(&bar_slot_full[t]);
             mbar_arrive_expect_tx(full, kXBytes);
-            tma_load_2d_hint(smem_base + x_off + t * kXBytes, &tm_x, kx * 64, m0, full, pol_x);
+            tma_load_2d_hint(smem_base + x_off + t * kXBytes, &tm_x, pair0 * 256 + kx * 64, m0, full, pol_x);
             if (++kx == S) kx = 0;
             ++sx;
             rx.advance(kSlots);
@@ -309,12 +311,18 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         uint32_t v[16];
         tmem_ld_16(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kW4fAccCol + c0, v);
         tc_wait_ld();
+        if constexpr (SPLIT) {  // this slice's sums, for the cluster's sum below
+          float* const part = reinterpret_cast<float*>(smem_gen + x_off);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) part[(c0 + j) * 128 + nl] = __uint_as_float(v[j]);
+          continue;
+        }
 #pragma unroll
         for (int j = 0; j < 16; ++j) stage[(c0 + j) * 128 + nl] = __float2bfloat16_rn(__uint_as_float(v[j]) + bias);
       }
       fence_proxy_async_smem();
       asm volatile("bar.sync 1, 384;" ::: "memory");
-      if (warp == kEpiWarp0 && lane == 0) {
+      if (!SPLIT && warp == kEpiWarp0 && lane == 0) {
         for (int r0 = 0; r0 < rows; r0 += 32)
           tma_store_2d(&tm_o, smem_u32(stage + r0 * 128), n0, m0 + r0);
         tma_store_commit();
@@ -323,6 +331,10 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     }
   }
 
+  if constexpr (SPLIT) {
+    __syncwarp();  // the single-lane roles rejoin their warps
+    w4_reduce_splits(p, smem_base + x_off, min(BN, p.m - m0), n0, m0, &abort_flag);
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {

@@ -205,3 +205,18 @@ def test_invalid_arguments_are_refused_before_any_launch(H):
     assert lib.rk_gemm_w4a16_g128(*args(8, 128, 256, -1)) == _lib.RK_EINVAL
     torch.cuda.synchronize()
     assert (out == 3.0).all()
+
+
+@pytest.mark.parametrize("shape", [(2, 200, 1664), (16, 8, 1536), (33, 2048, 2048), (50, 136, 16384), (64, 264, 3328),
+                                   (65, 136, 1664), (130, 264, 2176), (257, 520, 3072), (300, 2048, 8192)])
+def test_k_slices_of_a_cluster_add_up(H, shape):
+    """Few tiles and a long K: clusters share tiles (odd group counts, ragged last slices, ragged tiles).  The slices are
+    summed in fp32, so what remains is the bf16 rounding of the result (2^-9 of a value) plus the fp32 sums."""
+    m, n, k = shape
+    x, w, bias = H.randn_bf16((m, k), 1.0, 31), H.randn_bf16((n, k), 0.02, 32), H.randn_bf16((n,), 0.5, 33)
+    q, s = pack(H, w.to(H.DEVICE))
+    out = H.to_np(run_gemm(H, x.to(H.DEVICE), q, s, bias.to(H.DEVICE), m, n, k))
+    ep, es, _ = OW.pack_weight(H.to_np(w))
+    _, want = (OW.gemm if m <= 64 else OW.gemm_folded)(H.to_np(x), ep, es, H.to_np(bias))
+    assert H.rel_frobenius(out, want) < 2.0 ** -8
+    assert np.abs(out - want).max() <= 2.0 ** -8 * np.abs(want).max() + 1e-6
