@@ -3,6 +3,8 @@
 
 #include <cuda.h>
 
+#include <algorithm>
+
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -199,6 +201,39 @@ int block_scaled_tile_rows(int64_t rows) {
   return best;
 }
 
+// How many clusters of `size` CTAs with a whole SM each the current device runs at once.  A cluster lives inside one
+// GPC, so this is less than SMs / size; one cluster too many doubles the time of a launch.
+int max_clusters(int size) {
+  static std::mutex mu;
+  static int known[64][9] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  int& entry = known[dev & 63][size];
+  if (entry == 0) {
+    auto kernel = rk_gemm_w4a16_fold_kernel<256, true>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 1024);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1, 1, size);
+    cfg.blockDim = dim3(kW4fThreads);
+    cfg.dynamicSmemBytes = kSmemBudget;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = size;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = kNumSms / (2 * size);
+    }
+    entry = n;
+  }
+  return entry;
+}
+
 // `tactic` only nudges the shape of the decomposition (it can never change integer results and
 // only reorders fp32 partial sums): bit 0 forbids swap, bit 1 forbids split-K, bit 2 halves bn.
 Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
@@ -250,8 +285,16 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
     // with the same loop - beat both wide tiles and split-K (whose exchange costs more than it saves
     // unless the tiles are very few).
     if (!block_scaled && !(tactic & 4) && bn >= 64) {
+      const int64_t tiles_a = (n + 127) / 128;
       const int half = static_cast<int>(round_up(bn / 2, 32));
-      if (((n + 127) / 128) * ((m + half - 1) / half) <= kNumSms) bn = half;
+      if (tiles_a * ((m + half - 1) / half) <= kNumSms) {
+        bn = half;
+      } else if (kblocks >= 32 && tiles_a < kNumSms) {
+        // A long K loop runs at the rate at which an SM takes operands from L2, (128 + bn) x 128 bytes a block: as many
+        // chunks as there are SMs (FP8 816 x 2048 x 16384: 31.7 us with 112 CTAs of 128 rows, 28.4 with 144 of 96).
+        const int64_t fit = kNumSms / tiles_a;
+        bn = std::min(bn, static_cast<int>(round_up((m + fit - 1) / fit, 32)));
+      }
     }
     pl.bn = bn;
     pl.tiles_a = static_cast<int>((n + 127) / 128);
@@ -272,16 +315,19 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
   // split-K across a cluster when the tiles cannot occupy the machine; >= 2 K blocks per CTA
   const long long tiles = static_cast<long long>(pl.tiles_a) * pl.tiles_b;
   pl.splits = 1;
-  // A split costs a cluster launch and the exchange through distributed shared memory (+1 ... +7 us
-  // measured on K loops of 4 ... 16 blocks: 64 x 2048 x 2048 W8A8 6.5 us split eight ways, 5.75 us
-  // unsplit), so it is taken only when the K loop it shortens is long: 32 blocks of 128 bytes for the
-  // direct kinds, 8 for the rewriting kinds, whose stages take ~1 us each.
+  // A split costs a cluster launch and the exchange through distributed shared memory, so it is taken only when
+  // the K loop it shortens is long - 32 blocks of 128 bytes for the direct kinds, 8 for the rewriting kinds, whose
+  // stages take ~1 us each - and at least three ways, the largest cluster whose copies all run at once (one too many
+  // costs a second wave: 50 x 1024 x 4096 W8A8 10.2 us in 16 clusters of eight, 6.1 in clusters of six, 8.4 whole;
+  // 1 x 2048 x 8192 11.7, 6.9 and 13.5; 200 x 1024 x 4096 8.1 us four ways, 9.0 whole, 8.4 two ways).
   const bool long_loop = rewriting ? kblocks >= 8 : kblocks >= 32;
-  if (!(tactic & 2) && tiles * 4 <= kNumSms && long_loop) {  // a two-way split does not pay for its exchange
-    int s = static_cast<int>(kNumSms / tiles);
-    if (s > 8) s = 8;
-    if (s > kblocks / 2) s = kblocks / 2;
-    if (s > 1) pl.splits = s;
+  if (!(tactic & 2) && long_loop) {
+    for (int s = static_cast<int>(std::min<long long>(8, std::min<long long>(kNumSms / tiles, kblocks / 2))); s > 2; --s) {
+      if (tiles <= max_clusters(s)) {
+        pl.splits = s;
+        break;
+      }
+    }
   }
   // shared memory: pipeline stages + output staging + per-tile vectors
   const int stage = gemm_stage_bytes(kind, pl.bn, pl.sfb_blocks);
@@ -302,15 +348,15 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
   return pl;
 }
 
-template <int KIND, bool RESIDUAL = false>
-int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
+template <int KIND, bool RESIDUAL, bool SPLIT>
+int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
               const Plan& pl, cudaStream_t st) {
   static bool configured_dev[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   bool& configured = configured_dev[dev & 63];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc_kernel<KIND, RESIDUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc_kernel<KIND, RESIDUAL, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBudget + 1024);
     if (e != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured = true;
@@ -329,12 +375,19 @@ int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMa
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc_kernel<KIND, RESIDUAL>, tm_a, tm_b, tm_out, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc_kernel<KIND, RESIDUAL, SPLIT>, tm_a, tm_b, tm_out, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(RK_ECUDA, "rk_gemm_tc_kernel launch: %s", cudaGetErrorString(e));
   }
   return RK_OK;
+}
+
+template <int KIND, bool RESIDUAL = false>
+int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
+              const Plan& pl, cudaStream_t st) {
+  return pl.splits > 1 ? launch_tc_kernel<KIND, RESIDUAL, true>(tm_a, tm_b, tm_out, p, pl, st)
+                       : launch_tc_kernel<KIND, RESIDUAL, false>(tm_a, tm_b, tm_out, p, pl, st);
 }
 
 // RK_B200_ISSUE_BLOCK=0 issues every tensor-core instruction under its own predicate instead of the
@@ -1280,39 +1333,6 @@ int launch_w4_fold2(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUte
     return fail(RK_ECUDA, "rk_gemm_w4a16_fold2_kernel launch: %s", cudaGetErrorString(e));
   }
   return RK_OK;
-}
-
-// How many clusters of `size` CTAs with a whole SM each the current device runs at once.  A cluster lives inside one
-// GPC, so this is less than SMs / size; one cluster too many doubles the time of a launch.
-int max_clusters(int size) {
-  static std::mutex mu;
-  static int known[64][9] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  int& entry = known[dev & 63][size];
-  if (entry == 0) {
-    auto kernel = rk_gemm_w4a16_fold_kernel<256, true>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 1024);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(1, 1, size);
-    cfg.blockDim = dim3(kW4fThreads);
-    cfg.dynamicSmemBytes = kSmemBudget;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = size;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      n = kNumSms / (2 * size);
-    }
-    entry = n;
-  }
-  return entry;
 }
 
 // K slices per output tile.  A launch of few tiles leaves most SMs idle for a K loop of up to 128 groups, so a cluster

@@ -394,7 +394,8 @@ __device__ __forceinline__ void multicast_store_region(const GemmParams& p, cons
 // store descriptors of the column-parallel mode, one per rank, or null).
 // RESIDUAL: the epilogue applies GemmParams::residual (a separate instantiation: the 64 values it keeps
 // in flight would otherwise cost every launch of the kind its registers).
-template <int KIND, bool RESIDUAL = false>
+// SPLIT: the split-K schedule (GemmParams::splits > 1), its own instantiation for the same reason.
+template <int KIND, bool RESIDUAL = false, bool SPLIT = false>
 __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out,
                                              const CUtensorMap* peer_maps, const GemmParams& p) {
   using T = KindTraits<KIND>;
@@ -426,11 +427,11 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const uint32_t out_stage_off = p.stages * stage_bytes;
   const uint32_t vec_off = out_stage_off + p.out_bufs * kOutBufBytes;
 
-  const bool split_mode = p.splits > 1;
+  constexpr bool split_mode = SPLIT;
   const int num_tiles = p.tiles_a * p.tiles_b;
   const int tile_first = split_mode ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
   const int tile_step = split_mode ? num_tiles : static_cast<int>(gridDim.x);  // split mode: exactly one tile
-  const int split = split_mode ? static_cast<int>(blockIdx.z) : 0;
+  const int split = static_cast<int>(blockIdx.z);
   const int kb_begin = static_cast<int>((static_cast<long long>(p.kblocks) * split) / p.splits);
   const int kb_end = static_cast<int>((static_cast<long long>(p.kblocks) * (split + 1)) / p.splits);
   const int nkb = kb_end - kb_begin;
@@ -686,13 +687,16 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
           for (int k = 0; k < 4; ++k) {
             if (k < nmma) {
               const uint32_t accumulate = (i > 0 || k > 0) ? 1u : 0u;
-              // 32 bytes of K per MMA: advance the descriptor start address by 32 >> 4.
+              // 32 bytes of K per MMA: advance the descriptor start address by 32 >> 4.  The direct kinds branch on
+              // the elected lane around each MMA: the issuing warp paces their loop, and a branch is cheaper for it
+              // than the predicated form or one block per stage (50 x 1024 x 2048 W8A8 5.46, 6.49 and 5.95 us;
+              // 816 x 2048 x 16384 28.2, 33.4 and 30.0).
               const uint64_t ad = adesc + static_cast<uint64_t>(k * 2);
               const uint64_t bd = bdesc + static_cast<uint64_t>(k * 2);
               if constexpr (BK == KIND_I8) {
-                mma_i8(d_tmem, ad, bd, idesc, accumulate, on);
+                if (on) mma_i8_np(d_tmem, ad, bd, idesc, accumulate);
               } else if constexpr (BK == KIND_F8) {
-                mma_f8f6f4(d_tmem, ad, bd, idesc, accumulate, on);
+                if (on) mma_f8f6f4_np(d_tmem, ad, bd, idesc, accumulate);
               } else if constexpr (BK == KIND_MXF8) {
                 // four MMAs share one set of scale columns; byte k of each 32-bit column is theirs
                 // (scale-factor ids: bits [4,6) for B, [29,31) for A)
@@ -803,7 +807,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       tc_fence_after();
       const uint32_t t_acc = tmem_base + ab * p.acc_stride + (static_cast<uint32_t>(quad * 32) << 16);
 
-      if (split_mode) {
+      if constexpr (split_mode) {
         // ---- split-K: park the raw partial accumulators in shared memory, column-major [bn][128]
         uint32_t* const part = reinterpret_cast<uint32_t*>(smem_gen);
         for (int c0 = 0; c0 < p.bn; c0 += 16) {
@@ -1017,18 +1021,16 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   }
 
   // ---------------------------------------------------------------- split-K: reduce across the cluster
-  if (split_mode) {
+  if constexpr (split_mode) {
     __syncthreads();
     cluster_sync_all();  // every CTA's partial tile is in its shared memory
-    if (warp >= 2 && warp < 6) {
-      const int quad = warp & 3;
-      const int et = quad * 32 + lane;
-      const int tile = tile_first;
-      const int row_a0 = (tile / p.tiles_b) * kTileA;
-      const int row_b0 = (tile % p.tiles_b) * p.bn;
+    {
+      // every warp of the CTA takes part: an item is one column of the tile and four of its 128 rows, fetched from each
+      // peer with one 16-byte load (four warps with 4-byte loads spent up to 5 us here)
+      const int row_a0 = (tile_first / p.tiles_b) * kTileA;
+      const int row_b0 = (tile_first % p.tiles_b) * p.bn;
       const int lim_a = p.swap ? p.n : p.m;
       const int lim_b = p.swap ? p.m : p.n;
-      const int ra = row_a0 + et;
       const bool has_bias = p.bias != nullptr && p.acc_out == nullptr;
       float s_act_scalar = 1.0f, s_wgt_scalar = 1.0f;
       if constexpr (BK != KIND_I8) {
@@ -1038,12 +1040,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       // this CTA finishes columns [c_lo, c_hi) of the tile
       const int per = (p.bn + p.splits - 1) / p.splits;
       const int c_lo = static_cast<int>(cluster_ctarank()) * per;
-      const int c_hi = min(p.bn, c_lo + per);
-      float row_scale = 1.0f, row_bias = 0.0f;
-      if (ra < lim_a && p.acc_out == nullptr) {
-        if constexpr (BK == KIND_I8) row_scale = p.swap ? p.scale_wgt[ra] : p.scale_act[ra];
-        if (p.swap && has_bias) row_bias = __bfloat162float(p.bias[ra]);
-      }
+      const int c_hi = min(min(p.bn, c_lo + per), lim_b - row_b0);
       const float* const vec_scale_r = reinterpret_cast<const float*>(smem_gen + vec_off);
       const float* const vec_bias_r = vec_scale_r + 256;
       // shared::cluster base address of every peer's partial tile
@@ -1054,54 +1051,55 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
         if (q < p.splits)
           asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer[q]) : "r"(smem_base), "r"(q));
       }
-      for (int c4 = c_lo; c4 < c_hi; c4 += 4) {
-        // issue the loads of four columns from every peer back to back, then add in rank order
-        uint32_t v[4][8];
+      const bool dead = *reinterpret_cast<volatile int*>(&abort_flag) != 0;
+      for (int i = threadIdx.x; i < (c_hi - c_lo) * 32 && !dead; i += static_cast<int>(blockDim.x)) {
+        const int c = c_lo + (i >> 5), r0 = (i & 31) * 4;
+        const int ra = row_a0 + r0, rbj = row_b0 + c;
+        uint32_t v[8][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            v[u][q] = 0u;
-            if (q < p.splits && c4 + u < c_hi)
-              asm volatile("ld.shared::cluster.u32 %0, [%1];"
-                           : "=r"(v[u][q])
-                           : "r"(peer[q] + static_cast<uint32_t>((c4 + u) * 128 + et) * 4u)
-                           : "memory");
-          }
+        for (int q = 0; q < 8; ++q) {
+          v[q][0] = v[q][1] = v[q][2] = v[q][3] = 0u;
+          if (q < p.splits)
+            asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(v[q][0]), "=r"(v[q][1]), "=r"(v[q][2]), "=r"(v[q][3])
+                         : "r"(peer[q] + static_cast<uint32_t>(c * 128 + r0) * 4u)
+                         : "memory");
         }
+        float val[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int c = c4 + u;
-          if (c >= c_hi) continue;
           uint32_t total = 0;
           float ftotal = 0.0f;
 #pragma unroll
           for (int q = 0; q < 8; ++q) {  // fixed order: rank 0, 1, ... (absent ranks contribute zero)
-            if constexpr (BK == KIND_I8) total += v[u][q];
-            else ftotal += __uint_as_float(v[u][q]);
+            if constexpr (BK == KIND_I8) total += v[q][u];
+            else ftotal += __uint_as_float(v[q][u]);
           }
           if constexpr (BK != KIND_I8) total = __float_as_uint(ftotal);
-          const int rbj = row_b0 + c;
-          if (ra >= lim_a || rbj >= lim_b || abort_flag) continue;
-          const long long om = p.swap ? rbj : ra, on = p.swap ? ra : rbj;
+          val[u] = 0.0f;
+          if (ra + u >= lim_a) continue;
+          const long long om = p.swap ? rbj : ra + u, on = p.swap ? ra + u : rbj;
           if (p.acc_out != nullptr) {
             p.acc_out[om * p.n + on] = static_cast<int>(total);
             continue;
           }
-          float val;
           // B-role scale and bias of this column were staged in shared memory by the epilogue prologue
-          const float bias_v = p.swap ? row_bias : vec_bias_r[c];
+          const float bias_v = p.swap ? (has_bias ? __bfloat162float(p.bias[ra + u]) : 0.0f) : vec_bias_r[c];
           if constexpr (BK == KIND_I8) {
-            const float other = vec_scale_r[c];
-            val = p.swap ? finish_value<BK>(total, other, row_scale, has_bias, bias_v)
-                         : finish_value<BK>(total, row_scale, other, has_bias, bias_v);
+            const float own = p.swap ? p.scale_wgt[ra + u] : p.scale_act[ra + u], other = vec_scale_r[c];
+            val[u] = p.swap ? finish_value<BK>(total, other, own, has_bias, bias_v) : finish_value<BK>(total, own, other, has_bias, bias_v);
           } else {
-            val = finish_value<BK>(total, s_act_scalar, s_wgt_scalar, has_bias, bias_v);
+            val[u] = finish_value<BK>(total, s_act_scalar, s_wgt_scalar, has_bias, bias_v);
           }
-          if constexpr (RESIDUAL) val = with_residual(p, val, static_cast<int>(om), static_cast<int>(on));
-          p.out[om * p.ldo + on] = __float2bfloat16_rn(val);
+          if constexpr (RESIDUAL) val[u] = with_residual(p, val[u], static_cast<int>(om), static_cast<int>(on));
+          if (!p.swap) p.out[om * p.ldo + on] = __float2bfloat16_rn(val[u]);
         }
+        // swapped tile: four consecutive channels of one row (n is a multiple of 8: they exist whole or not at all)
+        if (p.swap && p.acc_out == nullptr && ra < lim_a)
+          *reinterpret_cast<uint2*>(p.out + static_cast<long long>(rbj) * p.ldo + ra) =
+              make_uint2(pack_bf16x2(val[0], val[1]), pack_bf16x2(val[2], val[3]));
       }
+      __syncwarp();
     }
     cluster_sync_all();  // nobody leaves while a peer may still read its shared memory
   }
@@ -1116,11 +1114,11 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   }
 }
 
-template <int KIND, bool RESIDUAL = false>
+template <int KIND, bool RESIDUAL, bool SPLIT>
 __global__ void __launch_bounds__(KindTraits<KIND>::kThreads, 1)
 rk_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                   const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
-  gemm_tc_body<KIND, RESIDUAL>(tm_a, tm_b, tm_out, nullptr, p);
+  gemm_tc_body<KIND, RESIDUAL, SPLIT>(tm_a, tm_b, tm_out, nullptr, p);
 }
 
 // The per-tensor FP8 GEMM in column-parallel mode: one store descriptor per rank instead of one output map.

@@ -113,11 +113,9 @@ def _widen_first(m, n, kpad):
     GEMM?  Inside, a 128 x 128 x 128 stage costs about 0.8 us of rewriting and each tile is rewritten for every tile it
     meets; the copies cost one pass of (m + n) * kpad bytes through L2.  Measured, copies against inside:
     1764 x 8192 x 2048 28.3 / 90.9 us, 1764 x 2048 x 8192 29.6 / 100.6, 256 x 2048 x 2048 8.3 / 15.7, 50 x 8192 x 2048
-    10.4 / 16.7, 1 x 1024 x 1024 5.8 / 11.5.  Inside stays for few rows with a long K (50 x 1000 x 4096: 12.5 / 11.1), for
-    many rows of a tiny weight (1764 x 256 x 256: 7.6 / 6.3) and where the copies would take over 256 MiB."""
-    if (m + n) * kpad > 1 << 28 or (m > 1024 and n * kpad < 1 << 18):
-        return False
-    return m >= 192 or kpad < 4096
+    10.4 / 16.7, 50 x 1000 x 4096 7.6 / 10.8, 1 x 1024 x 1024 5.8 / 11.5.  Inside stays for many rows of a tiny weight
+    (1764 x 256 x 256: 7.5 / 6.3) and where the copies would take over 256 MiB."""
+    return (m + n) * kpad <= 1 << 28 and not (m > 1024 and n * kpad < 1 << 18)
 
 
 def integer_gemm(a, sa, b, sb, bias, bits, tactic, residual=None, gate=None):
