@@ -13,14 +13,19 @@
 // 128 CTAs.  Per CTA:
 //   1. S = Q K^T for its slice with tcgen05 kind::f16 MMAs (Q and the K slice staged by TMA in the
 //      128-byte swizzle), fp32 accumulators in TMEM;
-//   2. softmax threads (one per row) find the slice's maximum, the KS CTAs exchange the maxima
-//      through distributed shared memory, exp(score - max) is taken once per score and summed, the
-//      sums are exchanged: every CTA knows the exact global max and sum;
+//   2. softmax threads (two per row) find the maximum m_t of their own scores, take exp(score - m_t) once
+//      per score and sum it to l_t; ONE exchange of the pairs (m_t, l_t) through distributed shared memory
+//      gives every thread the row's maximum m and sum l = sum_t l_t exp(m_t - m), and its own
+//      probabilities are exp(score - m_t) * (exp(m_t - m) / l);
 //   3. p is written back to TMEM as packed bf16 (over the scores it replaces) and is the TMEM
 //      A operand of the second MMA, O_slice = P V, against V^T tiles (keys contiguous) from TMA;
 //   4. the partial outputs are parked in shared memory and summed across the cluster in rank
 //      order; each CTA finishes 256 / KS of the head's columns and stores bf16 rows.
 // No global scratch, no atomics, fixed summation order.  Every wait is bounded.
+//
+// Bound by latency: three dependent passes over a row, two exchanges and four short MMA phases.  With one exchange
+// (maxima first, sums in a second one before), the keys and values asked into L2 before the dependency wait, and
+// partial outputs parked by rows and fetched 16 bytes at a time: see the launch for the figures.
 //
 // Warp roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2..9 =
 // softmax / epilogue: warp w works on TMEM lanes 32 * (w % 4) .. + 31 (one thread per query row) and
@@ -40,6 +45,7 @@ constexpr int kAttnDim = 256;                 // head dimension this kernel is b
 constexpr int kAttnQBytes = 128 * 128;        // one 64-element column block of the query tile
 constexpr int kAttnSlotBytes = 256 * 128;     // ring slot: a K block (keys x 128 B) or a V^T block (256 x 128 B)
 constexpr int kAttnSlots = 4;
+constexpr int kAttnPartPitch = kAttnDim + 4;  // floats between two rows of a parked partial output
 constexpr int kAttnSmem = 4 * kAttnQBytes + kAttnSlots * kAttnSlotBytes + 1024;
 
 struct AttnParams {
@@ -106,6 +112,16 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int kblocks_v = (p.keys + 63) >> 6;         // V^T blocks of 64 keys
 
   pdl_launch_dependents();
+  if (threadIdx.x == 64) {
+    // the cached keys and values start their way from DRAM to L2 while the kernel before this one appends to them
+    // (L2 is the coherence point: an early fetch is never stale)
+    for (int i = 0; i < 4; ++i)
+      asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                   ::"l"(reinterpret_cast<uint64_t>(&tm_k)), "r"(i * 64), "r"(key0), "r"(b * p.kv_heads + kv_head) : "memory");
+    for (int i = 0; i < kblocks_v; ++i)
+      asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                   ::"l"(reinterpret_cast<uint64_t>(&tm_vt)), "r"(key0 + i * 64), "r"(0), "r"(b * p.kv_heads + kv_head) : "memory");
+  }
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&bar_q), 1);
     for (int s = 0; s < kAttnSlots; ++s) {
@@ -198,7 +214,6 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
     if (alive) tc_commit(smem_u32(&bar_s_full), on);
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1b
     // O = P V: the probabilities are the TMEM A operand (two bf16 per column), V^T blocks of 64 keys
     alive = alive && mbar_wait_bounded(smem_u32(&bar_p_full), 0, &abort_flag, p.status, RK_DEV_TIMEOUT_XFORM);
     tc_fence_after();
@@ -243,20 +258,9 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if (c0 + j < valid) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(a[j]));
     }
     const float m_raw = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-    row_max[half][r] = m_raw > -INFINITY ? attn_score(__float_as_uint(m_raw), p.scaling) : -INFINITY;
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1
-    // the exact global maximum: every thread reads the 2 * KS partial maxima of its row
-    float m_glob = -INFINITY;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      if (q < p.splits) {
-        uint32_t am;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(am) : "r"(smem_u32(&row_max[0][r])), "r"(q));
-        m_glob = fmaxf(m_glob, fmaxf(dsmem_ld_f32(am), dsmem_ld_f32(am + 128u * 4u)));
-      }
-    }
-    // pass 2: e = exp(score - max) once per score, summed, and written back over the score (fp32)
-    const float mneg = -m_glob * log2e;
+    const float m_own = m_raw > -INFINITY ? attn_score(__float_as_uint(m_raw), p.scaling) : -INFINITY;
+    // pass 2: e = exp(score - m_own) once per score, summed, and written back over the score (fp32)
+    const float mneg = -m_own * log2e;
     float ls[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int c0 = half * 32; c0 < p.keys; c0 += 64) {
       uint32_t a[32];
@@ -274,19 +278,32 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tmem_st_32(tmem_s + lane_addr + c0, a);
     }
     tc_wait_st();
+    row_max[half][r] = m_own;
     row_sum[half][r] = (ls[0] + ls[1]) + (ls[2] + ls[3]);
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1b
-    float l_glob = 0.0f;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1
+    // the row's 2 * KS pairs (maximum, sum)
+    float pm[16], pl[16];
+    float m_glob = -INFINITY;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {  // fixed order: slice 0 (even chunks, odd chunks), slice 1, ...
+    for (int q = 0; q < 8; ++q) {
+      pm[2 * q] = pm[2 * q + 1] = -INFINITY;
+      pl[2 * q] = pl[2 * q + 1] = 0.0f;
       if (q < p.splits) {
-        uint32_t al;
+        uint32_t am, al;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(am) : "r"(smem_u32(&row_max[0][r])), "r"(q));
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(al) : "r"(smem_u32(&row_sum[0][r])), "r"(q));
-        l_glob += dsmem_ld_f32(al);
-        l_glob += dsmem_ld_f32(al + 128u * 4u);
+        pm[2 * q] = dsmem_ld_f32(am), pm[2 * q + 1] = dsmem_ld_f32(am + 128u * 4u);
+        pl[2 * q] = dsmem_ld_f32(al), pl[2 * q + 1] = dsmem_ld_f32(al + 128u * 4u);
       }
     }
-    const float inv_l = l_glob > 0.0f ? __fdiv_rn(1.0f, l_glob) : 0.0f;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) m_glob = fmaxf(m_glob, pm[q]);
+    float l_glob = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 16; ++q)  // fixed order: slice 0 (even chunks, odd chunks), slice 1, ...; a part without keys adds zero
+      l_glob = fmaf(pl[q], pm[q] > -INFINITY ? attn_ex2((pm[q] - m_glob) * log2e) : 0.0f, l_glob);
+    const float own = m_own > -INFINITY ? attn_ex2((m_own - m_glob) * log2e) : 0.0f;
+    const float inv_l = l_glob > 0.0f ? __fdiv_rn(own, l_glob) : 0.0f;
     // pass 3: probabilities as packed bf16 over the values they replace.  Packed column j covers the
     // fp32 columns 2j, 2j + 1; chunk c lands in the first (c even) or second (c odd) half of chunk
     // c / 2, which one of the row's two threads read in this step or an earlier one: a barrier of
@@ -318,63 +335,58 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     ok = mbar_wait_group(smem_u32(&bar_o_full), 0, threadIdx.x == 64, 1, kAttnSoftmaxThreads, &abort_flag, p.status,
                          RK_DEV_TIMEOUT_ACC, verdict, 1) && ok;
     tc_fence_after();
-    // park this slice's partial output, column-major [256][128] fp32, over the operand buffers
-    // (every MMA that read them has completed); each of the row's two threads takes 128 columns
-    float* const part = reinterpret_cast<float*>(smem_gen);
+    // park this slice's partial output by rows ([128][kAttnPartPitch] fp32; the pitch spreads a column's 16-byte
+    // stores over all banks) over the operand buffers: every MMA that read them has completed.  Each of the row's two
+    // threads takes 128 columns.
+    float* const part = reinterpret_cast<float*>(smem_gen) + r * kAttnPartPitch;
     for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
       uint32_t a[32];
       __syncwarp();
       tmem_ld_32(tmem_o + lane_addr + c0, a);
       tc_wait_ld();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) part[(c0 + j) * 128 + r] = ok ? __uint_as_float(a[j]) : 0.0f;
+      for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<uint4*>(part + c0 + j) = ok ? make_uint4(a[j], a[j + 1], a[j + 2], a[j + 3]) : make_uint4(0u, 0u, 0u, 0u);
     }
   }
   if (warp == 0) {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1b
   }
 
   // ---------------------------------------------------------------- sum the slices across the cluster
   __syncthreads();
   cluster_sync_all();  // #2: every CTA's partial output is in its shared memory
-  if (warp >= 2) {
-    const int r = (warp & 3) * 32 + lane;
-    const int per = 128 / p.splits;  // columns this thread finishes: the CTA takes 256 / splits, each of the row's two threads half
-    const int c_lo = split * 2 * per + ((warp - 2) >> 2) * per;
+  {
+    // this CTA finishes 256 / splits columns of every row: an item is four columns of a row
+    const int quads = 64 / p.splits;           // items per row: 64, 32, 16 or 8
+    const int shift = 31 - __clz(quads);
+    const int c_lo = split * 4 * quads;
     uint32_t peer[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       peer[q] = 0;
       if (q < p.splits) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer[q]) : "r"(smem_base), "r"(q));
     }
-    const int token = r / p.group, head = head0 + r % p.group;
-    __nv_bfloat16* const dst =
-        p.out + ((static_cast<long long>(b) * p.tokens + token) * p.heads + head) * kAttnDim + c_lo;
-    for (int c8 = 0; c8 < per; c8 += 8) {
-      // all loads of eight columns from every slice first (up to 64 in flight), then the sums in slice order
-      float x[8][8];
+    const bool dead = *reinterpret_cast<volatile int*>(&abort_flag) != 0;
+    for (int i = threadIdx.x; i < (rows_valid << shift) && !dead; i += kAttnThreads) {
+      const int r = i >> shift, c = c_lo + (i & (quads - 1)) * 4;
+      float4 x[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          x[q][u] = 0.0f;
-          if (q < p.splits) x[q][u] = dsmem_ld_f32(peer[q] + static_cast<uint32_t>((c_lo + c8 + u) * 128 + r) * 4u);
-        }
+      for (int q = 0; q < 8; ++q) {  // all loads first, then the sums in slice order
+        x[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (q < p.splits)
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(x[q].x), "=f"(x[q].y), "=f"(x[q].z), "=f"(x[q].w)
+                       : "r"(peer[q] + static_cast<uint32_t>(r * kAttnPartPitch + c) * 4u) : "memory");
       }
-      float v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        float t = x[0][u];
-#pragma unroll
-        for (int q = 1; q < 8; ++q)
-          if (q < p.splits) t += x[q][u];
-        v[u] = t;
-      }
-      if (r < rows_valid && !abort_flag)
-        *reinterpret_cast<uint4*>(dst + c8) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
-                                                          pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+      for (int q = 1; q < 8; ++q)
+        if (q < p.splits) x[0].x += x[q].x, x[0].y += x[q].y, x[0].z += x[q].z, x[0].w += x[q].w;
+      const int token = r / p.group, head = head0 + r % p.group;
+      *reinterpret_cast<uint2*>(p.out + ((static_cast<long long>(b) * p.tokens + token) * p.heads + head) * kAttnDim + c) =
+          make_uint2(pack_bf16x2(x[0].x, x[0].y), pack_bf16x2(x[0].z, x[0].w));
     }
+    __syncwarp();
   }
   cluster_sync_all();  // #3: nobody leaves while a peer may still read its shared memory
 

@@ -1610,9 +1610,15 @@ extern "C" int rk_attention_prefix(const void* q, const void* k_cache, const voi
       break;
     }
   const int tiles = static_cast<int>(heads / group);
-  // key slices: enough CTAs to occupy the machine, at most 256 keys each, a power of two up to 8
+  // Key slices: a power of two, as many as all run at once, at most 256 keys each.  Four are enough for 768 keys: eight
+  // shorten the passes over a row less than their exchange costs (50 tokens, 613 keys: 13.3 us in four, 13.7 in eight;
+  // 866 keys: 15.2 and 14.2).  Against two exchanges and 4-byte fetches: one environment, 613 keys 15.6 -> 13.3 us; eight,
+  // 866 keys 18.8 -> 17.2; four environments took eight slices in two waves, 30.7 -> 13.3.
+  const int most = kv_len > 768 ? 8 : 4;
   int splits = 1;
-  while (splits < 8 && (tiles * batch * splits * 2 <= kNumSms || (kv_len + splits - 1) / splits > 256)) splits *= 2;
+  while (splits < most && ((tiles * batch * splits * 2 <= kNumSms && tiles * batch <= max_clusters(splits * 2)) ||
+                        (kv_len + splits - 1) / splits > 256))
+    splits *= 2;
   const int keys = static_cast<int>(round_up((kv_len + splits - 1) / splits, 32));
   if (keys > 256) return fail(RK_EUNSUPPORTED, "%s: key slices above 256 keys", who);
   CUtensorMap tm_q, tm_k, tm_vt;

@@ -104,3 +104,17 @@ def test_attention_argument_errors():
     assert lib.rk_attention_prefix(*args(tokens=200)) == _lib.RK_EINVAL
     assert lib.rk_attention_prefix(*args(kv_len=65)) == _lib.RK_EINVAL
     assert lib.rk_attention_prefix(*args(pitch=60)) == _lib.RK_EINVAL
+
+
+@pytest.mark.parametrize("batch,prefix", [(1, 718), (1, 719), (3, 719), (4, 718), (4, 719), (5, 40)])
+def test_attention_with_any_number_of_key_slices(batch, prefix):
+    """Four slices up to 768 keys, eight above if that many clusters run at once (16 tiles of eight slices do not), slices
+    without keys: one exchange of (maximum, sum) pairs, with a score range that makes the pairs differ widely."""
+    q, k, v, kv_len, pitch = make_inputs(batch, 50, 8, 1, prefix, 23)
+    k[:, :, ::7] *= 6.0  # slices and threads with very different maxima
+    vt_all = torch.zeros((batch, 1, 256, pitch), dtype=torch.bfloat16)
+    vt_all[..., :kv_len] = v.transpose(-1, -2)
+    got = attention_prefix(q.to(DEVICE), k.to(DEVICE), vt_all.to(DEVICE), kv_len).float().cpu().numpy()
+    want = OA.attention(q.permute(0, 2, 1, 3).float().numpy(), k.float().numpy(), v.float().numpy(), 256 ** -0.5)
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < TOL
+    assert _lib.read_status(_lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)) == 0
