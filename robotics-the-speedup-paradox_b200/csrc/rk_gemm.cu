@@ -386,8 +386,8 @@ int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUt
 template <int KIND, bool RESIDUAL = false>
 int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
               const Plan& pl, cudaStream_t st) {
-  return pl.splits > 1 ? launch_tc_kernel<KIND, RESIDUAL, true>(tm_a, tm_b, tm_out, p, pl, st)
-                       : launch_tc_kernel<KIND, RESIDUAL, false>(tm_a, tm_b, tm_out, p, pl, st);
+  if (pl.splits > 1 || KindTraits<KIND>::kBlockScaled) return launch_tc_kernel<KIND, RESIDUAL, true>(tm_a, tm_b, tm_out, p, pl, st);
+  return launch_tc_kernel<KIND, RESIDUAL, KindTraits<KIND>::kBlockScaled>(tm_a, tm_b, tm_out, p, pl, st);
 }
 
 // RK_B200_ISSUE_BLOCK=0 issues every tensor-core instruction under its own predicate instead of the
@@ -440,15 +440,15 @@ int launch_tc_peer(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const PeerM
   return RK_OK;
 }
 
-template <int KIND>
-int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
+template <int KIND, bool REPACK>
+int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
                const CUtensorMap& tm_sfb, const Gemm2Params& p, int smem, cudaStream_t st) {
   static bool configured_dev[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   bool& configured = configured_dev[dev & 63];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc2_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc2_kernel<KIND, REPACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBudget + 1024);
     if (e != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured = true;
@@ -457,7 +457,7 @@ int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorM
   const int clusters = tiles < kNumSms / 2 ? tiles : kNumSms / 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * clusters, 1, 1);
-  cfg.blockDim = dim3(p.sw_q != nullptr ? kGemm2ThreadsSwiglu : kGemmThreads);
+  cfg.blockDim = dim3(REPACK ? kGemm2ThreadsSwiglu : kGemmThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -469,12 +469,21 @@ int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorM
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc2_kernel<KIND>, tm_a, tm_b, tm_out, tm_sfa, tm_sfb, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc2_kernel<KIND, REPACK>, tm_a, tm_b, tm_out, tm_sfa, tm_sfb, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(RK_ECUDA, "rk_gemm_tc2_kernel launch: %s", cudaGetErrorString(e));
   }
   return RK_OK;
+}
+
+template <int KIND>
+int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
+               const CUtensorMap& tm_sfb, const Gemm2Params& p, int smem, cudaStream_t st) {
+  if constexpr (KIND == KIND_MXF8 || KIND == KIND_NVF4) {
+    if (p.sw_q != nullptr) return launch_tc2_kernel<KIND, true>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, p, smem, st);
+  }
+  return launch_tc2_kernel<KIND, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, p, smem, st);
 }
 
 // A box of the 16 x U4 -> 16-byte-aligned tensor-map type writes 128 bytes per row into shared memory

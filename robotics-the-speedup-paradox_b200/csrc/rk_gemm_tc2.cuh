@@ -175,8 +175,9 @@ __host__ __device__ inline int gemm2_stage_bytes(int kind, int bn, int sfb_block
   return ((kTileA + bn / 2) * kStageKBytes + chunks * 512 * (1 + sfb_blocks) + 1023) / 1024 * 1024;
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(kGemm2ThreadsSwiglu, 1)
+// REPACK: the epilogues that never write the bf16 tile (sw_q set), on sixteen warps.
+template <int KIND, bool REPACK>
+__global__ void __launch_bounds__(REPACK ? kGemm2ThreadsSwiglu : kGemmThreads, 1)
 rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                    const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_sfa,
                    const __grid_constant__ CUtensorMap tm_sfb, const Gemm2Params p) {
@@ -214,7 +215,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_acc_full[b]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[b]), p.sw_q != nullptr ? 8 * kGemm2SwigluSets : 8);  // the epilogue warps of both CTAs of the pair
+      mbar_init(smem_u32(&bar_acc_empty[b]), REPACK ? 8 * kGemm2SwigluSets : 8);  // the epilogue warps of both CTAs of the pair
     }
     abort_flag = 0;
     sw_amax_bits = 0u;
@@ -379,9 +380,9 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             if (k < nmma) {
               const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
               if constexpr (KIND == KIND_I8) {
-                mma2_i8(d_tmem, adesc + k * 2, bdesc + k * 2, idesc, accumulate, on);
+                if (on) mma2_i8_np(d_tmem, adesc + k * 2, bdesc + k * 2, idesc, accumulate);
               } else if constexpr (KIND == KIND_F8) {
-                mma2_f8f6f4(d_tmem, adesc + k * 2, bdesc + k * 2, idesc, accumulate, on);
+                if (on) mma2_f8f6f4_np(d_tmem, adesc + k * 2, bdesc + k * 2, idesc, accumulate);
               } else if constexpr (KIND == KIND_MXF8) {
                 mma2_mxf8(d_tmem, adesc + k * 2, bdesc + k * 2,
                           idesc | (static_cast<uint32_t>(k) << 4) | (static_cast<uint32_t>(k) << 29), tmem_sfa,
@@ -416,7 +417,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     const uint32_t acc_empty_leader1 = mapa_u32(smem_u32(&bar_acc_empty[1]), 0);
     Ring racc{0, 0};
     uint32_t epi_iter = 0;
-    int pending_store = 0, obuf = 0;
+    int pending_store = 0, obuf = 0, sw_parity = 0;
     for (int tile = tile_first; tile < num_tiles; tile += tile_step, racc.advance(p.acc_bufs)) {
       const int ab = racc.stage;
       const int row_a0 = (tile / p.tiles_n) * 256 + static_cast<int>(rank) * kTileA;  // this CTA's 128 rows
@@ -426,35 +427,42 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       if constexpr (KIND == KIND_I8) {
         if (ra < p.m) row_scale = p.scale_act[ra];
       }
-      epi_sync(epi_threads);
-      for (int j = et; j < p.bn; j += 128) {
-        const int rb = row_b0 + j;
-        float sv = 1.0f, bv = 0.0f;
-        if (rb < p.n) {
-          if constexpr (KIND == KIND_I8) sv = p.scale_wgt[rb];
-          if (has_bias) bv = __bfloat162float(p.bias[rb]);
+      if constexpr (!REPACK) {
+        epi_sync(epi_threads);
+        for (int j = et; j < p.bn; j += 128) {
+          const int rb = row_b0 + j;
+          float sv = 1.0f, bv = 0.0f;
+          if (rb < p.n) {
+            if constexpr (KIND == KIND_I8) sv = p.scale_wgt[rb];
+            if (has_bias) bv = __bfloat162float(p.bias[rb]);
+          }
+          vec_scale[j] = sv;
+          vec_bias[j] = bv;
         }
-        vec_scale[j] = sv;
-        vec_bias[j] = bv;
+        epi_sync(epi_threads);
       }
-      epi_sync(epi_threads);
       const bool ok = mbar_wait_group(smem_u32(&bar_acc_full[ab]), racc.phase, threadIdx.x == 64, 1, epi_threads, &abort_flag, p.status,
                                       RK_DEV_TIMEOUT_ACC, verdict_epi, epi_iter++);
       tc_fence_after();
       const uint32_t t_acc = tmem_base + ab * 256 + (static_cast<uint32_t>(quad * 32) << 16);
-      if (p.sw_q != nullptr) {
+      if constexpr (REPACK) {
         // ---- SwiGLU + NVFP4 re-pack: this thread owns one activation row of the tile.  Per 128 output
         // columns: 64 `up` then 64 `gate` values -> 64 activations = four 16-element blocks = 32 code
         // bytes and 4 scale bytes (one aligned word of the swizzled layout).  The arithmetic is the
         // two-launch path's, step for step: bf16(alpha * acc), SwiGLU in bf16 steps, block pack.  Four warps
         // share a row: each takes one of the group's four blocks.
         const float alpha = s_act_scalar * s_wgt_scalar;
+        // bf16(alpha * acc) of two neighbouring columns
+        auto scaled_pair = [&](const uint32_t (&r)[16], int j) {
+          return pack_bf16x2(__fmul_rn(alpha, __uint_as_float(r[2 * j])), __fmul_rn(alpha, __uint_as_float(r[2 * j + 1])));
+        };
         const int rows_sf = (p.m + 127) & ~127;  // the scale buffer covers whole 128-row blocks; padding rows get zeros
         if (p.sw_mode == 2) {
           // ---- the activation itself as bf16 (the arithmetic of the table mode of the row quantizers) + its maximum
           __nv_bfloat16* const prod = reinterpret_cast<__nv_bfloat16*>(p.sw_q);
-          float amax = 0.0f;
+          uint32_t amax = 0u;  // bits of a bf16 magnitude
           for (int cc = 0; cc < p.bn; cc += 128) {
+            const uint32_t amax_before = amax;
             const int col0 = row_b0 + cc;
             const int ch0 = col0 >> 1;
             const int c0 = set * 16;
@@ -463,20 +471,18 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             tmem_ld_16(t_acc + cc + c0, ru);
             tmem_ld_16(t_acc + cc + 64 + c0, rg);
             tc_wait_ld();
+            const unsigned short* const table = reinterpret_cast<const unsigned short*>(p.sw_table);
             uint32_t w[8];
 #pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-              float v2[2];
-#pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const float up = round_bf16(__fmul_rn(alpha, __uint_as_float(ru[j + u])));
-                const float gate = round_bf16(__fmul_rn(alpha, __uint_as_float(rg[j + u])));
-                v2[u] = round_bf16(__fmul_rn(__bfloat162float(p.sw_table[__float_as_uint(gate) >> 16]), up));
-                const float a = fabsf(v2[u]);
-                if (a <= 3.4028234664e38f && ra < p.m && col0 < p.n) amax = fmaxf(amax, a);
-              }
-              w[j >> 1] = (__float_as_uint(v2[0]) >> 16) | (__float_as_uint(v2[1]) & 0xFFFF0000u);
+            for (int j = 0; j < 8; ++j) {
+              const uint32_t up = scaled_pair(ru, j), gate = scaled_pair(rg, j);
+              w[j] = mul_bf16x2(table[gate & 0xFFFFu] | (static_cast<uint32_t>(table[gate >> 16]) << 16), up);
+              // magnitudes order like their bit patterns; infinities and NaN count as zero
+              const uint32_t lo = w[j] & 0x7FFFu, hi = (w[j] >> 16) & 0x7FFFu;
+              amax = max(amax, lo < 0x7F80u ? lo : 0u);
+              amax = max(amax, hi < 0x7F80u ? hi : 0u);
             }
+            if (ra >= p.m || col0 >= p.n) amax = amax_before;
             if (ok && col0 < p.n && ra < p.m) {
               uint4* const dst = reinterpret_cast<uint4*>(prod + static_cast<long long>(ra) * (p.n >> 1) + ch0 + c0);
               dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -487,17 +493,17 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
           if (p.sw_sf != nullptr) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-            if (lane == 0 && ok && amax > 0.0f) atomicMax(&sw_amax_bits, __float_as_uint(amax));
+            amax = __reduce_max_sync(0xffffffffu, amax);
+            if (lane == 0 && ok && amax != 0u) atomicMax(&sw_amax_bits, amax << 16);
           }
           continue;
         }
         if (p.sw_mode == 1) {
           // ---- MXFP8 output: blocks of 32 channels = two warp sets; the sets of a pair exchange their 16 channels'
           // maximum (and whether a value was not finite) through shared memory, then each converts its own half
-          float* const part_max = reinterpret_cast<float*>(smem_gen + out_stage_off);  // [4 sets][128 rows]
-          uint32_t* const part_bad = reinterpret_cast<uint32_t*>(part_max + 4 * 128);    // [4 sets][128 rows]
+          // [2 parities][4 sets][128 rows]: magnitude bits of the larger value, bit 31 set when one is not finite
+          uint32_t* const part = reinterpret_cast<uint32_t*>(smem_gen + out_stage_off);
+          const unsigned short* const table = reinterpret_cast<const unsigned short*>(p.sw_table);
           for (int cc = 0; cc < p.bn; cc += 128) {
             const int col0 = row_b0 + cc;
             const int ch0 = col0 >> 1;
@@ -507,32 +513,35 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             tmem_ld_16(t_acc + cc + c0, ru);
             tmem_ld_16(t_acc + cc + 64 + c0, rg);
             tc_wait_ld();
-            float v[16];
-            float amax = 0.0f;
-            uint32_t bad = 0;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float up = round_bf16(__fmul_rn(alpha, __uint_as_float(ru[j])));
-              const float gate = round_bf16(__fmul_rn(alpha, __uint_as_float(rg[j])));
-              v[j] = round_bf16(__fmul_rn(__bfloat162float(p.sw_table[__float_as_uint(gate) >> 16]), up));
-              amax = fmaxf(amax, fabsf(v[j]));
-              bad |= !(fabsf(v[j]) <= 3.4028234664e38f);
+            if (cc + 128 >= p.bn) {  // the tile is in registers: hand the accumulator back before the arithmetic
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
             }
-            part_max[set * 128 + et] = amax;
-            part_bad[set * 128 + et] = bad;
-            epi_sync(epi_threads);
-            amax = fmaxf(amax, part_max[(set ^ 1) * 128 + et]);
-            bad |= part_bad[(set ^ 1) * 128 + et];
-            const uint32_t e = mxfp8_block_scale(amax, bad != 0);
+            uint32_t v[8];
+            uint32_t m = 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint32_t up = scaled_pair(ru, j), gate = scaled_pair(rg, j);
+              v[j] = mul_bf16x2(table[gate & 0xFFFFu] | (static_cast<uint32_t>(table[gate >> 16]) << 16), up);
+              m = max(m, max(v[j] & 0x7FFFu, (v[j] >> 16) & 0x7FFFu));  // NaN and infinities order above every number
+            }
+            // the two sets of a block exchange through alternating slots: one barrier of their two warps each time
+            uint32_t* const slot = part + (sw_parity & 1) * 512;
+            sw_parity ^= 1;
+            slot[set * 128 + et] = m;
+            asm volatile("bar.sync %0, 64;" ::"r"(2 + (set >> 1) * 4 + quad) : "memory");
+            m = max(m, slot[(set ^ 1) * 128 + et]);
+            const uint32_t e = mxfp8_block_scale(__uint_as_float(m << 16), m >= 0x7F80u);
             const float inverse = mxfp8_inverse_scale(e);
             uint32_t w[4];
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
-              w[q4] = 0;
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                w[q4] |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(__fmul_rn(v[4 * q4 + i], inverse), __NV_SATFINITE, __NV_E4M3))
-                         << (8 * i);
+              const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(bf16_lo(v[2 * q4]), inverse), __fmul_rn(bf16_hi(v[2 * q4]), inverse)),
+                                                           __NV_SATFINITE, __NV_E4M3);
+              const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(bf16_lo(v[2 * q4 + 1]), inverse), __fmul_rn(bf16_hi(v[2 * q4 + 1]), inverse)),
+                                                           __NV_SATFINITE, __NV_E4M3);
+              w[q4] = lo | (hi << 16);
             }
             if (ok && col0 < p.n) {
               if (ra < p.m)
@@ -540,11 +549,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
               if ((set & 1) == 0 && ra < rows_sf)
                 p.sw_sf[sf_offset(ra, (ch0 >> 5) + (set >> 1), p.sw_kt)] = ra < p.m ? static_cast<uint8_t>(e) : static_cast<uint8_t>(0);
             }
-            epi_sync(epi_threads);  // the exchange words are free again
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
           continue;
         }
         for (int cc = 0; cc < p.bn; cc += 128) {
@@ -557,13 +562,14 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           tmem_ld_16(t_acc + cc + c0, ru);
           tmem_ld_16(t_acc + cc + 64 + c0, rg);
           tc_wait_ld();
-          float v[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float up = round_bf16(__fmul_rn(alpha, __uint_as_float(ru[j])));
-            const float gate = round_bf16(__fmul_rn(alpha, __uint_as_float(rg[j])));
-            v[j] = swiglu_bf16_steps(gate, up);
+          if (cc + 128 >= p.bn) {  // the tile is in registers: hand the accumulator back before the arithmetic
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
           }
+          uint32_t v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = swiglu_bf16x2_steps(scaled_pair(rg, j), scaled_pair(ru, j));
           uint8_t code;
           const unsigned long long packed = nvfp4_block(v, &code);
           if (ok && col0 < p.n) {
@@ -572,9 +578,6 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             if (ra < rows_sf) p.sw_sf[sf_offset(ra, (ch0 >> 4) + set, p.sw_kt)] = ra < p.m ? code : static_cast<uint8_t>(0);
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
         continue;
       }
       for (int cc = 0; cc < p.bn; cc += 64, obuf = (p.out_bufs == 2) ? (obuf ^ 1) : 0) {
@@ -622,7 +625,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       }
     }
     if (et == 0) tma_store_wait_read<0>();  // the staging memory has been read; the writes drain after the CTA has left
-    if (p.sw_mode == 2 && p.sw_sf != nullptr) {
+    if (REPACK && p.sw_mode == 2 && p.sw_sf != nullptr) {
       epi_sync(epi_threads);  // every warp has added its maximum
       if (threadIdx.x == 64 && sw_amax_bits != 0u) atomicMax(reinterpret_cast<unsigned*>(p.sw_sf), sw_amax_bits);
     }

@@ -145,23 +145,6 @@ __device__ __forceinline__ float row_scale_from_max(float maximum, float limit, 
 // innocuous - except for products below the normal range, where one rounding is the closer one.
 // The row kernels are bound by instructions per element (36 -> about 17 for the modulated norm), not by
 // bytes: see the launch rule below for the figures.
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-  const __nv_bfloat162 r = __hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
-__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
-  const __nv_bfloat162 r = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
-// running maximum of magnitudes; like fmaxf, a NaN loses against a number
-__device__ __forceinline__ uint32_t absmax_bf16x2(uint32_t m, uint32_t v) {
-  v &= 0x7FFF7FFFu;
-  const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&m), *reinterpret_cast<const __nv_bfloat162*>(&v));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
-__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-
 struct Packed8 {
   uint32_t w[4];
 };
@@ -871,25 +854,31 @@ pack_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, long long rows, long long
 __device__ __forceinline__ float swiglu_f32(float gate, float up) {
   return round_bf16(__fmul_rn(__fdiv_rn(gate, __fadd_rn(1.0f, expf(-gate))), up));
 }
-// Eight consecutive SwiGLU outputs of row-major gate_up [rows, 2 * inter]: gate first, then up; or
-// `interleaved`: blocks of 128 columns, 64 up values followed by their 64 gate values (the layout a
-// fused gate/up projection writes: blackwell/csrc/fp4_cutlass_linear.cu:958-965).
-template <bool BF16_STEPS>
-__device__ __forceinline__ void load8_swiglu(const __nv_bfloat16* gate_up, long long inter, long long idx, int valid,
-                                             float (&v)[8], bool interleaved = false) {
+// Eight consecutive fp32-step SwiGLU outputs of row-major gate_up [rows, 2 * inter], gate first.
+__device__ __forceinline__ void load8_swiglu(const __nv_bfloat16* gate_up, long long inter, long long idx, float (&v)[8]) {
   const long long row = idx / inter, col = idx - row * inter;
+  const __nv_bfloat16* g = gate_up + row * 2 * inter + col;
+  float gv[8], uv[8];
+  const bool vec = (inter % 8) == 0;
+  load8(g, vec, 8, gv);
+  load8(g + inter, vec, 8, uv);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = swiglu_f32(gv[i], uv[i]);
+}
+// Eight consecutive outputs of `row` in bf16 steps: gate first, then up; or `interleaved`: blocks of 128 columns, 64 up
+// values followed by their 64 gate values (the layout a fused gate/up projection writes:
+// blackwell/csrc/fp4_cutlass_linear.cu:958-965).  inter % 8 == 0.
+__device__ __forceinline__ void load8_swiglu_bf16(const __nv_bfloat16* gate_up, long long inter, long long row, long long col,
+                                                  uint32_t* v, bool interleaved) {
   const __nv_bfloat16* g = gate_up + row * 2 * inter + col;
   const __nv_bfloat16* u = g + inter;
   if (interleaved) {  // eight consecutive columns never straddle a 64-column block
     u = gate_up + row * 2 * inter + (col >> 6) * 128 + (col & 63);
     g = u + 64;
   }
-  float gv[8], uv[8];
-  const bool vec = (inter % 8) == 0;
-  load8(g, vec, valid, gv);
-  load8(u, vec, valid, uv);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = i < valid ? (BF16_STEPS ? swiglu_bf16_steps(gv[i], uv[i]) : swiglu_f32(gv[i], uv[i])) : 0.0f;
+  const uint4 gw = *reinterpret_cast<const uint4*>(g), uw = *reinterpret_cast<const uint4*>(u);
+  v[0] = swiglu_bf16x2_steps(gw.x, uw.x), v[1] = swiglu_bf16x2_steps(gw.y, uw.y);
+  v[2] = swiglu_bf16x2_steps(gw.z, uw.z), v[3] = swiglu_bf16x2_steps(gw.w, uw.w);
 }
 
 // SwiGLU -> MXFP8 with power-of-two (ceil) block scales, the activation side of W4A8-MX
@@ -957,7 +946,7 @@ swiglu_amax_kernel(const __nv_bfloat16* __restrict__ gate_up, long long rows, lo
   for (long long idx = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8; idx < elements;
        idx += stride) {
     float v[8];
-    load8_swiglu<false>(gate_up, inter, idx, 8, v);  // inter % 8 == 0: a vector never straddles rows
+    load8_swiglu(gate_up, inter, idx, v);  // inter % 8 == 0: a vector never straddles rows
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float a = fabsf(v[i]);
@@ -985,7 +974,7 @@ swiglu_to_fp8_kernel(const __nv_bfloat16* __restrict__ gate_up, long long rows, 
   for (long long idx = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8; idx < elements;
        idx += stride) {
     float v[8];
-    load8_swiglu<false>(gate_up, inter, idx, 8, v);
+    load8_swiglu(gate_up, inter, idx, v);
     uint32_t c[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -1017,9 +1006,9 @@ swiglu_pack_nvfp4_kernel(const __nv_bfloat16* __restrict__ gate_up, long long ro
     sf[sfi] = 0;
     return;
   }
-  float v[16];
-  load8_swiglu<true>(gate_up, inter, row * inter + group * 16, 8, *reinterpret_cast<float(*)[8]>(&v[0]), interleaved != 0);
-  load8_swiglu<true>(gate_up, inter, row * inter + group * 16 + 8, 8, *reinterpret_cast<float(*)[8]>(&v[8]), interleaved != 0);
+  uint32_t v[8];
+  load8_swiglu_bf16(gate_up, inter, row, group * 16, &v[0], interleaved != 0);
+  load8_swiglu_bf16(gate_up, inter, row, group * 16 + 8, &v[4], interleaved != 0);
   uint8_t code;
   const unsigned long long packed = nvfp4_block(v, &code);
   *reinterpret_cast<unsigned long long*>(q + row * (inter / 2) + group * 8) = packed;
@@ -1036,9 +1025,10 @@ silu_mul_bf16_kernel(const __nv_bfloat16* __restrict__ gate_up, long long rows, 
   const long long total = rows * inter;
   for (long long idx = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8; idx < total;
        idx += static_cast<long long>(gridDim.x) * blockDim.x * 8) {
-    float v[8];
-    load8_swiglu<true>(gate_up, inter, idx, 8, v, interleaved != 0);  // inter % 8 == 0: a vector never straddles rows
-    store8(out + idx, true, 8, v);
+    Packed8 v;
+    const long long row = idx / inter;
+    load8_swiglu_bf16(gate_up, inter, row, idx - row * inter, v.w, interleaved != 0);  // inter % 8 == 0: one row per vector
+    store8p(out + idx, true, 8, v);
   }
 }
 
@@ -1113,12 +1103,13 @@ rmsnorm_producer_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 #pragma unroll
   for (int it = 0; it < kMaxVec; ++it) {
     const int idx = (it * kRowThreads + threadIdx.x) * 8;  // warp-uniform validity: k % 256 handled by the mask below
-    float v[16];
+    uint32_t v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float other = __shfl_xor_sync(0xffffffffu, vals[it][i], 1);
-      v[i] = (threadIdx.x & 1) ? other : vals[it][i];
-      v[8 + i] = (threadIdx.x & 1) ? vals[it][i] : other;
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t own = pack_bf16x2(vals[it][2 * i], vals[it][2 * i + 1]);  // bf16 values already: nothing is rounded
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+      v[i] = (threadIdx.x & 1) ? other : own;
+      v[4 + i] = (threadIdx.x & 1) ? own : other;
     }
     if (idx < k) {
       uint8_t code;

@@ -366,3 +366,18 @@ def test_nvfp4_gate_up_gemm_with_gelu_epilogue_equals_the_two_launches(H, shape,
                                            "down", global_scale=global_scale)
     out = fused.forward_into(down, x.reshape(1, m, k))
     assert out.shape == (1, m, 264) and torch.equal(out.reshape(m, 264), down(want))
+
+
+@pytest.mark.parametrize("up", [1.0, -3.0, 0.00146, 97.0, 1e30])
+def test_swiglu_steps_on_every_bf16_gate(up):
+    """The packed two-at-a-time evaluation (approximate reciprocal, one rounding per step) against the same steps as torch
+    takes them in fp32 with a rounding after each: equal for all 65536 gates, infinities and NaN included."""
+    from rk_b200.fp4_linear import cutlass_silu_mul_bf16
+
+    gate = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16).view(32, 2048)
+    ups = torch.full_like(gate, up)
+    got = cutlass_silu_mul_bf16(torch.cat([gate, ups], 1).contiguous(), 2048)
+    e = torch.exp(-gate.float()).bfloat16()
+    r = (1.0 / (1.0 + e.float()).bfloat16().float()).bfloat16()
+    want = ((gate.float() * r.float()).bfloat16().float() * ups.float()).bfloat16()
+    assert torch.equal(torch.nan_to_num(got.float(), nan=-7.5), torch.nan_to_num(want.float(), nan=-7.5))
