@@ -281,6 +281,11 @@ int rk_rmsnorm_quant_fp8(const void* x, const void* residual, const void* weight
  *   gate_up bf16 [rows, 2*inter]; q e4m3 [rows, inter]; inter % 16 == 0. */
 int rk_swiglu_quant_fp8(const void* gate_up, int64_t rows, int64_t inter, const float* scale_in, void* q,
                         float* scale_out, void* workspace, size_t workspace_bytes, void* stream);
+/* rk_swiglu_quant_fp8 with a computed scale for callers with room for the activation itself: a is written to
+ * `product` (bf16 [rows, inter], 16-byte aligned, contents free before and after) by the pass that finds its
+ * maximum and converted from there, instead of being evaluated twice.  Same codes, same scale. */
+int rk_swiglu_quant_fp8_product(const void* gate_up, int64_t rows, int64_t inter, void* product, void* q,
+                                float* scale_out, void* workspace, size_t workspace_bytes, void* stream);
 
 /* The "producer" form of the FP8 GEMM: bf16 activations with a UNIT activation scale are converted
  * to e4m3 (clamped to +-448) inside the kernel - raw bf16 rows land in shared memory by TMA and

@@ -52,6 +52,7 @@ SIGNATURES = {
     "rk_quant_tensor_fp8_with_scale": (_int, [_vp, _i64, _vp, _vp, _vp]),
     "rk_rmsnorm_quant_fp8": (_int, [_vp, _vp, _vp, _i64, _i64, _f32, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "rk_swiglu_quant_fp8": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "rk_swiglu_quant_fp8_product": (_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp, _sz, _vp]),
     "rk_gemm_fp8": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _int, _vp, _sz, _vp]),
     "rk_gemm_fp8_producer": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _int, _vp, _sz, _vp]),
     "rk_gemm_fp8_column_parallel": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp, _i64, _i64, _vp, _int, _int, _vp, _vp, _sz, _vp]),

@@ -123,9 +123,17 @@ def quantize_swiglu_bf16(gate_up, intermediate_size, scale=None):
     out_scale = scale if scale is not None else torch.empty(1, device=gate_up.device, dtype=torch.float32)
     with torch.cuda.device(gate_up.device):
         ws = _lib.workspace(gate_up.device, _lib.WORKSPACE_HEADER)
-        code = _lib.load().rk_swiglu_quant_fp8(_lib.ptr(gate_up), rows, inter, _lib.ptr(scale), _lib.ptr(q),
-                                               _lib.ptr(out_scale), _lib.ptr(ws), ws.numel(),
-                                               _lib.stream_ptr(gate_up.device))
+        if scale is None and rows * inter <= 1 << 29:
+            # the pass that finds the maximum keeps the activation (a per-call buffer half the size of the input), so that
+            # it is evaluated once: 816 x 16384 38.2 -> 28.1 us
+            product = torch.empty((rows, inter), device=gate_up.device, dtype=torch.bfloat16)
+            code = _lib.load().rk_swiglu_quant_fp8_product(_lib.ptr(gate_up), rows, inter, _lib.ptr(product), _lib.ptr(q),
+                                                           _lib.ptr(out_scale), _lib.ptr(ws), ws.numel(),
+                                                           _lib.stream_ptr(gate_up.device))
+        else:
+            code = _lib.load().rk_swiglu_quant_fp8(_lib.ptr(gate_up), rows, inter, _lib.ptr(scale), _lib.ptr(q),
+                                                   _lib.ptr(out_scale), _lib.ptr(ws), ws.numel(),
+                                                   _lib.stream_ptr(gate_up.device))
     _lib.check(code, "quantize_swiglu_bf16")
     return q, out_scale
 

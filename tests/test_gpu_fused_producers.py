@@ -381,3 +381,26 @@ def test_swiglu_steps_on_every_bf16_gate(up):
     r = (1.0 / (1.0 + e.float()).bfloat16().float()).bfloat16()
     want = ((gate.float() * r.float()).bfloat16().float() * ups.float()).bfloat16()
     assert torch.equal(torch.nan_to_num(got.float(), nan=-7.5), torch.nan_to_num(want.float(), nan=-7.5))
+
+
+@pytest.mark.parametrize("rows,inter", [(1, 16), (37, 48), (3, 2064), (130, 4112), (816, 16384)])
+def test_kept_swiglu_product_gives_the_same_codes(rows, inter):
+    """`rk_swiglu_quant_fp8_product` (activation kept by the pass that finds the maximum) against `rk_swiglu_quant_fp8`
+    (activation evaluated twice): the same scale and codes, infinities and NaN included."""
+    lib, ptr = _lib.load(), _lib.ptr
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    gate_up = (torch.randn(rows, 2 * inter, generator=gen, device="cuda") * 3).bfloat16()
+    gate_up[0, :3] = torch.tensor([float("inf"), float("nan"), -3e38], device="cuda")
+    ws = _lib.workspace(gate_up.device, _lib.WORKSPACE_HEADER)
+    product = torch.full((rows, inter), 5.0, device="cuda", dtype=torch.bfloat16)
+    results = []
+    for kept in (False, True):
+        q = torch.full((rows, inter), 77, device="cuda", dtype=torch.uint8)
+        scale = torch.zeros(1, device="cuda")
+        tail = (ptr(q), ptr(scale), ptr(ws), ws.numel(), _lib.stream_ptr(gate_up.device))
+        if kept:
+            _lib.check(lib.rk_swiglu_quant_fp8_product(ptr(gate_up), rows, inter, ptr(product), *tail), "kept")
+        else:
+            _lib.check(lib.rk_swiglu_quant_fp8(ptr(gate_up), rows, inter, None, *tail), "twice")
+        results.append((q, scale))
+    assert torch.equal(results[0][1], results[1][1]) and torch.equal(results[0][0], results[1][0])
