@@ -12,6 +12,7 @@
 #include <cuda_fp4.h>
 #include <cuda_fp8.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "rk_blockscale.cuh"
@@ -265,7 +266,7 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const
     if constexpr (MODE != RK_ACT_PLAIN) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        v.w[i] = static_cast<uint32_t>(table[v.w[i] & 0xFFFFu]) | (static_cast<uint32_t>(table[v.w[i] >> 16]) << 16);
+        v.w[i] = static_cast<uint32_t>(__ldg(table + (v.w[i] & 0xFFFFu))) | (static_cast<uint32_t>(__ldg(table + (v.w[i] >> 16))) << 16);
         if constexpr (MODE == RK_ACT_LUT_MUL) v.w[i] = mul_bf16x2(v.w[i], u.w[i]);
       }
     }
@@ -315,45 +316,176 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const
   }
 }
 
+// ------------------------------------------------------------------ table activations with the table on chip
+// A gather of 32 random entries of the 128 KB table takes an SM's L1 about 20 cycles (one tag look-up per line) and
+// bounds the kernels above once there is enough work; from shared memory it takes three or four (bank conflicts
+// only).  So for large tensors one CTA of 1024 threads per SM copies the whole table first and then walks the rows.
+constexpr int kTableThreads = 1024;
+constexpr int kTableBytes = 65536 * 2;
+// Elements from which the table pays (long rows leave the L1 form few CTAs).  Measured, table in L1 against on chip - row
+// quantizer: 300 x 8192 8.1 -> 6.9 us, 1764 x 8192 17.9 -> 15.0, 196 x 8192 7.7 -> 7.0, 100 x 8192 5.4 -> 6.7, 1764 x 2048
+// 8.6 -> 6.9, 1300 x 2048 7.9 -> 6.7, 1000 x 2048 6.4 -> 6.8; product and maximum: 400 x 4096 5.2 -> 4.3, 816 x 2048
+// 5.1 -> 4.3, 1764 x 2048 7.4 -> 5.3, 400 x 1024 3.6 -> 3.6, 50 x 4096 3.1 -> 3.6.
+constexpr int64_t kTableRowsLine = 2400000, kTableLongRowsLine = 1300000;  // k up to 4096, beyond
+constexpr int64_t kTableProductLine = 1ll << 20;
+
+// every thread of the CTA: starts copying the table (eight 16-byte pieces each); table_arrive() completes it
+__device__ __forceinline__ void table_copy(const __nv_bfloat16* lut, uint8_t* smem) {
+  const uint32_t dst = smem_u32(smem);
+#pragma unroll
+  for (int i = 0; i < kTableBytes / 16 / kTableThreads; ++i) {
+    const uint32_t off = (i * kTableThreads + threadIdx.x) * 16;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + off), "l"(reinterpret_cast<const uint8_t*>(lut) + off)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void table_arrive() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+}
+__device__ __forceinline__ uint32_t table_pair(const unsigned short* table, uint32_t w) {
+  return static_cast<uint32_t>(table[w & 0xFFFFu]) | (static_cast<uint32_t>(table[w >> 16]) << 16);
+}
+
+// GROUP threads per row, four vectors of eight each (k <= GROUP * 32): the CTA holds 1024 / GROUP rows at a time and every
+// group walks on by itself (named barriers).  Values, codes and scales are those of quant_rows_kernel.
+template <int BITS, int MODE, int GROUP>
+__global__ void __launch_bounds__(kTableThreads, 1)
+quant_rows_table_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const __nv_bfloat16* __restrict__ up,
+                        long long up_stride, const __nv_bfloat16* __restrict__ lut, int k, int kpad, int n_rows,
+                        uint8_t* __restrict__ q, float* __restrict__ scales, int vec_ok) {
+  pdl_launch_dependents();  // every thread, before any return: see launch_pdl
+  pdl_wait();
+  extern __shared__ __align__(16) uint8_t smem_table[];
+  __shared__ float scratch[kTableThreads / 32];
+  table_copy(lut, smem_table);
+  const unsigned short* const table = reinterpret_cast<const unsigned short*>(smem_table);
+  constexpr int kGroups = kTableThreads / GROUP, kWarps = GROUP / 32;
+  const int group = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
+  float* const part = scratch + group * kWarps;
+  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(GROUP) : "memory"); };
+  const float limit = static_cast<float>((1 << (BITS - 1)) - 1);
+  bool first = true;
+  for (int row0 = blockIdx.x * kGroups; row0 < n_rows; row0 += gridDim.x * kGroups) {  // uniform over the CTA
+    const int row = row0 + group;
+    const bool live = row < n_rows;
+    Packed8 v[kMaxVec], u[MODE == RK_ACT_LUT_MUL ? kMaxVec : 1];
+#pragma unroll
+    for (int it = 0; it < kMaxVec; ++it) {
+      const int idx = (it * GROUP + t) * 8, valid = live ? k - idx : 0;
+      v[it] = load8p(x + row * x_stride + idx, vec_ok, valid);
+      if constexpr (MODE == RK_ACT_LUT_MUL) u[it] = load8p(up + row * up_stride + idx, vec_ok, valid);
+    }
+    if (first) table_arrive();  // the first rows are on their way meanwhile
+    first = false;
+    if (!live) continue;
+    uint32_t m = 0u;
+#pragma unroll
+    for (int it = 0; it < kMaxVec; ++it) {
+      const int idx = (it * GROUP + t) * 8;
+      if (idx >= k) continue;  // zeros stay zeros, whatever the table says
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[it].w[i] = table_pair(table, v[it].w[i]);
+        if constexpr (MODE == RK_ACT_LUT_MUL) v[it].w[i] = mul_bf16x2(v[it].w[i], u[it].w[i]);
+      }
+      if (idx + 8 > k) mask8(v[it], k - idx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m = absmax_bf16x2(m, v[it].w[i]);
+    }
+    const float local = warp_max(fmaxf(bf16_lo(m), bf16_hi(m)));
+    group_sync();  // the previous row's maxima have been read
+    if ((t & 31) == 0) part[t >> 5] = local;
+    group_sync();
+    float maximum = part[0];
+#pragma unroll
+    for (int w = 1; w < kWarps; ++w) maximum = fmaxf(maximum, part[w]);
+    const float scale = row_scale_from_max(maximum, limit, false);
+    if (t == 0) scales[row] = scale;
+    const float rcp = __frcp_rn(scale);
+    uint8_t* const qrow = q + static_cast<long long>(row) * (BITS == 8 ? kpad : kpad / 2);
+#pragma unroll
+    for (int it = 0; it < kMaxVec; ++it) {
+      const int idx = (it * GROUP + t) * 8;
+      if (idx < kpad) {
+        float f[8];
+        unpack8(v[it], f);
+        quantize_store8<BITS>(qrow, idx, f, scale, rcp, limit);
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------ table activation * up -> bf16 + tensor amax
 // out = bf16(table[x] * up) element by element (the arithmetic of the GELU-table mode of the row
 // quantizer above) and the absolute maximum of the finite results, for a per-tensor scale that a
 // block packer needs before it can run.  Eight elements per thread and step; rows may be strided.
-__global__ void __launch_bounds__(256)
+// ON_CHIP: 1024 threads per CTA, the table in shared memory (see quant_rows_table_kernel); else 256 threads, the table
+// gathered through L1.
+template <bool ON_CHIP>
+__global__ void __launch_bounds__(ON_CHIP ? kTableThreads : 256, 1)
 lut_mul_amax_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const __nv_bfloat16* __restrict__ up,
                     long long up_stride, const __nv_bfloat16* __restrict__ lut, long long rows, int k,
                     __nv_bfloat16* __restrict__ out, unsigned* __restrict__ staging) {
   pdl_launch_dependents();  // every thread, before any return: see launch_pdl
   pdl_wait();
-  __shared__ float scratch[8];
+  constexpr int kUnroll = 2;
+  extern __shared__ __align__(16) uint8_t smem_table[];
+  __shared__ uint32_t scratch[kTableThreads / 32];
+  const unsigned short* table = reinterpret_cast<const unsigned short*>(lut);
+  if constexpr (ON_CHIP) {
+    table_copy(lut, smem_table);
+    table = reinterpret_cast<const unsigned short*>(smem_table);
+  }
   const int per_row = k >> 3;
   const long long total = rows * per_row;
-  float local = 0.0f;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long row = i / per_row;
-    const int col = static_cast<int>(i - row * per_row) << 3;
-    const uint4 xv = *reinterpret_cast<const uint4*>(x + row * x_stride + col);
-    const uint4 uv = *reinterpret_cast<const uint4*>(up + row * up_stride + col);
-    const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
-    const uint32_t uw[4] = {uv.x, uv.y, uv.z, uv.w};
-    uint32_t ow[4];
+  const bool short_index = total < (1ll << 32);  // a 64-bit division costs as much as four gathers
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  uint32_t m = 0u;
+  bool first = true;
+  // the trip count is the same for every thread of the CTA: the first trip holds a barrier
+  for (long long base = static_cast<long long>(blockIdx.x) * blockDim.x; base < total; base += kUnroll * step) {
+    uint4 xv[kUnroll], uv[kUnroll];
+    long long dst[kUnroll];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float t0 = __bfloat162float(lut[xw[w] & 0xFFFFu]);
-      const float t1 = __bfloat162float(lut[xw[w] >> 16]);
-      const float r0 = round_bf16(__fmul_rn(t0, __uint_as_float(uw[w] << 16)));
-      const float r1 = round_bf16(__fmul_rn(t1, __uint_as_float(uw[w] & 0xFFFF0000u)));
-      const float a0 = fabsf(r0), a1 = fabsf(r1);
-      if (a0 <= 3.4028234664e38f) local = fmaxf(local, a0);
-      if (a1 <= 3.4028234664e38f) local = fmaxf(local, a1);
-      ow[w] = (__float_as_uint(r0) >> 16) | (__float_as_uint(r1) & 0xFFFF0000u);
+    for (int j = 0; j < kUnroll; ++j) {
+      const long long i = base + j * step + threadIdx.x;
+      dst[j] = -1;
+      if (i < total) {
+        const long long row = short_index ? static_cast<unsigned>(i) / static_cast<unsigned>(per_row) : i / per_row;
+        const int col = static_cast<int>(i - row * per_row) << 3;
+        xv[j] = *reinterpret_cast<const uint4*>(x + row * x_stride + col);
+        uv[j] = *reinterpret_cast<const uint4*>(up + row * up_stride + col);
+        dst[j] = row * k + col;
+      }
     }
-    *reinterpret_cast<uint4*>(out + row * k + col) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    if (ON_CHIP && first) table_arrive();
+    first = false;
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j) {
+      if (dst[j] < 0) continue;
+      uint32_t w[4] = {xv[j].x, xv[j].y, xv[j].z, xv[j].w};
+      const uint32_t u[4] = {uv[j].x, uv[j].y, uv[j].z, uv[j].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        w[i] = mul_bf16x2(table_pair(table, w[i]), u[i]);
+        // magnitudes order like their bit patterns; infinities and NaN count as zero
+        const uint32_t lo = w[i] & 0x7FFFu, hi = (w[i] >> 16) & 0x7FFFu;
+        m = max(m, lo < 0x7F80u ? lo : 0u);
+        m = max(m, hi < 0x7F80u ? hi : 0u);
+      }
+      *reinterpret_cast<uint4*>(out + dst[j]) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
   }
   if (staging != nullptr) {
-    const float block_max = block_reduce(local, true, scratch);
-    if (threadIdx.x == 0 && block_max > 0.0f) atomicMax(staging, __float_as_uint(block_max));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      m = threadIdx.x < (blockDim.x >> 5) ? scratch[threadIdx.x] : 0u;
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (threadIdx.x == 0 && m != 0u) atomicMax(staging, m << 16);  // the float of those upper bits
+    }
   }
 }
 
@@ -1169,6 +1301,28 @@ void with_row_shape(int64_t rows, int64_t kpad, F&& f) {
   else pick(integral_constant<int, 256>{});
 }
 
+// Table in shared memory or gathered through L1?  Copying it costs an SM about 2 us and leaves it one CTA, so there must be
+// enough work: `line` elements.
+bool table_on_chip(const void* lut, int64_t rows, int64_t k, int64_t line) { return aligned16(lut) && rows * k >= line; }
+// one CTA per SM (at most `blocks`) of a kernel whose dynamic shared memory is the table
+template <typename... KArgs, typename... Args>
+int launch_with_table(void (*kernel)(KArgs...), int64_t blocks, cudaStream_t st, Args&&... args) {
+  const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes);
+  if (set != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(set));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>(blocks, 148)));
+  cfg.blockDim = dim3(kTableThreads);
+  cfg.dynamicSmemBytes = kTableBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  return check_launch("table kernel");
+}
+
 template <int BITS>
 int launch_quant_rows(const void* x, int64_t rows, int64_t total_rows, int64_t k, int64_t xs, const void* up,
                       int64_t us, const void* lut, int mode, void* q, float* scales, int true_division,
@@ -1180,6 +1334,20 @@ int launch_quant_rows(const void* x, int64_t rows, int64_t total_rows, int64_t k
   auto lb = static_cast<const __nv_bfloat16*>(lut);
   auto qb = static_cast<uint8_t*>(q);
   const dim3 grid(static_cast<unsigned>(total_rows));
+  if (mode != RK_ACT_PLAIN && total_rows == rows && !true_division && kpad <= kCachedK && table_on_chip(lut, rows, k, k > 4096 ? kTableLongRowsLine : kTableRowsLine)) {
+    auto launch_table = [&](auto kernel, int group) {
+      return launch_with_table(kernel, (rows + kTableThreads / group - 1) / (kTableThreads / group), st, xb, xs, ub, us, lb,
+                               static_cast<int>(k), kpad, static_cast<int>(rows), qb, scales, vec_ok);
+    };
+    auto by_group = [&](auto mode_c) {
+      constexpr int kMode = decltype(mode_c)::value;
+      if (kpad <= 64 * 32) return launch_table(quant_rows_table_kernel<BITS, kMode, 64>, 64);
+      if (kpad <= 128 * 32) return launch_table(quant_rows_table_kernel<BITS, kMode, 128>, 128);
+      return launch_table(quant_rows_table_kernel<BITS, kMode, 256>, 256);
+    };
+    return mode == RK_ACT_LUT_MUL ? by_group(std::integral_constant<int, RK_ACT_LUT_MUL>{})
+                                  : by_group(std::integral_constant<int, RK_ACT_LUT>{});
+  }
   const int threads = row_threads(total_rows, kpad);
   const int vecs = row_vectors(threads, kpad);
   auto launch = [&](auto kernel) {
@@ -1359,10 +1527,17 @@ extern "C" int rk_lut_mul_tensor_scale(const void* x, int64_t x_stride, const vo
     staging = reinterpret_cast<unsigned*>(static_cast<uint8_t*>(workspace) + 64);  // zero between calls
   }
   const long long vectors = rows * (k / 8);
-  const unsigned blocks = static_cast<unsigned>(std::min<long long>((vectors + 255) / 256, 148LL * 8));
   auto b = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
-  launch_pdl(lut_mul_amax_kernel, blocks, 256, as_stream(stream), b(x), x_stride, b(up), up_stride, b(lut), rows,
-                                                             static_cast<int>(k), static_cast<__nv_bfloat16*>(out), staging);
+  if (table_on_chip(lut, rows, k, kTableProductLine)) {
+    const int rc = launch_with_table(lut_mul_amax_kernel<true>, (vectors + kTableThreads - 1) / kTableThreads, as_stream(stream),
+                                     b(x), x_stride, b(up), up_stride, b(lut), rows, static_cast<int>(k),
+                                     static_cast<__nv_bfloat16*>(out), staging);
+    if (rc != RK_OK) return rc;
+  } else {
+    const unsigned blocks = static_cast<unsigned>(std::min<long long>((vectors + 255) / 256, 148LL * 8));
+    launch_pdl(lut_mul_amax_kernel<false>, blocks, 256, as_stream(stream), b(x), x_stride, b(up), up_stride, b(lut), rows,
+               static_cast<int>(k), static_cast<__nv_bfloat16*>(out), staging);
+  }
   if (staging != nullptr) launch_pdl(finalize_scale_kernel, 1, 1, as_stream(stream), staging, divisor, scale_out);
   return check_launch(who);
 }

@@ -59,3 +59,40 @@ def test_the_shape_of_a_launch_never_changes_a_row(k, bits):
 
     for tall, few in zip(_bits(run(TALL)), _bits(run(FEW))):
         assert torch.equal(tall, few)
+
+
+@pytest.mark.parametrize("rows,k", [(1200, 2048), (331, 4100), (160, 8190), (1181, 2056), (150, 8192)])
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("strided", [False, True])
+def test_table_on_chip_equals_the_gathered_table(rows, k, bits, strided):
+    """Enough elements for the table in shared memory: rows equal the same rows in small launches (table through L1), for dense
+    and strided inputs, with groups of threads that run out of rows."""
+    lib, dev, ptr = _lib.load(), torch.device("cuda:0"), _lib.ptr
+    gen = torch.Generator(device=dev).manual_seed(rows + k)
+    pitch = k + 24 if strided else k
+    x, up = _randn(gen, rows, pitch)[:, :k], _randn(gen, rows, pitch)[:, :k]
+    table = _randn(gen, 65536)
+    table[0x4000:0x4010] = float("nan")
+    width = (k + 127) // 128 * 128 * bits // 8
+    ws = torch.zeros(_lib.WORKSPACE_HEADER, device=dev, dtype=torch.uint8)
+
+    def quantized(mode, first, count):
+        q, s = torch.full((count, width), 9, device=dev, dtype=torch.uint8), torch.zeros(count, device=dev)
+        _lib.check(lib.rk_quant_rows(ptr(x[first:]), count, k, pitch, ptr(up[first:]), pitch, ptr(table), mode, bits, ptr(q),
+                                     ptr(s), _lib.stream_ptr(dev)), "rows")
+        return q, s
+
+    for mode in (_lib.ACT_LUT_MUL, _lib.ACT_LUT):
+        q, s = quantized(mode, 0, rows)
+        for first in (0, rows // 2, rows - 20):
+            few_q, few_s = quantized(mode, first, 20)
+            assert torch.equal(q[first:first + 20], few_q) and torch.equal(s[first:first + 20], few_s)
+    if k % 8 == 0 and pitch % 8 == 0:
+        out, one = torch.zeros(rows, k, device=dev, dtype=torch.bfloat16), torch.zeros(1, device=dev)
+        _lib.check(lib.rk_lut_mul_tensor_scale(ptr(x), pitch, ptr(up), pitch, ptr(table), rows, k, 2688.0, ptr(out), ptr(one),
+                                               ptr(ws), ws.numel(), _lib.stream_ptr(dev)), "product")
+        index = x.contiguous().view(torch.int16).to(torch.int64) & 0xFFFF
+        want = (table[index].float() * up.float()).bfloat16()
+        assert torch.equal(torch.nan_to_num(out.float(), nan=-7.5), torch.nan_to_num(want.float(), nan=-7.5))
+        finite = want.float()[torch.isfinite(want)].abs().max().item()
+        assert one.item() == np.float32(finite) / np.float32(2688.0)
