@@ -327,8 +327,9 @@ class GemmaStack(nn.Module):
                 param.copy_((torch.randn(param.shape, generator=gen) * std).to(param.dtype))
         return self
 
-    def forward(self, x, positions, past=None, cond=None):
-        cos, sin = rope_tables(positions, self.cfg.head_dim, self.cfg.rope_theta, x.dtype)
+    def forward(self, x, positions, past=None, cond=None, rope=None):
+        """`rope`: the (cos, sin) tables of `positions`, for a caller that runs the stack on the same positions repeatedly."""
+        cos, sin = rope if rope is not None else rope_tables(positions, self.cfg.head_dim, self.cfg.rope_theta, x.dtype)
         presents = []
         pending = None
         for index, layer in enumerate(self.layers):
@@ -419,12 +420,15 @@ class ActionExpert(nn.Module):
             self._conditions[key] = compute()
         return self._conditions[key]
 
-    def denoise_step(self, x_t, time, prefix_kv, prefix_len, step=None):
-        b = x_t.shape[0]
+    def positions(self, batch, prefix_len, device):
+        """Positions of the chunk tokens behind a prefix: the same in every denoising step."""
+        return prefix_len + torch.arange(self.chunk, device=device)[None, :].expand(batch, -1)
+
+    def denoise_step(self, x_t, time, prefix_kv, prefix_len, step=None, rope=None):
         cond = self.condition(time, step)
         tokens = self.action_in_proj(x_t).to(torch.bfloat16)
-        positions = prefix_len + torch.arange(self.chunk, device=x_t.device)[None, :].expand(b, -1)
-        hidden, _ = self.stack(tokens, positions, past=prefix_kv, cond=cond)
+        positions = self.positions(x_t.shape[0], prefix_len, x_t.device) if rope is None else None
+        hidden, _ = self.stack(tokens, positions, past=prefix_kv, cond=cond, rope=rope)
         return self.action_out_proj(hidden.float())
 
     def forward(self, noise, prefix_k, prefix_v):
@@ -448,11 +452,13 @@ class ActionExpert(nn.Module):
             prefix_kv = [(k_all[i], v_all[i], prefix_len, vt_all[i]) for i in range(depth)]
         else:
             prefix_kv = [(k_all[i], v_all[i], prefix_len) for i in range(depth)]
+        # every step has the same positions: one set of rotary tables instead of a dozen small launches per step
+        rope = rope_tables(self.positions(b, prefix_len, noise.device), self.cfg.head_dim, self.cfg.rope_theta, torch.bfloat16)
         dt = -1.0 / self.steps
         x_t = noise
         for step in range(self.steps):
             time = torch.full((b,), 1.0 + step * dt, device=noise.device, dtype=torch.float32)
-            x_t = x_t + dt * self.denoise_step(x_t, time, prefix_kv, prefix_len, step)
+            x_t = x_t + dt * self.denoise_step(x_t, time, prefix_kv, prefix_len, step, rope)
         return x_t
 
 
