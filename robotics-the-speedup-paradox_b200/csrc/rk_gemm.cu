@@ -442,7 +442,7 @@ int launch_tc_peer(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const PeerM
 
 template <int KIND, bool REPACK>
 int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
-               const CUtensorMap& tm_sfb, const Gemm2Params& p, int smem, cudaStream_t st) {
+               const CUtensorMap& tm_sfb, const CUtensorMap& tm_tail, const Gemm2Params& p, int smem, cudaStream_t st) {
   static bool configured_dev[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -457,7 +457,7 @@ int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CU
   const int clusters = tiles < kNumSms / 2 ? tiles : kNumSms / 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * clusters, 1, 1);
-  cfg.blockDim = dim3(REPACK ? kGemm2ThreadsSwiglu : kGemmThreads);
+  cfg.blockDim = dim3(gemm2_threads(KIND, REPACK));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -469,7 +469,7 @@ int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CU
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc2_kernel<KIND, REPACK>, tm_a, tm_b, tm_out, tm_sfa, tm_sfb, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc2_kernel<KIND, REPACK>, tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(RK_ECUDA, "rk_gemm_tc2_kernel launch: %s", cudaGetErrorString(e));
@@ -479,11 +479,11 @@ int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CU
 
 template <int KIND>
 int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
-               const CUtensorMap& tm_sfb, const Gemm2Params& p, int smem, cudaStream_t st) {
+               const CUtensorMap& tm_sfb, const CUtensorMap& tm_tail, const Gemm2Params& p, int smem, cudaStream_t st) {
   if constexpr (KIND == KIND_MXF8 || KIND == KIND_NVF4) {
-    if (p.sw_q != nullptr) return launch_tc2_kernel<KIND, true>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, p, smem, st);
+    if (p.sw_q != nullptr) return launch_tc2_kernel<KIND, true>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
   }
-  return launch_tc2_kernel<KIND, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, p, smem, st);
+  return launch_tc2_kernel<KIND, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
 }
 
 // A box of the 16 x U4 -> 16-byte-aligned tensor-map type writes 128 bytes per row into shared memory
@@ -565,7 +565,22 @@ int run_tc(const TcArgs& a) {
       return v ? std::atoi(v) : 0;
     }();
     if (!block_scaled) {
-      p2.bn = ((a.tactic & 4) || a.n < 256) ? 128 : 256;
+      // A stage costs an SM the operands it takes from L2 (about 64 bytes a clock: 256 + bn cycles; its MMAs take 2 bn), the
+      // launch as many stages as its busiest pair: the width with the least of that, in the steps of 32 that a pair's MMA
+      // takes.  1764 rows are 7 pair tiles: 2048 columns are 56 tiles of 256 or 70 of 224 for 74 pairs, 8192 columns 224 of
+      // 256 (four rounds, the last for two tiles) or 259 of 224.  256 columns against the rule's choice, W8A8: 1764 x 2048 x
+      // 8192 24.6 -> 22.7 us (224), 1764 x 6144 x 2048 20.0 -> 18.6 (224), 1100 x 1024 x 4096 14.4 -> 9.8 (128), 3264 x 2048 x
+      // 16384 81.9 -> 74.8 (192), 1200 x 3000 x 896 12.3 -> 8.2 (224); 4096 x 8192 x 8192 stays at 256.
+      p2.bn = 128;
+      if (!(a.tactic & 4) && a.n >= 256) {
+        const int64_t tiles_m = (a.m + 255) / 256;
+        int64_t best = -1;
+        for (int bn = 256; bn >= 128; bn -= 32) {
+          const int64_t rounds = (tiles_m * ((a.n + bn - 1) / bn) + kNumSms / 2 - 1) / (kNumSms / 2);
+          const int64_t cost = rounds * kblocks * (256 + bn) + 10 * bn;
+          if (best < 0 || cost < best) best = cost, p2.bn = bn;
+        }
+      }
       p2.acc_bufs = 2;
     } else {
       // The scale factors need tensor-memory columns of their own: 128- and 192-column tiles keep two
@@ -617,7 +632,7 @@ int run_tc(const TcArgs& a) {
     p2.sw_mode = a.swiglu_mode;
     p2.sw_kt = a.swiglu_table != nullptr ? static_cast<int>((a.n / 2 / 32 + 3) / 4) : static_cast<int>(a.n / 128);
     p2.status = ws.status;
-    CUtensorMap t_act, t_wgt, t_out, t_sfa, t_sfb;
+    CUtensorMap t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail;
     rc = make_map_2d(&t_act, a.act, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.k_bytes, a.m, a.k_bytes, kStageKBytes, kTileA,
                      CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != RK_OK) return rc;
@@ -637,6 +652,11 @@ int run_tc(const TcArgs& a) {
     }
     t_sfa = t_act;
     t_sfb = t_act;
+    t_tail = t_out;
+    if (p2.bn % 64 != 0) {  // the last 32 columns of every tile leave through boxes of their own
+      rc = make_map_2d(&t_tail, a.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.n, a.m, a.n * 2, 32, 128, CU_TENSOR_MAP_SWIZZLE_64B);
+      if (rc != RK_OK) return rc;
+    }
     if (block_scaled) {
       // scale buffers as [chunks, 128] 32-bit words; one box = the chunks of one stage and row block
       const uint32_t chunks = a.kind == KIND_NVF4 ? 4 : 1;
@@ -649,10 +669,10 @@ int run_tc(const TcArgs& a) {
     }
     const int smem = p2.stages * stage + 2 * kOutBufBytes + kVecBytes + 1024;
     switch (a.kind) {
-      case KIND_I8: return launch_tc2<KIND_I8>(t_act, t_wgt, t_out, t_sfa, t_sfb, p2, smem, a.stream);
-      case KIND_F8: return launch_tc2<KIND_F8>(t_act, t_wgt, t_out, t_sfa, t_sfb, p2, smem, a.stream);
-      case KIND_MXF8: return launch_tc2<KIND_MXF8>(t_act, t_wgt, t_out, t_sfa, t_sfb, p2, smem, a.stream);
-      default: return launch_tc2<KIND_NVF4>(t_act, t_wgt, t_out, t_sfa, t_sfb, p2, smem, a.stream);
+      case KIND_I8: return launch_tc2<KIND_I8>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);
+      case KIND_F8: return launch_tc2<KIND_F8>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);
+      case KIND_MXF8: return launch_tc2<KIND_MXF8>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);
+      default: return launch_tc2<KIND_NVF4>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);
     }
   }
   const Plan pl = make_plan(a.kind, a.m, a.n, kblocks, a.tactic);

@@ -21,8 +21,8 @@
 // 64 bytes per clock): a pair halves the weight bytes per SM and MMA, which is where the speed-up
 // over the one-CTA kernel comes from.
 //
-// Warp roles per CTA (192 threads): warp 0 = TMA producer, warp 1 = TMEM allocation (+ MMA issue
-// in the leader), warps 2..5 = epilogue.
+// Warp roles per CTA: warp 0 = TMA producer, warp 1 = TMEM allocation (+ MMA issue in the leader), the others =
+// epilogue: four warps, eight for the kinds without block scales, sixteen for the re-packing epilogues.
 #pragma once
 
 #include <cuda.h>
@@ -38,11 +38,18 @@ namespace rk {
 // four.  816 x 32768 x 2048: 131.7 us with four warps, 82.5 with eight.
 constexpr int kGemm2SwigluSets = 4;
 constexpr int kGemm2ThreadsSwiglu = 64 + 128 * kGemm2SwigluSets;
+// The plain epilogue of the kinds without block scales: two sets of four warps take alternate 64-column chunks, each
+// with its own staging buffer.  It halves the tail after the last tile, which nothing hides (with the tile widths of
+// run_tc and the early weight fetch: four W8A8 video-diffusion blocks of 1764 tokens 538 -> 514 us).
+__host__ __device__ constexpr int gemm2_epi_sets(int kind, bool repack) {
+  return repack ? kGemm2SwigluSets : (kind == KIND_I8 || kind == KIND_F8 ? 2 : 1);
+}
+__host__ __device__ constexpr int gemm2_threads(int kind, bool repack) { return 64 + 128 * gemm2_epi_sets(kind, repack); }
 
 struct Gemm2Params {
   int m, n, kblocks;
   int k_valid_mmas_last;
-  int bn;        // weight rows per pair tile (128, 192 or 256); each CTA loads bn / 2
+  int bn;        // weight rows per pair tile (a multiple of 32, 128 .. 256); each CTA loads bn / 2
   int stages;
   int out_bufs;
   int acc_bufs;  // accumulator buffers in tensor memory (2, or 1 when bn = 256 shares it with scale columns)
@@ -177,12 +184,13 @@ __host__ __device__ inline int gemm2_stage_bytes(int kind, int bn, int sfb_block
 
 // REPACK: the epilogues that never write the bf16 tile (sw_q set), on sixteen warps.
 template <int KIND, bool REPACK>
-__global__ void __launch_bounds__(REPACK ? kGemm2ThreadsSwiglu : kGemmThreads, 1)
+__global__ void __launch_bounds__(gemm2_threads(KIND, REPACK), 1)
 rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                    const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_sfa,
-                   const __grid_constant__ CUtensorMap tm_sfb, const Gemm2Params p) {
+                   const __grid_constant__ CUtensorMap tm_sfb, const __grid_constant__ CUtensorMap tm_tail, const Gemm2Params p) {
   using T = KindTraits<KIND>;
   constexpr int kC = T::kSfChunksPerStage;  // scale chunks per stage and 128-row block
+  constexpr int kSets = gemm2_epi_sets(KIND, REPACK);  // epilogue warp sets
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t bar_full[kMaxStages];    // used in the leader: both CTAs' loads land
   __shared__ __align__(8) uint64_t bar_empty[kMaxStages];   // per CTA: the MMAs have read this stage
@@ -208,6 +216,12 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   const int tile_step = static_cast<int>(gridDim.x >> 1);
 
   pdl_launch_dependents();
+  if (!T::kBlockScaled && threadIdx.x == 64 && tile_first < num_tiles) {
+    // the weight rows of the first tile start their way from DRAM to L2 while the preceding kernel drains (weights are
+    // parameters, never that kernel's output; the block-scaled kinds measured 0.3 us slower with it)
+    const int row_b0 = (tile_first % p.tiles_n) * p.bn + static_cast<int>(rank) * half_bn;
+    for (int kb = 0; kb < min(p.kblocks, p.stages) && row_b0 < p.n; ++kb) tma_prefetch_l2_2d(&tm_b, kb * kStageKBytes, row_b0);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
@@ -215,7 +229,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_acc_full[b]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[b]), REPACK ? 8 * kGemm2SwigluSets : 8);  // the epilogue warps of both CTAs of the pair
+      mbar_init(smem_u32(&bar_acc_empty[b]), 8 * kSets);  // the epilogue warps of both CTAs of the pair
     }
     abort_flag = 0;
     sw_amax_bits = 0u;
@@ -225,6 +239,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     tma_prefetch_desc(&tm_a);
     tma_prefetch_desc(&tm_b);
     tma_prefetch_desc(&tm_out);
+    tma_prefetch_desc(&tm_tail);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -410,7 +425,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       if (p.scale_act) s_act_scalar = *p.scale_act;
       if (p.scale_wgt) s_wgt_scalar = *p.scale_wgt;
     }
-    const int epi_threads = static_cast<int>(blockDim.x) - 64;  // 128, or 512 with the re-packing epilogue
+    constexpr int epi_threads = 128 * kSets;
     const int set = (warp - 2) >> 2;                              // which of a lane quadrant's warps (re-packing epilogue)
     auto epi_sync = [](int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); };
     const uint32_t acc_empty_leader0 = mapa_u32(smem_u32(&bar_acc_empty[0]), 0);
@@ -429,7 +444,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       }
       if constexpr (!REPACK) {
         epi_sync(epi_threads);
-        for (int j = et; j < p.bn; j += 128) {
+        for (int j = set * 128 + et; j < p.bn; j += epi_threads) {
           const int rb = row_b0 + j;
           float sv = 1.0f, bv = 0.0f;
           if (rb < p.n) {
@@ -580,45 +595,65 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         }
         continue;
       }
-      for (int cc = 0; cc < p.bn; cc += 64, obuf = (p.out_bufs == 2) ? (obuf ^ 1) : 0) {
-        uint8_t* const stage = smem_gen + out_stage_off + obuf * kOutBufBytes;
+      // one set alternates between both staging buffers, two sets own one each
+      auto set_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + set) : "memory"); };
+      for (int cc = set * 64; cc < p.bn; cc += 64 * kSets, obuf ^= 1) {
+        uint8_t* const stage = smem_gen + out_stage_off + (kSets == 1 ? obuf : set) * kOutBufBytes;
         if (et == 0 && pending_store) {
-          if (p.out_bufs == 2) tma_store_wait_read<1>();
+          if (kSets == 1) tma_store_wait_read<1>();
           else tma_store_wait_read<0>();
         }
-        epi_bar_sync();
+        set_sync();
+        const int cols = T::kBlockScaled ? 64 : min(64, p.bn - cc);  // 64, or 32 for the tail of a tile whose width is not a multiple of 64
 #pragma unroll
-        for (int c0 = 0; c0 < 64; c0 += 16) {
-          uint32_t r[16];
+        for (int c0 = 0; c0 < 64; c0 += 32) {
+          if (c0 >= cols) break;
+          uint32_t r0[16], r1[16];
           __syncwarp();
-          tmem_ld_16(t_acc + cc + c0, r);
+          tmem_ld_16(t_acc + cc + c0, r0);
+          if (!T::kBlockScaled) tmem_ld_16(t_acc + cc + c0 + 16, r1);
           tc_wait_ld();
-          float v[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            if constexpr (KIND == KIND_I8)
-              v[j] = finish_value<KIND>(r[j], row_scale, vec_scale[cc + c0 + j], has_bias, vec_bias[cc + c0 + j]);
-            else
-              v[j] = finish_value<KIND>(r[j], s_act_scalar, s_wgt_scalar, has_bias, vec_bias[cc + c0 + j]);
+          for (int h = 0; h < 2; ++h) {
+            if (T::kBlockScaled && h == 1) {  // one load at a time measured faster beside the scale copies (112.7 / 114.0 us)
+              __syncwarp();
+              tmem_ld_16(t_acc + cc + c0 + 16, r1);
+              tc_wait_ld();
+            }
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const uint32_t bits = h == 0 ? r0[j] : r1[j];
+              const int col = cc + c0 + h * 16 + j;
+              if constexpr (KIND == KIND_I8)
+                v[j] = finish_value<KIND>(bits, row_scale, vec_scale[col], has_bias, vec_bias[col]);
+              else
+                v[j] = finish_value<KIND>(bits, s_act_scalar, s_wgt_scalar, has_bias, vec_bias[col]);
+            }
+            const uint4 lo = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                        pack_bf16x2(v[6], v[7]));
+            const uint4 hi = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
+                                        pack_bf16x2(v[14], v[15]));
+            const int ch = (c0 >> 3) + 2 * h;
+            if (cols == 64) {  // rows of 128 bytes in the 128-byte swizzle
+              *reinterpret_cast<uint4*>(stage + et * 128 + ((ch ^ (et & 7)) << 4)) = lo;
+              *reinterpret_cast<uint4*>(stage + et * 128 + (((ch + 1) ^ (et & 7)) << 4)) = hi;
+            } else {           // rows of 64 bytes in the 64-byte swizzle
+              *reinterpret_cast<uint4*>(stage + et * 64 + ((ch ^ ((et >> 1) & 3)) << 4)) = lo;
+              *reinterpret_cast<uint4*>(stage + et * 64 + (((ch + 1) ^ ((et >> 1) & 3)) << 4)) = hi;
+            }
           }
-          const uint4 lo = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
-                                      pack_bf16x2(v[6], v[7]));
-          const uint4 hi = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
-                                      pack_bf16x2(v[14], v[15]));
-          const int ch = c0 >> 3;
-          *reinterpret_cast<uint4*>(stage + et * 128 + ((ch ^ (et & 7)) << 4)) = lo;
-          *reinterpret_cast<uint4*>(stage + et * 128 + (((ch + 1) ^ (et & 7)) << 4)) = hi;
         }
-        if (cc + 64 >= p.bn) {
-          // accumulator drained: tell the leader's MMA thread (its barrier counts both CTAs' warps)
+        if (cc + 64 * kSets >= p.bn) {
+          // this warp has drained its chunks: tell the leader's MMA thread (its barrier counts both CTAs' warps)
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
         }
         fence_proxy_async_smem();
-        epi_bar_sync();
+        set_sync();
         if (et == 0) {
-          if (ok) tma_store_2d(&tm_out, smem_u32(stage), row_b0 + cc, row_a0);
+          if (ok) tma_store_2d(cols == 64 ? &tm_out : &tm_tail, smem_u32(stage), row_b0 + cc, row_a0);
           tma_store_commit();
           pending_store = 1;
         }

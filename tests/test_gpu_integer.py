@@ -306,3 +306,37 @@ def test_residual_epilogue_refuses_bad_arguments(H):
     assert lib.rk_gemm_int_residual(*args(_lib.ptr(stream), 7)) == _lib.RK_EINVAL
     assert lib.rk_gemm_int_residual(*args(_lib.ptr(stream), 0)) == _lib.RK_EINVAL
     assert lib.rk_gemm_int_residual(*args(_lib.ptr(stream), 60)) == _lib.RK_OK
+
+
+# pair tiles of 224 (the second tile row ends 32 columns in), 256, 192, 160 and 128 columns; ragged rows and columns
+@pytest.mark.parametrize("m,n,k", [(1764, 2048, 2048), (1764, 6144, 1024), (2048, 2048, 1024), (3264, 2048, 2048), (2304, 1200, 256),
+                                   (1025, 264, 384), (1100, 2376, 384), (1300, 3000, 896), (1030, 4640, 1024)])
+@pytest.mark.parametrize("kind", ["int8", "fp8"])
+def test_pair_tiles_of_every_width(m, n, k, kind):
+    """W8A8 and FP8 above 1024 rows: small integer operands make every product and sum exact, so the outputs are known."""
+    from rk_b200 import _lib
+
+    lib, ptr, dev = _lib.load(), _lib.ptr, torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(m + n)
+    high = 128 if kind == "int8" else 9  # e4m3 holds the integers up to 16
+    a = torch.randint(1 - high, high, (m, k), generator=gen, device=dev)
+    b = torch.randint(1 - high, high, (n, k), generator=gen, device=dev)
+    bias = torch.randn(n, generator=gen, device=dev).bfloat16()
+    acc = (a.double() @ b.double().t()).float()  # below 2^24 for fp8, rounded once from the exact integer for int8
+    buf = torch.full((m + 2, n), 7.0, device=dev, dtype=torch.bfloat16)
+    out, ws = buf[1:m + 1], _lib.workspace(dev, _lib.WORKSPACE_HEADER)
+    tail = (ptr(bias), ptr(out), m, n, k)
+    if kind == "int8":
+        qa, qb = a.to(torch.int8), b.to(torch.int8)
+        sa, sb = torch.rand(m, generator=gen, device=dev) * 0.01, torch.rand(n, generator=gen, device=dev) * 0.01
+        code = lib.rk_gemm_int(ptr(qa), ptr(sa), ptr(qb), ptr(sb), *tail, 8, 0, ptr(ws), ws.numel(), _lib.stream_ptr(dev))
+        want = (acc * sa[:, None]) * sb[None, :] + bias.float()[None, :]
+    else:
+        qa, qb = a.to(torch.float8_e4m3fn), b.to(torch.float8_e4m3fn)
+        sa, sb = torch.full((1,), 0.03125, device=dev), torch.full((1,), 0.0078125, device=dev)
+        code = lib.rk_gemm_fp8(ptr(qa), ptr(sa), ptr(qb), ptr(sb), *tail, 0, ptr(ws), ws.numel(), _lib.stream_ptr(dev))
+        want = acc * (sa * sb) + bias.float()[None, :]
+    _lib.check(code, kind)
+    assert torch.equal(out.view(torch.int16), want.bfloat16().view(torch.int16))
+    assert (buf[0] == 7.0).all() and (buf[m + 1] == 7.0).all()
+    assert _lib.read_status(ws) == 0
