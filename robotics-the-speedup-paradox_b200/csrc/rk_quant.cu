@@ -361,9 +361,12 @@ quant_rows_table_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride,
   table_copy(lut, smem_table);
   const unsigned short* const table = reinterpret_cast<const unsigned short*>(smem_table);
   constexpr int kGroups = kTableThreads / GROUP, kWarps = GROUP / 32;
+  // One named barrier per group.  A CTA has sixteen, 0 to 15, and GROUP = 64 needs them all: group 0 takes barrier 0, which is
+  // free again because its only other use, table_arrive(), lies before the first group_sync() of every thread.
+  static_assert(kGroups <= 16, "a CTA has sixteen named barriers");
   const int group = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
   float* const part = scratch + group * kWarps;
-  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(GROUP) : "memory"); };
+  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(group), "n"(GROUP) : "memory"); };
   const float limit = static_cast<float>((1 << (BITS - 1)) - 1);
   bool first = true;
   for (int row0 = blockIdx.x * kGroups; row0 < n_rows; row0 += gridDim.x * kGroups) {  // uniform over the CTA

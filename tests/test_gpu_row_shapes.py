@@ -96,3 +96,32 @@ def test_table_on_chip_equals_the_gathered_table(rows, k, bits, strided):
         assert torch.equal(torch.nan_to_num(out.float(), nan=-7.5), torch.nan_to_num(want.float(), nan=-7.5))
         finite = want.float()[torch.isfinite(want)].abs().max().item()
         assert one.item() == np.float32(finite) / np.float32(2688.0)
+
+
+@pytest.mark.parametrize("k,group", [(2048, 64), (520, 64), (2056, 128), (4096, 128), (8190, 256)])
+@pytest.mark.parametrize("mode", ["gelu", "gelu times up"])
+def test_every_row_of_every_trip_of_the_table_kernel(k, group, mode):
+    """Two full trips of 148 CTAs with 1024 / `group` rows each and a third for five rows, so every group of threads of a CTA
+    (sixteen with 64 threads per row: as many as it has named barriers) takes several rows.  Every row equals the same
+    row in small launches, which gather the table through L1."""
+    lib, dev, ptr = _lib.load(), torch.device("cuda:0"), _lib.ptr
+    rows, few = 2 * 148 * (1024 // group) + 5, 1200000 // k  # fewer elements than the table in shared memory asks for
+    gen = torch.Generator(device=dev).manual_seed(k)
+    # rows of very different size: a maximum taken from another row or another warp's half shows in the scale
+    x = _randn(gen, rows, k) * torch.logspace(-2, 2, 31, device=dev)[torch.arange(rows, device=dev) % 31, None].bfloat16()
+    up = _randn(gen, rows, k)
+    table = torch.nn.functional.gelu(torch.arange(65536, device=dev, dtype=torch.int32).to(torch.int16).view(torch.bfloat16))
+    act = _lib.ACT_LUT if mode == "gelu" else _lib.ACT_LUT_MUL
+    width = (k + 127) // 128 * 128
+
+    def quantized(first, count):
+        q, s = torch.full((count, width), 9, device=dev, dtype=torch.int8), torch.zeros(count, device=dev)
+        _lib.check(lib.rk_quant_rows(ptr(x[first:]), count, k, k, ptr(up[first:]), k, ptr(table), act, 8, ptr(q), ptr(s),
+                                     _lib.stream_ptr(dev)), mode)
+        return q, s
+
+    q, s = quantized(0, rows)
+    for first in range(0, rows, few):
+        count = min(few, rows - first)
+        few_q, few_s = quantized(first, count)
+        assert torch.equal(q[first:first + count], few_q) and torch.equal(s[first:first + count], few_s)
