@@ -259,8 +259,10 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
     const float m_raw = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
     const float m_own = m_raw > -INFINITY ? attn_score(__float_as_uint(m_raw), p.scaling) : -INFINITY;
-    // pass 2: e = exp(score - m_own) once per score, summed, and written back over the score (fp32)
-    const float mneg = -m_own * log2e;
+    // pass 2: e = exp(score - m_own) once per score, summed, and written back over the score (fp32).  A share of -infinities,
+    // or of scores so low (below -2.3e38) that m_own * log2e overflows, gives e = 0 and a sum of zero, not infinity - infinity:
+    // beside any larger score of the row it weighs nothing.
+    const float mneg = fminf(-m_own * log2e, 3.4028234664e38f);
     float ls[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int c0 = half * 32; c0 < p.keys; c0 += 64) {
       uint32_t a[32];
@@ -303,7 +305,8 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     for (int q = 0; q < 16; ++q)  // fixed order: slice 0 (even chunks, odd chunks), slice 1, ...; a part without keys adds zero
       l_glob = fmaf(pl[q], pm[q] > -INFINITY ? attn_ex2((pm[q] - m_glob) * log2e) : 0.0f, l_glob);
     const float own = m_own > -INFINITY ? attn_ex2((m_own - m_glob) * log2e) : 0.0f;
-    const float inv_l = l_glob > 0.0f ? __fdiv_rn(own, l_glob) : 0.0f;
+    // a row with nothing above those lowest scores has no probabilities: NaN, as softmax of all -infinity gives
+    const float inv_l = l_glob > 0.0f ? __fdiv_rn(own, l_glob) : (m_glob < 0.0f ? __uint_as_float(0x7FC00000u) : 0.0f);
     // pass 3: probabilities as packed bf16 over the values they replace.  Packed column j covers the
     // fp32 columns 2j, 2j + 1; chunk c lands in the first (c even) or second (c odd) half of chunk
     // c / 2, which one of the row's two threads read in this step or an earlier one: a barrier of

@@ -118,3 +118,34 @@ def test_attention_with_any_number_of_key_slices(batch, prefix):
     want = OA.attention(q.permute(0, 2, 1, 3).float().numpy(), k.float().numpy(), v.float().numpy(), 256 ** -0.5)
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < TOL
     assert _lib.read_status(_lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)) == 0
+
+
+@pytest.mark.parametrize("batch", [1, 5])
+@pytest.mark.parametrize("case", ["two shares", "last key", "every key"])
+def test_attention_where_a_share_of_the_keys_weighs_nothing(case, batch):
+    """Scores of -infinity and near the type's lowest value.  "two shares": with 613 keys in four slices of 160, one thread's
+    keys (alternate chunks of 32 in a slice) all at -infinity, another's at -3e38.  "last key": 385 keys are slices of 128 and
+    the last holds one key, at -infinity.  Such keys weigh zero and every row stays finite; a row of -infinities is NaN, as
+    in the tensor ops."""
+    prefix, scaling = (335, 256 ** -0.5) if case == "last key" else (563, 1.0)
+    q, k, v, kv_len, pitch = make_inputs(batch, 50, 8, 1, prefix, 24)
+    q *= 0.0625
+    q[..., 0] = 1.0
+    if case == "two shares":
+        for chunk in (160 + 32, 160 + 96):
+            k[:, :, chunk:chunk + 32, 0] = float("-inf")
+        for chunk in (320, 320 + 64, 320 + 128):
+            k[:, :, chunk:chunk + 32, 0] = -3e38
+    elif case == "last key":
+        k[:, :, kv_len - 1, 0] = float("-inf")
+    else:
+        k[..., 0] = float("-inf")
+    vt_all = torch.zeros((batch, 1, 256, pitch), dtype=torch.bfloat16)
+    vt_all[..., :kv_len] = v.transpose(-1, -2)
+    got = attention_prefix(q.to(DEVICE), k.to(DEVICE), vt_all.to(DEVICE), kv_len, scaling).float().cpu().numpy()
+    assert _lib.read_status(_lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)) == 0
+    if case == "every key":
+        assert np.isnan(got).all()
+        return
+    want = OA.attention(q.permute(0, 2, 1, 3).float().numpy(), k.float().numpy(), v.float().numpy(), scaling)
+    assert np.isfinite(got).all() and np.linalg.norm(got - want) / np.linalg.norm(want) < TOL
