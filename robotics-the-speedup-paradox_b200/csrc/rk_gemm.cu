@@ -1002,17 +1002,25 @@ extern "C" int rk_gemm_int(const void* a, const float* sa, const void* b, const 
                          "rk_gemm_int");
 }
 
-extern "C" int rk_gemm_int_residual(const void* a, const float* sa, const void* b, const float* sb, const void* bias,
-                                    const void* residual, const void* gate, int64_t tokens, void* out, int64_t m, int64_t n,
-                                    int64_t kpad, int bits, int tactic, void* workspace, size_t workspace_bytes,
-                                    void* stream) {
-  const char* who = "rk_gemm_int_residual";
+// The arguments of the residual epilogue (gate may be null).
+static int check_residual(const char* who, const void* residual, const void* gate, int64_t tokens, const void* out, int64_t m,
+                          int64_t n) {
   if (!residual || !out) return fail(RK_EINVAL, "%s: null pointer", who);
   if (tokens < 1 || m < 1 || m % tokens != 0) return fail(RK_EINVAL, "%s: m must be a positive multiple of tokens", who);
   if (static_cast<unsigned long long>(m) * static_cast<unsigned long long>(tokens) >= (1ull << 32))
     return fail(RK_EUNSUPPORTED, "%s: m * tokens must stay below 2^32", who);
   if (n % 8 != 0 || (reinterpret_cast<uintptr_t>(residual) & 1u) || (gate && (reinterpret_cast<uintptr_t>(gate) & 1u)))
     return fail(RK_EINVAL, "%s: n must be a multiple of 8 and the bf16 pointers 2-byte aligned", who);
+  return RK_OK;
+}
+
+extern "C" int rk_gemm_int_residual(const void* a, const float* sa, const void* b, const float* sb, const void* bias,
+                                    const void* residual, const void* gate, int64_t tokens, void* out, int64_t m, int64_t n,
+                                    int64_t kpad, int bits, int tactic, void* workspace, size_t workspace_bytes,
+                                    void* stream) {
+  const char* who = "rk_gemm_int_residual";
+  const int rc = check_residual(who, residual, gate, tokens, out, m, n);
+  if (rc != RK_OK) return rc;
   return gemm_int_common(a, sa, b, sb, bias, out, nullptr, m, n, kpad, bits, tactic, workspace, workspace_bytes, stream, who,
                          false, residual, gate, tokens);
 }
@@ -1031,8 +1039,13 @@ extern "C" int rk_gemm_int4_widened(const void* a, const float* sa, const void* 
     return fail(RK_EINVAL, "%s: operands and scratch must be 16-byte aligned", who);
   if (scratch_bytes < static_cast<size_t>(m + n) * static_cast<size_t>(kpad))
     return fail(RK_EWORKSPACE, "%s: scratch must hold (m + n) * kpad bytes", who);
+  // everything that the GEMM would refuse is refused here: a call that fails must not have queued work on the scratch
+  if (!aligned16(out)) return fail(RK_EINVAL, "%s: the output must be 16-byte aligned", who);
+  if (!residual && gate) return fail(RK_EINVAL, "%s: a gate needs a residual", who);
+  int rc = residual != nullptr ? check_residual(who, residual, gate, tokens, out, m, n) : RK_OK;
+  if (rc != RK_OK) return rc;
   Workspace ws;
-  int rc = carve_workspace(workspace, workspace_bytes, &ws, who);
+  rc = carve_workspace(workspace, workspace_bytes, &ws, who);
   if (rc != RK_OK) return rc;
   uint8_t* const a8 = static_cast<uint8_t*>(scratch);
   uint8_t* const b8 = a8 + static_cast<size_t>(m) * kpad;

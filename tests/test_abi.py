@@ -67,6 +67,26 @@ def test_argument_errors_are_reported_without_a_gpu(built_library):
         _lib.check(_lib.RK_EUNSUPPORTED, "probe")
 
 
+def test_widened_w4a4_gemm_refuses_bad_arguments_before_any_launch(built_library):
+    """Whatever the GEMM behind it would refuse: without a GPU a launch would fail with another code, so these codes show that
+    nothing was queued on the caller's scratch."""
+    from rk_b200 import _lib
+
+    lib = _lib.load()
+    m, n, k, buffer = 60, 128, 256, 1 << 20  # an aligned address; nothing reads it
+
+    def call(residual=buffer, gate=None, tokens=1, out=buffer, rows=m, workspace=buffer):
+        return lib.rk_gemm_int4_widened(buffer, buffer, buffer, buffer, None, residual, gate, tokens, out, rows, n, k, 0, buffer,
+                                        (rows + n) * k, workspace, _lib.WORKSPACE_HEADER, None)
+
+    assert call(tokens=7) == call(tokens=0) == _lib.RK_EINVAL  # 60 rows are not a multiple
+    assert call(tokens=1 << 20, rows=1 << 20) == _lib.RK_EUNSUPPORTED
+    assert call(residual=buffer + 1) == call(gate=buffer + 1) == _lib.RK_EINVAL
+    assert call(residual=None, gate=buffer) == _lib.RK_EINVAL
+    assert call(out=buffer + 8) == call(out=buffer + 8, residual=None) == _lib.RK_EINVAL
+    assert call(workspace=None) == _lib.RK_EWORKSPACE
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from rk_b200 import _lib
 
