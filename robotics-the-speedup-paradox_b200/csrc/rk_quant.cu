@@ -781,6 +781,13 @@ __device__ __forceinline__ uint2 to_fp8x8(const float (&v)[8], float inverse) {
   return make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
 }
 
+// the first `count` (below eight) of eight codes
+__device__ __forceinline__ void store_codes(uint8_t* q, uint2 codes, int count) {
+#pragma unroll
+  for (int i = 0; i < 7; ++i)
+    if (i < count) q[i] = static_cast<uint8_t>((i < 4 ? codes.x : codes.y) >> (8 * (i & 3)));
+}
+
 // Sixteen elements per thread and step: two 16-byte loads in flight, one 16-byte store (maximum and conversion of
 // 816 x 32768: 26.6 -> 20.1 us against eight elements and scalar conversions).
 __global__ void __launch_bounds__(256)
@@ -798,13 +805,14 @@ to_fp8_kernel(const __nv_bfloat16* __restrict__ x, long long elements, const flo
     load8(x + idx, true, valid, v);
     load8(x + idx + 8, true, valid - 8, w);
     const uint2 a = to_fp8x8(v, inverse), b = to_fp8x8(w, inverse);
-    if (valid == 16 && q16) {
+    if (valid == 16 && q16) {  // `q16`: the codes are 16-byte aligned; else they are 8-byte aligned
       *reinterpret_cast<uint4*>(q + idx) = make_uint4(a.x, a.y, b.x, b.y);
+    } else if (valid >= 8) {
+      *reinterpret_cast<uint2*>(q + idx) = a;
+      if (valid == 16) *reinterpret_cast<uint2*>(q + idx + 8) = b;
+      else store_codes(q + idx + 8, b, valid - 8);
     } else {
-      const uint32_t words[4] = {a.x, a.y, b.x, b.y};
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (i < valid) q[idx + i] = static_cast<uint8_t>(words[i >> 2] >> (8 * (i & 3)));
+      store_codes(q + idx, a, valid);
     }
   }
 }

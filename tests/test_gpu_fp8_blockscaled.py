@@ -84,6 +84,18 @@ def test_fp8_quantize_with_supplied_scale(H):
     assert np.array_equal(q.cpu().numpy(), OF.quantize_with_scale(H.to_np(x), np.float32(0.0125)))
 
 
+@pytest.mark.parametrize("elements", [5, 8, 13, 24, 31, 4096, 100003])
+def test_quantize_with_scale_writes_codes_at_any_8_byte_boundary(H, elements):
+    """Codes are stored 16 bytes at a time where the destination allows it and 8 otherwise: the same codes, nothing around them."""
+    x = H.randn_bf16((elements,), 3.0, 15).to(H.DEVICE)
+    scale = torch.tensor([0.03], dtype=torch.float32, device=H.DEVICE)
+    buffers = [torch.full((elements + 32,), 77, dtype=torch.uint8, device=H.DEVICE) for _ in range(2)]
+    for offset, buffer in zip((16, 8), buffers):
+        H.call("rk_quant_tensor_fp8_with_scale", _lib.ptr(x), elements, _lib.ptr(scale), _lib.ptr(buffer[offset:]), H.stream())
+    assert torch.equal(buffers[0][16:16 + elements], buffers[1][8:8 + elements])
+    assert (buffers[1][:8] == 77).all() and (buffers[1][8 + elements:] == 77).all()
+
+
 # ---------------------------------------------------------------- MXFP8
 def mx_pack(H, x):
     rows, k = x.shape
