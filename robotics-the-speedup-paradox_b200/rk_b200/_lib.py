@@ -180,6 +180,15 @@ def gemm_workspace(op, device, m, n, k):
     return workspace(device, need)
 
 
+def scratch(shape, device, dtype):
+    """Uninitialised scratch for one call, from the caching allocator (concurrent streams and captured graphs each get
+    their own), or None where the device has no room left: the caller then takes its form without scratch."""
+    try:
+        return torch.empty(shape, device=device, dtype=dtype)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def read_status(buf, device=None):
     """Device status word of a workspace tensor; `buf=None` reads the scratch array built into the
     library (the one `rk_gemm_int4_noalloc` uses) on `device`."""

@@ -123,10 +123,11 @@ def quantize_swiglu_bf16(gate_up, intermediate_size, scale=None):
     out_scale = scale if scale is not None else torch.empty(1, device=gate_up.device, dtype=torch.float32)
     with torch.cuda.device(gate_up.device):
         ws = _lib.workspace(gate_up.device, _lib.WORKSPACE_HEADER)
-        if scale is None and rows * inter <= 1 << 29:
-            # the pass that finds the maximum keeps the activation (a per-call buffer half the size of the input), so that
-            # it is evaluated once: 816 x 16384 38.2 -> 28.1 us
-            product = torch.empty((rows, inter), device=gate_up.device, dtype=torch.bfloat16)
+        # the pass that finds the maximum keeps the activation (a per-call buffer half the size of the input, up to 1 GiB), so
+        # that it is evaluated once: 816 x 16384 38.2 -> 28.1 us; without room for it, it is evaluated twice
+        keep = scale is None and rows * inter <= 1 << 29
+        product = _lib.scratch((rows, inter), gate_up.device, torch.bfloat16) if keep else None
+        if product is not None:
             code = _lib.load().rk_swiglu_quant_fp8_product(_lib.ptr(gate_up), rows, inter, _lib.ptr(product), _lib.ptr(q),
                                                            _lib.ptr(out_scale), _lib.ptr(ws), ws.numel(),
                                                            _lib.stream_ptr(gate_up.device))

@@ -114,7 +114,7 @@ def _widen_first(m, n, kpad):
     meets; the copies cost one pass of (m + n) * kpad bytes through L2.  Measured, copies against inside:
     1764 x 8192 x 2048 28.3 / 90.9 us, 1764 x 2048 x 8192 29.6 / 100.6, 256 x 2048 x 2048 8.3 / 15.7, 50 x 8192 x 2048
     10.4 / 16.7, 50 x 1000 x 4096 7.6 / 10.8, 1 x 1024 x 1024 5.8 / 11.5.  Inside stays for many rows of a tiny weight
-    (1764 x 256 x 256: 7.5 / 6.3) and where the copies would take over 256 MiB."""
+    (1764 x 256 x 256: 7.5 / 6.3), where the copies would take over 256 MiB and where the device has no room for them."""
     return (m + n) * kpad <= 1 << 28 and not (m > 1024 and n * kpad < 1 << 18)
 
 
@@ -123,7 +123,8 @@ def integer_gemm(a, sa, b, sb, bias, bits, tactic, residual=None, gate=None):
 
     With `residual` [M, N] (bf16, contiguous) the epilogue writes the decoder layer's new residual
     stream instead of the projection: residual + y, or residual + y * gate[row // (M / B)] for a
-    `gate` [B, N] (`rk_gemm_int_residual`; the same roundings as the tensor ops)."""
+    `gate` [B, N] (`rk_gemm_int_residual`; the same roundings as the tensor ops).  W4A4 products take
+    up to 256 MiB of scratch for the call (`_widen_first`) where the device has room for it."""
     if not (a.is_cuda and b.is_cuda and sa.is_cuda and sb.is_cuda):
         raise RuntimeError("integer GEMM operands must be CUDA tensors")
     if a.dim() != 2 or b.dim() != 2 or a.size(1) != b.size(1) or not a.is_contiguous() or not b.is_contiguous():
@@ -148,9 +149,8 @@ def integer_gemm(a, sa, b, sb, bias, bits, tactic, residual=None, gate=None):
         raise RuntimeError("integer GEMM: a gate needs a residual")
     with torch.cuda.device(a.device):
         ws = _lib.workspace(a.device, _lib.WORKSPACE_HEADER)
-        if bits == 4 and _widen_first(m, n, kpad):
-            # per call, from the caching allocator: concurrent streams and captured graphs each have their own
-            scratch = torch.empty((m + n) * kpad, device=a.device, dtype=torch.int8)
+        scratch = _lib.scratch((m + n) * kpad, a.device, torch.int8) if bits == 4 and _widen_first(m, n, kpad) else None
+        if scratch is not None:
             code = _lib.load().rk_gemm_int4_widened(
                 _lib.ptr(a), _lib.ptr(sa), _lib.ptr(b), _lib.ptr(sb), _lib.ptr(bias), _lib.ptr(residual), _lib.ptr(gate),
                 tokens, _lib.ptr(out), m, n, kpad, tactic, _lib.ptr(scratch), scratch.numel(), _lib.ptr(ws), ws.numel(),

@@ -177,3 +177,46 @@ def test_w4a4_widened_copies_match_the_in_kernel_form(m, n, k, form):
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     assert _lib.read_status(ws) == 0
     assert lib.rk_gemm_int4_widened(*call, scratch.numel() - 1, *tail) == _lib.RK_EWORKSPACE
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_w4a4_without_room_for_the_copies_takes_the_in_kernel_form(H, monkeypatch, gated):
+    """A device without room for the scratch of a faster form still gets the result, from the form that needs none."""
+    from rk_b200 import _lib
+    from rk_b200 import integer as I
+
+    gen = torch.Generator(device=H.DEVICE).manual_seed(4)
+    linear = torch.nn.Linear(384, 136, dtype=torch.bfloat16, device=H.DEVICE)
+    layer = I.IntegerLinear.from_linear(linear, bits=4)
+    x = torch.randn(70, 384, generator=gen, device=H.DEVICE).bfloat16()
+    extra = {}
+    if gated:
+        extra = {"residual": torch.randn(70, 136, generator=gen, device=H.DEVICE).bfloat16(),
+                 "gate": torch.randn(2, 136, generator=gen, device=H.DEVICE).bfloat16()}
+    packed = layer.pack_input(x)
+    want = layer.forward_packed(packed, **extra)
+    refuse_allocations_of(monkeypatch, (70 + 136) * 384)
+    assert _lib.scratch((70 + 136) * 384, H.DEVICE, torch.int8) is None
+    assert torch.equal(layer.forward_packed(packed, **extra), want)
+
+
+def test_fp8_swiglu_without_room_for_the_activation_evaluates_it_twice(H, monkeypatch):
+    from rk_b200 import fp8_linear as F8
+
+    gate_up = torch.randn(37, 2 * 48, device=H.DEVICE).bfloat16()
+    want_q, want_scale = F8.quantize_swiglu_bf16(gate_up, 48)
+    refuse_allocations_of(monkeypatch, (37, 48), torch.bfloat16)
+    q, scale = F8.quantize_swiglu_bf16(gate_up, 48)
+    assert torch.equal(q.view(torch.uint8), want_q.view(torch.uint8)) and torch.equal(scale, want_scale)
+
+
+def refuse_allocations_of(monkeypatch, shape, dtype=torch.int8):
+    """torch.empty of this shape and type fails as on a full device."""
+    empty = torch.empty
+
+    def full(*args, **kwargs):
+        if args == (shape,) and kwargs.get("dtype") == dtype:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*args, **kwargs)
+
+    monkeypatch.setattr(torch, "empty", full)
