@@ -440,7 +440,7 @@ int launch_tc_peer(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const PeerM
   return RK_OK;
 }
 
-template <int KIND, bool REPACK>
+template <int KIND, bool REPACK, bool TAIL>
 int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
                const CUtensorMap& tm_sfb, const CUtensorMap& tm_tail, const Gemm2Params& p, int smem, cudaStream_t st) {
   static bool configured_dev[64] = {};
@@ -448,7 +448,7 @@ int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CU
   cudaGetDevice(&dev);
   bool& configured = configured_dev[dev & 63];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc2_kernel<KIND, REPACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc2_kernel<KIND, REPACK, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBudget + 1024);
     if (e != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured = true;
@@ -469,7 +469,7 @@ int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CU
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc2_kernel<KIND, REPACK>, tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc2_kernel<KIND, REPACK, TAIL>, tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(RK_ECUDA, "rk_gemm_tc2_kernel launch: %s", cudaGetErrorString(e));
@@ -481,9 +481,12 @@ template <int KIND>
 int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
                const CUtensorMap& tm_sfb, const CUtensorMap& tm_tail, const Gemm2Params& p, int smem, cudaStream_t st) {
   if constexpr (KIND == KIND_MXF8 || KIND == KIND_NVF4) {
-    if (p.sw_q != nullptr) return launch_tc2_kernel<KIND, true>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
+    if (p.sw_q != nullptr) return launch_tc2_kernel<KIND, true, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
   }
-  return launch_tc2_kernel<KIND, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
+  if constexpr (KIND == KIND_I8 || KIND == KIND_F8) {
+    if (p.bn % 64 != 0) return launch_tc2_kernel<KIND, false, true>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
+  }
+  return launch_tc2_kernel<KIND, false, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
 }
 
 // A box of the 16 x U4 -> 16-byte-aligned tensor-map type writes 128 bytes per row into shared memory
@@ -565,19 +568,21 @@ int run_tc(const TcArgs& a) {
       return v ? std::atoi(v) : 0;
     }();
     if (!block_scaled) {
-      // A stage costs an SM the operands it takes from L2 (about 64 bytes a clock: 256 + bn cycles; its MMAs take 2 bn), the
-      // launch as many stages as its busiest pair: the width with the least of that, in the steps of 32 that a pair's MMA
-      // takes.  1764 rows are 7 pair tiles: 2048 columns are 56 tiles of 256 or 70 of 224 for 74 pairs, 8192 columns 224 of
-      // 256 (four rounds, the last for two tiles) or 259 of 224.  256 columns against the rule's choice, W8A8: 1764 x 2048 x
-      // 8192 24.6 -> 22.7 us (224), 1764 x 6144 x 2048 20.0 -> 18.6 (224), 1100 x 1024 x 4096 14.4 -> 9.8 (128), 3264 x 2048 x
-      // 16384 81.9 -> 74.8 (192), 1200 x 3000 x 896 12.3 -> 8.2 (224); 4096 x 8192 x 8192 stays at 256.
+      // A stage costs an SM the operands it takes from L2 (about 64 bytes a clock: 256 + bn cycles; its MMAs take 2 bn), a tile
+      // some 900 cycles more whatever its width (hand-over of the accumulator, chunks of the epilogue), the launch as many as
+      // its busiest pair has: the width with the least of that, in the steps of 32 that a pair's MMA takes.  1764 rows are 7 pair
+      // tiles: 2048 columns are 56 tiles of 256 or 70 of 224 for 74 pairs, 8192 columns 224 of 256 (four rounds, the last for two
+      // tiles) or 259 of 224.  256 columns against the rule's choice, W8A8: 1764 x 2048 x 8192 24.6 -> 22.7 us (224), 1764 x 6144 x
+      // 2048 20.0 -> 18.6 (224), 1100 x 1024 x 4096 14.4 -> 9.8 (128), 3264 x 2048 x 16384 81.9 -> 74.8 (192); 4096 x 8192 x 8192
+      // stays at 256.  The 900 cycles decide short loops: 3264 x 2560 x 256 13.2 us in two rounds of 256, 14.9 in three of 160,
+      // which the stages alone would choose.
       p2.bn = 128;
       if (!(a.tactic & 4) && a.n >= 256) {
         const int64_t tiles_m = (a.m + 255) / 256;
         int64_t best = -1;
         for (int bn = 256; bn >= 128; bn -= 32) {
           const int64_t rounds = (tiles_m * ((a.n + bn - 1) / bn) + kNumSms / 2 - 1) / (kNumSms / 2);
-          const int64_t cost = rounds * kblocks * (256 + bn) + 10 * bn;
+          const int64_t cost = rounds * (kblocks * (256 + bn) + 900) + 10 * bn;
           if (best < 0 || cost < best) best = cost, p2.bn = bn;
         }
       }
@@ -667,7 +672,10 @@ int run_tc(const TcArgs& a) {
                        chunks, CU_TENSOR_MAP_SWIZZLE_NONE);
       if (rc != RK_OK) return rc;
     }
-    const int smem = p2.stages * stage + 2 * kOutBufBytes + kVecBytes + 1024;
+    // More than half of an SM's shared memory, however short the K loop: a pair holds all 512 columns of tensor memory, so a CTA
+    // of the next launch that found room beside it would only wait for them, and the rest of its launch behind it (K = 256, behind
+    // a quantizer: FP8 1764 x 1024 9.9 -> 6.0 us, 1025 x 6144 18.0 -> 9.9).
+    const int smem = std::max(p2.stages * stage + 2 * kOutBufBytes + kVecBytes + 1024, 118 * 1024);
     switch (a.kind) {
       case KIND_I8: return launch_tc2<KIND_I8>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);
       case KIND_F8: return launch_tc2<KIND_F8>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);

@@ -22,7 +22,7 @@
 // over the one-CTA kernel comes from.
 //
 // Warp roles per CTA: warp 0 = TMA producer, warp 1 = TMEM allocation (+ MMA issue in the leader), the others =
-// epilogue: four warps, eight for the kinds without block scales, sixteen for the re-packing epilogues.
+// epilogue: four warps, eight for W8A8, sixteen for the re-packing epilogues.
 #pragma once
 
 #include <cuda.h>
@@ -38,11 +38,12 @@ namespace rk {
 // four.  816 x 32768 x 2048: 131.7 us with four warps, 82.5 with eight.
 constexpr int kGemm2SwigluSets = 4;
 constexpr int kGemm2ThreadsSwiglu = 64 + 128 * kGemm2SwigluSets;
-// The plain epilogue of the kinds without block scales: two sets of four warps take alternate 64-column chunks, each
+// W8A8, whose epilogue applies a scale per row and column: two sets of four warps take alternate 64-column chunks, each
 // with its own staging buffer.  It halves the tail after the last tile, which nothing hides (with the tile widths of
-// run_tc and the early weight fetch: four W8A8 video-diffusion blocks of 1764 tokens 538 -> 514 us).
+// run_tc and the early weight fetch: four W8A8 video-diffusion blocks of 1764 tokens 538 -> 514 us).  FP8 has one scale and
+// is faster with one set that alternates between both buffers: 2304 x 8192 x 512 16.5 -> 15.2 us, 3264 x 4096 x 1024 17.0 -> 16.2.
 __host__ __device__ constexpr int gemm2_epi_sets(int kind, bool repack) {
-  return repack ? kGemm2SwigluSets : (kind == KIND_I8 || kind == KIND_F8 ? 2 : 1);
+  return repack ? kGemm2SwigluSets : (kind == KIND_I8 ? 2 : 1);
 }
 __host__ __device__ constexpr int gemm2_threads(int kind, bool repack) { return 64 + 128 * gemm2_epi_sets(kind, repack); }
 
@@ -183,7 +184,9 @@ __host__ __device__ inline int gemm2_stage_bytes(int kind, int bn, int sfb_block
 }
 
 // REPACK: the epilogues that never write the bf16 tile (sw_q set), on sixteen warps.
-template <int KIND, bool REPACK>
+// TAIL: tiles whose width is not a multiple of 64 (W8A8 and FP8), a form of its own because the choice in every chunk costs the
+// others up to 8 % (FP8 2304 x 8192 x 512 16.3 -> 15.2 us, W8A8 19.2 -> 18.4).
+template <int KIND, bool REPACK, bool TAIL>
 __global__ void __launch_bounds__(gemm2_threads(KIND, REPACK), 1)
 rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                    const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_sfa,
@@ -216,9 +219,10 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   const int tile_step = static_cast<int>(gridDim.x >> 1);
 
   pdl_launch_dependents();
-  if (!T::kBlockScaled && threadIdx.x == 64 && tile_first < num_tiles) {
-    // the weight rows of the first tile start their way from DRAM to L2 while the preceding kernel drains (weights are
-    // parameters, never that kernel's output; the block-scaled kinds measured 0.3 us slower with it)
+  if (KIND == KIND_I8 && threadIdx.x == 64 && tile_first < num_tiles) {
+    // the weight rows of the first tile start their way from DRAM to L2 while the preceding kernel drains.  A request to L2
+    // alone: that kernel may still be writing them (the int8 copies of rk_gemm_int4_widened), so no load may move up here.
+    // W8A8 only: FP8 (1764 x 4096 x 1024 12.8 us against 12.5) and the block-scaled kinds (0.3 us) are slower with it.
     const int row_b0 = (tile_first % p.tiles_n) * p.bn + static_cast<int>(rank) * half_bn;
     for (int kb = 0; kb < min(p.kblocks, p.stages) && row_b0 < p.n; ++kb) tma_prefetch_l2_2d(&tm_b, kb * kStageKBytes, row_b0);
   }
@@ -339,7 +343,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             // whole K blocks of the block-scaled kinds: the stage's up to 17 tensor-core instructions as one
             // straight-line block of the elected lane (the issuing thread's cost per instruction paces
             // these kinds; one instruction here drives both SMs, which is what makes the pair faster);
-            // the kinds without scale copies measured faster in the predicated form below
+            // the kinds without scale copies measured faster with a branch around each MMA, below
             if (on) {
               const uint32_t accumulate0 = kb > 0 ? 1u : 0u;
               if constexpr (T::kBlockScaled) {
@@ -604,10 +608,10 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           else tma_store_wait_read<0>();
         }
         set_sync();
-        const int cols = T::kBlockScaled ? 64 : min(64, p.bn - cc);  // 64, or 32 for the tail of a tile whose width is not a multiple of 64
+        const int cols = TAIL ? min(64, p.bn - cc) : 64;  // 64, or 32 at the end of the tile
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
-          if (c0 >= cols) break;
+          if (TAIL && c0 >= cols) break;
           uint32_t r0[16], r1[16];
           __syncwarp();
           tmem_ld_16(t_acc + cc + c0, r0);
@@ -635,7 +639,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             const uint4 hi = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
                                         pack_bf16x2(v[14], v[15]));
             const int ch = (c0 >> 3) + 2 * h;
-            if (cols == 64) {  // rows of 128 bytes in the 128-byte swizzle
+            if (!TAIL || cols == 64) {  // rows of 128 bytes in the 128-byte swizzle
               *reinterpret_cast<uint4*>(stage + et * 128 + ((ch ^ (et & 7)) << 4)) = lo;
               *reinterpret_cast<uint4*>(stage + et * 128 + (((ch + 1) ^ (et & 7)) << 4)) = hi;
             } else {           // rows of 64 bytes in the 64-byte swizzle
@@ -653,7 +657,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         fence_proxy_async_smem();
         set_sync();
         if (et == 0) {
-          if (ok) tma_store_2d(cols == 64 ? &tm_out : &tm_tail, smem_u32(stage), row_b0 + cc, row_a0);
+          if (ok) tma_store_2d(!TAIL || cols == 64 ? &tm_out : &tm_tail, smem_u32(stage), row_b0 + cc, row_a0);
           tma_store_commit();
           pending_store = 1;
         }

@@ -308,9 +308,11 @@ def test_residual_epilogue_refuses_bad_arguments(H):
     assert lib.rk_gemm_int_residual(*args(_lib.ptr(stream), 60)) == _lib.RK_OK
 
 
-# pair tiles of 224 (the second tile row ends 32 columns in), 256, 192, 160 and 128 columns; ragged rows and columns
+# pair tiles of 224 (the second tile row ends 32 columns in), 256, 192, 160 and 128 columns; ragged rows and columns; one and
+# two stages of K with two tiles per pair
 @pytest.mark.parametrize("m,n,k", [(1764, 2048, 2048), (1764, 6144, 1024), (2048, 2048, 1024), (3264, 2048, 2048), (2304, 1200, 256),
-                                   (1025, 264, 384), (1100, 2376, 384), (1300, 3000, 896), (1030, 4640, 1024)])
+                                   (1025, 264, 384), (1100, 2376, 384), (1300, 3000, 896), (1030, 4640, 1024),
+                                   (3264, 2560, 128), (1025, 6144, 256)])
 @pytest.mark.parametrize("kind", ["int8", "fp8"])
 def test_pair_tiles_of_every_width(m, n, k, kind):
     """W8A8 and FP8 above 1024 rows: small integer operands make every product and sum exact, so the outputs are known."""
