@@ -111,11 +111,23 @@ def quantize_weight(weight, bits):
 def _widen_first(m, n, kpad):
     """W4A4: widen both operands to int8 copies once and run the int8 kernels on them, or widen every tile inside the
     GEMM?  Inside, a 128 x 128 x 128 stage costs about 0.8 us of rewriting and each tile is rewritten for every tile it
-    meets; the copies cost one pass of (m + n) * kpad bytes through L2.  Measured, copies against inside:
+    meets; the copies cost a launch and one pass of (m + n) * kpad bytes through L2.  Measured, copies against inside:
     1764 x 8192 x 2048 28.3 / 90.9 us, 1764 x 2048 x 8192 29.6 / 100.6, 256 x 2048 x 2048 8.3 / 15.7, 50 x 8192 x 2048
-    10.4 / 16.7, 50 x 1000 x 4096 7.6 / 10.8, 1 x 1024 x 1024 5.8 / 11.5.  Inside stays for many rows of a tiny weight
-    (1764 x 256 x 256: 7.5 / 6.3), where the copies would take over 256 MiB and where the device has no room for them."""
-    return (m + n) * kpad <= 1 << 28 and not (m > 1024 and n * kpad < 1 << 18)
+    10.4 / 16.7, 50 x 1000 x 4096 7.6 / 10.8, 1 x 1024 x 1024 5.8 / 11.5.
+
+    Inside stays where the copies would take over 256 MiB or the device has no room for them, for a tiny weight
+    (1764 x 256 x 256: 7.5 / 6.3; 400 x 64 x 128: 6.9 / 6.3), and up to 1024 rows on a K loop of few stages where the launch and
+    the int8 kernel's coarser waves (tiles of 256 rows) cost more than the rewriting - behind a row quantizer, weights
+    from HBM: one full wave of 128 x 128 tiles inside, 400 x 4096 x 128 9.6 / 8.7 (two waves: 400 x 6144 x 256 10.3 / 11.9), or
+    more than two, 1024 x 6144 x 128 18.9 / 14.7 and, with full tiles of 256 rows, 1024 x 6144 x 512 20.8 / 18.7."""
+    if (m + n) * kpad > 1 << 28:
+        return False
+    if m > 1024:
+        return n * kpad >= 1 << 18
+    tiles = -(-m // 128) * -(-n // 128)
+    if kpad <= 256:
+        return not (n * kpad <= 1 << 14 and m > 32) and not 96 <= tiles <= 148 and tiles <= 2 * 148
+    return not (kpad <= 512 and m > 896 and tiles > 2 * 148)
 
 
 def integer_gemm(a, sa, b, sb, bias, bits, tactic, residual=None, gate=None):

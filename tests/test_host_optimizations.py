@@ -365,3 +365,16 @@ def test_packed_nvfp4_activation_carrier():
         _fake_fp4(256, 64, True).pack_input(carrier)      # feature count
     with pytest.raises(ValueError):
         _fake_fp4(128, 64, False).pack_input(carrier)     # a per-tensor scale the layer does not expect
+
+
+def test_w4a4_takes_the_widened_copies_only_where_they_measured_faster():
+    """Sizes with both forms timed behind a row quantizer; the copies win or lose there by more than 2 % of the pair."""
+    from rk_b200.integer import _widen_first
+
+    faster = [(1, 4096, 128), (100, 2048, 256), (200, 16384, 128), (400, 6144, 256), (512, 8192, 256), (1024, 4096, 256), (50, 64, 512),
+              (800, 8192, 512), (400, 16384, 512), (1024, 6144, 1024), (1024, 64, 1024), (1025, 8192, 128), (1764, 8192, 2048)]
+    slower = [(400, 64, 128), (512, 64, 256), (1024, 64, 256), (400, 4096, 128), (200, 8192, 256), (800, 2048, 256), (1024, 2048, 128),
+              (800, 6144, 128), (1024, 6144, 256), (1024, 16384, 256), (512, 16384, 128), (1024, 6144, 512), (1764, 256, 256)]
+    assert [_widen_first(*size) for size in faster] == [True] * len(faster)
+    assert [_widen_first(*size) for size in slower] == [False] * len(slower)
+    assert not _widen_first(1 << 15, 8192, 8192)  # copies above 256 MiB
