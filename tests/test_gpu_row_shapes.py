@@ -16,8 +16,8 @@ def _randn(gen, *shape, std=1.0):
     return (torch.randn(*shape, generator=gen, device="cuda") * std).bfloat16()
 
 
-def _bits(tensors):
-    return [t[:FEW].contiguous().view(torch.uint8) for t in tensors]
+def _bits(tensors, rows):
+    return [t[rows].contiguous().view(torch.uint8) for t in tensors]
 
 
 @pytest.mark.parametrize("k", [8, 250, 333, 512, 1000, 1032, 2048, 2056, 4096, 4100, 8192])
@@ -25,15 +25,19 @@ def _bits(tensors):
 def test_the_shape_of_a_launch_never_changes_a_row(k, bits):
     lib, dev, ptr = _lib.load(), torch.device("cuda:0"), _lib.ptr
     gen = torch.Generator(device=dev).manual_seed(k)
-    x, y = _randn(gen, TALL, k), _randn(gen, TALL, k)
-    scale, shift, gate = (_randn(gen, TALL // 48, k, std=0.1) for _ in range(3))
-    x[1] = 0.0
-    x[2, 0], x[3, 0], x[4, 0] = float("inf"), float("nan"), 3e38
+    x_all, y_all = _randn(gen, TALL, k), _randn(gen, TALL, k)
+    scale_all, shift_all, gate_all = (_randn(gen, TALL // 48, k, std=0.1) for _ in range(3))
+    x_all[1] = 0.0
+    x_all[2, 0], x_all[3, 0], x_all[4, 0] = float("inf"), float("nan"), 3e38
     table = torch.nn.functional.gelu(torch.arange(65536, device=dev, dtype=torch.int32).to(torch.int16).view(torch.bfloat16))
     ws = torch.zeros(_lib.WORKSPACE_HEADER, device=dev, dtype=torch.uint8)
     width = (k + 127) // 128 * 128 * bits // 8
 
-    def run(rows):
+    def run(first, rows):
+        part = slice(first, first + rows)
+        vectors = slice(first // 48, (first + rows) // 48)
+        x, y = x_all[part].clone(), y_all[part].clone()  # at aligned addresses, whatever k
+        scale, shift, gate = (t[vectors].clone() for t in (scale_all, shift_all, gate_all))
         q, s = torch.zeros(rows, width, device=dev, dtype=torch.uint8), torch.zeros(rows, device=dev)
         stream, results = _lib.stream_ptr(dev), []
         for mode in (_lib.ACT_PLAIN, _lib.ACT_LUT_MUL, _lib.ACT_LUT):
@@ -50,15 +54,17 @@ def test_the_shape_of_a_launch_never_changes_a_row(k, bits):
         results += [q.clone(), s.clone(), res, normed]
         if bits == 8:
             res, normed, one = torch.zeros_like(res), torch.zeros_like(normed), torch.zeros(1, device=dev)
-            _lib.check(lib.rk_rmsnorm_tensor_scale(ptr(x), ptr(y), ptr(scale), None, 0, rows, k, 1e-6, 2688.0, ptr(res),
+            _lib.check(lib.rk_rmsnorm_tensor_scale(ptr(x), ptr(y), ptr(scale_all), None, 0, rows, k, 1e-6, 2688.0, ptr(res),
                                                    ptr(normed), ptr(one), ptr(ws), ws.numel(), stream), "tensor scale")
             finite = normed.float()[torch.isfinite(normed)].abs().max().item()
             assert one.item() == max(np.float32(finite) / np.float32(2688.0), np.float32(1e-12))  # the IEEE quotient
             results += [res, normed]
         return results
 
-    for tall, few in zip(_bits(run(TALL)), _bits(run(FEW))):
-        assert torch.equal(tall, few)
+    all_rows = run(0, TALL)
+    for first in (0, TALL - FEW):  # rows that a CTA takes first and rows it comes to last
+        for tall, few in zip(_bits(all_rows, slice(first, first + FEW)), _bits(run(first, FEW), slice(FEW))):
+            assert torch.equal(tall, few)
 
 
 @pytest.mark.parametrize("rows,k", [(1200, 2048), (331, 4100), (160, 8190), (1181, 2056), (150, 8192)])
