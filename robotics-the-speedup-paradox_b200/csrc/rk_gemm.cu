@@ -348,7 +348,7 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
   return pl;
 }
 
-template <int KIND, bool RESIDUAL, bool SPLIT>
+template <int KIND, bool RESIDUAL, int SCHED>
 int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
               const Plan& pl, cudaStream_t st) {
   static bool configured_dev[64] = {};
@@ -356,7 +356,7 @@ int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUt
   cudaGetDevice(&dev);
   bool& configured = configured_dev[dev & 63];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc_kernel<KIND, RESIDUAL, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rk_gemm_tc_kernel<KIND, RESIDUAL, SCHED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBudget + 1024);
     if (e != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured = true;
@@ -375,7 +375,7 @@ int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUt
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc_kernel<KIND, RESIDUAL, SPLIT>, tm_a, tm_b, tm_out, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemm_tc_kernel<KIND, RESIDUAL, SCHED>, tm_a, tm_b, tm_out, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(RK_ECUDA, "rk_gemm_tc_kernel launch: %s", cudaGetErrorString(e));
@@ -383,11 +383,24 @@ int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUt
   return RK_OK;
 }
 
+// A launch that does not split K runs in a kernel without the code of the split, or in the one that holds both schedules, by
+// what the compiler makes of the issue and epilogue loops.  Both: the rewriting and the block-scaled kinds (which never split)
+// - FP8 producer 1764 x 8192 x 1024 60.3 us against 61.9, W4A4 in the kernel 1024 x 16384 x 512 31.2 / 31.8, NVFP4 300 x 8192 x 1024
+// 6.8 / 7.2 - and W8A8 where a CTA walks several tiles, 1024 x 16384 x 512 32.0 / 32.3.  Without: FP8 (816 x 32768 x 2048 56.4 us
+// against 58.1), the residual epilogue (50 x 1024 x 1024 5.71 / 5.84) and W8A8 in one round, where the shorter code counts in a
+// chain of different kernels (action chunk of one environment 10.15 / 10.23 ms).
 template <int KIND, bool RESIDUAL = false>
 int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
               const Plan& pl, cudaStream_t st) {
-  if (pl.splits > 1 || KindTraits<KIND>::kBlockScaled) return launch_tc_kernel<KIND, RESIDUAL, true>(tm_a, tm_b, tm_out, p, pl, st);
-  return launch_tc_kernel<KIND, RESIDUAL, KindTraits<KIND>::kBlockScaled>(tm_a, tm_b, tm_out, p, pl, st);
+  constexpr bool direct = KIND == KIND_I8 || KIND == KIND_F8;
+  if constexpr (!KindTraits<KIND>::kBlockScaled) {
+    if (pl.splits > 1) return launch_tc_kernel<KIND, RESIDUAL, SCHED_SPLIT>(tm_a, tm_b, tm_out, p, pl, st);
+  }
+  if constexpr (KIND == KIND_I8 && !RESIDUAL) {
+    if (static_cast<long long>(pl.tiles_a) * pl.tiles_b > kNumSms)
+      return launch_tc_kernel<KIND, RESIDUAL, SCHED_EITHER>(tm_a, tm_b, tm_out, p, pl, st);
+  }
+  return launch_tc_kernel<KIND, RESIDUAL, direct ? SCHED_WHOLE : SCHED_EITHER>(tm_a, tm_b, tm_out, p, pl, st);
 }
 
 // RK_B200_ISSUE_BLOCK=0 issues every tensor-core instruction under its own predicate instead of the

@@ -394,9 +394,10 @@ __device__ __forceinline__ void multicast_store_region(const GemmParams& p, cons
 // store descriptors of the column-parallel mode, one per rank, or null).
 // RESIDUAL: the epilogue applies GemmParams::residual (a separate instantiation: the 64 values it keeps
 // in flight would otherwise cost every launch of the kind its registers).
-// SPLIT: the split-K schedule (GemmParams::splits > 1), its own instantiation for the same reason; the block-scaled kinds
-// have one for both (their issue loop measured slower alone: NVFP4 300 x 8192 x 1024 6.8 -> 7.2 us).
-template <int KIND, bool RESIDUAL = false, bool SPLIT = false>
+// SCHED: whole K per CTA, K split over a cluster (GemmParams::splits > 1), or either as `splits` says; see launch_tc for which
+// form a launch takes.
+enum Schedule : int { SCHED_WHOLE, SCHED_SPLIT, SCHED_EITHER };
+template <int KIND, bool RESIDUAL = false, int SCHED = SCHED_WHOLE>
 __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out,
                                              const CUtensorMap* peer_maps, const GemmParams& p) {
   using T = KindTraits<KIND>;
@@ -428,9 +429,9 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const uint32_t out_stage_off = p.stages * stage_bytes;
   const uint32_t vec_off = out_stage_off + p.out_bufs * kOutBufBytes;
 
-  const bool split_mode = T::kBlockScaled ? p.splits > 1 : SPLIT;
+  const bool split_mode = SCHED == SCHED_EITHER ? p.splits > 1 : SCHED == SCHED_SPLIT;
   const int num_tiles = p.tiles_a * p.tiles_b;
-  const int tile_first = split_mode ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
+  const int tile_first = static_cast<int>(blockIdx.x);
   const int tile_step = split_mode ? num_tiles : static_cast<int>(gridDim.x);  // split mode: exactly one tile
   const int split = static_cast<int>(blockIdx.z);
   const int kb_begin = static_cast<int>((static_cast<long long>(p.kblocks) * split) / p.splits);
@@ -1115,11 +1116,11 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   }
 }
 
-template <int KIND, bool RESIDUAL, bool SPLIT>
+template <int KIND, bool RESIDUAL, int SCHED>
 __global__ void __launch_bounds__(KindTraits<KIND>::kThreads, 1)
 rk_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                   const __grid_constant__ CUtensorMap tm_out, const GemmParams p) {
-  gemm_tc_body<KIND, RESIDUAL, SPLIT>(tm_a, tm_b, tm_out, nullptr, p);
+  gemm_tc_body<KIND, RESIDUAL, SCHED>(tm_a, tm_b, tm_out, nullptr, p);
 }
 
 // The per-tensor FP8 GEMM in column-parallel mode: one store descriptor per rank instead of one output map.
