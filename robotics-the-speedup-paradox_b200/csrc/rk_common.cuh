@@ -163,8 +163,9 @@ __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
 // Asks L2 to fetch one box of a tiled tensor; nothing is delivered to this kernel.  Used for
-// weights and scales before the dependency wait: they are parameters, not outputs of the kernel
-// that runs before this one, and L2 is the coherence point, so an early fetch can never be stale.
+// weights and scales before the dependency wait: L2 is the coherence point, so an early fetch can
+// never be stale, not even where the kernel that runs before this one still writes the box (the
+// int8 copies of rk_gemm_int4_widened).  A load that delivers data must stay behind the wait.
 __device__ __forceinline__ void tma_prefetch_l2_2d(const void* tmap, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
                ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y) : "memory");
@@ -357,19 +358,14 @@ __host__ __device__ constexpr uint32_t umma_idesc_bs(uint32_t afmt, uint32_t bfm
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T; issued by one thread.
-#define RK_DEFINE_MMA(NAME, KIND)                                                                           \
-  __device__ __forceinline__ void NAME(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,     \
-                                       uint32_t accumulate, uint32_t on = 1u) {                             \
-    asm volatile(                                                                                           \
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"                        \
-        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, p;\n\t}"                              \
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on)                         \
-        : "memory");                                                                                        \
-  }
-RK_DEFINE_MMA(mma_i8, "i8")
-RK_DEFINE_MMA(mma_f16, "f16")
-RK_DEFINE_MMA(mma_f8f6f4, "f8f6f4")
-#undef RK_DEFINE_MMA
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate, uint32_t on = 1u) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on)
+      : "memory");
+}
 
 // D[tmem] (+)= A[tmem] * B[smem]^T: the A operand is a TMEM tile (one row per lane, K along columns)
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,

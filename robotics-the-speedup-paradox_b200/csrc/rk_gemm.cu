@@ -403,8 +403,8 @@ int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMa
   return launch_tc_kernel<KIND, RESIDUAL, direct ? SCHED_WHOLE : SCHED_EITHER>(tm_a, tm_b, tm_out, p, pl, st);
 }
 
-// RK_B200_ISSUE_BLOCK=0 issues every tensor-core instruction under its own predicate instead of the
-// straight-line block of the elected lane (kept for comparison).
+// RK_B200_ISSUE_BLOCK=0 issues every tensor-core instruction of the block-scaled kinds under its own predicate instead of
+// in the straight-line block of the elected lane (kept for comparison); the other kinds branch around each MMA either way.
 int issue_block_mode() {
   static const int mode = [] {
     const char* v = std::getenv("RK_B200_ISSUE_BLOCK");

@@ -441,7 +441,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   pdl_launch_dependents();
   if (threadIdx.x == 64) {  // first thing, by a thread that has no part in the set-up
     // The weight rows of this CTA's first tile start their way from DRAM to L2 during set-up, while
-    // the preceding kernel drains (weights are parameters, never that kernel's output).
+    // the preceding kernel drains (a request to L2 alone: see tma_prefetch_l2_2d).
     if (tile_first < num_tiles) {
       const int row_a0 = (tile_first / p.tiles_b) * kTileA;
       const int row_b0 = (tile_first % p.tiles_b) * p.bn;

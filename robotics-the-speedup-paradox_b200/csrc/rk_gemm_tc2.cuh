@@ -107,18 +107,6 @@ __device__ __forceinline__ void tc2_commit_both(uint32_t bar, uint32_t on = 1u) 
       ::"r"(bar), "h"(static_cast<uint16_t>(3)), "r"(on)
       : "memory");
 }
-#define RK_DEFINE_MMA2(NAME, KIND)                                                                          \
-  __device__ __forceinline__ void NAME(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,     \
-                                       uint32_t accumulate, uint32_t on = 1u) {                             \
-    asm volatile(                                                                                           \
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"                        \
-        "@q tcgen05.mma.cta_group::2.kind::" KIND " [%0], %1, %2, %3, p;\n\t}"                              \
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on)                         \
-        : "memory");                                                                                        \
-  }
-RK_DEFINE_MMA2(mma2_i8, "i8")
-RK_DEFINE_MMA2(mma2_f8f6f4, "f8f6f4")
-#undef RK_DEFINE_MMA2
 __device__ __forceinline__ void mma2_mxf8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate, uint32_t on = 1u) {
   asm volatile(
