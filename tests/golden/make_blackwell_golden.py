@@ -466,7 +466,7 @@ def main_silu(out_dir):
 
 if __name__ == "__main__":
     args = [a for a in sys.argv[1:] if not a.startswith("--")]
-    target = args[0] if args else "gpurun_out"
+    target = args[0] if args else "golden_out"
     if "--ext" in sys.argv:
         main_ext(target)
     elif "--silu" in sys.argv:
