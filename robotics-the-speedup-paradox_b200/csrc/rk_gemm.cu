@@ -386,19 +386,15 @@ int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUt
 // A launch that does not split K runs in a kernel without the code of the split, or in the one that holds both schedules, by
 // what the compiler makes of the issue and epilogue loops.  Both: the rewriting and the block-scaled kinds (which never split)
 // - FP8 producer 1764 x 8192 x 1024 60.3 us against 61.9, W4A4 in the kernel 1024 x 16384 x 512 31.2 / 31.8, NVFP4 300 x 8192 x 1024
-// 6.8 / 7.2 - and W8A8 where a CTA walks several tiles, 1024 x 16384 x 512 32.0 / 32.3.  Without: FP8 (816 x 32768 x 2048 56.4 us
-// against 58.1), the residual epilogue (50 x 1024 x 1024 5.71 / 5.84) and W8A8 in one round, where the shorter code counts in a
-// chain of different kernels (action chunk of one environment 10.15 / 10.23 ms).
+// 6.8 / 7.2.  Without: FP8 (816 x 32768 x 2048 56.4 us against 58.1) and W8A8, whose single launches gain from the other form
+// (1024 x 16384 x 512 32.0 / 32.3) while its chains of different kernels lose, more code being fetched by each: four
+// video-diffusion blocks of 600 tokens 337 us against 347, action chunk of one environment 10.15 ms against 10.23.
 template <int KIND, bool RESIDUAL = false>
 int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
               const Plan& pl, cudaStream_t st) {
   constexpr bool direct = KIND == KIND_I8 || KIND == KIND_F8;
   if constexpr (!KindTraits<KIND>::kBlockScaled) {
     if (pl.splits > 1) return launch_tc_kernel<KIND, RESIDUAL, SCHED_SPLIT>(tm_a, tm_b, tm_out, p, pl, st);
-  }
-  if constexpr (KIND == KIND_I8 && !RESIDUAL) {
-    if (static_cast<long long>(pl.tiles_a) * pl.tiles_b > kNumSms)
-      return launch_tc_kernel<KIND, RESIDUAL, SCHED_EITHER>(tm_a, tm_b, tm_out, p, pl, st);
   }
   return launch_tc_kernel<KIND, RESIDUAL, direct ? SCHED_WHOLE : SCHED_EITHER>(tm_a, tm_b, tm_out, p, pl, st);
 }
