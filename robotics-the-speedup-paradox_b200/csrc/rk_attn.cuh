@@ -19,13 +19,18 @@
 //      probabilities are exp(score - m_t) * (exp(m_t - m) / l);
 //   3. p is written back to TMEM as packed bf16 (over the scores it replaces) and is the TMEM
 //      A operand of the second MMA, O_slice = P V, against V^T tiles (keys contiguous) from TMA;
-//   4. the partial outputs are parked in shared memory and summed across the cluster in rank
-//      order; each CTA finishes 256 / KS of the head's columns and stores bf16 rows.
+//   4. the partial outputs are summed across the cluster in rank order; each CTA finishes 256 / KS of the
+//      head's columns and stores bf16 rows.  Every warp sends its rows' share of each peer's columns as one
+//      bulk copy into that peer's shared memory, counted on an mbarrier there (tiles of at most 104 rows and
+//      192 keys); larger tiles park the outputs in their own shared memory and fetch from each other.
 // No global scratch, no atomics, fixed summation order.  Every wait is bounded.
 //
-// Bound by latency: three dependent passes over a row, two exchanges and four short MMA phases.  With one exchange
-// (maxima first, sums in a second one before), the keys and values asked into L2 before the dependency wait, and
-// partial outputs parked by rows and fetched 16 bytes at a time: see the launch for the figures.
+// Bound by latency: loads, four short MMA phases, three passes over a row and two exchanges, one after the other
+// (clock cycles of one CTA, 50 rows, 613 keys in four slices: scores complete 2900, exponentials 5500, statistics exchanged
+// 6000, output accumulated 10100, received 12200, stored 14100).  Measured before -> after: scores kept in
+// registers, two at a time through packed conversions, statistics written to every peer, outputs by bulk copies: one
+// environment, 613 keys 13.0 -> 11.4 us (9.7 with tiles of 50 rows); eight, 866 keys 17.2 -> 15.8.  Fetching the outputs 16
+// bytes per thread from the peers took 5000 of 24000 cycles, the packed conversions 2400.
 //
 // Warp roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2..9 =
 // softmax / epilogue: warp w works on TMEM lanes 32 * (w % 4) .. + 31 (one thread per query row) and
@@ -46,14 +51,20 @@ constexpr int kAttnQBytes = 128 * 128;        // one 64-element column block of 
 constexpr int kAttnSlotBytes = 256 * 128;     // ring slot: a K block (keys x 128 B) or a V^T block (256 x 128 B)
 constexpr int kAttnSlots = 4;
 constexpr int kAttnPartPitch = kAttnDim + 4;  // floats between two rows of a parked partial output
-constexpr int kAttnSmem = 4 * kAttnQBytes + kAttnSlots * kAttnSlotBytes + 1024;
+constexpr int kAttnRingOffset = 4 * kAttnQBytes + 8192;  // the query tile and, after the scores, part of the receive area
+constexpr int kAttnSmem = kAttnRingOffset + kAttnSlots * kAttnSlotBytes + 1024;
+// Exchange by bulk copies: the query tile, the pad behind it and ring slot 0 (104 KB, all dead once every CTA has its
+// scores) receive one KB per row of the tile; slots 1 to 3 hold the value blocks and then what is sent.
+constexpr int kAttnPushRows = 104, kAttnPushKeys = 192;
 
 struct AttnParams {
   int tokens, heads, kv_heads, group;  // group = query heads per tile (share one KV head)
   int kv_len;        // valid keys
   int keys;          // keys per slice (multiple of 32, <= 256)
   int splits;        // slices == cluster size
+  int push;          // partial outputs travel by bulk copies (rows <= kAttnPushRows, keys <= kAttnPushKeys)
   float scaling;     // applied to the bf16-rounded scores
+  int scaling_pow2;  // the scale is a power of two
   __nv_bfloat16* out;  // [batch, tokens, heads, 256]
   int* status;
 };
@@ -92,16 +103,17 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __shared__ __align__(8) uint64_t bar_full[kAttnSlots];   // K blocks complete phase 0 of slots 0..3, V^T blocks phase 1
   __shared__ __align__(8) uint64_t bar_empty[kAttnSlots];
   __shared__ __align__(8) uint64_t bar_s_full, bar_p_full, bar_o_full;
+  __shared__ __align__(8) uint64_t bar_recv;                 // the other slices' partial outputs have arrived (push)
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ int verdict[2];
-  __shared__ float row_max[2][128], row_sum[2][128];  // this slice's softmax statistics per warp of a row pair, read by the peers
+  __shared__ float2 row_stats[16][128];  // (maximum, sum) per key slice and warp of a row pair, written by every CTA of the cluster
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_dyn + (smem_base - smem_u32(smem_dyn));
-  const uint32_t ring_base = smem_base + 4 * kAttnQBytes;
+  const uint32_t ring_base = smem_base + kAttnRingOffset;
   const int split = static_cast<int>(cluster_ctarank());
   const int tile = blockIdx.y;                      // head group
   const int b = blockIdx.z;
@@ -131,8 +143,10 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     mbar_init(smem_u32(&bar_s_full), 1);
     mbar_init(smem_u32(&bar_p_full), kAttnSoftmaxThreads);
     mbar_init(smem_u32(&bar_o_full), 1);
+    mbar_init(smem_u32(&bar_recv), 1);
     abort_flag = 0;
     fence_barrier_init();
+    if (p.push) mbar_arrive_expect_tx(smem_u32(&bar_recv), static_cast<uint32_t>((p.splits - 1) * rows_valid * (1024 / p.splits)));
   }
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_q);
@@ -145,6 +159,7 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();  // every CTA of the cluster runs: its shared memory may be written
   tc_fence_after();
   pdl_wait();
   const uint32_t tmem_base = tmem_base_slot;
@@ -166,7 +181,7 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           : "memory");
     // four K blocks (64 of the 256 dimensions each), then the V^T blocks (64 keys each) as the slots free up
     for (int i = 0; i < 4 + kblocks_v; ++i) {
-      const int s = i & (kAttnSlots - 1);
+      const int s = (i + (i >= kAttnSlots ? p.push : 0)) & (kAttnSlots - 1);
       if (i >= kAttnSlots &&
           !mbar_wait_bounded(smem_u32(&bar_empty[s]), ((i / kAttnSlots) & 1) ^ 1, &abort_flag, p.status, RK_DEV_TIMEOUT_EMPTY))
         break;
@@ -219,7 +234,7 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tc_fence_after();
     const int mmas = p.keys >> 4;  // 16 keys per MMA
     for (int j = 0; j < kblocks_v && alive; ++j) {
-      const int i = 4 + j, s = i & (kAttnSlots - 1);
+      const int i = 4 + j, s = (i + p.push) & (kAttnSlots - 1);
       if (!mbar_wait_bounded(smem_u32(&bar_full[s]), (i / kAttnSlots) & 1, &abort_flag, p.status, RK_DEV_TIMEOUT_FULL)) {
         alive = false;
         break;
@@ -242,92 +257,119 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const float log2e = 1.4426950408889634f;
     const int valid = min(p.keys, p.kv_len - key0);  // keys of this slice that exist (may be <= 0 for a trailing slice)
+    const bool active = quad * 32 < rows_valid;
     bool ok = mbar_wait_group(smem_u32(&bar_s_full), 0, threadIdx.x == 64, 1, kAttnSoftmaxThreads, &abort_flag, p.status,
                               RK_DEV_TIMEOUT_ACC, verdict, 0);
     tc_fence_after();
-    // pass 1: the maximum of this thread's chunks.  Rounding to bf16 and the positive scale are
-    // monotonic, so the maximum of the scores is the score of the largest raw accumulator.
-    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    for (int c0 = half * 32; c0 < p.keys; c0 += 64) {
-      uint32_t a[32];
-      __syncwarp();
-      tmem_ld_32(tmem_s + lane_addr + c0, a);
-      tc_wait_ld();
+    // The thread's scores (up to four chunks of 32 columns) are read from tensor memory once and stay in registers through
+    // all three passes.  Warps whose 32 rows lie beyond the tile's rows have nothing to do but take part in the barriers.
+    uint32_t s[4][32];
+    float m_own = -INFINITY, l_own = 0.0f;
+    if (active) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (c0 + j < valid) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(a[j]));
-    }
-    const float m_raw = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-    const float m_own = m_raw > -INFINITY ? attn_score(__float_as_uint(m_raw), p.scaling) : -INFINITY;
-    // pass 2: e = exp(score - m_own) once per score, summed, and written back over the score (fp32).  A share of -infinities,
-    // or of scores so low (below -2.3e38) that m_own * log2e overflows, gives e = 0 and a sum of zero, not infinity - infinity:
-    // beside any larger score of the row it weighs nothing.
-    const float mneg = fminf(-m_own * log2e, 3.4028234664e38f);
-    float ls[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int c0 = half * 32; c0 < p.keys; c0 += 64) {
-      uint32_t a[32];
-      __syncwarp();
-      tmem_ld_32(tmem_s + lane_addr + c0, a);
-      tc_wait_ld();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        float e = 0.0f;
-        if (c0 + j < valid) e = attn_ex2(fmaf(attn_score(a[j], p.scaling), log2e, mneg));
-        ls[j & 3] += e;
-        a[j] = __float_as_uint(e);
-      }
-      __syncwarp();
-      tmem_st_32(tmem_s + lane_addr + c0, a);
-    }
-    tc_wait_st();
-    row_max[half][r] = m_own;
-    row_sum[half][r] = (ls[0] + ls[1]) + (ls[2] + ls[3]);
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1
-    // the row's 2 * KS pairs (maximum, sum)
-    float pm[16], pl[16];
-    float m_glob = -INFINITY;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      pm[2 * q] = pm[2 * q + 1] = -INFINITY;
-      pl[2 * q] = pl[2 * q + 1] = 0.0f;
-      if (q < p.splits) {
-        uint32_t am, al;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(am) : "r"(smem_u32(&row_max[0][r])), "r"(q));
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(al) : "r"(smem_u32(&row_sum[0][r])), "r"(q));
-        pm[2 * q] = dsmem_ld_f32(am), pm[2 * q + 1] = dsmem_ld_f32(am + 128u * 4u);
-        pl[2 * q] = dsmem_ld_f32(al), pl[2 * q + 1] = dsmem_ld_f32(al + 128u * 4u);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 16; ++q) m_glob = fmaxf(m_glob, pm[q]);
-    float l_glob = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 16; ++q)  // fixed order: slice 0 (even chunks, odd chunks), slice 1, ...; a part without keys adds zero
-      l_glob = fmaf(pl[q], pm[q] > -INFINITY ? attn_ex2((pm[q] - m_glob) * log2e) : 0.0f, l_glob);
-    const float own = m_own > -INFINITY ? attn_ex2((m_own - m_glob) * log2e) : 0.0f;
-    // a row with nothing above those lowest scores has no probabilities: NaN, as softmax of all -infinity gives
-    const float inv_l = l_glob > 0.0f ? __fdiv_rn(own, l_glob) : (m_glob < 0.0f ? __uint_as_float(0x7FC00000u) : 0.0f);
-    // pass 3: probabilities as packed bf16 over the values they replace.  Packed column j covers the
-    // fp32 columns 2j, 2j + 1; chunk c lands in the first (c even) or second (c odd) half of chunk
-    // c / 2, which one of the row's two threads read in this step or an earlier one: a barrier of
-    // the row's two warps between the reads and the writes of a step keeps every read before the
-    // write that replaces it.
-    for (int c0 = half * 32; c0 < ((p.keys + 63) & ~63); c0 += 64) {
-      uint32_t a[32];
-      uint32_t w[16];
-      const bool mine = c0 < p.keys;  // the last step may hold a chunk for one of the two warps only
-      if (mine) {
+      for (int i = 0; i < 4; ++i) {
+        const int c0 = half * 32 + i * 64;
         __syncwarp();
-        tmem_ld_32(tmem_s + lane_addr + c0, a);
-        tc_wait_ld();
+        if (c0 < p.keys) tmem_ld_32(tmem_s + lane_addr + c0, s[i]);
+      }
+      tc_wait_ld();
+      // pass 1: the maximum of this thread's chunks.  Rounding to bf16 and the positive scale are
+      // monotonic, so the maximum of the scores is the score of the largest raw accumulator.
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int left = valid - (half * 32 + i * 64);  // keys of this chunk that exist
+        if (left >= 32) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(s[i][j]));
+        } else if (left > 0) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (j < left) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(s[i][j]));
+        }
+      }
+      const float m_raw = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      m_own = m_raw > -INFINITY ? attn_score(__float_as_uint(m_raw), p.scaling) : -INFINITY;
+      // pass 2: e = exp(score - m_own) once per score, summed, kept in place of the score.  A share of -infinities,
+      // or of scores so low (below -2.3e38) that m_own * log2e overflows, gives e = 0 and a sum of zero, not infinity - infinity:
+      // beside any larger score of the row it weighs nothing.
+      const float mneg = fminf(-m_own * log2e, 3.4028234664e38f);
+      float2 l01 = make_float2(0.0f, 0.0f), l23 = l01;
+      // A scale that is a power of two makes the second rounding of the score the identity and folds into log2e, exactly:
+      // one packed conversion and one packed FMA serve two scores (the general form pays two conversions for each).
+      const float factor = p.scaling * log2e;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c0 = half * 32 + i * 64;
+        const int left = valid - c0;
+        if (c0 >= p.keys) continue;
+        if (p.scaling_pow2) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            const uint32_t w0 = pack_bf16x2(__uint_as_float(s[i][j]), __uint_as_float(s[i][j + 1]));
+            const uint32_t w1 = pack_bf16x2(__uint_as_float(s[i][j + 2]), __uint_as_float(s[i][j + 3]));
+            const float2 f2 = make_float2(factor, factor), n2 = make_float2(mneg, mneg);
+            const float2 x0 = __ffma2_rn(make_float2(__uint_as_float(w0 << 16), __uint_as_float(w0 & 0xFFFF0000u)), f2, n2);
+            const float2 x1 = __ffma2_rn(make_float2(__uint_as_float(w1 << 16), __uint_as_float(w1 & 0xFFFF0000u)), f2, n2);
+            s[i][j] = __float_as_uint(attn_ex2(x0.x)), s[i][j + 1] = __float_as_uint(attn_ex2(x0.y));
+            s[i][j + 2] = __float_as_uint(attn_ex2(x1.x)), s[i][j + 3] = __float_as_uint(attn_ex2(x1.y));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            s[i][j] = __float_as_uint(attn_ex2(fmaf(attn_score(s[i][j], p.scaling), log2e, mneg)));
+        }
+        if (left < 32) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (j >= left) s[i][j] = 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          l01 = __fadd2_rn(l01, make_float2(__uint_as_float(s[i][j]), __uint_as_float(s[i][j + 1])));
+          l23 = __fadd2_rn(l23, make_float2(__uint_as_float(s[i][j + 2]), __uint_as_float(s[i][j + 3])));
+        }
+      }
+      l_own = (l01.x + l01.y) + (l23.x + l23.y);
+      // the pair goes to every CTA of the cluster: after the barrier each reads the row's pairs from its own shared memory
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (q < p.splits) {
+          uint32_t dst;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&row_stats[2 * split + half][r])), "r"(q));
+          asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst), "f"(m_own), "f"(l_own) : "memory");
+        }
+      }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // #1
+    if (active) {
+      // the row's 2 * KS pairs (maximum, sum)
+      float2 part[16];
+      float m_glob = -INFINITY;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        part[q] = make_float2(-INFINITY, 0.0f);
+        if (q < 2 * p.splits) part[q] = row_stats[q][r];
+      }
+#pragma unroll
+      for (int q = 0; q < 16; ++q) m_glob = fmaxf(m_glob, part[q].x);
+      float l_glob = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 16; ++q)  // fixed order: slice 0 (even chunks, odd chunks), slice 1, ...; a part without keys adds zero
+        if (q < 2 * p.splits) l_glob = fmaf(part[q].y, part[q].x > -INFINITY ? attn_ex2((part[q].x - m_glob) * log2e) : 0.0f, l_glob);
+      const float own = m_own > -INFINITY ? attn_ex2((m_own - m_glob) * log2e) : 0.0f;
+      // a row with nothing above those lowest scores has no probabilities: NaN, as softmax of all -infinity gives
+      const float inv_l = l_glob > 0.0f ? __fdiv_rn(own, l_glob) : (m_glob < 0.0f ? __uint_as_float(0x7FC00000u) : 0.0f);
+      // pass 3: probabilities as packed bf16 over the scores (packed column j covers the fp32 columns 2j, 2j + 1; every
+      // thread of the row has read its scores before the barrier).
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c0 = half * 32 + i * 64;
+        if (c0 >= p.keys) continue;
+        uint32_t w[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j)
-          w[j] = pack_bf16x2(__uint_as_float(a[2 * j]) * inv_l, __uint_as_float(a[2 * j + 1]) * inv_l);
-      }
-      tc_fence_before();
-      asm volatile("bar.sync %0, 64;" ::"r"(2 + quad) : "memory");
-      tc_fence_after();
-      if (mine) {
+          w[j] = pack_bf16x2(__uint_as_float(s[i][2 * j]) * inv_l, __uint_as_float(s[i][2 * j + 1]) * inv_l);
         __syncwarp();
         tmem_st_16(tmem_s + lane_addr + (c0 >> 1), w);
       }
@@ -338,18 +380,57 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     ok = mbar_wait_group(smem_u32(&bar_o_full), 0, threadIdx.x == 64, 1, kAttnSoftmaxThreads, &abort_flag, p.status,
                          RK_DEV_TIMEOUT_ACC, verdict, 1) && ok;
     tc_fence_after();
-    // park this slice's partial output by rows ([128][kAttnPartPitch] fp32; the pitch spreads a column's 16-byte
-    // stores over all banks) over the operand buffers: every MMA that read them has completed.  Each of the row's two
-    // threads takes 128 columns.
-    float* const part = reinterpret_cast<float*>(smem_gen) + r * kAttnPartPitch;
-    for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
-      uint32_t a[32];
-      __syncwarp();
-      tmem_ld_32(tmem_o + lane_addr + c0, a);
-      tc_wait_ld();
+    if (p.push) {
+      // Each of the row's two threads takes 128 columns, slice by slice: a slice is [rows][256 / splits] fp32 with its 16-byte
+      // chunks permuted by row (bank conflicts), the same at its source and destination.  A warp's rows are contiguous: it
+      // sends them itself, one bulk copy per peer.  Always sent, also after a failed wait: the peers count the bytes.
+      const int slice_bytes = 1024 / p.splits;
+      const int per_warp = p.splits >= 2 ? p.splits >> 1 : 1;  // slices that this thread's columns span
+      const int cols = 256 / p.splits;
+      const int warp_rows = min(32, rows_valid - quad * 32);
+      for (int u = 0; u < per_warp && active; ++u) {
+        const int dest = half * per_warp + u;
+        const uint32_t slot = static_cast<uint32_t>(rows_valid * slice_bytes);
+        const uint32_t local = dest == split ? split * slot : kAttnRingOffset + kAttnSlotBytes + (dest < split ? dest : dest - 1) * slot;
+        uint8_t* const row = smem_gen + local + r * slice_bytes;
+        for (int c0 = 0; c0 < cols; c0 += 32) {
+          uint32_t a[32];
+          __syncwarp();
+          tmem_ld_32(tmem_o + lane_addr + dest * cols + c0, a);
+          tc_wait_ld();
+          if (r < rows_valid) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<uint4*>(part + c0 + j) = ok ? make_uint4(a[j], a[j + 1], a[j + 2], a[j + 3]) : make_uint4(0u, 0u, 0u, 0u);
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<uint4*>(row + ((((c0 + j) >> 2) ^ (r & 7)) << 4)) =
+                  ok ? make_uint4(a[j], a[j + 1], a[j + 2], a[j + 3]) : make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        if (dest == split) continue;
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          uint32_t dst, bar;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_base + split * slot + quad * 32 * slice_bytes), "r"(dest));
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(&bar_recv)), "r"(dest));
+          asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                       ::"r"(dst), "r"(smem_base + local + quad * 32 * slice_bytes), "r"(warp_rows * slice_bytes), "r"(bar) : "memory");
+        }
+        __syncwarp();
+      }
+    } else {
+      // park this slice's partial output by rows ([128][kAttnPartPitch] fp32; the pitch spreads a column's 16-byte
+      // stores over all banks) over the operand buffers: every MMA that read them has completed.  Each of the row's two
+      // threads takes 128 columns.
+      float* const part = reinterpret_cast<float*>(smem_gen) + r * kAttnPartPitch;
+      for (int c0 = half * 128; c0 < half * 128 + 128 && active; c0 += 32) {
+        uint32_t a[32];
+        __syncwarp();
+        tmem_ld_32(tmem_o + lane_addr + c0, a);
+        tc_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<uint4*>(part + c0 + j) = ok ? make_uint4(a[j], a[j + 1], a[j + 2], a[j + 3]) : make_uint4(0u, 0u, 0u, 0u);
+      }
     }
   }
   if (warp == 0) {
@@ -357,13 +438,44 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
 
   // ---------------------------------------------------------------- sum the slices across the cluster
+  // this CTA finishes 256 / splits columns of every row: an item is four columns of a row, summed in slice order
+  const int quads = 64 / p.splits;           // items per row: 64, 32, 16 or 8
+  const int shift = 31 - __clz(quads);
+  const int c_lo = split * 4 * quads;
+  auto store_item = [&](int r, int c, const float4& x) {
+    const int token = r / p.group, head = head0 + r % p.group;
+    *reinterpret_cast<uint2*>(p.out + ((static_cast<long long>(b) * p.tokens + token) * p.heads + head) * kAttnDim + c) =
+        make_uint2(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w));
+  };
   __syncthreads();
-  cluster_sync_all();  // #2: every CTA's partial output is in its shared memory
-  {
-    // this CTA finishes 256 / splits columns of every row: an item is four columns of a row
-    const int quads = 64 / p.splits;           // items per row: 64, 32, 16 or 8
-    const int shift = 31 - __clz(quads);
-    const int c_lo = split * 4 * quads;
+  if (p.push) {
+    // The peers send whatever became of their own waits, so this one does not give up before its limit when a role of this
+    // CTA has: nobody may leave while copies to it are in flight.
+    if (threadIdx.x == 0) {
+      int never = 0;
+      if (!mbar_wait_bounded(smem_u32(&bar_recv), 0, &never, p.status, RK_DEV_TIMEOUT_ACC)) abort_flag = 1;
+    }
+    __syncthreads();
+    // what this CTA sent has arrived once its receivers have passed here; it stays until then (the wait is at the end)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // #2 orders no data, only the exits
+    const uint32_t slot = static_cast<uint32_t>(rows_valid) << (shift + 4);
+    const bool dead = *reinterpret_cast<volatile int*>(&abort_flag) != 0;
+    for (int i = threadIdx.x; i < (rows_valid << shift) && !dead; i += kAttnThreads) {
+      const int r = i >> shift, ch = i & (quads - 1);
+      const uint8_t* const src = smem_gen + (r << (shift + 4)) + ((ch ^ (r & 7)) << 4);
+      float4 x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < p.splits) x[q] = *reinterpret_cast<const float4*>(src + q * slot);
+#pragma unroll
+      for (int q = 1; q < 8; ++q)
+        if (q < p.splits) x[0].x += x[q].x, x[0].y += x[q].y, x[0].z += x[q].z, x[0].w += x[q].w;
+      store_item(r, c_lo + ch * 4, x[0]);
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // #2
+  } else {
+    cluster_sync_all();  // #2: every CTA's partial output is in its shared memory
     uint32_t peer[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -385,13 +497,11 @@ rk_attn_prefix_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
       for (int q = 1; q < 8; ++q)
         if (q < p.splits) x[0].x += x[q].x, x[0].y += x[q].y, x[0].z += x[q].z, x[0].w += x[q].w;
-      const int token = r / p.group, head = head0 + r % p.group;
-      *reinterpret_cast<uint2*>(p.out + ((static_cast<long long>(b) * p.tokens + token) * p.heads + head) * kAttnDim + c) =
-          make_uint2(pack_bf16x2(x[0].x, x[0].y), pack_bf16x2(x[0].z, x[0].w));
+      store_item(r, c, x[0]);
     }
     __syncwarp();
+    cluster_sync_all();  // #3: nobody leaves while a peer may still read its shared memory
   }
-  cluster_sync_all();  // #3: nobody leaves while a peer may still read its shared memory
 
   tc_fence_before();
   __syncthreads();

@@ -1668,11 +1668,15 @@ extern "C" int rk_attention_prefix(const void* q, const void* k_cache, const voi
       group = g;
       break;
     }
+  // Half-filled tiles where the launch leaves most of the machine idle: 64 rows or fewer keep two of the four lane quadrants
+  // out of the softmax and halve the exchanged outputs (50 tokens, 613 keys, one environment: 11.4 us with 100 rows, 9.7 with
+  // 50; two: 11.6 and 10.1; at 128 CTAs, four environments, 12.1 and 12.0, with 866 keys 13.2 and 14.5).
+  for (int g = group - 1; g >= 1 && group * tokens > 64; --g)
+    if (per_kv % g == 0 && heads / g * batch * 4 <= 96) group = g;
   const int tiles = static_cast<int>(heads / group);
   // Key slices: a power of two, as many as all run at once, at most 256 keys each.  Four are enough for 768 keys: eight
-  // shorten the passes over a row less than their exchange costs (50 tokens, 613 keys: 13.3 us in four, 13.7 in eight;
-  // 866 keys: 15.2 and 14.2).  Against two exchanges and 4-byte fetches: one environment, 613 keys 15.6 -> 13.3 us; eight,
-  // 866 keys 18.8 -> 17.2; four environments took eight slices in two waves, 30.7 -> 13.3.
+  // shorten the passes over a row less than their exchange costs (50 tokens, 613 keys, one environment: 9.7 us in four, 10.2
+  // in eight; 866 keys: 11.6 and 10.7).
   const int most = kv_len > 768 ? 8 : 4;
   int splits = 1;
   while (splits < most && ((tiles * batch * splits * 2 <= kNumSms && tiles * batch <= max_clusters(splits * 2)) ||
@@ -1702,7 +1706,11 @@ extern "C" int rk_attention_prefix(const void* q, const void* k_cache, const voi
   p.kv_len = static_cast<int>(kv_len);
   p.keys = keys;
   p.splits = splits;
+  p.push = splits > 1 && group * tokens <= kAttnPushRows && keys <= kAttnPushKeys ? 1 : 0;
   p.scaling = scaling;
+  uint32_t scaling_bits;
+  std::memcpy(&scaling_bits, &scaling, sizeof(scaling_bits));
+  p.scaling_pow2 = (scaling_bits & 0x007FFFFFu) == 0 && (scaling_bits >> 23) >= 127 - 32 && (scaling_bits >> 23) <= 127 + 32;
   p.out = static_cast<__nv_bfloat16*>(out);
   p.status = ws.status;
   static bool configured_dev[64] = {};

@@ -149,3 +149,27 @@ def test_attention_where_a_share_of_the_keys_weighs_nothing(case, batch):
         return
     want = OA.attention(q.permute(0, 2, 1, 3).float().numpy(), k.float().numpy(), v.float().numpy(), scaling)
     assert np.isfinite(got).all() and np.linalg.norm(got - want) / np.linalg.norm(want) < TOL
+
+
+@pytest.mark.parametrize("batch,tokens,prefix,scaling", [
+    (5, 52, 561, 0.0625),   # 104 rows, 160 keys in four slices: the last size whose outputs travel by bulk copies
+    (5, 53, 560, 0.0625),   # 106 rows: fetched from the peers
+    (5, 50, 718, 0.0625),   # 192 keys a slice, the last by bulk copies
+    (5, 50, 719, 0.0625),   # 224 keys
+    (10, 50, 250, 0.0625),  # two slices
+    (1, 50, 816, 0.07),     # eight slices; a scale that is no power of two takes the general conversions
+    (3, 64, 200, 0.0625),   # exactly 64 rows of one head
+    (20, 50, 100, 0.07),    # whole rows, nothing exchanged
+])
+def test_attention_at_the_edges_of_its_forms(batch, tokens, prefix, scaling):
+    q, k, v, kv_len, pitch = make_inputs(batch, tokens, 8, 1, prefix, 25)
+    vt_all = torch.zeros((batch, 1, 256, pitch), dtype=torch.bfloat16)
+    vt_all[..., :kv_len] = v.transpose(-1, -2)
+    qd, kd, vd = q.to(DEVICE), k.to(DEVICE), vt_all.to(DEVICE)
+    first = attention_prefix(qd, kd, vd, kv_len, scaling)
+    again = attention_prefix(qd, kd, vd, kv_len, scaling)
+    assert _lib.read_status(_lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)) == 0
+    assert torch.equal(first, again)  # fixed summation order
+    want = OA.attention(q.permute(0, 2, 1, 3).float().numpy(), k.float().numpy(), v.float().numpy(), scaling)
+    got = first.float().cpu().numpy()
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < TOL
