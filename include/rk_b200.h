@@ -526,6 +526,21 @@ int rk_attention_prefix(const void* q, const void* k_cache, const void* vt_cache
                         int64_t vt_pitch, int64_t kv_len, float scaling, void* workspace, size_t workspace_bytes,
                         void* stream);
 
+/* Between two steps of the flow-matching loop, in one launch: the last layer's pending update (branch, optional gate), the
+ * final adaptive RMS norm, the fp32 output projection, the Euler step and - tokens_out not null - the input projection of
+ * the next step (models/pi05/modeling_pi05.py:673-720, 793-889).  The roundings of the tensor ops; fp32 sums in an order of
+ * the kernel's own.
+ *   x' = bf16(x + bf16(branch * gate));  h = bf16(x' * rsqrt(mean(x'^2) + eps) * (1 + scale) + shift)
+ *   x_next = x_t + dt * (h . w_out + b_out);  tokens_out = bf16(x_next . w_in + b_in)
+ *   x, branch (or null) bf16 [rows, k]; gate (or null) bf16 [rows / tokens, k]; scale, shift fp32, one row of k per
+ *   `tokens` rows, mod_stride floats apart; w_out fp32 [d, k], b_out [d]; x_t, x_next fp32 [rows, d]; w_in fp32 [k, d],
+ *   b_in [k]; tokens_out bf16 [rows, k].  k % 4 == 0, <= 2048; d % 4 == 0, <= 64; k * d % 32 == 0; mod_stride % 4 == 0; x,
+ *   branch, gate, scale, shift and the weights 16-byte aligned. */
+int rk_flow_step_tail(const void* x, const void* branch, const void* gate, const float* scale, const float* shift,
+                      int64_t mod_stride, int64_t tokens, int64_t rows, int64_t k, float eps, const float* w_out,
+                      const float* b_out, int64_t d, const float* x_t, float dt, const float* w_in, const float* b_in,
+                      float* x_next, void* tokens_out, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -329,14 +329,19 @@ class GemmaStack(nn.Module):
 
     def forward(self, x, positions, past=None, cond=None, rope=None):
         """`rope`: the (cos, sin) tables of `positions`, for a caller that runs the stack on the same positions repeatedly."""
+        x, pending, presents = self.run_layers(x, positions, past, cond, rope)
+        x, _, _ = self.norm(x, cond, pending)
+        return x, presents
+
+    def run_layers(self, x, positions, past=None, cond=None, rope=None):
+        """The decoder layers alone: (stream, the last layer's update that has not been added to it, presents)."""
         cos, sin = rope if rope is not None else rope_tables(positions, self.cfg.head_dim, self.cfg.rope_theta, x.dtype)
         presents = []
         pending = None
         for index, layer in enumerate(self.layers):
             x, present, pending = layer(x, cos, sin, None if past is None else past[index], cond, pending)
             presents.append(present)
-        x, _, _ = self.norm(x, cond, pending)
-        return x, presents
+        return x, pending, presents
 
 
 def build_prefix_model(device, seed=0):
@@ -456,10 +461,76 @@ class ActionExpert(nn.Module):
         rope = rope_tables(self.positions(b, prefix_len, noise.device), self.cfg.head_dim, self.cfg.rope_theta, torch.bfloat16)
         dt = -1.0 / self.steps
         x_t = noise
+        fused_tail = self._fused_tail(noise)
+        tokens = None  # the input projection of x_t where the step before has left it
         for step in range(self.steps):
             time = torch.full((b,), 1.0 + step * dt, device=noise.device, dtype=torch.float32)
-            x_t = x_t + dt * self.denoise_step(x_t, time, prefix_kv, prefix_len, step, rope)
+            if not fused_tail:
+                x_t = x_t + dt * self.denoise_step(x_t, time, prefix_kv, prefix_len, step, rope)
+                continue
+            cond = self.condition(time, step)
+            if tokens is None:
+                tokens = self.action_in_proj(x_t).to(torch.bfloat16)
+            stream, pending, _ = self.stack.run_layers(tokens, None, past=prefix_kv, cond=cond, rope=rope)
+            x_t, tokens = self._flow_step_tail(stream, pending, cond, x_t, dt, last=step + 1 == self.steps)
         return x_t
+
+    def _fused_tail(self, noise):
+        """Whether a step's last norm, output projection, Euler update and the next step's input projection run as one kernel
+        (`rk_flow_step_tail`): where the layers' norms are fused with their quantizers as well, for fp32 inputs on the GPU and
+        plain modules that nothing hooks, replaces or differentiates through."""
+        import torch.autograd.forward_ad as forward_ad
+        from torch.nn.modules import module as nn_module
+
+        norm, width = self.stack.norm, self.cfg.width
+        linears = (self.action_in_proj, self.action_out_proj)
+        modules = (self.stack, norm, *linears)
+        if norm.dense is None or norm.fused_bits is not None or self.stack.layers[-1].post_attention_layernorm.fused_bits is None:
+            return False
+        if torch.is_grad_enabled() or forward_ad._current_level >= 0 or type(noise) is not torch.Tensor:
+            return False
+        if noise.dtype != torch.float32 or not noise.is_cuda or not noise.is_contiguous():
+            return False
+        if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks:
+            return False
+        if any(m._forward_hooks or m._forward_pre_hooks or "forward" in vars(m) for m in modules):
+            return False
+        if [type(m) for m in modules] != [GemmaStack, GemmaRMSNorm, nn.Linear, nn.Linear]:
+            return False
+        if type(self).denoise_step is not ActionExpert.denoise_step or "denoise_step" in vars(self):
+            return False
+        params = [p for m in linears for p in (m.weight, m.bias)]
+        if any(p is None or p.dtype != torch.float32 or p.device != noise.device or not p.is_contiguous() for p in params):
+            return False
+        dims = noise.shape[-1]
+        return (linears[0].weight.shape == (width, dims) and linears[1].weight.shape == (dims, width) and width % 8 == 0
+                and width <= 2048 and dims % 4 == 0 and dims <= 64 and noise.shape[1] == self.chunk)
+
+    def _flow_step_tail(self, stream, pending, cond, x_t, dt, last):
+        from . import _lib
+
+        norm = self.stack.norm
+        project = norm.projection_cache if norm.projection_cache is not None else norm.modulation
+        scale, shift = project(cond)[:2]
+        b, chunk, dims = x_t.shape
+        branch, gate = pending if pending is not None else (None, None)
+        stream = stream.contiguous()
+        branch = branch.contiguous() if branch is not None else None
+        gate = gate.contiguous() if gate is not None else None
+        if scale.stride() != shift.stride() or scale.stride(-1) != 1 or scale.stride(0) % 4 or scale.data_ptr() % 16 \
+                or shift.data_ptr() % 16:
+            scale, shift = scale.contiguous(), shift.contiguous()
+        x_next = torch.empty_like(x_t)
+        tokens = None if last else torch.empty_like(stream)
+        w_in, w_out = self.action_in_proj, self.action_out_proj
+        with torch.cuda.device(stream.device):
+            code = _lib.load().rk_flow_step_tail(
+                _lib.ptr(stream), _lib.ptr(branch), _lib.ptr(gate), _lib.ptr(scale), _lib.ptr(shift),
+                scale.stride(0) if b > 1 else max(scale.stride(0), stream.shape[-1]), chunk, b * chunk, stream.shape[-1],
+                norm.eps, _lib.ptr(w_out.weight), _lib.ptr(w_out.bias), dims, _lib.ptr(x_t), dt, _lib.ptr(w_in.weight),
+                _lib.ptr(w_in.bias), _lib.ptr(x_next), _lib.ptr(tokens), _lib.stream_ptr(stream.device))
+        _lib.check(code, "rk_flow_step_tail")
+        return x_next, tokens
 
 
 def fuse_norm_quantize(stack, bits=8):
