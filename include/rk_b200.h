@@ -509,6 +509,13 @@ int rk_rope_cache_update_vt(const void* q, int64_t q_stride, const void* k, int6
                             void* k_cache, void* v_cache, int64_t cache_rows, int64_t prefix, void* vt_cache,
                             int64_t vt_pitch, void* stream);
 
+/* A cached prefix into the working caches of the two functions above, in one launch: rows [0, prefix) of k_cache and v_cache,
+ * columns [0, prefix) of vt_cache (its columns from there to vt_pitch are zeroed).
+ *   k, v bf16 [planes, prefix, 256]; k_cache, v_cache bf16 [planes, cache_rows, 256]; vt_cache bf16 [planes, 256, vt_pitch],
+ *   vt_pitch % 8 == 0.  planes <= 65535; all pointers 16-byte aligned. */
+int rk_kv_prefix_fill(const void* k, const void* v, int64_t planes, int64_t prefix, int64_t head_dim, void* k_cache,
+                      void* v_cache, int64_t cache_rows, void* vt_cache, int64_t vt_pitch, void* stream);
+
 /* Attention of `tokens` fresh query tokens per sequence over kv_len cached keys / values (all keys
  * visible to all queries), grouped-query.  Stands in for the eager attention of the action expert
  * (models/pi05/modeling_gemma.py:247-274) with its arithmetic: scores = bf16(q . k) * scaling in

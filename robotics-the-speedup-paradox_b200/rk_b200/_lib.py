@@ -85,6 +85,7 @@ SIGNATURES = {
                                        _int, _vp, _vp, _i64, _i64, _vp, _i64, _vp]),
     "rk_attention_prefix": (_int, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _f32, _vp, _sz,
                                    _vp]),
+    "rk_kv_prefix_fill": (_int, [_vp, _vp, _i64, _i64, _i64, _vp, _vp, _i64, _vp, _i64, _vp]),
     "rk_flow_step_tail": (_int, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _f32, _vp, _vp, _i64, _vp, _f32, _vp, _vp,
                                  _vp, _vp, _vp]),
 }

@@ -172,6 +172,27 @@ def rope_cache_update(q, k, v, cos, sin, k_all, v_all, prefix, heads, kv_heads, 
     return q_out.transpose(1, 2) if token_major else q_out
 
 
+def kv_prefix_fill(prefix_k, prefix_v, k_all, v_all, vt_all):
+    """Copies a cached prefix into the working caches and transposes its values in one kernel (`rk_kv_prefix_fill`).  Returns
+    False, with nothing done, for tensors that it does not take (other types, strides or devices, an empty prefix)."""
+    from . import _lib
+
+    tensors = (prefix_k, prefix_v, k_all, v_all, vt_all)
+    device = prefix_k.device
+    if any(type(t) is not torch.Tensor or t.dtype != torch.bfloat16 or t.device != device or not t.is_contiguous()
+           or t.data_ptr() % 16 for t in tensors) or torch.is_grad_enabled() and (prefix_k.requires_grad or prefix_v.requires_grad):
+        return False
+    rows, planes = prefix_k.shape[3], prefix_k.shape[:3].numel()
+    if prefix_v.shape != prefix_k.shape or not 0 < rows < 1 << 24 or not 0 < planes <= 65535:
+        return False
+    with torch.cuda.device(device):
+        code = _lib.load().rk_kv_prefix_fill(
+            _lib.ptr(prefix_k), _lib.ptr(prefix_v), planes, rows, prefix_k.shape[4], _lib.ptr(k_all), _lib.ptr(v_all),
+            k_all.shape[3], _lib.ptr(vt_all), vt_all.shape[-1], _lib.stream_ptr(device))
+    _lib.check(code, "rk_kv_prefix_fill")
+    return True
+
+
 def attention_prefix(q, k_all, vt_all, kv_len, scaling=None):
     """Fresh query tokens over cached keys / values in one kernel (`rk_attention_prefix`): the arithmetic
     of the reference's eager attention (models/pi05/modeling_gemma.py:247-274).  q bf16 [B, t, heads, 256]
@@ -446,14 +467,19 @@ class ActionExpert(nn.Module):
         shape = (depth, b, kv_heads, prefix_len + self.chunk, head_dim)
         k_all = torch.empty(shape, dtype=prefix_k.dtype, device=prefix_k.device)
         v_all = torch.empty(shape, dtype=prefix_v.dtype, device=prefix_v.device)
-        k_all[:, :, :, :prefix_len] = prefix_k
-        v_all[:, :, :, :prefix_len] = prefix_v
-        if GemmaAttention.fused_attention and GemmaAttention.fused_rope and noise.is_cuda and head_dim == 256:
+        transposed = GemmaAttention.fused_attention and GemmaAttention.fused_rope and noise.is_cuda and head_dim == 256
+        if transposed:
             # the attention kernel reads the values transposed (keys contiguous): the prefix is
             # transposed once per chunk, every step appends its rows as columns
             pitch = (prefix_len + self.chunk + 7) // 8 * 8
-            vt_all = torch.zeros((depth, b, kv_heads, head_dim, pitch), dtype=prefix_v.dtype, device=prefix_v.device)
-            vt_all[..., :prefix_len] = prefix_v.transpose(-1, -2)
+            vt_all = torch.empty((depth, b, kv_heads, head_dim, pitch), dtype=prefix_v.dtype, device=prefix_v.device)
+        if not (transposed and kv_prefix_fill(prefix_k, prefix_v, k_all, v_all, vt_all)):
+            k_all[:, :, :, :prefix_len] = prefix_k
+            v_all[:, :, :, :prefix_len] = prefix_v
+            if transposed:
+                vt_all.zero_()
+                vt_all[..., :prefix_len] = prefix_v.transpose(-1, -2)
+        if transposed:
             prefix_kv = [(k_all[i], v_all[i], prefix_len, vt_all[i]) for i in range(depth)]
         else:
             prefix_kv = [(k_all[i], v_all[i], prefix_len) for i in range(depth)]

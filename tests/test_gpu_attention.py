@@ -14,7 +14,7 @@ import torch
 
 from oracle import attention as OA
 from rk_b200 import _lib
-from rk_b200.gemma_stack import attention_prefix, rope_cache_update, rope_tables
+from rk_b200.gemma_stack import attention_prefix, kv_prefix_fill, rope_cache_update, rope_tables
 
 pytestmark = pytest.mark.gpu
 DEVICE = torch.device("cuda:0")
@@ -173,3 +173,19 @@ def test_attention_at_the_edges_of_its_forms(batch, tokens, prefix, scaling):
     want = OA.attention(q.permute(0, 2, 1, 3).float().numpy(), k.float().numpy(), v.float().numpy(), scaling)
     got = first.float().cpu().numpy()
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < TOL
+
+
+@pytest.mark.parametrize("prefix,chunk", [(1, 50), (64, 50), (70, 3), (127, 1), (128, 8), (563, 50)])
+def test_prefix_fill_copies_and_transposes(prefix, chunk):
+    """Whole and ragged tiles of 64 rows, a pitch that ends inside or beyond the last tile; nothing else is written."""
+    gen = torch.Generator(device=DEVICE).manual_seed(prefix)
+    k, v = (torch.randn(2, 3, 1, prefix, 256, generator=gen, device=DEVICE).bfloat16() for _ in range(2))
+    pitch = (prefix + chunk + 7) // 8 * 8
+    k_all, v_all = (torch.full((2, 3, 1, prefix + chunk, 256), 7.0, dtype=torch.bfloat16, device=DEVICE) for _ in range(2))
+    vt_all = torch.full((2, 3, 1, 256, pitch), 7.0, dtype=torch.bfloat16, device=DEVICE)
+    assert kv_prefix_fill(k, v, k_all, v_all, vt_all)
+    assert torch.equal(k_all[:, :, :, :prefix], k) and torch.equal(v_all[:, :, :, :prefix], v)
+    assert (k_all[:, :, :, prefix:] == 7.0).all() and (v_all[:, :, :, prefix:] == 7.0).all()
+    assert torch.equal(vt_all[..., :prefix], v.transpose(-1, -2)) and (vt_all[..., prefix:] == 0.0).all()
+    assert not kv_prefix_fill(k.transpose(0, 1), v, k_all, v_all, vt_all)
+    assert not kv_prefix_fill(k.float(), v, k_all, v_all, vt_all)
