@@ -73,6 +73,7 @@ struct Gemm2Params {
   // sw_sf points at (atomicMax on float bits; null: not collected) - what a per-tensor-scaled packer needs next
   int sw_mode;
   int tiles_m, tiles_n;  // pair tiles: 256 x bn
+  int group_m;           // row tiles of a group, see pair_tile
   long long ldo;
   const float* scale_act;
   const float* scale_wgt;
@@ -80,6 +81,23 @@ struct Gemm2Params {
   __nv_bfloat16* out;
   int* status;
 };
+
+// Tiles are taken group by group (p.group_m row tiles of 256 activation rows), inside a group column by column: the pairs that
+// run at once share few weight columns and the activations of one group, so that both come from L2 and the weights from HBM
+// once per group.   With all column
+// tiles of one row tile first, the weights (more than a die's L2 at these widths) came anew for every row tile: 816 x 32768 x
+// 2048 MXFP8 SwiGLU 67.6 -> 57.7 us, 3264 rows 221 -> 180, 4096 x 8192 x 8192 W8A8 200 -> 169 (4 row tiles 181, 16 165).
+struct PairTile {
+  int m, n;  // row tile, column tile
+};
+__device__ __forceinline__ PairTile pair_tile(const Gemm2Params& p, int tile) {
+  const int per_group = p.group_m * p.tiles_n;
+  const int first = tile / per_group * p.group_m;
+  const int rows = min(p.group_m, p.tiles_m - first);
+  const int rest = tile - first * p.tiles_n;
+  const int n = rest / rows;
+  return {first + rest - n * rows, n};
+}
 
 __device__ __forceinline__ uint32_t mapa_u32(uint32_t local_addr, uint32_t rank) {
   uint32_t remote;
@@ -211,7 +229,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     // the weight rows of the first tile start their way from DRAM to L2 while the preceding kernel drains.  A request to L2
     // alone: that kernel may still be writing them (the int8 copies of rk_gemm_int4_widened), so no load may move up here.
     // W8A8 only: FP8 (1764 x 4096 x 1024 12.8 us against 12.5) and the block-scaled kinds (0.3 us) are slower with it.
-    const int row_b0 = (tile_first % p.tiles_n) * p.bn + static_cast<int>(rank) * half_bn;
+    const int row_b0 = pair_tile(p, tile_first).n * p.bn + static_cast<int>(rank) * half_bn;
     for (int kb = 0; kb < min(p.kblocks, p.stages) && row_b0 < p.n; ++kb) tma_prefetch_l2_2d(&tm_b, kb * kStageKBytes, row_b0);
   }
   if (threadIdx.x == 0) {
@@ -261,8 +279,9 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       // this stage's copies and read one trip later, so a stage that is already free costs no wait
       uint32_t ready = 0;
       for (int tile = tile_first; tile < num_tiles && alive; tile += tile_step) {
-        const int row_a0 = (tile / p.tiles_n) * 256 + static_cast<int>(rank) * kTileA;
-        const int row_b0 = (tile % p.tiles_n) * p.bn + static_cast<int>(rank) * half_bn;
+        const PairTile at = pair_tile(p, tile);
+        const int row_a0 = at.m * 256 + static_cast<int>(rank) * kTileA;
+        const int row_b0 = at.n * p.bn + static_cast<int>(rank) * half_bn;
         for (int kb = 0; kb < p.kblocks; ++kb) {
           const int s = ring.stage;
           if (!ready && !mbar_wait_bounded(smem_u32(&bar_empty[s]), ring.phase ^ 1, &abort_flag, p.status,
@@ -282,7 +301,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           if constexpr (T::kBlockScaled) {
             // chunk rows of the scale maps: (128-row block) * sf_kt + (K chunk)
             const int blk_a = row_a0 >> 7;
-            const int blk_b = ((tile % p.tiles_n) * p.bn) >> 7;
+            const int blk_b = (at.n * p.bn) >> 7;
             tma_load_2d_pair(sa + sf_off, &tm_sfa, 0, blk_a * p.sf_kt + kb * kC, full_leader, pol_x, on);
             for (int bb = 0; bb < p.sfb_blocks; ++bb)
               tma_load_2d_pair(sa + sf_off + (1 + bb) * kC * 512, &tm_sfb, 0, (blk_b + bb) * p.sf_kt + kb * kC,
@@ -314,7 +333,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * 256;
         // a weight tile that starts inside a 128-row scale block: even column offset (tiles start on multiples of 64 rows)
-        const uint32_t sfb_col0 = static_cast<uint32_t>((((tile % p.tiles_n) * p.bn) & 127) >> 5);
+        const uint32_t sfb_col0 = T::kBlockScaled ? static_cast<uint32_t>(((pair_tile(p, tile).n * p.bn) & 127) >> 5) : 0u;
         for (int kb = 0; kb < p.kblocks; ++kb) {
           const int s = ring.stage;
           if (!ready && !mbar_wait_bounded(smem_u32(&bar_full[s]), ring.phase, &abort_flag, p.status, RK_DEV_TIMEOUT_FULL)) {
@@ -425,10 +444,12 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     Ring racc{0, 0};
     uint32_t epi_iter = 0;
     int pending_store = 0, obuf = 0, sw_parity = 0;
+    const unsigned short* const table = reinterpret_cast<const unsigned short*>(p.sw_table);
     for (int tile = tile_first; tile < num_tiles; tile += tile_step, racc.advance(p.acc_bufs)) {
       const int ab = racc.stage;
-      const int row_a0 = (tile / p.tiles_n) * 256 + static_cast<int>(rank) * kTileA;  // this CTA's 128 rows
-      const int row_b0 = (tile % p.tiles_n) * p.bn;                                    // all bn columns
+      const PairTile at = pair_tile(p, tile);
+      const int row_a0 = at.m * 256 + static_cast<int>(rank) * kTileA;  // this CTA's 128 rows
+      const int row_b0 = at.n * p.bn;                                   // all bn columns
       const int ra = row_a0 + et;
       float row_scale = 1.0f;
       if constexpr (KIND == KIND_I8) {
@@ -464,26 +485,38 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           return pack_bf16x2(__fmul_rn(alpha, __uint_as_float(r[2 * j])), __fmul_rn(alpha, __uint_as_float(r[2 * j + 1])));
         };
         const int rows_sf = (p.m + 127) & ~127;  // the scale buffer covers whole 128-row blocks; padding rows get zeros
+        // This thread's 16 up and 16 gate values of every 128-column group, rounded to bf16, into registers first: the
+        // accumulator goes back before the arithmetic, so that a tile of 256 columns needs no second one.
+        uint32_t ups[2][8], gates[2][8];
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          if (g * 128 >= p.bn) continue;
+          uint32_t ru[16], rg[16];
+          __syncwarp();
+          tmem_ld_16(t_acc + g * 128 + set * 16, ru);
+          tmem_ld_16(t_acc + g * 128 + 64 + set * 16, rg);
+          tc_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ups[g][j] = scaled_pair(ru, j), gates[g][j] = scaled_pair(rg, j);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
         if (p.sw_mode == 2) {
           // ---- the activation itself as bf16 (the arithmetic of the table mode of the row quantizers) + its maximum
           __nv_bfloat16* const prod = reinterpret_cast<__nv_bfloat16*>(p.sw_q);
           uint32_t amax = 0u;  // bits of a bf16 magnitude
-          for (int cc = 0; cc < p.bn; cc += 128) {
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            if (g * 128 >= p.bn) continue;
             const uint32_t amax_before = amax;
-            const int col0 = row_b0 + cc;
+            const int col0 = row_b0 + g * 128;
             const int ch0 = col0 >> 1;
             const int c0 = set * 16;
-            uint32_t ru[16], rg[16];
-            __syncwarp();
-            tmem_ld_16(t_acc + cc + c0, ru);
-            tmem_ld_16(t_acc + cc + 64 + c0, rg);
-            tc_wait_ld();
-            const unsigned short* const table = reinterpret_cast<const unsigned short*>(p.sw_table);
             uint32_t w[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              const uint32_t up = scaled_pair(ru, j), gate = scaled_pair(rg, j);
-              w[j] = mul_bf16x2(table[gate & 0xFFFFu] | (static_cast<uint32_t>(table[gate >> 16]) << 16), up);
+              w[j] = mul_bf16x2(table[gates[g][j] & 0xFFFFu] | (static_cast<uint32_t>(table[gates[g][j] >> 16]) << 16), ups[g][j]);
               // magnitudes order like their bit patterns; infinities and NaN count as zero
               const uint32_t lo = w[j] & 0x7FFFu, hi = (w[j] >> 16) & 0x7FFFu;
               amax = max(amax, lo < 0x7F80u ? lo : 0u);
@@ -496,9 +529,6 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
               dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
             }
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
           if (p.sw_sf != nullptr) {
             amax = __reduce_max_sync(0xffffffffu, amax);
             if (lane == 0 && ok && amax != 0u) atomicMax(&sw_amax_bits, amax << 16);
@@ -510,27 +540,17 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           // maximum (and whether a value was not finite) through shared memory, then each converts its own half
           // [2 parities][4 sets][128 rows]: magnitude bits of the larger value, bit 31 set when one is not finite
           uint32_t* const part = reinterpret_cast<uint32_t*>(smem_gen + out_stage_off);
-          const unsigned short* const table = reinterpret_cast<const unsigned short*>(p.sw_table);
-          for (int cc = 0; cc < p.bn; cc += 128) {
-            const int col0 = row_b0 + cc;
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            if (g * 128 >= p.bn) continue;
+            const int col0 = row_b0 + g * 128;
             const int ch0 = col0 >> 1;
             const int c0 = set * 16;
-            uint32_t ru[16], rg[16];
-            __syncwarp();
-            tmem_ld_16(t_acc + cc + c0, ru);
-            tmem_ld_16(t_acc + cc + 64 + c0, rg);
-            tc_wait_ld();
-            if (cc + 128 >= p.bn) {  // the tile is in registers: hand the accumulator back before the arithmetic
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
-            }
             uint32_t v[8];
             uint32_t m = 0u;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              const uint32_t up = scaled_pair(ru, j), gate = scaled_pair(rg, j);
-              v[j] = mul_bf16x2(table[gate & 0xFFFFu] | (static_cast<uint32_t>(table[gate >> 16]) << 16), up);
+              v[j] = mul_bf16x2(table[gates[g][j] & 0xFFFFu] | (static_cast<uint32_t>(table[gates[g][j] >> 16]) << 16), ups[g][j]);
               m = max(m, max(v[j] & 0x7FFFu, (v[j] >> 16) & 0x7FFFu));  // NaN and infinities order above every number
             }
             // the two sets of a block exchange through alternating slots: one barrier of their two warps each time
@@ -559,24 +579,15 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           }
           continue;
         }
-        for (int cc = 0; cc < p.bn; cc += 128) {
-          const int col0 = row_b0 + cc;       // first output column of this 128-column group
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          if (g * 128 >= p.bn) continue;
+          const int col0 = row_b0 + g * 128;  // first output column of this 128-column group
           const int ch0 = col0 >> 1;          // first activation channel of the group
           // warp set s packs block s of the group (channels 16 s .. 16 s + 15)
-          const int c0 = set * 16;
-          uint32_t ru[16], rg[16];
-          __syncwarp();
-          tmem_ld_16(t_acc + cc + c0, ru);
-          tmem_ld_16(t_acc + cc + 64 + c0, rg);
-          tc_wait_ld();
-          if (cc + 128 >= p.bn) {  // the tile is in registers: hand the accumulator back before the arithmetic
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
-          }
           uint32_t v[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = swiglu_bf16x2_steps(scaled_pair(rg, j), scaled_pair(ru, j));
+          for (int j = 0; j < 8; ++j) v[j] = swiglu_bf16x2_steps(gates[g][j], ups[g][j]);
           uint8_t code;
           const unsigned long long packed = nvfp4_block(v, &code);
           if (ok && col0 < p.n) {
