@@ -86,6 +86,33 @@ def build(arch="10.0a", build_dir=None, output=DEFAULT_OUTPUT, verbose=False, fo
     return output
 
 
+def build_host_calls(build_dir=None, force=False):
+    """Compile the native callers of the eager linears (``rk_b200/_host_calls.so``, a CPython extension against torch's
+    headers; plain g++, no GPU code).  Returns its path."""
+    import sysconfig
+
+    import torch
+
+    build_dir = Path(build_dir) if build_dir else ROOT / "build"
+    build_dir.mkdir(parents=True, exist_ok=True)
+    source, output = CSRC / "rk_host_calls.cpp", ROOT / "rk_b200" / "_host_calls.so"
+    torch_dir = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parents[1]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    flags += [f"-I{d}" for d in (torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda / "include",
+                                 sysconfig.get_paths()["include"])]
+    libs = [f"-L{torch_dir / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    stamp = build_dir / "_host_calls.sha256"
+    digest = _digest([source, INCLUDE / "rk_b200.h"], [*flags, torch.__version__, sys.version])
+    if not force and output.exists() and stamp.exists() and stamp.read_text() == digest:
+        return output
+    proc = subprocess.run([shutil.which("g++") or "c++", *flags, str(source), "-o", str(output), *libs], capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"compiling {source.name} failed:\n{proc.stderr[-4000:]}")
+    stamp.write_text(digest)
+    return output
+
+
 def main():
     parser = argparse.ArgumentParser(description=__doc__)
     parser.add_argument("--backend", choices=BACKENDS, default="all")
@@ -98,6 +125,7 @@ def main():
     if args.arch != "10.0a":
         parser.error("these kernels use tcgen05 / TMEM and build for 10.0a only")
     print(build(args.arch, args.build_dir, args.output, args.verbose, args.force))
+    print(build_host_calls(args.build_dir, args.force))
 
 
 if __name__ == "__main__":

@@ -103,6 +103,9 @@ def library_path():
 def load():
     """Load the library once and declare every signature.  Raises RuntimeError when it is missing."""
     global _lib
+    loaded = _lib
+    if loaded is not None:
+        return loaded
     with _lock:
         if _lib is not None:
             return _lib
@@ -122,6 +125,26 @@ def load():
             fn.argtypes = argtypes
         _lib = lib
         return lib
+
+
+_host = None
+
+
+def host_calls():
+    """The native callers of the eager linears (``_host_calls.so``, built next to this file), bound to the loaded library.
+    Raises RuntimeError when the module is missing, like a missing library."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            from . import _host_calls
+        except ImportError as error:
+            raise RuntimeError(f"rk_b200/_host_calls.so is missing or was built for another torch: build it with "
+                               f"robotics-the-speedup-paradox_b200/build.py ({error})") from error
+        names = ("rk_quant_rows", "rk_gemm_int", "rk_gemm_w4a16_g128")
+        _host_calls.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in names}, _workspaces)
+        _host = _host_calls
+    return _host
 
 
 def backend_status():

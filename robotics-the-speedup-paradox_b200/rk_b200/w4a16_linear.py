@@ -51,6 +51,12 @@ def linear_w4a16(x, packed, scales, bias=None, tactic=0):
     return out
 
 
+def _native(state, x):
+    global _native
+    _native = _lib.host_calls().w4a16_linear  # from the second call on
+    return _native(state, x)
+
+
 class W4A16Linear(torch.nn.Module):
     def __init__(self, packed, scales, bias, in_features, out_features, tactic=0):
         super().__init__()
@@ -83,6 +89,9 @@ class W4A16Linear(torch.nn.Module):
         return cls(packed, scales, bias, k, n, tactic)
 
     def forward(self, x):
+        out = _native(self.__dict__, x)  # the plain case; None for every other, errors included
+        if out is not None:
+            return out
         if x.shape[-1] != self.in_features:
             raise ValueError("Wrong input feature count")
         flat = x.reshape(-1, self.in_features)
