@@ -851,6 +851,36 @@ int widen_int4_operands(const void* a, void* a8, long long a_bytes, const void* 
   return check_launch("widen_int4_kernel");
 }
 
+template <int TILES8, int WARPS>
+int launch_gemv(const GemvParams& g, cudaStream_t st) {
+  static bool configured_dev[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured_dev[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(rk_gemv_w4a16_kernel<TILES8, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         gemv_smem_limit(WARPS));
+    if (e != cudaSuccess) return fail(RK_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    configured_dev[dev & 63] = true;
+  }
+  const int tiles = (g.n + kGemvRows - 1) / kGemvRows, per_cta = WARPS / g.share;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((tiles + per_cta - 1) / per_cta);
+  cfg.blockDim = dim3(WARPS * 32);
+  cfg.dynamicSmemBytes = gemv_smem(g.m, g.k, TILES8, WARPS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemv_w4a16_kernel<TILES8, WARPS>, g);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(RK_ECUDA, "rk_gemv_w4a16_kernel launch: %s", cudaGetErrorString(e));
+  }
+  return RK_OK;
+}
+
 template <int BN, int UW, bool SPLIT>
 int launch_w4(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUtensorMap& tm_s, const CUtensorMap& tm_o,
               const W4Params& p, int tiles_n, int tiles_m, int smem, cudaStream_t st) {
@@ -1481,37 +1511,34 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
   p.groups = static_cast<int>(k / 128);
   if (k > 32768) return fail(RK_EUNSUPPORTED, "%s: k > 32768", who);
   if (!aligned16(scales)) return fail(RK_EINVAL, "%s: scales must be 16-byte aligned", who);
-  const int64_t gemv_slabs = k / kGemvSlab;
-  const bool gemv_shape = k % kGemvSlab == 0 && (gemv_slabs == 1 || gemv_slabs == 2 || gemv_slabs == 4 || gemv_slabs % 8 == 0);
-  if (m == 1 && tactic == 0 && gemv_shape && aligned16(x) && aligned16(q) && aligned16(out)) {
-    // one activation row: byte-streaming work for the CUDA cores (any tactic bit keeps the tensor-core kernels)
+  // A handful of activation rows: the streaming kernel.  Up to eight rows cost it little more than one, nine to sixteen a second
+  // fragment, which large weights repay only in the tensor-memory kernels.  Against those, 16384 x 2048 with 1 / 8 / 16 rows
+  // 7.1 / 8.0 / 10.4 us and 9.1 / 9.1 / 9.1; 4096 x 4096 4.7 / 6.1 / 6.8 and 7.6 / 7.8 / 8.0; 1024 x 1024 2.1 / 2.4 / 3.0 and 5.4;
+  // 17 to 24 rows would gain 0.9 us at 4096 x 2048 and lose 3 at 16384 x 2048.  Any tactic bit keeps the other kernels.
+  const bool few_rows = m <= 8 || (m <= 16 && n * k <= (1 << 24));
+  if (few_rows && tactic == 0 && aligned16(x) && aligned16(q) && aligned16(out)) {
     GemvParams g{};
     g.q = static_cast<const uint8_t*>(q);
     g.scales = static_cast<const __nv_bfloat16*>(scales);
     g.x = static_cast<const __nv_bfloat16*>(x);
     g.bias = static_cast<const __nv_bfloat16*>(bias);
     g.out = static_cast<__nv_bfloat16*>(out);
+    g.m = static_cast<int>(m);
     g.n = static_cast<int>(n);
     g.k = static_cast<int>(k);
-    const int slabs = static_cast<int>(k / kGemvSlab);
-    const int share = slabs < kGemvWarps ? slabs : kGemvWarps;
-    const int batches = static_cast<int>(n / kGemvRows);
-    const int per_cta = kGemvWarps / share;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((batches + per_cta - 1) / per_cta);
-    cfg.blockDim = dim3(kGemvWarps * 32);
-    cfg.stream = as_stream(stream);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, rk_gemv_w4a16_kernel, g);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(RK_ECUDA, "rk_gemv_w4a16_kernel launch: %s", cudaGetErrorString(e));
+    // warps per channel tile: as many as keep the launch in one wave of sixteen warps per SM, one group each at least
+    const int tiles = (g.n + kGemvRows - 1) / kGemvRows, tiles8 = m <= 8 ? 1 : 2;
+    g.share = 1;
+    while (g.share < 16 && tiles * g.share * 2 <= 16 * kNumSms && g.share * 2 <= g.k / 128) g.share *= 2;
+    // CTAs of sixteen warps where a tile wants them all, where two CTAs' activations do not fit, or two fragments meet a long K
+    // (8192 x 2048, 16 rows: 6.4 us against 7.0; 1024 x 1024: 3.3 against 3.0)
+    const bool wide = g.share == 16 || gemv_smem(g.m, g.k, tiles8, 8) > gemv_smem_limit(8) || (tiles8 == 2 && g.k >= 2048);
+    if (!wide && g.share > 8) g.share = 8;
+    if (gemv_smem(g.m, g.k, tiles8, wide ? 16 : 8) <= gemv_smem_limit(wide ? 16 : 8)) {
+      cudaStream_t st = as_stream(stream);
+      if (wide) return tiles8 == 1 ? launch_gemv<1, 16>(g, st) : launch_gemv<2, 16>(g, st);
+      return tiles8 == 1 ? launch_gemv<1, 8>(g, st) : launch_gemv<2, 8>(g, st);
     }
-    return RK_OK;
   }
   if (m > 64 && !(tactic & 2)) {  // tactic bit 1 keeps the per-group-accumulator kernel for any m
     p.ldo = n;

@@ -1,30 +1,25 @@
-// W4A16 group-wise int4 GEMV: ONE activation row (decode batch 1).
+// W4A16 group-wise int4 products with a handful of activation rows (decode batches of one to sixteen).
 //
-// With a single activation row the tensor pipe is the wrong tool: a `tcgen05.mma` of K = 16 costs
-// 64 cycles whatever N <= 128 is, which puts a floor of 4.3 us per CTA under the kernels of
-// rk_gemm_w4.cuh at K = 2048, above the 2.65 us the packed weights need to arrive from HBM.  One
-// row is 2 flops per weight - byte-streaming work - so this kernel does it on the CUDA cores and is
-// bound by the weight stream.
+// Byte-streaming work: two flops per weight and row.  The tensor-memory kernels of rk_gemm_w4.cuh take 128 output channels
+// per CTA and expand them through one ring, which leaves them at the latency of that ring; here every warp streams its own
+// weights straight into registers and expands them there, and the warps of an SM hide each other's latency.  The
+// expanded weights are the A operand of warp-level m16n8k16 MMAs (bf16, fp32 accumulation): sixteen output channels by
+// eight activation rows, so that up to eight rows cost what one does.  tcgen05 has nothing to offer at this size: its A
+// tile is 128 channels from shared or tensor memory.
 //
-// K is cut into slabs of 1024; a warp owns eight consecutive output channels and one slab at a time:
-// lane l holds the 32 activations of the slab's chunk l in registers (fp32) and, per channel, loads
-// the matching 16-byte piece of the packed row - the eight loads are issued before the first is
-// used.  The warps of a CTA that share a row batch take different slabs (so that all their loads are
-// in flight together) and combine their partial sums through shared memory.
+// A warp owns sixteen output channels and a contiguous share of K's groups; `share` warps of a CTA split a channel tile
+// along K and add their totals through shared memory in a fixed order.  Lane (g, t) = (lane / 4, lane % 4) loads the 16
+// bytes t of a group's 64 for channels g and g + 8: 32 consecutive weights of each, which are also the K positions that
+// the MMA fragments of lane t stand for (any order of K serves, as long as both operands use the same).  The loads
+// of four groups are in flight while two are computed.  The activations lie in shared memory in fragment order.
 //
-// Arithmetic per weight: the offset-binary nibble u = q + 8, isolated in its own byte with bit 7
-// set, is placed by one byte-permute under the exponent byte 0x3F: the float 1 + u / 128, exactly;
-// acc += x * f.  Per chunk the identity
-//   sum x * q = 128 * acc - 136 * sum x
-// recovers the group's partial sum (11 integer operations per eight weights and one FMA per
-// weight; no int -> float conversion, which runs at an eighth of the FMA rate).  The partial sums are
-// scaled by their bf16 group scale in fp32, reduced over the warp by shuffles and over the slabs in
-// shared memory; eight bf16 outputs leave in one store.  Summation is fp32 throughout (a different
-// order than the tensor-core kernels; same tolerance).
+// Arithmetic of the kernels above it: nibbles to exact bf16 integers, the group's partial sum in fp32, times the group
+// scale in fp32, summed in fp32.
 //
-// The kernel is issue bound, not latency bound: a variant that streamed the packed rows through
-// per-team shared-memory rings with bulk copies (192 KB of weights in flight per SM instead of
-// 64 KB at best) measured 9.0 us against 8.2 us for this form at N = 16384, K = 2048.
+// Bound by the integer pipe (7 of some 14 instructions per eight weights are masks and byte permutes) and by the launch
+// and the first loads.  16384 x 2048, one row 8.3 -> 7.1 us, 1024 x 1024 2.9 -> 2.1, 2048 x 16384 8.3 -> 7.9, against a kernel that
+// multiplied on the FMA pipe (a byte permute and half a packed FMA per weight); eight rows against rk_gemm_w4.cuh 9.1 -> 8.0, 5.4
+// -> 2.4 and 13.0 (their activations do not fit here).  Deeper batches (four groups) and three CTAs per SM measured slower.
 //
 // Packed word format as everywhere: byte b of a word holds weights k_b (low nibble) and k_{b+4}.
 #pragma once
@@ -32,132 +27,167 @@
 #include <cuda_bf16.h>
 
 #include "rk_common.cuh"
+#include "rk_gemm_w4.cuh"
 
 namespace rk {
 
-constexpr int kGemvSlab = 1024;   // K elements per pass: 32 chunks of 32, one per lane
-constexpr int kGemvRows = 8;      // output channels per warp
-constexpr int kGemvWarps = 8;
+constexpr int kGemvRows = 16;   // output channels per warp
+constexpr int kGemvBatch = 2;   // groups per batch of loads; two batches are in flight
+// activations and totals of a CTA: two CTAs of eight warps or one of sixteen share an SM
+__host__ __device__ constexpr int gemv_smem_limit(int warps) { return warps == 8 ? 96 * 1024 : 200 * 1024; }
 
 struct GemvParams {
   const uint8_t* q;              // [n, k / 2]
   const __nv_bfloat16* scales;   // [k / 128, n]
-  const __nv_bfloat16* x;        // [k]
+  const __nv_bfloat16* x;        // [m, k]
   const __nv_bfloat16* bias;     // [n] or null
-  __nv_bfloat16* out;            // [n]
-  int n, k;
+  __nv_bfloat16* out;            // [m, n]
+  int m, n, k;
+  int share;                     // warps per channel tile (a power of two up to the warps of a CTA)
 };
 
-// sum over the 32 weights of one 16-byte piece of x[e] * (1 + u / 128).  xs2[4 * j + b] holds the
-// chunk's activations (8 j + b, 8 j + 4 + b): the two weights that share byte b of word j.  One packed
-// `fma.rn.f32x2` advances both running sums (the same two chains, rounded identically, as two FMAs).
-__device__ __forceinline__ float gemv_chunk(const uint4& piece, const float2 (&xs2)[16]) {
-  const uint32_t words[4] = {piece.x, piece.y, piece.z, piece.w};
-  float2 acc = make_float2(0.0f, 0.0f);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    // bytes of `lo`: 0x80 | (k_b + 8) for weights k_0..k_3 of the word, of `hi`: k_4..k_7
-    // (one logic op each: inside the mask the xor flips the sign bit of the nibble, outside it sets bit 7)
-    const uint32_t lo = (words[j] & 0x0F0F0F0Fu) ^ 0x88888888u;
-    const uint32_t hi = ((words[j] >> 4) & 0x0F0F0F0Fu) ^ 0x88888888u;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      // result bytes (low to high): 0, 0, byte b of the source, 0x3F
-      const float f_lo = __uint_as_float(__byte_perm(lo, 0x3F000000u, 0x7044u | (b << 8)));
-      const float f_hi = __uint_as_float(__byte_perm(hi, 0x3F000000u, 0x7044u | (b << 8)));
-      acc = __ffma2_rn(xs2[4 * j + b], make_float2(f_lo, f_hi), acc);
-    }
-  }
-  return acc.x + acc.y;
+// bytes of one activation row in fragment order: 64 more than the row, so that the eight rows of a fragment spread over the banks
+__host__ __device__ constexpr int gemv_row_bytes(int k) { return 2 * k + 64; }
+// activation rows (one of zeros behind them where they do not fill the fragments), then the totals
+__host__ __device__ constexpr int gemv_sums_offset(int m, int k) { return (m + (m % 8 != 0 ? 1 : 0)) * gemv_row_bytes(k); }
+__host__ __device__ constexpr int gemv_smem(int m, int k, int tiles8, int warps) { return gemv_sums_offset(m, k) + warps * tiles8 * 8 * kGemvRows * 4; }
+
+__device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(kGemvWarps * 32, 2)
+struct GemvBatch {
+  uint4 w[kGemvBatch][2];             // the 32 weights of channels g and g + 8
+  unsigned short scale[kGemvBatch][2];
+};
+
+// TILES8: blocks of eight activation rows (m <= 8 * TILES8)
+template <int TILES8, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 rk_gemv_w4a16_kernel(const GemvParams p) {
-  __shared__ float partial[kGemvWarps][kGemvRows];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int slabs = p.k / kGemvSlab;
-  const int share = slabs < kGemvWarps ? slabs : kGemvWarps;  // warps of this CTA per row batch (1, 2, 4 or 8)
-  const int batches_per_cta = kGemvWarps / share;
-  const int batch = blockIdx.x * batches_per_cta + warp / share;
-  const int first_slab = warp % share;
-  const int n0 = batch * kGemvRows;
-  const bool active = n0 < p.n;  // n is a multiple of 8: a batch's eight channels exist or none does
+  extern __shared__ __align__(16) uint8_t gemv_smem_dyn[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int tiles_per_cta = WARPS / p.share;
+  const int part = warp % p.share;                                  // which share of K
+  const int n0 = (blockIdx.x * tiles_per_cta + warp / p.share) * kGemvRows;
+  const int groups = p.k >> 7;
+  const int first = groups * part / p.share, last = n0 < p.n ? groups * (part + 1) / p.share : 0;
+  const long long row_bytes = p.k >> 1;
+  // channels beyond n (a multiple of eight: the tile's second half) read the last channel and are not stored
+  const int ch[2] = {min(n0 + g, p.n - 1), min(n0 + g + 8, p.n - 1)};
   pdl_launch_dependents();
+  if (lane < kGemvRows && n0 + lane < p.n && first < last) {
+    // this warp's rows start their way to L2 while the preceding kernel drains (a request to L2 alone)
+    const uint8_t* const row = p.q + (n0 + lane) * row_bytes + first * 64;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row), "r"((last - first) * 64) : "memory");
+  }
   pdl_wait();  // the activations (and, in tests, freshly packed weights) come from the preceding kernel
-  const int row_bytes = p.k >> 1;
-  float total[kGemvRows];
+
+  const uint8_t* src[2] = {p.q + ch[0] * row_bytes + first * 64 + t * 16, p.q + ch[1] * row_bytes + first * 64 + t * 16};
+  const unsigned short* scale[2] = {reinterpret_cast<const unsigned short*>(p.scales) + static_cast<long long>(first) * p.n + ch[0],
+                                    reinterpret_cast<const unsigned short*>(p.scales) + static_cast<long long>(first) * p.n + ch[1]};
+  // loads the next `count` groups (the same in all lanes) and moves on
+  auto load = [&](GemvBatch& b, int count) {
 #pragma unroll
-  for (int r = 0; r < kGemvRows; ++r) total[r] = 0.0f;
-  for (int slab = first_slab; active && slab < slabs; slab += share) {
-    const int k0 = slab * kGemvSlab;
-    // the weight pieces of all eight channels first, streaming (read once)
-    uint4 piece[kGemvRows];
+    for (int j = 0; j < kGemvBatch; ++j) {
+      if (j >= count) break;
 #pragma unroll
-    for (int r = 0; r < kGemvRows; ++r) {
-      const uint8_t* row = p.q + static_cast<long long>(n0 + r) * row_bytes + (k0 >> 1);
-      piece[r] = __ldcs(reinterpret_cast<const uint4*>(row + lane * 16));
+      for (int h = 0; h < 2; ++h) {
+        b.w[j][h] = __ldcs(reinterpret_cast<const uint4*>(src[h]));
+        b.scale[j][h] = __ldg(scale[h]);
+        src[h] += 64;
+        scale[h] += p.n;
+      }
     }
-    // this lane's chunk of the slab: activations to registers (paired as gemv_chunk wants them), and their plain sum
-    float2 xs2[16];
-    float xsum = 0.0f;
-    {
-      const uint4* src = reinterpret_cast<const uint4*>(p.x + k0 + lane * 32);
-      float2 sum2 = make_float2(0.0f, 0.0f);
+  };
+  GemvBatch batch[2];
+  load(batch[0], last - first);
+  load(batch[1], last - first - kGemvBatch);
+
+  // activations in fragment order: eight elements (one word's weights) of group j, lane t, word w at j * 256 + w * 64 + t * 16;
+  // the fragment's rows beyond m read a row of zeros
+  const int pitch = gemv_row_bytes(p.k);
+  for (int i = threadIdx.x; i < p.m * (p.k >> 3); i += WARPS * 32) {
+    const int r = i / (p.k >> 3), c = i - r * (p.k >> 3);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;"
+                 ::"r"(smem_u32(gemv_smem_dyn) + r * pitch + (c >> 4) * 256 + (c & 3) * 64 + ((c >> 2) & 3) * 16),
+                   "l"(p.x + static_cast<long long>(r) * p.k + c * 8) : "memory");
+  }
+  if (p.m % 8 != 0)
+    for (int i = threadIdx.x; i < p.k >> 3; i += WARPS * 32)
+      *reinterpret_cast<uint4*>(gemv_smem_dyn + p.m * pitch + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+
+  const uint8_t* xrow[TILES8];
+  float total[TILES8][4];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {  // eight activations: words 0, 1 hold elements 0..3, words 2, 3 elements 4..7
-        const uint4 t = src[v];
-        const uint32_t tw[4] = {t.x, t.y, t.z, t.w};
+  for (int u = 0; u < TILES8; ++u) {
+    xrow[u] = gemv_smem_dyn + min(u * 8 + g, p.m) * pitch + first * 256 + t * 16;
+    total[u][0] = total[u][1] = total[u][2] = total[u][3] = 0.0f;
+  }
+  auto compute = [&](const GemvBatch& b, int count) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          xs2[4 * v + 2 * c] = make_float2(__uint_as_float(tw[c] << 16), __uint_as_float(tw[c + 2] << 16));
-          xs2[4 * v + 2 * c + 1] = make_float2(__uint_as_float(tw[c] & 0xFFFF0000u), __uint_as_float(tw[c + 2] & 0xFFFF0000u));
+    for (int j = 0; j < kGemvBatch; ++j) {
+      if (j >= count) break;
+      const uint32_t lo[4] = {b.w[j][0].x, b.w[j][0].y, b.w[j][0].z, b.w[j][0].w};
+      const uint32_t hi[4] = {b.w[j][1].x, b.w[j][1].y, b.w[j][1].z, b.w[j][1].w};
+      float acc[TILES8][2][4];  // two chains, so that an MMA does not wait for the one before it
+#pragma unroll
+      for (int u = 0; u < TILES8; ++u)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) acc[u][c][0] = acc[u][c][1] = acc[u][c][2] = acc[u][c][3] = 0.0f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const uint4 a = w4_unpack8(lo[w]), c = w4_unpack8(hi[w]);
+#pragma unroll
+        for (int u = 0; u < TILES8; ++u) {
+          const uint4 x = *reinterpret_cast<const uint4*>(xrow[u] + w * 64);
+          mma_m16n8k16(acc[u][0], a.x, c.x, a.y, c.y, x.x, x.y);
+          mma_m16n8k16(acc[u][1], a.z, c.z, a.w, c.w, x.z, x.w);
         }
       }
+      const float s0 = bf16_bits_to_float(b.scale[j][0]), s1 = bf16_bits_to_float(b.scale[j][1]);
 #pragma unroll
-      for (int e = 0; e < 16; ++e) sum2 = __fadd2_rn(sum2, xs2[e]);
-      xsum = sum2.x + sum2.y;
+      for (int u = 0; u < TILES8; ++u) {
+        xrow[u] += 256;
+        total[u][0] = fmaf(s0, acc[u][0][0] + acc[u][1][0], total[u][0]);
+        total[u][1] = fmaf(s0, acc[u][0][1] + acc[u][1][1], total[u][1]);
+        total[u][2] = fmaf(s1, acc[u][0][2] + acc[u][1][2], total[u][2]);
+        total[u][3] = fmaf(s1, acc[u][0][3] + acc[u][1][3], total[u][3]);
+      }
     }
-    // group scales of the eight channels: chunk c lies in group c / 4
-    const int group = (k0 >> 7) + (lane >> 2);
-    const uint4 sc = *reinterpret_cast<const uint4*>(p.scales + static_cast<long long>(group) * p.n + n0);
-    const uint32_t sw[4] = {sc.x, sc.y, sc.z, sc.w};
-#pragma unroll
-    for (int r = 0; r < kGemvRows; ++r) {
-      const float acc = gemv_chunk(piece[r], xs2);
-      const float dot = fmaf(128.0f, acc, -136.0f * xsum);  // sum x * q over the chunk
-      const float scale = (r & 1) ? __uint_as_float(sw[r >> 1] & 0xFFFF0000u) : __uint_as_float(sw[r >> 1] << 16);
-      total[r] = fmaf(scale, dot, total[r]);
-    }
+  };
+  for (int left = last - first; left > 0; left -= 2 * kGemvBatch) {
+    compute(batch[0], left);
+    load(batch[0], left - 2 * kGemvBatch);
+    compute(batch[1], left - kGemvBatch);
+    load(batch[1], left - 3 * kGemvBatch);
   }
+
+  // totals to shared memory as [warp][activation row][channel], then added over the shares of K in order
+  float* const sums = reinterpret_cast<float*>(gemv_smem_dyn + gemv_sums_offset(p.m, p.k));
 #pragma unroll
-  for (int r = 0; r < kGemvRows; ++r) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) total[r] += __shfl_xor_sync(0xffffffffu, total[r], off);
-  }
-  if (lane < kGemvRows) {
-    float mine = total[0];
-#pragma unroll
-    for (int r = 1; r < kGemvRows; ++r) mine = lane == r ? total[r] : mine;
-    partial[warp][lane] = mine;
+  for (int u = 0; u < TILES8; ++u) {
+    float* const dst = sums + (warp * TILES8 + u) * 8 * kGemvRows;
+    dst[2 * t * kGemvRows + g] = total[u][0];
+    dst[(2 * t + 1) * kGemvRows + g] = total[u][1];
+    dst[2 * t * kGemvRows + g + 8] = total[u][2];
+    dst[(2 * t + 1) * kGemvRows + g + 8] = total[u][3];
   }
   __syncthreads();
-  if (active && first_slab == 0 && lane == 0) {
-    uint32_t o[4];
-#pragma unroll
-    for (int r = 0; r < kGemvRows; r += 2) {
-      float a = 0.0f, b = 0.0f;
-      for (int s = 0; s < share; ++s) {  // fixed order: deterministic
-        a += partial[warp + s][r];
-        b += partial[warp + s][r + 1];
-      }
-      if (p.bias != nullptr) {
-        a += __bfloat162float(p.bias[n0 + r]);
-        b += __bfloat162float(p.bias[n0 + r + 1]);
-      }
-      o[r >> 1] = pack_bf16x2(a, b);
-    }
-    *reinterpret_cast<uint4*>(p.out + n0) = make_uint4(o[0], o[1], o[2], o[3]);
+  for (int i = threadIdx.x; i < tiles_per_cta * p.m * kGemvRows; i += WARPS * 32) {
+    const int channel = i & (kGemvRows - 1), rest = i / kGemvRows;
+    const int tile = rest / p.m, row = rest - tile * p.m;
+    const int n = (blockIdx.x * tiles_per_cta + tile) * kGemvRows + channel;
+    if (n >= p.n) continue;
+    float sum = 0.0f;
+    for (int s = 0; s < p.share; ++s) sum += sums[((tile * p.share + s) * TILES8 * 8 + row) * kGemvRows + channel];
+    if (p.bias != nullptr) sum += __bfloat162float(p.bias[n]);
+    p.out[static_cast<long long>(row) * p.n + n] = __float2bfloat16_rn(sum);
   }
 }
 
