@@ -10,6 +10,7 @@
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -184,13 +185,14 @@ PyObject* integer_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     at::Tensor out;
     Py_BEGIN_ALLOW_THREADS;
     try {
-      at::Tensor codes = at::empty({m, kpad}, x->options().dtype(at::kChar));
-      at::Tensor scales = at::empty({m}, x->options().dtype(at::kFloat));
+      // the row codes and their scales live for this call only: one block of the caching allocator, on the current stream
+      const c10::DataPtr codes = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(m) * kpad + static_cast<size_t>(m) * 4);
+      float* const scales = reinterpret_cast<float*>(static_cast<uint8_t*>(codes.get()) + static_cast<size_t>(m) * kpad);
       out = at::empty(shape, x->options());
-      code = g_quant_rows(px, m, k, k, nullptr, k, nullptr, 0, 8, codes.data_ptr(), static_cast<float*>(scales.data_ptr()), stream);
+      code = g_quant_rows(px, m, k, k, nullptr, k, nullptr, 0, 8, codes.get(), scales, stream);
       if (code == RK_OK)
-        code = g_gemm_int(codes.data_ptr(), static_cast<const float*>(scales.data_ptr()), pw, ps, pb, out.data_ptr(), m, n, kpad, 8,
-                          static_cast<int>(layer.tactic), ws, ws_bytes, stream);
+        code = g_gemm_int(codes.get(), scales, pw, ps, pb, out.data_ptr(), m, n, kpad, 8, static_cast<int>(layer.tactic), ws, ws_bytes,
+                          stream);
     } catch (...) {
       code = RK_ECUDA;
     }
