@@ -1407,7 +1407,7 @@ int launch_w4_fold2(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const CUte
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(tiles_n, tiles_m, 1);
-  cfg.blockDim = dim3(kW4fThreads);
+  cfg.blockDim = dim3(kW4f2Threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];

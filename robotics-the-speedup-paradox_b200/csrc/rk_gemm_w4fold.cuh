@@ -16,7 +16,8 @@
 // of 128 channels per copy.  slot_full: unpack warps + activation copy -> MMA thread; slot_empty:
 // MMA commit -> unpack warps and producer.  All multi-warp waits poll with the non-blocking probe.
 //
-// Warp roles: 0 = TMA producer, 1 = TMEM owner + MMA issuer, 2..9 = unpack, 10..13 = epilogue.
+// Warp roles: 0 = TMA producer of the activations, 1 = TMEM owner + MMA issuer, 2..17 = unpack, then epilogue, 18 = TMA
+// producer of the raw weights.
 #pragma once
 
 #include <cuda.h>
@@ -26,8 +27,8 @@
 
 namespace rk {
 
-constexpr int kW4fUnpackWarps = 8;
-constexpr int kW4fThreads = 32 * (2 + kW4fUnpackWarps + 4);
+constexpr int kW4fUnpackWarps = 16;
+constexpr int kW4fThreads = 32 * (2 + kW4fUnpackWarps + 1);
 constexpr int kW4fStepCols = 32;  // TMEM columns of one expanded step: 64 bf16 of K per lane
 constexpr int kW4fAccCol = 256;   // the accumulator occupies TMEM columns [256, 256 + BN)
 constexpr int kW4fMaxSlots = 8;
@@ -44,7 +45,6 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   constexpr int kXBytes = BN * 128;  // one 64-element column block of BN rows
   constexpr int kSlots = w4f_slots(BN);
   constexpr uint32_t kTmemCols = 512;
-  constexpr int kEpiWarp0 = 2 + UW;
   static_assert(kSlots * kW4fStepCols <= kW4fAccCol, "expanded-weight ring overlaps the accumulator");
 
   extern __shared__ uint8_t smem_dyn[];
@@ -97,7 +97,7 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       mbar_init(smem_u32(&bar_w_empty[s]), UW);
     }
     for (int t = 0; t < kSlots; ++t) {
-      mbar_init(smem_u32(&bar_slot_full[t]), UW / 2 + 1);  // the four unpack warps of the step + the activation copy
+      mbar_init(smem_u32(&bar_slot_full[t]), 4 + 1);       // the four unpack warps of the step + the activation copy
       mbar_init(smem_u32(&bar_slot_empty[t]), 1);      // MMA commit
     }
     mbar_init(smem_u32(&bar_acc_full), 1);
@@ -123,56 +123,41 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   const uint32_t tmem_base = tmem_base_slot;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      const uint64_t pol_w = l2_policy_evict_first();
-      const uint64_t pol_x = l2_policy_evict_last();
-      mbar_arrive_expect_tx(smem_u32(&bar_scales), static_cast<uint32_t>(p.scale_rows) * 256u);
-      tma_load_2d_hint(smem_base + scales_off, &tm_s, n0, 2 * pair0, smem_u32(&bar_scales), pol_w);
-      int gw = 0, sx = 0;
-      int kw = rot_copies, kx = rot_steps;  // rotated positions along K
-      Ring rw{0, 0}, rx{0, 0};
-      uint32_t idle = 0;
-      while ((gw < P || sx < S) && !*reinterpret_cast<volatile int*>(&abort_flag)) {
-        bool progressed = false;
-        if (gw < P) {
-          const int s = rw.stage;
-          if (mbar_test_wait(smem_u32(&bar_w_empty[s]), rw.phase ^ 1)) {
-            const uint32_t full = smem_u32(&bar_w_full[s]);
-            mbar_arrive_expect_tx(full, kW4PairBytes);
-            tma_load_2d_hint(smem_base + w_off + s * kW4PairBytes, &tm_w, (pair0 + kw) * 128, n0, full, pol_w);
-            if (++kw == P) kw = 0;
-            ++gw;
-            rw.advance(p.w_stages);
-            progressed = true;
-          }
-        }
-        if (sx < S) {
-          const int t = rx.stage;
-          if (mbar_test_wait(smem_u32(&bar_slot_empty[t]), rx.phase ^ 1)) {
-            const uint32_t full = smem_u32(&bar_slot_full[t]);
-            mbar_arrive_expect_tx(full, kXBytes);
-            tma_load_2d_hint(smem_base + x_off + t * kXBytes, &tm_x, pair0 * 256 + kx * 64, m0, full, pol_x);
-            if (++kx == S) kx = 0;
-            ++sx;
-            rx.advance(kSlots);
-            progressed = true;
-          }
-        }
-        if (progressed) {
-          idle = 0;
-        } else if (gw == P && sx < S) {
-          // only activation copies remain: park on the slot's barrier instead of spinning, so that
-          // this thread stops taking issue slots from the unpack warps of its scheduler
-          if (!mbar_wait_bounded(smem_u32(&bar_slot_empty[rx.stage]), rx.phase ^ 1, &abort_flag, p.status,
-                                 RK_DEV_TIMEOUT_EMPTY)) break;
-        } else if (++idle > kWaitSpinMax) {
-          abort_flag = 1;
-          atomicCAS(p.status, 0, RK_DEV_TIMEOUT_EMPTY);
-        } else {
-          __nanosleep(idle > kWaitSpinFast ? 256 : 128);
-        }
-      }
+    // ------------------------------------------------------------ TMA producer of the activations, one copy per step
+    // (one thread that fed both rings, probing one after the other, took 540 to 700 cycles a step and paced the whole kernel)
+    const uint32_t on = elect_one();
+    const uint64_t pol_x = l2_policy_evict_last();
+    // first the scales and the first raw copy: behind the activations of all slots (160 KB) they came 1400 cycles later
+    mbar_arrive_expect_tx(smem_u32(&bar_scales), static_cast<uint32_t>(p.scale_rows) * 256u, on);
+    tma_load_2d_hint(smem_base + scales_off, &tm_s, n0, 2 * pair0, smem_u32(&bar_scales), pol_x, on);
+    mbar_arrive_expect_tx(smem_u32(&bar_w_full[0]), kW4PairBytes, on);
+    tma_load_2d_hint(smem_base + w_off, &tm_w, (pair0 + rot_copies) * 128, n0, smem_u32(&bar_w_full[0]), l2_policy_evict_first(), on);
+    Ring rx{0, 0};
+    int kx = rot_steps;  // rotated position along K
+    uint32_t ready = 0;
+    for (int s = 0; s < S; ++s) {
+      const int t = rx.stage;
+      if (!ready && !mbar_wait_bounded(smem_u32(&bar_slot_empty[t]), rx.phase ^ 1, &abort_flag, p.status, RK_DEV_TIMEOUT_EMPTY)) break;
+      rx.advance(kSlots);
+      ready = mbar_test_wait(smem_u32(&bar_slot_empty[rx.stage]), rx.phase ^ 1);
+      const uint32_t full = smem_u32(&bar_slot_full[t]);
+      mbar_arrive_expect_tx(full, kXBytes, on);
+      tma_load_2d_hint(smem_base + x_off + t * kXBytes, &tm_x, pair0 * 256 + kx * 64, m0, full, pol_x, on);
+      if (++kx == S) kx = 0;
+    }
+  } else if (warp == 2 + UW) {
+    // ------------------------------------------------------------ TMA producer of the raw weights from the second copy on
+    const uint32_t on = elect_one();
+    const uint64_t pol_w = l2_policy_evict_first();
+    Ring rw{0, 0};
+    rw.advance(p.w_stages);
+    int kw = rot_copies + 1 == P ? 0 : rot_copies + 1;
+    for (int i = 1; i < P; ++i, rw.advance(p.w_stages)) {
+      if (!mbar_wait_bounded(smem_u32(&bar_w_empty[rw.stage]), rw.phase ^ 1, &abort_flag, p.status, RK_DEV_TIMEOUT_EMPTY)) break;
+      const uint32_t full = smem_u32(&bar_w_full[rw.stage]);
+      mbar_arrive_expect_tx(full, kW4PairBytes, on);
+      tma_load_2d_hint(smem_base + w_off + rw.stage * kW4PairBytes, &tm_w, (pair0 + kw) * 128, n0, full, pol_w, on);
+      if (++kw == P) kw = 0;
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer: four MMAs of K = 16 per step
@@ -207,12 +192,13 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       if (alive) tc_commit(smem_u32(&bar_acc_full), on);
     }
   } else {
-    if (warp < kEpiWarp0) {
+    {
       // ------------------------------------------------------------ unpack: int4 -> bf16(q * scale) into TMEM
-      // row = 32 * (warp % 4) + lane (a warp writes only the TMEM lanes of its quadrant).  One loop
-      // trip covers a scale group, i.e. two steps: warps 0..3 expand the group's first step, warps
-      // 4..7 its second, each into its own slot - 64 weights per thread and one barrier probe, one
-      // arrival and one scale fetch per trip.
+      // row = 32 * (warp % 4) + lane (a warp writes only the TMEM lanes of its quadrant).  One loop trip covers a raw copy, i.e.
+      // two scale groups or four steps: set h of four warps expands the copy's step h into that step's slot - 64 weights per
+      // thread and one barrier probe, one arrival and one scale fetch per trip.  The expansion is a chain of short dependent
+      // operations (some 900 cycles a step for a warp): with two sets it paced the loop at 550 cycles a step, with four the tensor
+      // pipe nearly does.  With the two producers 128 rows x 16384 x 2048 14.3 -> 12.6 us, 65 rows 13.8 -> 12.0, 256 rows 17.0 -> 16.5.
       const int uw = warp - 2;
       const int quad = warp & 3;
       const int r = quad * 32 + lane;
@@ -220,43 +206,43 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       bool alive = mbar_poll_warp(smem_u32(&bar_scales), 0, &abort_flag, p.status, RK_DEV_TIMEOUT_FULL);
       const __nv_bfloat16* my_scales = reinterpret_cast<const __nv_bfloat16*>(smem_gen + scales_off) + r;
       Ring rw{0, 0};
-      Ring rt{h % kSlots, 0};  // slot of step 2 g + h
-      int kg = rot_copies * 2;  // rotated group index along K
+      Ring rt{h, 0};  // slot of step 4 i + h (there are more than four)
+      static_assert(kSlots > 4 && UW == 16, "four sets of four warps, a slot each");
+      int kc = rot_copies;  // rotated position along K, in raw copies
       // the barrier probes for the next trip are issued right after this trip's loads and consumed one
       // trip later (their latency hides behind the conversion); a warp stops to poll only on "not yet"
       uint32_t ready = 0;
-      for (int g = 0; g < G && alive; ++g) {
+      for (int i = 0; i < P && alive; ++i) {
         const int sw = rw.stage;
         const int t = rt.stage;
-        const int odd = g & 1;  // second group of the raw copy
+        const bool live = 2 * i + (h >> 1) < G;  // an odd last group: the copy's second half holds zeros beyond K, no step
         if (!__all_sync(0xffffffffu, ready != 0)) {
-          bool ok = true;
-          if (!odd) ok = mbar_poll_lane(smem_u32(&bar_w_full[sw]), rw.phase, &abort_flag, p.status, RK_DEV_TIMEOUT_RAW);
-          ok = ok && mbar_poll_lane(smem_u32(&bar_slot_empty[t]), rt.phase ^ 1, &abort_flag, p.status, RK_DEV_TIMEOUT_XFORM);
+          bool ok = mbar_poll_lane(smem_u32(&bar_w_full[sw]), rw.phase, &abort_flag, p.status, RK_DEV_TIMEOUT_RAW);
+          if (live) ok = ok && mbar_poll_lane(smem_u32(&bar_slot_empty[t]), rt.phase ^ 1, &abort_flag, p.status, RK_DEV_TIMEOUT_XFORM);
           if (!__all_sync(0xffffffffu, ok)) break;
         }
-        // 128-byte swizzle of the raw copy: 16-byte chunk c of row r sits at c ^ (r & 7); the step of
-        // this warp owns chunks 4 * odd + 2 * h and the next one
+        if (!live) {
+          if (lane == 0) mbar_arrive(smem_u32(&bar_w_empty[sw]));
+          break;
+        }
+        // 128-byte swizzle of the raw copy: 16-byte chunk c of row r sits at c ^ (r & 7); step h owns chunks 2 h and 2 h + 1
         const uint8_t* raw = smem_gen + w_off + sw * kW4PairBytes + r * 128;
-        const int c = odd * 4 + h * 2;
+        const int c = h * 2;
         const uint4 pk0 = *reinterpret_cast<const uint4*>(raw + ((c ^ (r & 7)) << 4));
         const uint4 pk1 = *reinterpret_cast<const uint4*>(raw + (((c + 1) ^ (r & 7)) << 4));
-        const __nv_bfloat162 ss = __bfloat162bfloat162(my_scales[kg * 128]);
-        if (++kg == G) kg = 0;
-        const bool raw_done = odd || g == G - 1;
-        // next trip: this warp's slot two steps on, and - when it opens a new raw copy - that copy
+        const __nv_bfloat162 ss = __bfloat162bfloat162(my_scales[(2 * kc + (h >> 1)) * 128]);
+        if (++kc == P) kc = 0;
+        // next trip: this set's slot four steps on and the next raw copy
         Ring rt2 = rt, rw2 = rw;
-        rt2.stage += 2;
+        rt2.stage += 4;
         if (rt2.stage >= kSlots) {
           rt2.stage -= kSlots;
           rt2.phase ^= 1u;
         }
-        if (raw_done) rw2.advance(p.w_stages);
+        rw2.advance(p.w_stages);
         ready = 0;
-        if (g + 1 < G) {
-          ready = mbar_test_wait(smem_u32(&bar_slot_empty[rt2.stage]), rt2.phase ^ 1);
-          if (odd) ready &= mbar_test_wait(smem_u32(&bar_w_full[rw2.stage]), rw2.phase);
-        }
+        if (2 * (i + 1) + (h >> 1) < G)
+          ready = mbar_test_wait(smem_u32(&bar_slot_empty[rt2.stage]), rt2.phase ^ 1) & mbar_test_wait(smem_u32(&bar_w_full[rw2.stage]), rw2.phase);
         tc_fence_after();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + t * kW4fStepCols;
         const uint32_t words[8] = {pk0.x, pk0.y, pk0.z, pk0.w, pk1.x, pk1.y, pk1.z, pk1.w};
@@ -280,34 +266,33 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(smem_u32(&bar_slot_full[t]));
-          if (raw_done) mbar_arrive(smem_u32(&bar_w_empty[sw]));
+          mbar_arrive(smem_u32(&bar_w_empty[sw]));
         }
         rt = rt2;
         rw = rw2;
       }
     }
-    // ------------------------------------------------------------ epilogue: all twelve unpack and epilogue warps
+    // ------------------------------------------------------------ epilogue: the sixteen unpack warps
     // The accumulator holds one output channel per lane; the output is [m][n] with n contiguous.
     // Storing it straight from registers would be one 2-byte store per element.  Instead the tile
     // is transposed through shared memory (the activation slots are free by now) as [m][128 n]
     // rows and leaves by TMA stores of 32 rows each, which also clip the ragged edges.
-    // The unpack warps have nothing left to do once their last group is written, and a warp may read
-    // any TMEM column of its own lane quadrant: the 16-column chunks of the accumulator are dealt
-    // round-robin to the three warps of each quadrant.
+    // A warp may read any TMEM column of its own lane quadrant: the 16-column chunks of the accumulator are dealt
+    // round-robin to the four warps of each quadrant.
     const int quad = warp & 3;
-    const int part = (warp - 2) >> 2;  // 0, 1: unpack warps; 2: epilogue warps
+    const int part = (warp - 2) >> 2;
     const int nl = quad * 32 + lane;
     const int n = n0 + nl;
     const bool alive = mbar_poll_warp(smem_u32(&bar_acc_full), 0, &abort_flag, p.status, RK_DEV_TIMEOUT_ACC);
     tc_fence_after();
-    // every one of the twelve warps reaches this rendezvous, whether it saw the accumulator complete or gave up
+    // every one of the sixteen warps reaches this rendezvous, whether it saw the accumulator complete or gave up
     if (!alive) *reinterpret_cast<volatile int*>(&epi_dead) = 1;
-    asm volatile("bar.sync 1, 384;" ::: "memory");
+    asm volatile("bar.sync 1, 512;" ::: "memory");
     if (*reinterpret_cast<volatile int*>(&epi_dead) == 0) {
       const float bias = (p.bias && n < p.n) ? __bfloat162float(p.bias[n]) : 0.0f;
       const int rows = p.m - m0 < BN ? p.m - m0 : BN;
       __nv_bfloat16* stage = reinterpret_cast<__nv_bfloat16*>(smem_gen + x_off);
-      for (int c0 = part * 16; c0 < rows; c0 += 48) {  // warp-uniform bound: tcgen05.ld is a warp-wide instruction
+      for (int c0 = part * 16; c0 < rows; c0 += 64) {  // warp-uniform bound: tcgen05.ld is a warp-wide instruction
         uint32_t v[16];
         tmem_ld_16(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kW4fAccCol + c0, v);
         tc_wait_ld();
@@ -321,8 +306,8 @@ rk_gemm_w4a16_fold_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
         for (int j = 0; j < 16; ++j) stage[(c0 + j) * 128 + nl] = __float2bfloat16_rn(__uint_as_float(v[j]) + bias);
       }
       fence_proxy_async_smem();
-      asm volatile("bar.sync 1, 384;" ::: "memory");
-      if (!SPLIT && warp == kEpiWarp0 && lane == 0) {
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      if (!SPLIT && warp == 2 && lane == 0) {
         for (int r0 = 0; r0 < rows; r0 += 32)
           tma_store_2d(&tm_o, smem_u32(stage + r0 * 128), n0, m0 + r0);
         tma_store_commit();

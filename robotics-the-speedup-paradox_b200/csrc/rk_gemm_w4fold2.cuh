@@ -43,11 +43,14 @@ __device__ __forceinline__ void mma2_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       : "memory");
 }
 
-__global__ void __launch_bounds__(kW4fThreads, 1)
+constexpr int kW4f2UnpackWarps = 8;
+constexpr int kW4f2Threads = 32 * (2 + kW4f2UnpackWarps + 4);
+
+__global__ void __launch_bounds__(kW4f2Threads, 1)
 rk_gemm_w4a16_fold2_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                            const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_o,
                            const W4Params p) {
-  constexpr int UW = kW4fUnpackWarps;
+  constexpr int UW = kW4f2UnpackWarps;
   constexpr int BN = 256;  // activation rows per pair tile
   constexpr int kSlots = kW4f2Slots;
   constexpr uint32_t kTmemCols = 512;
