@@ -176,7 +176,7 @@ int pow2_at_least(int v, int lo) {
 
 // ------------------------------------------------------------------ tile selection
 struct Plan {
-  int swap, bn, tiles_a, tiles_b, splits, stages, tmem_cols, acc_stride, acc_bufs, out_bufs, smem_bytes, grid_x;
+  int swap, bn, tiles_a, tiles_b, splits, stages, tmem_cols, acc_stride, acc_bufs, out_bufs, smem_bytes, grid_x, dual;
   int sfb_blocks;
 };
 
@@ -284,7 +284,13 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
     // the tile width), so while the machine is not full, narrower activation chunks - more CTAs, each
     // with the same loop - beat both wide tiles and split-K (whose exchange costs more than it saves
     // unless the tiles are very few).
-    if (!block_scaled && !(tactic & 4) && bn >= 64) {
+    if (kind == KIND_I8 && !(tactic & 4) && n <= 128 * kNumSms) {
+      // With two issuing warps the loop runs at the rate at which an SM takes operands from L2, (128 + bn) x 128 bytes a block:
+      // as many chunks as there are SMs, of 32 rows at least (400 x 1024 x 2048 5.4 us with chunks of 64 rows, 4.9 of 32; 400 x
+      // 1024 x 4096 7.7 and 7.0; 816 x 2048 x 2048 7.5 of 128, 7.1 of 96; 600 x 2048 x 2048 7.3 of 128, 6.8 of 96).
+      const int64_t fit = kNumSms / ((n + 127) / 128);
+      bn = std::min(bn, static_cast<int>(round_up((m + fit - 1) / fit, 32)));
+    } else if (!block_scaled && !(tactic & 4) && bn >= 64) {
       const int64_t tiles_a = (n + 127) / 128;
       const int half = static_cast<int>(round_up(bn / 2, 32));
       if (tiles_a * ((m + half - 1) / half) <= kNumSms) {
@@ -343,6 +349,22 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
   if (pl.stages > kb_per_cta) pl.stages = kb_per_cta < 2 ? 2 : kb_per_cta;
   // the split-K exchange parks a bn x 128 x 4-byte tile in the stage memory
   while (pl.splits > 1 && pl.stages * stage < pl.bn * 512) ++pl.stages;
+  // W8A8 with one tile per CTA leaves an accumulator buffer over: two warps issue alternate K blocks, an accumulator each (see
+  // GemmParams::dual).  A stage has to belong to the same warp in every round of the ring - a warp that skipped a phase of its
+  // "full" barrier would wait on a parity that has already passed - so a ring that wraps has an even number of stages.
+  // (Not above 128 rows: four MMAs take longer than issuing them, and the epilogue reads twice: 400 x 8192 x 1024 8.2 -> 8.4 us.)
+  // The issuing warp paced the loop with five tensor-core instructions a block, 50 to 60 cycles each: 816 x 2048 x 16384 35.5 ->
+  // 28.5 us, 50 x 1024 x 2048 5.5 -> 4.7, 400 x 1024 x 4096 8.7 -> 7.7; chunk of one environment 9.00 -> 8.77 ms.
+  pl.dual = kind == KIND_I8 && pl.bn <= 128 && pl.acc_bufs == 2 && (pl.splits > 1 || tiles <= kNumSms) && kb_per_cta >= 2 ? 1 : 0;
+  if (pl.dual && pl.stages < kb_per_cta && pl.stages % 2 != 0) {
+    if (pl.out_bufs == 2 && pl.stages < kMaxStages && (pl.stages + 1) * stage <= budget + kOutBufBytes) {
+      pl.out_bufs = 1, ++pl.stages;
+    } else if (pl.splits == 1 || (pl.stages - 1) * stage >= pl.bn * 512) {
+      --pl.stages;
+    } else {
+      pl.dual = 0;
+    }
+  }
   pl.smem_bytes = pl.stages * stage + pl.out_bufs * kOutBufBytes + kVecBytes + 1024;
   pl.grid_x = pl.splits > 1 ? static_cast<int>(tiles) : static_cast<int>(tiles < kNumSms ? tiles : kNumSms);
   return pl;
@@ -743,6 +765,7 @@ int run_tc(const TcArgs& a) {
   p.tmem_cols = pl.tmem_cols;
   p.acc_stride = pl.acc_stride;
   p.acc_bufs = pl.acc_bufs;
+  p.dual = pl.dual;
   p.out_bufs = pl.out_bufs;
   p.tiles_a = pl.tiles_a;
   p.tiles_b = pl.tiles_b;

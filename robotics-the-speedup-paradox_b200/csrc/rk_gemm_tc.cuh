@@ -71,6 +71,8 @@ struct GemmParams {
   int tmem_cols;
   int acc_stride;  // TMEM columns between the accumulator buffers
   int acc_bufs;    // 1 or 2 accumulator buffers in TMEM
+  int dual;        // KIND_I8, one tile per CTA: two warps issue alternate K blocks, each into an accumulator buffer of its own;
+                   // `stages` is even if the ring wraps, so that a stage is always the same warp's
   int out_bufs;    // 1 or 2 output staging buffers in shared memory
   int tiles_a, tiles_b;
   long long ldo;  // output row stride (elements)
@@ -123,6 +125,7 @@ struct NoXform {
 };
 template <>
 struct KindTraits<KIND_I8> : NoXform {
+  static constexpr int kThreads = kGemmThreads + 32;  // a second issuing warp, see GemmParams::dual
   static constexpr int kBase = KIND_I8;
   static constexpr bool kBlockScaled = false;
   static constexpr int kSfChunksPerStage = 0;
@@ -437,6 +440,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const int kb_begin = static_cast<int>((static_cast<long long>(p.kblocks) * split) / p.splits);
   const int kb_end = static_cast<int>((static_cast<long long>(p.kblocks) * (split + 1)) / p.splits);
   const int nkb = kb_end - kb_begin;
+  constexpr bool kDual = KIND == KIND_I8;
+  const bool dual = kDual && p.dual && nkb > 1;
 
   pdl_launch_dependents();
   if (threadIdx.x == 64) {  // first thing, by a thread that has no part in the set-up
@@ -460,7 +465,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       mbar_init(smem_u32(&bar_raw_empty[s]), kXformWarps);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&bar_acc_full[b]), 1);
+      mbar_init(smem_u32(&bar_acc_full[b]), dual ? 2 : 1);
       mbar_init(smem_u32(&bar_acc_empty[b]), 128);
     }
     abort_flag = 0;
@@ -587,7 +592,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 || (dual && warp == 6)) {
     // ------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop (uniform control flow); the tcgen05 instructions execute in one
     // elected lane.  Every lane takes part in the barrier waits.
@@ -595,6 +600,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       const uint32_t on = elect_one();
       Ring ring{0, 0}, racc{0, 0};
       bool alive = true;
+      const int first = kDual && warp == 6 ? 1 : 0, step = dual ? 2 : 1;
+      if (first) ring.advance(p.stages);
       uint32_t ready = 0;  // answer of the early probe of the next stage's "full" barrier
       // instruction descriptor(s) and the descriptor of stage 0 are loop invariants
       uint32_t idesc = 0;
@@ -611,11 +618,11 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
         if (!mbar_wait_bounded(smem_u32(&bar_acc_empty[ab]), racc.phase ^ 1, &abort_flag, p.status,
                                RK_DEV_TIMEOUT_ACC_FREE, spin_max)) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + ab * p.acc_stride;
+        const uint32_t d_tmem = tmem_base + (ab + first) * p.acc_stride;
         // a B tile that starts inside a 128-row scale block reads its factors from the matching
         // column of the block's four (one 32-bit column per 32 rows)
         const uint32_t sfb_col0 = static_cast<uint32_t>((((tile % p.tiles_b) * p.bn) & 127) >> 5);
-        for (int i = 0; i < nkb; ++i) {
+        for (int i = first; i < nkb; i += step) {
           const int s = ring.stage;
           const uint32_t ph = ring.phase;
           if (!ready && !mbar_wait_bounded(smem_u32(&bar_full[s]), ph, &abort_flag, p.status, RK_DEV_TIMEOUT_FULL, spin_max)) {
@@ -624,6 +631,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
           }
           tc_fence_after();
           ring.advance(p.stages);  // probe the next stage now, read the answer after this stage's MMAs
+          if (dual) ring.advance(p.stages);
           ready = mbar_test_wait(smem_u32(&bar_full[ring.stage]), ring.phase);
           const uint32_t sa = smem_base + s * stage_bytes;
           const uint32_t sb = sa + kTileA * kStageKBytes;
@@ -688,7 +696,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             if (k < nmma) {
-              const uint32_t accumulate = (i > 0 || k > 0) ? 1u : 0u;
+              const uint32_t accumulate = (i > first || k > 0) ? 1u : 0u;
               // 32 bytes of K per MMA: advance the descriptor start address by 32 >> 4.  The direct kinds branch on
               // the elected lane around each MMA: the issuing warp paces their loop, and a branch is cheaper for it
               // than the predicated form or one block per stage (50 x 1024 x 2048 W8A8 5.46, 6.49 and 5.95 us;
@@ -808,6 +816,19 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
                                       RK_DEV_TIMEOUT_ACC, verdict_epi, epi_iter++, spin_max);
       tc_fence_after();
       const uint32_t t_acc = tmem_base + ab * p.acc_stride + (static_cast<uint32_t>(quad * 32) << 16);
+      // sixteen columns of the accumulator (of both, added, when two warps issued)
+      auto load16 = [&](int c, uint32_t (&r)[16]) {
+        tmem_ld_16(t_acc + c, r);
+        if constexpr (kDual) {
+          if (dual) {
+            uint32_t second[16];
+            tmem_ld_16(t_acc + p.acc_stride + c, second);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] += second[j];
+          }
+        }
+      };
 
       if (split_mode) {
         // ---- split-K: park the raw partial accumulators in shared memory, column-major [bn][128]
@@ -815,7 +836,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
         for (int c0 = 0; c0 < p.bn; c0 += 16) {
           uint32_t r[16];
           __syncwarp();
-          tmem_ld_16(t_acc + c0, r);
+          load16(c0, r);
           tc_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; ++j) part[(c0 + j) * 128 + et] = ok ? r[j] : 0u;
@@ -828,7 +849,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
         for (int c0 = 0; c0 < p.bn; c0 += 16) {
           uint32_t r[16];
           __syncwarp();
-          tmem_ld_16(t_acc + c0, r);
+          load16(c0, r);
           tc_wait_ld();
           if (ra_ok && ok) {
 #pragma unroll
@@ -864,9 +885,9 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
           const bool two = c0 + 32 <= p.bn;  // warp-uniform
           uint32_t r0[16], r1[16];
           __syncwarp();
-          tmem_ld_16(t_acc + c0, r0);
+          load16(c0, r0);
           if (two) {
-            tmem_ld_16(t_acc + c0 + 16, r1);
+            load16(c0 + 16, r1);
           } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) r1[j] = 0u;
@@ -938,7 +959,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
         for (int c0 = 0; c0 < ncols; c0 += 16) {
           uint32_t r[16];
           __syncwarp();
-          tmem_ld_16(t_acc + cc + c0, r);
+          load16(cc + c0, r);
           tc_wait_ld();
           float v[16];
 #pragma unroll

@@ -342,3 +342,36 @@ def test_pair_tiles_of_every_width(m, n, k, kind):
     assert torch.equal(out.view(torch.int16), want.bfloat16().view(torch.int16))
     assert (buf[0] == 7.0).all() and (buf[m + 1] == 7.0).all()
     assert _lib.read_status(ws) == 0
+
+
+# One tile per CTA, so two warps issue alternate K blocks: K of one block (one warp), two, three, a ring that wraps with 32, 64,
+# 96, 128 and 224 rows a tile (an odd number of stages would fit at 64 and 96), split K, a ragged last block and ragged edges
+@pytest.mark.parametrize("m,n,k", [(50, 1024, 128), (50, 1024, 256), (50, 264, 384), (50, 2560, 1024), (50, 1024, 2080),
+                                   (400, 2560, 1152), (400, 1024, 2048), (400, 1024, 4096), (400, 1000, 4224), (600, 1024, 4096),
+                                   (816, 2048, 4096), (1000, 1000, 2304), (400, 8192, 1024), (448, 8192, 640), (7, 1024, 4096),
+                                   (200, 1024, 4096), (96, 512, 8192)])
+def test_two_issuing_warps_add_up(m, n, k):
+    from rk_b200 import _lib
+
+    lib, ptr, dev = _lib.load(), _lib.ptr, torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(m + n + k)
+    kpad = (k + 127) // 128 * 128
+    qa, qb = (torch.zeros(rows, kpad, device=dev, dtype=torch.int8) for rows in (m, n))
+    qa[:, :k] = torch.randint(-127, 128, (m, k), generator=gen, device=dev)
+    qb[:, :k] = torch.randint(-127, 128, (n, k), generator=gen, device=dev)
+    sa, sb = (torch.rand(rows, generator=gen, device=dev) * 0.01 for rows in (m, n))
+    bias = torch.randn(n, generator=gen, device=dev).bfloat16()
+    acc = qa.double() @ qb.double().t()
+    want = ((acc.float() * sa[:, None]) * sb[None, :] + bias.float()[None, :]).bfloat16()
+    ws = _lib.gemm_workspace(_lib.OP_W8A8, dev, m, n, kpad)
+    got = torch.full((m + 2, n), 7.0, device=dev, dtype=torch.bfloat16)
+    raw = torch.full((m + 2, n), 7, device=dev, dtype=torch.int32)
+    for _ in range(20):  # the two warps meet data in any order
+        _lib.check(lib.rk_gemm_int(ptr(qa), ptr(sa), ptr(qb), ptr(sb), ptr(bias), ptr(got[1:]), m, n, kpad, 8, 0, ptr(ws), ws.numel(),
+                                   _lib.stream_ptr(dev)), "scaled")
+        _lib.check(lib.rk_gemm_int_acc(ptr(qa), ptr(qb), ptr(raw[1:]), m, n, kpad, 8, 0, ptr(ws), ws.numel(), _lib.stream_ptr(dev)), "raw")
+        assert torch.equal(got[1:m + 1].view(torch.int16), want.view(torch.int16)) and torch.equal(raw[1:m + 1].double(), acc)
+        for edge in (0, m + 1):
+            assert (got[edge] == 7.0).all() and (raw[edge] == 7).all()
+        got[1:m + 1], raw[1:m + 1] = 0, 0
+    assert _lib.read_status(ws) == 0
