@@ -579,15 +579,29 @@ int run_tc(const TcArgs& a) {
   const bool two_cta_kind = a.acc_out == nullptr && (a.out != nullptr || a.swiglu_q != nullptr) && a.kind <= KIND_NVF4 && a.peer == nullptr &&
                             a.residual == nullptr;  // the residual epilogue lives in the one-CTA kernel
   const int mode = two_cta_mode();
-  // CTA pairs: from 512 activation rows on for the block-scaled kinds, whose main loop is paced by
+  // CTA pairs: from 385 activation rows on for the block-scaled kinds, whose main loop is paced by
   // the issuing thread (scale copies + MMAs: up to 17 tensor-core instructions per stage; one
-  // instruction of a pair drives two SMs), beyond 1024 rows for the others (no gain below: measured)
+  // instruction of a pair drives two SMs), and from 193 if the one-CTA tiles are few (one-CTA against pairs, MXFP8 / NVFP4: 400 x
+  // 32768 x 2048 36.7 -> 31.0 / 23.7 -> 19.8 us, 400 x 2048 x 16384 35.3 -> 33.8 / 22.2 -> 21.1, 264 x 2048 x 16384 44.6 -> 33.6 /
+  // 26.1 -> 21.0, 200 x 2048 x 2048 7.8 -> 7.6 / 6.4 -> 6.0; but 264 x 32768 x 2048 28.1 -> 29.6 / 23.2 -> 19.4 and 264 x 8192 x
+  // 2048 10.2 -> 10.8 / 7.8 -> 8.0, pair tiles being half padding there).  Beyond 1024 rows for the others, and from 321 where the one-CTA plan has more than
+  // one tile for a CTA: both are bound by the operands an SM takes from L2, and a pair's SMs share the weights (one-CTA against pairs,
+  // W8A8 / FP8: 400 x 10240 x 2048 18.4 -> 12.7 / 16.7 -> 12.3 us, 816 x 16384 x 2048 31.7 -> 24.1 / 27.9 -> 24.6, 816 x 32768 x
+  // 2048 52.7 -> 45.5 / 48.5 -> 46.6, 1000 x 12288 x 256 22.1 -> 11.9 / 18.9 -> 10.7; 300 x 32768 x 2048 25.4 -> 24.4 / 23.5 -> 26.0).
+  // Pair tiles have 256 rows: with more than a quarter of them padding a long K loop gains nothing (560 x 12288 x 8192 48.5 -> 48.4
+  // / 49.1 -> 51.1).  In one wave the narrow chunks of the one-CTA plan are as fast or faster (816 x 2048 x 2048 7.1 against 8.0).
   static const int64_t pair_min_env = [] {
     const char* v = std::getenv("RK_B200_TWO_CTA_MIN_M");
     return v ? static_cast<int64_t>(std::atoll(v)) : static_cast<int64_t>(0);
   }();
-  const int64_t pair_min_m = pair_min_env > 0 ? pair_min_env : (block_scaled ? 512 : 1025);
-  if (two_cta_kind && ((mode != 0 && ((mode == 1 && a.m > 256) || a.m >= pair_min_m) && a.n >= 128) || a.swiglu_q != nullptr)) {
+  const int64_t pair_min_m = pair_min_env > 0 ? pair_min_env : (block_scaled ? 385 : 1025);
+  const bool pair_below = pair_min_env == 0 && a.m < pair_min_m && [&] {
+    if (a.m <= (block_scaled ? 192 : 320) || !(block_scaled || kblocks <= 32 || 4 * a.m >= 3 * round_up(a.m, 256))) return false;
+    const Plan one = make_plan(a.kind, a.m, a.n, kblocks, a.tactic);
+    const int64_t tiles = static_cast<int64_t>(one.tiles_a) * one.tiles_b;
+    return block_scaled ? tiles <= kNumSms / 2 : one.splits == 1 && tiles > one.grid_x;
+  }();
+  if (two_cta_kind && ((mode != 0 && ((mode == 1 && a.m > 256) || a.m >= pair_min_m || pair_below) && a.n >= 128) || a.swiglu_q != nullptr)) {
     Gemm2Params p2{};
     p2.m = static_cast<int>(a.m);
     p2.n = static_cast<int>(a.n);
