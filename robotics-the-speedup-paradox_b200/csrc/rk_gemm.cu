@@ -176,7 +176,7 @@ int pow2_at_least(int v, int lo) {
 
 // ------------------------------------------------------------------ tile selection
 struct Plan {
-  int swap, bn, tiles_a, tiles_b, splits, stages, tmem_cols, acc_stride, acc_bufs, out_bufs, smem_bytes, grid_x, dual;
+  int swap, bn, tiles_a, tiles_b, splits, stages, tmem_cols, acc_stride, acc_bufs, out_bufs, smem_bytes, grid_x, dual, few;
   int sfb_blocks;
 };
 
@@ -365,9 +365,45 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
       pl.dual = 0;
     }
   }
-  pl.smem_bytes = pl.stages * stage + pl.out_bufs * kOutBufBytes + kVecBytes + 1024;
+  // more than half of an SM's, for the reason given in few_rows_plan (chains of short loops: 816 x 2560 x 256 W8A8 6.0 -> 5.0 us)
+  pl.smem_bytes = std::max(pl.stages * stage + pl.out_bufs * kOutBufBytes + kVecBytes + 1024, 118 * 1024);
   pl.grid_x = pl.splits > 1 ? static_cast<int>(tiles) : static_cast<int>(tiles < kNumSms ? tiles : kNumSms);
   return pl;
+}
+
+// W8A8, up to 128 activation rows: the rows take the 128-lane axis, and only those that exist are fetched; every CTA has one
+// tile of weights, as narrow as gives each SM one (multiples of 16).  A block of K then costs an SM (m + bn) x 128 bytes from L2
+// instead of (128 + 32) x 128 with the weights on the lanes, the copies are spread over more SMs, and a row of the tile is stored
+// from registers.  Bound by the producer's two copies and the issuing warps (about 165 cycles a block).  Against `pl`: 50 x 1024
+// x 2048 4.5 -> 3.8 us, 100 x 8192 x 1024 5.5 -> 4.6, 64 x 4096 x 4096 7.6 -> 6.4, 128 x 2048 x 8192 11.8 -> 10.0, 1 x 1024 x 2048
+// 4.4 -> 3.8; chunk of one environment 8.78 -> 8.07 ms.  Not for
+// - tiles much wider than the rows are many: 16 x 8192 x 1024 4.0 against 4.4 us, 32 rows 4.2 and 4.4, 50 x 16384 x 2048 8.0 and
+//   8.2 (64 x 8192 x 1024 4.6 -> 4.4, 100 x 16384 x 2048 8.9 -> 8.5);
+// - a long loop that `pl` splits: 50 x 2048 x 8192 8.2 against 8.8, 50 x 256 x 4096 4.7 against 5.1 in eight; at 32 blocks in six
+//   or fewer it still gains (50 x 1024 x 4096 5.6 -> 5.4, 100 rows 6.4 -> 5.5).
+Plan few_rows_plan(const Plan& pl, int64_t m, int64_t n, int kblocks, int tactic) {
+  const int bn = static_cast<int>(round_up((n + kNumSms - 1) / kNumSms, 16));
+  if (m > 128 || (tactic & 5) || bn > pow2_at_least(static_cast<int>(m), 16) || pl.splits > (kblocks <= 32 ? 6 : 1)) return pl;
+  Plan few{};
+  few.few = 1;
+  few.dual = kblocks >= 2 ? 1 : 0;
+  few.bn = bn;
+  few.tiles_a = 1;
+  few.tiles_b = few.grid_x = static_cast<int>((n + bn - 1) / bn);
+  few.splits = 1;
+  few.acc_stride = static_cast<int>(round_up(bn, 32));
+  few.acc_bufs = 2;
+  few.tmem_cols = pow2_at_least(2 * few.acc_stride, 32);
+  few.out_bufs = 1;  // nothing is staged: an MMA reads 128 rows from the start of a stage, beyond the end of the last
+  const int stage = static_cast<int>(round_up(m, 8) + bn) * kStageKBytes;
+  few.stages = std::min((kSmemBudget - kVecBytes - kOutBufBytes) / stage, kMaxStagesFew);
+  if (few.stages < kblocks) few.stages &= ~1;  // a ring that wraps, as in make_plan
+  else few.stages = std::max(kblocks, 2);
+  // More than half of an SM's shared memory, however little the stages need: CTAs of the next launch that start early would crowd
+  // into the SMs that this one uses, two or three to an SM, beside idle ones (chains: 50 x 2560 x 1024 3.9 -> 3.5 us, 17 x 8192 x
+  // 1024 5.0 -> 4.4, 1 x 2048 x 2048 5.9 -> 4.4).
+  few.smem_bytes = std::max(few.stages * stage + kOutBufBytes + kVecBytes + 1024, 118 * 1024);
+  return few;
 }
 
 template <int KIND, bool RESIDUAL, int SCHED>
@@ -415,6 +451,9 @@ template <int KIND, bool RESIDUAL = false>
 int launch_tc(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const GemmParams& p,
               const Plan& pl, cudaStream_t st) {
   constexpr bool direct = KIND == KIND_I8 || KIND == KIND_F8;
+  if constexpr (KIND == KIND_I8) {
+    if (pl.few) return launch_tc_kernel<KIND, RESIDUAL, SCHED_FEW>(tm_a, tm_b, tm_out, p, pl, st);
+  }
   if constexpr (!KindTraits<KIND>::kBlockScaled) {
     if (pl.splits > 1) return launch_tc_kernel<KIND, RESIDUAL, SCHED_SPLIT>(tm_a, tm_b, tm_out, p, pl, st);
   }
@@ -731,10 +770,11 @@ int run_tc(const TcArgs& a) {
       default: return launch_tc2<KIND_NVF4>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);
     }
   }
-  const Plan pl = make_plan(a.kind, a.m, a.n, kblocks, a.tactic);
+  Plan pl = make_plan(a.kind, a.m, a.n, kblocks, a.tactic);
+  if (a.kind == KIND_I8 && a.acc_out == nullptr && a.peer == nullptr) pl = few_rows_plan(pl, a.m, a.n, kblocks, a.tactic);
 
   CUtensorMap tm_act, tm_wgt, tm_out;
-  const uint32_t box_act = pl.swap ? pl.bn : kTileA;
+  const uint32_t box_act = pl.swap ? pl.bn : pl.few ? static_cast<uint32_t>(round_up(a.m, 8)) : kTileA;
   const uint32_t box_wgt = pl.swap ? kTileA : pl.bn;
   // an operand that is rewritten in shared memory is fetched as raw rows: `raw` bytes of every row per
   // 128 MMA bytes of K, unswizzled; its row pitch is k_bytes * raw / 128
@@ -780,6 +820,7 @@ int run_tc(const TcArgs& a) {
   p.acc_stride = pl.acc_stride;
   p.acc_bufs = pl.acc_bufs;
   p.dual = pl.dual;
+  p.a_rows = static_cast<int>(box_act);
   p.out_bufs = pl.out_bufs;
   p.tiles_a = pl.tiles_a;
   p.tiles_b = pl.tiles_b;

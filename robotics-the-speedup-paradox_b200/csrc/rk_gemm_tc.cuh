@@ -56,6 +56,7 @@ constexpr int kGemmThreadsXform = kGemmThreads + kXformThreads;
 constexpr int kTileA = 128;        // rows of the A-role tile (MMA M)
 constexpr int kStageKBytes = 128;  // bytes of K per pipeline stage (one 128-byte swizzle atom)
 constexpr int kMaxStages = 8;
+constexpr int kMaxStagesFew = 16;          // SCHED_FEW, whose stages are small
 constexpr int kOutBufBytes = 16 * 1024;    // one output staging buffer (one or two are carved)
 constexpr int kVecBytes = 2 * 1024;        // per-tile B-role scale and bias vectors, 256 f32 entries each
 
@@ -75,6 +76,7 @@ struct GemmParams {
                    // `stages` is even if the ring wraps, so that a stage is always the same warp's
   int out_bufs;    // 1 or 2 output staging buffers in shared memory
   int tiles_a, tiles_b;
+  int a_rows;     // SCHED_FEW: activation rows of a stage (a multiple of 8; the MMA's other rows are whatever lies behind them)
   long long ldo;  // output row stride (elements)
   const float* scale_act;   // KIND_I8: [m] row scales.  other kinds: optional pointer to one scalar
   const float* scale_wgt;   // KIND_I8: [n] channel scales.  other kinds: optional pointer to one scalar
@@ -399,7 +401,9 @@ __device__ __forceinline__ void multicast_store_region(const GemmParams& p, cons
 // in flight would otherwise cost every launch of the kind its registers).
 // SCHED: whole K per CTA, K split over a cluster (GemmParams::splits > 1), or either as `splits` says; see launch_tc for which
 // form a launch takes.
-enum Schedule : int { SCHED_WHOLE, SCHED_SPLIT, SCHED_EITHER };
+// SCHED_FEW (KIND_I8): at most 128 activation rows on the 128-lane axis, of which only those that exist are fetched, one narrow
+// tile of weights per CTA; see few_rows_plan.
+enum Schedule : int { SCHED_WHOLE, SCHED_SPLIT, SCHED_EITHER, SCHED_FEW };
 template <int KIND, bool RESIDUAL = false, int SCHED = SCHED_WHOLE>
 __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out,
                                              const CUtensorMap* peer_maps, const GemmParams& p) {
@@ -407,8 +411,9 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   constexpr int BK = T::kBase;  // the MMA kind and epilogue this kind runs on
   constexpr bool kXform = T::kXformA != XF_NONE || T::kXformB != XF_NONE;
   extern __shared__ uint8_t smem_dyn[];
-  __shared__ __align__(8) uint64_t bar_full[kMaxStages];
-  __shared__ __align__(8) uint64_t bar_empty[kMaxStages];
+  constexpr bool kFew = SCHED == SCHED_FEW;
+  __shared__ __align__(8) uint64_t bar_full[kFew ? kMaxStagesFew : kMaxStages];
+  __shared__ __align__(8) uint64_t bar_empty[kFew ? kMaxStagesFew : kMaxStages];
   __shared__ __align__(8) uint64_t bar_raw_full[kMaxStages];   // raw operand bytes have landed (rewriting kinds)
   __shared__ __align__(8) uint64_t bar_raw_empty[kMaxStages];  // the rewriting warps have read them
   __shared__ __align__(8) uint64_t bar_acc_full[2];
@@ -422,7 +427,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_dyn + (smem_base - smem_u32(smem_dyn));  // generic pointer to smem_base
-  const int stage_bytes = gemm_stage_bytes(KIND, p.bn, p.sfb_blocks);
+  const int stage_bytes = kFew ? (p.a_rows + p.bn) * kStageKBytes : gemm_stage_bytes(KIND, p.bn, p.sfb_blocks);
+  const int a_bytes = (kFew ? p.a_rows : kTileA) * kStageKBytes;
   const int rb_b = p.sfb_blocks;  // 128-row scale blocks fetched per B tile
   const uint32_t spin_max = static_cast<uint32_t>(p.wait_limit);
   // offsets inside a stage: [A-role tile][B-role tile][scale chunks][raw A rows][raw B rows]
@@ -461,8 +467,10 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), kXform ? 1 + kXformWarps : 1);  // the producer's announcement (+ the rewriting warps)
       mbar_init(smem_u32(&bar_empty[s]), 1);
-      mbar_init(smem_u32(&bar_raw_full[s]), 1);
-      mbar_init(smem_u32(&bar_raw_empty[s]), kXformWarps);
+      if constexpr (kXform) {
+        mbar_init(smem_u32(&bar_raw_full[s]), 1);
+        mbar_init(smem_u32(&bar_raw_empty[s]), kXformWarps);
+      }
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bar_acc_full[b]), dual ? 2 : 1);
@@ -507,7 +515,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       // a barrier probe costs a shared-memory round trip: the probe of the NEXT stage is issued before
       // this stage's copies and read one trip later, so a stage that is already free costs no wait
       uint32_t ready = 0;
-      const uint32_t tx_data = (kTileA + p.bn) * kStageKBytes - p.tx_deficit;
+      const uint32_t tx_data = a_bytes + p.bn * kStageKBytes - p.tx_deficit;
       for (int tile = tile_first; tile < num_tiles && alive; tile += tile_step) {
         const int row_a0 = (tile / p.tiles_b) * kTileA;
         const int row_b0 = (tile % p.tiles_b) * p.bn;
@@ -539,7 +547,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
           }
           const uint32_t full = smem_u32(&bar_full[s]);
           const uint32_t sa = smem_base + s * stage_bytes;
-          const uint32_t sb = sa + kTileA * kStageKBytes;
+          const uint32_t sb = sa + a_bytes;
           const int kb = kb_begin + i;
           uint32_t tx = tx_data;
           // scale chunks present in this K block (the last block of a ragged K holds fewer)
@@ -610,7 +618,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       else if constexpr (BK == KIND_MXF8) idesc = umma_idesc_bs(p.fmt_a, p.fmt_b, 128, p.bn, 1, 0, 0);
       else idesc = umma_idesc_bs(FMT_E2M1_MXF4, FMT_E2M1_MXF4, 128, p.bn, 0, 0, 0);
       const uint64_t adesc0 = umma_desc_k128(smem_base);
-      const uint64_t bdesc0 = umma_desc_k128(smem_base + kTileA * kStageKBytes);
+      const uint64_t bdesc0 = umma_desc_k128(smem_base + a_bytes);
       const uint32_t stage_step = static_cast<uint32_t>(stage_bytes) >> 4;
       for (int tile = tile_first; tile < num_tiles && alive; tile += tile_step, racc.advance(p.acc_bufs)) {
         const int ab = racc.stage;
@@ -634,7 +642,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
           if (dual) ring.advance(p.stages);
           ready = mbar_test_wait(smem_u32(&bar_full[ring.stage]), ring.phase);
           const uint32_t sa = smem_base + s * stage_bytes;
-          const uint32_t sb = sa + kTileA * kStageKBytes;
+          const uint32_t sb = sa + a_bytes;
           const uint64_t adesc = adesc0 + static_cast<uint64_t>(s * stage_step);
           const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * stage_step);
           const int nmma = (kb_begin + i == p.kblocks - 1) ? p.k_valid_mmas_last : 4;
@@ -865,6 +873,32 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
         tc_fence_before();
         mbar_arrive(smem_u32(&bar_acc_empty[ab]));
         continue;
+      }
+
+      if constexpr (kFew) {
+        // ---- a thread's row of a narrow tile: 32 to 128 bytes, stored as they are
+        if (quad * 32 < p.m) {
+          __nv_bfloat16* const row_out = p.out + static_cast<long long>(ra) * p.ldo + row_b0;
+          for (int c0 = 0; c0 < p.bn; c0 += 16) {
+            uint32_t r[16];
+            __syncwarp();
+            load16(c0, r);
+            tc_wait_ld();
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = finish_value<BK>(r[j], row_scale, vec_scale[c0 + j], has_bias, vec_bias[c0 + j]);
+            if constexpr (RESIDUAL) with_residual16(p, v, row_b0 + c0, lim_b, ra, ra_ok, false);
+            if (ra_ok && ok) {
+#pragma unroll
+              for (int h = 0; h < 16; h += 8)
+                if (row_b0 + c0 + h < lim_b)  // n is a multiple of 8
+                  *reinterpret_cast<uint4*>(row_out + c0 + h) =
+                      make_uint4(pack_bf16x2(v[h], v[h + 1]), pack_bf16x2(v[h + 2], v[h + 3]), pack_bf16x2(v[h + 4], v[h + 5]),
+                                 pack_bf16x2(v[h + 6], v[h + 7]));
+            }
+          }
+        }
+        continue;  // the only tile
       }
 
       // ---- swapped tiles that fit: stage the whole tile once, then issue all its TMA stores.  The
