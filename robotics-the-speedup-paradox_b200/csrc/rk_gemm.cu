@@ -374,13 +374,16 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
 // W8A8, up to 128 activation rows: the rows take the 128-lane axis, and only those that exist are fetched; every CTA has one
 // tile of weights, as narrow as gives each SM one (multiples of 16).  A block of K then costs an SM (m + bn) x 128 bytes from L2
 // instead of (128 + 32) x 128 with the weights on the lanes, the copies are spread over more SMs, and a row of the tile is stored
-// from registers.  Bound by the producer's two copies and the issuing warps (about 165 cycles a block).  Against `pl`: 50 x 1024
-// x 2048 4.5 -> 3.8 us, 100 x 8192 x 1024 5.5 -> 4.6, 64 x 4096 x 4096 7.6 -> 6.4, 128 x 2048 x 8192 11.8 -> 10.0, 1 x 1024 x 2048
-// 4.4 -> 3.8; chunk of one environment 8.78 -> 8.07 ms.  Not for
+// from registers.  A stage is two blocks: one copy brings both of an operand (its descriptor has the blocks as a third dimension;
+// four copies a pair of blocks paced the loop, 170 cycles a block: 50 x 1024 x 2048 3.9 -> 3.7 us, chunk of one environment
+// 8.00 -> 7.78 ms), and each of two warps issues one block.  What is left is latency: 2.5 us at four blocks of K, 3.3 at eight,
+// then 95 ns a block, which neither a deeper ring nor prefetching all weights to L2 nor another order of blocks per CTA changes.
+// Against `pl`: 50 x 1024 x 2048 4.5 -> 3.7 us, 100 x 8192 x 1024 5.5 -> 4.5, 50 x 4096 x 4096 7.6 -> 6.1, 128 x 2048 x 2048
+// 4.9 -> 4.4, 1 x 1024 x 2048 4.4 -> 3.6; chunk of one environment 8.78 -> 7.78 ms.  Not for
 // - tiles much wider than the rows are many: 16 x 8192 x 1024 4.0 against 4.4 us, 32 rows 4.2 and 4.4, 50 x 16384 x 2048 8.0 and
 //   8.2 (64 x 8192 x 1024 4.6 -> 4.4, 100 x 16384 x 2048 8.9 -> 8.5);
 // - a long loop that `pl` splits: 50 x 2048 x 8192 8.2 against 8.8, 50 x 256 x 4096 4.7 against 5.1 in eight; at 32 blocks in six
-//   or fewer it still gains (50 x 1024 x 4096 5.6 -> 5.4, 100 rows 6.4 -> 5.5).
+//   or fewer it still gains (50 x 1024 x 4096 5.6 -> 5.2, 100 rows 6.4 -> 5.3).
 Plan few_rows_plan(const Plan& pl, int64_t m, int64_t n, int kblocks, int tactic) {
   const int bn = static_cast<int>(round_up((n + kNumSms - 1) / kNumSms, 16));
   if (m > 128 || (tactic & 5) || bn > pow2_at_least(static_cast<int>(m), 16) || pl.splits > (kblocks <= 32 ? 6 : 1)) return pl;
@@ -395,10 +398,8 @@ Plan few_rows_plan(const Plan& pl, int64_t m, int64_t n, int kblocks, int tactic
   few.acc_bufs = 2;
   few.tmem_cols = pow2_at_least(2 * few.acc_stride, 32);
   few.out_bufs = 1;  // nothing is staged: an MMA reads 128 rows from the start of a stage, beyond the end of the last
-  const int stage = static_cast<int>(round_up(m, 8) + bn) * kStageKBytes;
-  few.stages = std::min((kSmemBudget - kVecBytes - kOutBufBytes) / stage, kMaxStagesFew);
-  if (few.stages < kblocks) few.stages &= ~1;  // a ring that wraps, as in make_plan
-  else few.stages = std::max(kblocks, 2);
+  const int stage = 2 * static_cast<int>(round_up(m, 8) + bn) * kStageKBytes;  // two K blocks
+  few.stages = std::min({(kSmemBudget - kVecBytes - kOutBufBytes) / stage, kMaxStages, std::max((kblocks + 1) / 2, 2)});
   // More than half of an SM's shared memory, however little the stages need: CTAs of the next launch that start early would crowd
   // into the SMs that this one uses, two or three to an SM, beside idle ones (chains: 50 x 2560 x 1024 3.9 -> 3.5 us, 17 x 8192 x
   // 1024 5.0 -> 4.4, 1 x 2048 x 2048 5.9 -> 4.4).
@@ -771,7 +772,7 @@ int run_tc(const TcArgs& a) {
     }
   }
   Plan pl = make_plan(a.kind, a.m, a.n, kblocks, a.tactic);
-  if (a.kind == KIND_I8 && a.acc_out == nullptr && a.peer == nullptr) pl = few_rows_plan(pl, a.m, a.n, kblocks, a.tactic);
+  if (a.kind == KIND_I8 && a.acc_out == nullptr && a.peer == nullptr && a.k_bytes % kStageKBytes == 0) pl = few_rows_plan(pl, a.m, a.n, kblocks, a.tactic);
 
   CUtensorMap tm_act, tm_wgt, tm_out;
   const uint32_t box_act = pl.swap ? pl.bn : pl.few ? static_cast<uint32_t>(round_up(a.m, 8)) : kTileA;
@@ -779,14 +780,20 @@ int run_tc(const TcArgs& a) {
   // an operand that is rewritten in shared memory is fetched as raw rows: `raw` bytes of every row per
   // 128 MMA bytes of K, unswizzled; its row pitch is k_bytes * raw / 128
   const int raw_act = gemm_raw_bytes_a(a.kind), raw_wgt = gemm_raw_bytes_b(a.kind);
-  if (raw_act)
+  if (pl.few)  // [K block][row][128 bytes]: a box is two K blocks, tile after tile
+    rc = make_map_3d(&tm_act, a.act, CU_TENSOR_MAP_DATA_TYPE_UINT8, kStageKBytes, a.m, kblocks, a.k_bytes, kStageKBytes, kStageKBytes,
+                     box_act, 2, CU_TENSOR_MAP_SWIZZLE_128B);
+  else if (raw_act)
     rc = make_map_2d(&tm_act, a.act, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.k_bytes * raw_act / kStageKBytes, a.m,
                      a.k_bytes * raw_act / kStageKBytes, raw_act, box_act, CU_TENSOR_MAP_SWIZZLE_NONE);
   else
     rc = make_map_2d(&tm_act, a.act, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.k_bytes, a.m, a.k_bytes, kStageKBytes, box_act,
                      CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != RK_OK) return rc;
-  if (raw_wgt)
+  if (pl.few)
+    rc = make_map_3d(&tm_wgt, a.wgt, CU_TENSOR_MAP_DATA_TYPE_UINT8, kStageKBytes, a.n, kblocks, a.k_bytes, kStageKBytes, kStageKBytes,
+                     box_wgt, 2, CU_TENSOR_MAP_SWIZZLE_128B);
+  else if (raw_wgt)
     rc = make_map_2d(&tm_wgt, a.wgt, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.k_bytes * raw_wgt / kStageKBytes, a.n,
                      a.k_bytes * raw_wgt / kStageKBytes, raw_wgt, box_wgt, CU_TENSOR_MAP_SWIZZLE_NONE);
   else

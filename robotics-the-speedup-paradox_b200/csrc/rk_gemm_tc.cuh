@@ -56,7 +56,6 @@ constexpr int kGemmThreadsXform = kGemmThreads + kXformThreads;
 constexpr int kTileA = 128;        // rows of the A-role tile (MMA M)
 constexpr int kStageKBytes = 128;  // bytes of K per pipeline stage (one 128-byte swizzle atom)
 constexpr int kMaxStages = 8;
-constexpr int kMaxStagesFew = 16;          // SCHED_FEW, whose stages are small
 constexpr int kOutBufBytes = 16 * 1024;    // one output staging buffer (one or two are carved)
 constexpr int kVecBytes = 2 * 1024;        // per-tile B-role scale and bias vectors, 256 f32 entries each
 
@@ -76,7 +75,7 @@ struct GemmParams {
                    // `stages` is even if the ring wraps, so that a stage is always the same warp's
   int out_bufs;    // 1 or 2 output staging buffers in shared memory
   int tiles_a, tiles_b;
-  int a_rows;     // SCHED_FEW: activation rows of a stage (a multiple of 8; the MMA's other rows are whatever lies behind them)
+  int a_rows;     // SCHED_FEW: activation rows of a K block (a multiple of 8; the MMA's other rows are whatever lies behind them)
   long long ldo;  // output row stride (elements)
   const float* scale_act;   // KIND_I8: [m] row scales.  other kinds: optional pointer to one scalar
   const float* scale_wgt;   // KIND_I8: [n] channel scales.  other kinds: optional pointer to one scalar
@@ -402,7 +401,8 @@ __device__ __forceinline__ void multicast_store_region(const GemmParams& p, cons
 // SCHED: whole K per CTA, K split over a cluster (GemmParams::splits > 1), or either as `splits` says; see launch_tc for which
 // form a launch takes.
 // SCHED_FEW (KIND_I8): at most 128 activation rows on the 128-lane axis, of which only those that exist are fetched, one narrow
-// tile of weights per CTA; see few_rows_plan.
+// tile of weights per CTA, two K blocks to a stage: one copy brings both of an operand, two issuing warps take one each.  See
+// few_rows_plan.
 enum Schedule : int { SCHED_WHOLE, SCHED_SPLIT, SCHED_EITHER, SCHED_FEW };
 template <int KIND, bool RESIDUAL = false, int SCHED = SCHED_WHOLE>
 __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out,
@@ -412,8 +412,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   constexpr bool kXform = T::kXformA != XF_NONE || T::kXformB != XF_NONE;
   extern __shared__ uint8_t smem_dyn[];
   constexpr bool kFew = SCHED == SCHED_FEW;
-  __shared__ __align__(8) uint64_t bar_full[kFew ? kMaxStagesFew : kMaxStages];
-  __shared__ __align__(8) uint64_t bar_empty[kFew ? kMaxStagesFew : kMaxStages];
+  __shared__ __align__(8) uint64_t bar_full[kMaxStages];
+  __shared__ __align__(8) uint64_t bar_empty[kMaxStages];
   __shared__ __align__(8) uint64_t bar_raw_full[kMaxStages];   // raw operand bytes have landed (rewriting kinds)
   __shared__ __align__(8) uint64_t bar_raw_empty[kMaxStages];  // the rewriting warps have read them
   __shared__ __align__(8) uint64_t bar_acc_full[2];
@@ -427,7 +427,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_dyn + (smem_base - smem_u32(smem_dyn));  // generic pointer to smem_base
-  const int stage_bytes = kFew ? (p.a_rows + p.bn) * kStageKBytes : gemm_stage_bytes(KIND, p.bn, p.sfb_blocks);
+  const int stage_bytes = kFew ? 2 * (p.a_rows + p.bn) * kStageKBytes : gemm_stage_bytes(KIND, p.bn, p.sfb_blocks);
   const int a_bytes = (kFew ? p.a_rows : kTileA) * kStageKBytes;
   const int rb_b = p.sfb_blocks;  // 128-row scale blocks fetched per B tile
   const uint32_t spin_max = static_cast<uint32_t>(p.wait_limit);
@@ -456,9 +456,10 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
     if (tile_first < num_tiles) {
       const int row_a0 = (tile_first / p.tiles_b) * kTileA;
       const int row_b0 = (tile_first % p.tiles_b) * p.bn;
-      const int ahead = min(nkb, p.stages);
+      const int ahead = min(kFew ? (nkb + 1) / 2 : nkb, p.stages);
       for (int i = 0; i < ahead; ++i) {
-        if (p.swap) tma_prefetch_l2_2d(&tm_a, (kb_begin + i) * kStageKBytes, row_a0);
+        if constexpr (kFew) tma_prefetch_l2_3d(&tm_b, 0, row_b0, 2 * i);
+        else if (p.swap) tma_prefetch_l2_2d(&tm_a, (kb_begin + i) * kStageKBytes, row_a0);
         else tma_prefetch_l2_2d(&tm_b, (kb_begin + i) * kStageKBytes, row_b0);
       }
     }
@@ -466,7 +467,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), kXform ? 1 + kXformWarps : 1);  // the producer's announcement (+ the rewriting warps)
-      mbar_init(smem_u32(&bar_empty[s]), 1);
+      mbar_init(smem_u32(&bar_empty[s]), kFew && dual ? 2 : 1);
       if constexpr (kXform) {
         mbar_init(smem_u32(&bar_raw_full[s]), 1);
         mbar_init(smem_u32(&bar_raw_empty[s]), kXformWarps);
@@ -498,7 +499,51 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const uint32_t tmem_sfa = tmem_base + p.acc_bufs * p.acc_stride;
   const uint32_t tmem_sfb = tmem_sfa + 16;
 
-  if (warp == 0) {
+  if (kFew && warp == 0) {
+    // ------------------------------------------------------------ TMA producer, few rows: two K blocks a copy
+    const uint32_t on = elect_one();
+    const uint64_t pol_w = l2_policy_evict_first(), pol_x = l2_policy_evict_last();
+    Ring ring{0, 0};
+    uint32_t ready = 0;
+    for (int i = 0; 2 * i < nkb; ++i) {
+      const int s = ring.stage;
+      if (!ready && !mbar_wait_bounded(smem_u32(&bar_empty[s]), ring.phase ^ 1, &abort_flag, p.status, RK_DEV_TIMEOUT_EMPTY, spin_max)) break;
+      ring.advance(p.stages);
+      ready = mbar_test_wait(smem_u32(&bar_empty[ring.stage]), ring.phase ^ 1);
+      const uint32_t full = smem_u32(&bar_full[s]), sa = smem_base + s * stage_bytes;
+      mbar_arrive_expect_tx(full, stage_bytes + (p.debug_stall && i == 0 ? 16 : 0), on);
+      tma_load_3d_on(sa, &tm_a, 0, 0, 2 * i, full, pol_x, on);  // blocks beyond K arrive as zeros
+      tma_load_3d_on(sa + 2 * a_bytes, &tm_b, 0, tile_first * p.bn, 2 * i, full, pol_w, on);
+    }
+  } else if (kFew && (warp == 1 || (dual && warp == 6))) {
+    // ------------------------------------------------------------ MMA issuers, few rows: each its block of every stage
+    const uint32_t on = elect_one();
+    const int mine = warp == 6 ? 1 : 0;
+    const uint32_t idesc = umma_idesc(DFMT_S32, FMT_S8, FMT_S8, 128, p.bn);
+    const uint64_t adesc0 = umma_desc_k128(smem_base + mine * a_bytes);
+    const uint64_t bdesc0 = umma_desc_k128(smem_base + 2 * a_bytes + mine * p.bn * kStageKBytes);
+    const uint32_t stage_step = static_cast<uint32_t>(stage_bytes) >> 4;
+    const uint32_t d_tmem = tmem_base + mine * p.acc_stride;
+    Ring ring{0, 0};
+    bool alive = true;
+    uint32_t ready = 0;
+    for (int i = 0; 2 * i < nkb; ++i) {
+      const int s = ring.stage;
+      if (!ready && !mbar_wait_bounded(smem_u32(&bar_full[s]), ring.phase, &abort_flag, p.status, RK_DEV_TIMEOUT_FULL, spin_max)) {
+        alive = false;
+        break;
+      }
+      tc_fence_after();
+      ring.advance(p.stages);
+      ready = mbar_test_wait(smem_u32(&bar_full[ring.stage]), ring.phase);
+      const uint64_t adesc = adesc0 + static_cast<uint64_t>(s * stage_step), bdesc = bdesc0 + static_cast<uint64_t>(s * stage_step);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (on && 2 * i + mine < nkb) mma_i8_np(d_tmem, adesc + k * 2, bdesc + k * 2, idesc, (i > 0 || k > 0) ? 1u : 0u);
+      tc_commit(smem_u32(&bar_empty[s]), on);
+    }
+    if (alive) tc_commit(smem_u32(&bar_acc_full[0]), on);
+  } else if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     // the whole warp walks the loop (uniform control flow); the copies are issued by one elected lane
     {
