@@ -176,7 +176,7 @@ int pow2_at_least(int v, int lo) {
 
 // ------------------------------------------------------------------ tile selection
 struct Plan {
-  int swap, bn, tiles_a, tiles_b, splits, stages, tmem_cols, acc_stride, acc_bufs, out_bufs, smem_bytes, grid_x, dual, few;
+  int swap, bn, tiles_a, tiles_b, splits, stages, tmem_cols, acc_stride, acc_bufs, out_bufs, smem_bytes, grid_x, dual, few, a_rows;
   int sfb_blocks;
 };
 
@@ -371,7 +371,7 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
   return pl;
 }
 
-// W8A8, up to 128 activation rows: the rows take the 128-lane axis, and only those that exist are fetched; every CTA has one
+// W8A8, few activation rows: the rows take the 128-lane axis, and only those that exist are fetched; every CTA has one
 // tile of weights, as narrow as gives each SM one (multiples of 16).  A block of K then costs an SM (m + bn) x 128 bytes from L2
 // instead of (128 + 32) x 128 with the weights on the lanes, the copies are spread over more SMs, and a row of the tile is stored
 // from registers.  A stage is two blocks: one copy brings both of an operand (its descriptor has the blocks as a third dimension;
@@ -384,21 +384,28 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
 //   8.2 (64 x 8192 x 1024 4.6 -> 4.4, 100 x 16384 x 2048 8.9 -> 8.5);
 // - a long loop that `pl` splits: 50 x 2048 x 8192 8.2 against 8.8, 50 x 256 x 4096 4.7 against 5.1 in eight; at 32 blocks in six
 //   or fewer it still gains (50 x 1024 x 4096 5.6 -> 5.2, 100 rows 6.4 -> 5.3).
+// Above 128 rows equal tiles of at most 128: 200 x 2048 x 2048 5.2 -> 4.7 us, 300 x 2560 x 1024 4.8 -> 4.3, 400 x 1024 x 2048 4.9 ->
+// 4.6, 600 x 1024 x 2048 5.6 -> 5.0, 816 x 1024 x 512 4.1 -> 3.8.  Not where a block has more operand rows than `pl`'s (816 x
+// 2048 x 2048 6.9 against 7.2) or tiles are wide (300 x 8192 x 1024 6.8 and 7.4), nor above 256 rows for a long loop (400 x 2048 x
+// 8192 12.8 and 13.5, 816 rows 16.0 and 18.0; 200 rows 11.6 -> 10.1).
 Plan few_rows_plan(const Plan& pl, int64_t m, int64_t n, int kblocks, int tactic) {
-  const int bn = static_cast<int>(round_up((n + kNumSms - 1) / kNumSms, 16));
-  if (m > 128 || (tactic & 5) || bn > pow2_at_least(static_cast<int>(m), 16) || pl.splits > (kblocks <= 32 ? 6 : 1)) return pl;
+  const int64_t tiles_a = (m + 127) / 128, rows = round_up((m + tiles_a - 1) / tiles_a, 8), fit = kNumSms / tiles_a;
+  const int bn = static_cast<int>(round_up((n + fit - 1) / fit, 16));
+  if ((tactic & 5) || bn > std::min(128, pow2_at_least(static_cast<int>(m), 16)) || pl.splits > (kblocks <= 32 ? 6 : 1)) return pl;
+  if (m > 128 && (!pl.swap || rows + bn > kTileA + pl.bn || (m > 256 && kblocks > 32))) return pl;
   Plan few{};
   few.few = 1;
   few.dual = kblocks >= 2 ? 1 : 0;
   few.bn = bn;
-  few.tiles_a = 1;
-  few.tiles_b = few.grid_x = static_cast<int>((n + bn - 1) / bn);
+  few.a_rows = static_cast<int>(rows);
+  few.tiles_a = static_cast<int>(tiles_a);
+  few.tiles_b = few.grid_x = static_cast<int>((n + bn - 1) / bn);  // the row tiles are the grid's y
   few.splits = 1;
   few.acc_stride = static_cast<int>(round_up(bn, 32));
   few.acc_bufs = 2;
   few.tmem_cols = pow2_at_least(2 * few.acc_stride, 32);
   few.out_bufs = 1;  // nothing is staged: an MMA reads 128 rows from the start of a stage, beyond the end of the last
-  const int stage = 2 * static_cast<int>(round_up(m, 8) + bn) * kStageKBytes;  // two K blocks
+  const int stage = 2 * (few.a_rows + bn) * kStageKBytes;  // two K blocks
   few.stages = std::min({(kSmemBudget - kVecBytes - kOutBufBytes) / stage, kMaxStages, std::max((kblocks + 1) / 2, 2)});
   // More than half of an SM's shared memory, however little the stages need: CTAs of the next launch that start early would crowd
   // into the SMs that this one uses, two or three to an SM, beside idle ones (chains: 50 x 2560 x 1024 3.9 -> 3.5 us, 17 x 8192 x
@@ -421,7 +428,7 @@ int launch_tc_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUt
     configured = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(pl.grid_x, 1, pl.splits);
+  cfg.gridDim = dim3(pl.grid_x, SCHED == SCHED_FEW ? pl.tiles_a : 1, pl.splits);
   cfg.blockDim = dim3(KindTraits<KIND>::kThreads);
   cfg.dynamicSmemBytes = pl.smem_bytes;
   cfg.stream = st;
@@ -775,7 +782,7 @@ int run_tc(const TcArgs& a) {
   if (a.kind == KIND_I8 && a.acc_out == nullptr && a.peer == nullptr && a.k_bytes % kStageKBytes == 0) pl = few_rows_plan(pl, a.m, a.n, kblocks, a.tactic);
 
   CUtensorMap tm_act, tm_wgt, tm_out;
-  const uint32_t box_act = pl.swap ? pl.bn : pl.few ? static_cast<uint32_t>(round_up(a.m, 8)) : kTileA;
+  const uint32_t box_act = pl.swap ? pl.bn : pl.few ? pl.a_rows : kTileA;
   const uint32_t box_wgt = pl.swap ? kTileA : pl.bn;
   // an operand that is rewritten in shared memory is fetched as raw rows: `raw` bytes of every row per
   // 128 MMA bytes of K, unswizzled; its row pitch is k_bytes * raw / 128

@@ -75,7 +75,7 @@ struct GemmParams {
                    // `stages` is even if the ring wraps, so that a stage is always the same warp's
   int out_bufs;    // 1 or 2 output staging buffers in shared memory
   int tiles_a, tiles_b;
-  int a_rows;     // SCHED_FEW: activation rows of a K block (a multiple of 8; the MMA's other rows are whatever lies behind them)
+  int a_rows;     // SCHED_FEW: activation rows of a tile (a multiple of 8; the MMA's other rows are whatever lies behind them)
   long long ldo;  // output row stride (elements)
   const float* scale_act;   // KIND_I8: [m] row scales.  other kinds: optional pointer to one scalar
   const float* scale_wgt;   // KIND_I8: [n] channel scales.  other kinds: optional pointer to one scalar
@@ -400,7 +400,7 @@ __device__ __forceinline__ void multicast_store_region(const GemmParams& p, cons
 // in flight would otherwise cost every launch of the kind its registers).
 // SCHED: whole K per CTA, K split over a cluster (GemmParams::splits > 1), or either as `splits` says; see launch_tc for which
 // form a launch takes.
-// SCHED_FEW (KIND_I8): at most 128 activation rows on the 128-lane axis, of which only those that exist are fetched, one narrow
+// SCHED_FEW (KIND_I8): a tile's activation rows on the 128-lane axis, only those that exist being fetched, one narrow
 // tile of weights per CTA, two K blocks to a stage: one copy brings both of an operand, two issuing warps take one each.  See
 // few_rows_plan.
 enum Schedule : int { SCHED_WHOLE, SCHED_SPLIT, SCHED_EITHER, SCHED_FEW };
@@ -439,7 +439,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const uint32_t vec_off = out_stage_off + p.out_bufs * kOutBufBytes;
 
   const bool split_mode = SCHED == SCHED_EITHER ? p.splits > 1 : SCHED == SCHED_SPLIT;
-  const int num_tiles = p.tiles_a * p.tiles_b;
+  const int num_tiles = kFew ? static_cast<int>(gridDim.x) : p.tiles_a * p.tiles_b;  // few rows: the grid is columns x rows of tiles
   const int tile_first = static_cast<int>(blockIdx.x);
   const int tile_step = split_mode ? num_tiles : static_cast<int>(gridDim.x);  // split mode: exactly one tile
   const int split = static_cast<int>(blockIdx.z);
@@ -454,8 +454,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
     // The weight rows of this CTA's first tile start their way from DRAM to L2 during set-up, while
     // the preceding kernel drains (a request to L2 alone: see tma_prefetch_l2_2d).
     if (tile_first < num_tiles) {
-      const int row_a0 = (tile_first / p.tiles_b) * kTileA;
-      const int row_b0 = (tile_first % p.tiles_b) * p.bn;
+      const int row_a0 = kFew ? 0 : (tile_first / p.tiles_b) * kTileA;
+      const int row_b0 = (kFew ? tile_first : tile_first % p.tiles_b) * p.bn;
       const int ahead = min(kFew ? (nkb + 1) / 2 : nkb, p.stages);
       for (int i = 0; i < ahead; ++i) {
         if constexpr (kFew) tma_prefetch_l2_3d(&tm_b, 0, row_b0, 2 * i);
@@ -503,6 +503,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
     // ------------------------------------------------------------ TMA producer, few rows: two K blocks a copy
     const uint32_t on = elect_one();
     const uint64_t pol_w = l2_policy_evict_first(), pol_x = l2_policy_evict_last();
+    const int row_a0 = static_cast<int>(blockIdx.y) * p.a_rows, row_b0 = tile_first * p.bn;
     Ring ring{0, 0};
     uint32_t ready = 0;
     for (int i = 0; 2 * i < nkb; ++i) {
@@ -512,8 +513,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
       ready = mbar_test_wait(smem_u32(&bar_empty[ring.stage]), ring.phase ^ 1);
       const uint32_t full = smem_u32(&bar_full[s]), sa = smem_base + s * stage_bytes;
       mbar_arrive_expect_tx(full, stage_bytes + (p.debug_stall && i == 0 ? 16 : 0), on);
-      tma_load_3d_on(sa, &tm_a, 0, 0, 2 * i, full, pol_x, on);  // blocks beyond K arrive as zeros
-      tma_load_3d_on(sa + 2 * a_bytes, &tm_b, 0, tile_first * p.bn, 2 * i, full, pol_w, on);
+      tma_load_3d_on(sa, &tm_a, 0, row_a0, 2 * i, full, pol_x, on);  // blocks beyond K arrive as zeros
+      tma_load_3d_on(sa + 2 * a_bytes, &tm_b, 0, row_b0, 2 * i, full, pol_w, on);
     }
   } else if (kFew && (warp == 1 || (dual && warp == 6))) {
     // ------------------------------------------------------------ MMA issuers, few rows: each its block of every stage
@@ -841,10 +842,10 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
     int obuf = 0;
     for (int tile = tile_first; tile < num_tiles; tile += tile_step, racc.advance(p.acc_bufs)) {
       const int ab = racc.stage;
-      const int row_a0 = (tile / p.tiles_b) * kTileA;
-      const int row_b0 = (tile % p.tiles_b) * p.bn;
+      const int row_a0 = kFew ? static_cast<int>(blockIdx.y) * p.a_rows : (tile / p.tiles_b) * kTileA;
+      const int row_b0 = (kFew ? tile : tile % p.tiles_b) * p.bn;
       const int ra = row_a0 + et;
-      const bool ra_ok = ra < lim_a;
+      const bool ra_ok = ra < lim_a && (!kFew || et < p.a_rows);
       // per-thread constants of the A-role row, and the B-role vectors of this tile into shared memory
       float row_scale = 1.0f, row_bias = 0.0f;
       if (p.acc_out == nullptr) {
@@ -922,7 +923,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
 
       if constexpr (kFew) {
         // ---- a thread's row of a narrow tile: 32 to 128 bytes, stored as they are
-        if (quad * 32 < p.m) {
+        if (quad * 32 < p.a_rows) {
           __nv_bfloat16* const row_out = p.out + static_cast<long long>(ra) * p.ldo + row_b0;
           for (int c0 = 0; c0 < p.bn; c0 += 16) {
             uint32_t r[16];

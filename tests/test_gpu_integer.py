@@ -346,13 +346,15 @@ def test_pair_tiles_of_every_width(m, n, k, kind):
 
 # One tile per CTA, so two warps issue alternate K blocks: K of one block (one warp), two, three, a ring that wraps with 32, 64,
 # 96, 128 and 224 rows a tile (an odd number of stages would fit at 64 and 96), split K, a ragged last block and ragged edges;
-# then 17 to 128 rows on the lane axis: its bounds, weight tiles of 16 to 128 columns, rows and columns that end inside a tile
+# then rows on the lane axis, one tile of them and several: its bounds, weight tiles of 16 to 128 columns, rows and columns that end inside a tile
 @pytest.mark.parametrize("m,n,k", [(50, 1024, 128), (50, 1024, 256), (50, 264, 384), (50, 2560, 1024), (50, 1024, 2080),
                                    (400, 2560, 1152), (400, 1024, 2048), (400, 1024, 4096), (400, 1000, 4224), (600, 1024, 4096),
                                    (816, 2048, 4096), (1000, 1000, 2304), (400, 8192, 1024), (448, 8192, 640), (7, 1024, 4096),
                                    (200, 1024, 4096), (96, 512, 8192),
                                    (16, 520, 512), (17, 8, 128), (17, 520, 512), (31, 2376, 640), (33, 2368, 2176), (64, 9472, 256),
-                                   (65, 9480, 256), (97, 18944, 128), (127, 4104, 1920), (128, 2048, 4096), (128, 1000, 4224)])
+                                   (65, 9480, 256), (97, 18944, 128), (127, 4104, 1920), (128, 2048, 4096), (128, 1000, 4224),
+                                   (129, 2376, 640), (137, 8192, 384), (256, 1032, 4224), (257, 2048, 2176), (385, 2560, 1024),
+                                   (600, 1016, 4096), (1000, 1000, 512), (1024, 1032, 384)])
 def test_two_issuing_warps_add_up(m, n, k):
     from rk_b200 import _lib
 
