@@ -443,8 +443,9 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tm_a, const CUte
   const int tile_first = static_cast<int>(blockIdx.x);
   const int tile_step = split_mode ? num_tiles : static_cast<int>(gridDim.x);  // split mode: exactly one tile
   const int split = static_cast<int>(blockIdx.z);
-  const int kb_begin = static_cast<int>((static_cast<long long>(p.kblocks) * split) / p.splits);
-  const int kb_end = static_cast<int>((static_cast<long long>(p.kblocks) * (split + 1)) / p.splits);
+  constexpr bool kWhole = SCHED == SCHED_WHOLE || kFew;
+  const int kb_begin = kWhole ? 0 : static_cast<int>((static_cast<long long>(p.kblocks) * split) / p.splits);
+  const int kb_end = kWhole ? p.kblocks : static_cast<int>((static_cast<long long>(p.kblocks) * (split + 1)) / p.splits);
   const int nkb = kb_end - kb_begin;
   constexpr bool kDual = KIND == KIND_I8;
   const bool dual = kDual && p.dual && nkb > 1;
