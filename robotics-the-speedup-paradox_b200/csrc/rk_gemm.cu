@@ -389,6 +389,7 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
 // 2048 x 2048 6.9 against 7.2) or tiles are wide (300 x 8192 x 1024 6.8 and 7.4), nor above 256 rows for a long loop (400 x 2048 x
 // 8192 12.8 and 13.5, 816 rows 16.0 and 18.0; 200 rows 11.6 -> 10.1).
 Plan few_rows_plan(const Plan& pl, int64_t m, int64_t n, int kblocks, int tactic) {
+  if (m > 1024) return pl;  // nothing above is taken, and from 149 row tiles on no SM would be left for the columns (fit = 0)
   const int64_t tiles_a = (m + 127) / 128, rows = round_up((m + tiles_a - 1) / tiles_a, 8), fit = kNumSms / tiles_a;
   const int bn = static_cast<int>(round_up((n + fit - 1) / fit, 16));
   if ((tactic & 5) || bn > std::min(128, pow2_at_least(static_cast<int>(m), 16)) || pl.splits > (kblocks <= 32 ? 6 : 1)) return pl;
