@@ -174,7 +174,8 @@ def rope_cache_update(q, k, v, cos, sin, k_all, v_all, prefix, heads, kv_heads, 
 
 def kv_prefix_fill(prefix_k, prefix_v, k_all, v_all, vt_all):
     """Copies a cached prefix into the working caches and transposes its values in one kernel (`rk_kv_prefix_fill`).  Returns
-    False, with nothing done, for tensors that it does not take (other types, strides or devices, an empty prefix)."""
+    False, with nothing done, for tensors that it does not take (other types, strides or devices, an empty prefix, one that
+    the copy has to broadcast)."""
     from . import _lib
 
     tensors = (prefix_k, prefix_v, k_all, v_all, vt_all)
@@ -185,6 +186,8 @@ def kv_prefix_fill(prefix_k, prefix_v, k_all, v_all, vt_all):
     rows, planes = prefix_k.shape[3], prefix_k.shape[:3].numel()
     if prefix_v.shape != prefix_k.shape or not 0 < rows < 1 << 24 or not 0 < planes <= 65535:
         return False
+    if not prefix_k.shape[:3] == k_all.shape[:3] == v_all.shape[:3] == vt_all.shape[:3]:
+        return False  # one prefix for several environments: the tensor ops broadcast it
     with torch.cuda.device(device):
         code = _lib.load().rk_kv_prefix_fill(
             _lib.ptr(prefix_k), _lib.ptr(prefix_v), planes, rows, prefix_k.shape[4], _lib.ptr(k_all), _lib.ptr(v_all),

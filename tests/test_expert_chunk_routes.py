@@ -1,0 +1,42 @@
+"""Calls of the action expert that its fused kernels do not take keep going through the tensor ops."""
+
+import pytest
+import torch
+
+from rk_b200.gemma_stack import ActionExpert, GemmaAttention, GemmaConfig, kv_prefix_fill
+
+BF16 = torch.bfloat16
+
+
+@pytest.mark.parametrize("batch", [1, 2, 3])
+def test_prefix_fill_leaves_a_broadcast_prefix_to_the_tensor_ops(batch):
+    """One prefix for several environments (or any other pair of shapes that only broadcasting joins)."""
+    prefix = torch.zeros(2, batch, 1, 8, 256, dtype=BF16)
+    caches = torch.zeros(2, 2, 4, 1, 16, 256, dtype=BF16)
+    assert not kv_prefix_fill(prefix, prefix, caches[0], caches[1], torch.zeros(2, 4, 1, 256, 16, dtype=BF16))
+
+
+DEVICE = torch.device("cuda:0")
+
+
+def small_expert(head_dim, steps=3):
+    cfg = GemmaConfig(width=256, mlp_dim=512, depth=2, num_heads=2, num_kv_heads=1, head_dim=head_dim, adarms_cond_dim=256)
+    return ActionExpert(cfg, chunk=50, action_dim=32, steps=steps).init_random(1).to(DEVICE).eval()
+
+
+def draws(head_dim, noise_batch, prefix_batch, tokens=70):
+    gen = torch.Generator(device=DEVICE).manual_seed(7)
+    r = lambda *s: torch.randn(s, generator=gen, device=DEVICE)
+    return r(noise_batch, 50, 32), *(r(2, prefix_batch, 1, tokens, head_dim).to(BF16) for _ in range(2))
+
+
+@pytest.mark.gpu
+def test_one_prefix_for_several_environments(monkeypatch):
+    monkeypatch.setattr(GemmaAttention, "fused_rope", True)
+    monkeypatch.setattr(GemmaAttention, "fused_attention", True)
+    expert = small_expert(256)
+    noise, pk, pv = draws(256, 3, 1)
+    with torch.no_grad():
+        shared = expert(noise, pk, pv)
+        copied = expert(noise, *(t.expand(2, 3, 1, 70, 256).contiguous() for t in (pk, pv)))
+    assert torch.equal(shared, copied)
