@@ -529,7 +529,10 @@ class ActionExpert(nn.Module):
         if type(self).denoise_step is not ActionExpert.denoise_step or "denoise_step" in vars(self):
             return False
         params = [p for m in linears for p in (m.weight, m.bias)]
-        if any(p is None or p.dtype != torch.float32 or p.device != noise.device or not p.is_contiguous() for p in params):
+        if any(type(p) not in (nn.Parameter, torch.Tensor) or p.dtype != torch.float32 or p.device != noise.device
+               or not p.is_contiguous() for p in params):
+            return False
+        if any(m.weight.data_ptr() % 16 for m in linears):  # views into a flat buffer, for instance
             return False
         dims = noise.shape[-1]
         return (linears[0].weight.shape == (width, dims) and linears[1].weight.shape == (dims, width) and width % 8 == 0

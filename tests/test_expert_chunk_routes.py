@@ -40,3 +40,41 @@ def test_one_prefix_for_several_environments(monkeypatch):
         shared = expert(noise, pk, pv)
         copied = expert(noise, *(t.expand(2, 3, 1, 70, 256).contiguous() for t in (pk, pv)))
     assert torch.equal(shared, copied)
+
+
+def fused_step_expert():
+    """An expert whose steps take the fused tail (its norms are fused with the int8 quantizers), and what undoes that."""
+    from rk_b200.gemma_stack import expert_scope, fuse_norm_quantize
+    from rk_b200.optimizations import quantize_linears
+
+    expert = small_expert(128)
+    context = quantize_linears(expert, "int8", scopes=("expert",), selector=expert_scope, shared_quant=True, grouped=True)
+    context.__enter__()
+    fuse_norm_quantize(expert.stack)
+    return expert, lambda: context.__exit__(None, None, None)
+
+
+def stepwise(expert, *inputs):
+    """The same call with a hook in place, which keeps every step in tensor ops."""
+    handle = expert.action_out_proj.register_forward_hook(lambda *a: None)
+    try:
+        assert not expert._fused_tail(inputs[0])
+        return expert(*inputs)
+    finally:
+        handle.remove()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["action_in_proj", "action_out_proj"])
+def test_weights_at_any_address(name):
+    """A projection whose weight is a view into a flat buffer, four bytes off."""
+    expert, undo = fused_step_expert()
+    inputs = draws(128, 2, 2)
+    with torch.no_grad():
+        assert expert._fused_tail(inputs[0])
+        linear = getattr(expert, name)
+        flat = torch.empty(linear.weight.numel() + 1, device=DEVICE)[1:].view_as(linear.weight)
+        linear.weight.data = flat.copy_(linear.weight)
+        assert linear.weight.data_ptr() % 16 and not expert._fused_tail(inputs[0])
+        assert torch.equal(expert(*inputs), stepwise(expert, *inputs))
+    undo()
