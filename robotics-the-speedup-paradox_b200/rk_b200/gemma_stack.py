@@ -501,7 +501,11 @@ class ActionExpert(nn.Module):
             if tokens is None:
                 tokens = self.action_in_proj(x_t).to(torch.bfloat16)
             stream, pending, _ = self.stack.run_layers(tokens, None, past=prefix_kv, cond=cond, rope=rope)
-            x_t, tokens = self._flow_step_tail(stream, pending, cond, x_t, dt, last=step + 1 == self.steps)
+            tail = self._flow_step_tail(stream, pending, cond, x_t, dt, last=step + 1 == self.steps)
+            if tail is None:
+                hidden, _, _ = self.stack.norm(stream, cond, pending)
+                tail = x_t + dt * self.action_out_proj(hidden.float()), None
+            x_t, tokens = tail
         return x_t
 
     def _fused_tail(self, noise):
@@ -517,6 +521,8 @@ class ActionExpert(nn.Module):
         if norm.dense is None or norm.fused_bits is not None or self.stack.layers[-1].post_attention_layernorm.fused_bits is None:
             return False
         if torch.is_grad_enabled() or forward_ad._current_level >= 0 or type(noise) is not torch.Tensor:
+            return False
+        if torch.is_autocast_enabled("cuda"):  # the projections and the modulation are the autocast type's then
             return False
         if noise.dtype != torch.float32 or not noise.is_cuda or not noise.is_contiguous():
             return False
@@ -539,6 +545,8 @@ class ActionExpert(nn.Module):
                 and width <= 2048 and dims % 4 == 0 and dims <= 64 and noise.shape[1] == self.chunk)
 
     def _flow_step_tail(self, stream, pending, cond, x_t, dt, last):
+        """(x of the next step, its input projection or None), or None where the kernel does not take the tensors: a modulation
+        that is not fp32 (cached under autocast), another batch, layers that return another type."""
         from . import _lib
 
         norm = self.stack.norm
@@ -546,7 +554,13 @@ class ActionExpert(nn.Module):
         scale, shift = project(cond)[:2]
         b, chunk, dims = x_t.shape
         branch, gate = pending if pending is not None else (None, None)
-        stream = stream.contiguous()
+        width = self.cfg.width
+        expected = ((stream, torch.bfloat16, (b, chunk, width)), (branch, torch.bfloat16, (b, chunk, width)),
+                    (gate, torch.bfloat16, (b, 1, width)), (scale, torch.float32, (b, 1, width)),
+                    (shift, torch.float32, (b, 1, width)), (x_t, torch.float32, (b, chunk, dims)))
+        if any(t is not None and (t.dtype != dtype or t.shape != shape or t.device != x_t.device) for t, dtype, shape in expected):
+            return None
+        stream, x_t = stream.contiguous(), x_t.contiguous()
         branch = branch.contiguous() if branch is not None else None
         gate = gate.contiguous() if gate is not None else None
         if scale.stride() != shift.stride() or scale.stride(-1) != 1 or scale.stride(0) % 4 or scale.data_ptr() % 16 \
@@ -558,8 +572,8 @@ class ActionExpert(nn.Module):
         with torch.cuda.device(stream.device):
             code = _lib.load().rk_flow_step_tail(
                 _lib.ptr(stream), _lib.ptr(branch), _lib.ptr(gate), _lib.ptr(scale), _lib.ptr(shift),
-                scale.stride(0) if b > 1 else max(scale.stride(0), stream.shape[-1]), chunk, b * chunk, stream.shape[-1],
-                norm.eps, _lib.ptr(w_out.weight), _lib.ptr(w_out.bias), dims, _lib.ptr(x_t), dt, _lib.ptr(w_in.weight),
+                scale.stride(0) if b > 1 else max(scale.stride(0), width), chunk, b * chunk, width, norm.eps,
+                _lib.ptr(w_out.weight), _lib.ptr(w_out.bias), dims, _lib.ptr(x_t), dt, _lib.ptr(w_in.weight),
                 _lib.ptr(w_in.bias), _lib.ptr(x_next), _lib.ptr(tokens), _lib.stream_ptr(stream.device))
         _lib.check(code, "rk_flow_step_tail")
         return x_next, tokens

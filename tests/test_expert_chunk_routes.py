@@ -78,3 +78,46 @@ def test_weights_at_any_address(name):
         assert linear.weight.data_ptr() % 16 and not expert._fused_tail(inputs[0])
         assert torch.equal(expert(*inputs), stepwise(expert, *inputs))
     undo()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cached", [False, True])
+def test_autocast_and_projections_cached_under_it(cached):
+    """Under autocast the projections and the modulation are bf16; a projection cache filled there keeps such rows."""
+    expert, undo = fused_step_expert()
+    inputs = draws(128, 2, 2)
+    with torch.no_grad():
+        if cached:
+            expert.enable_condition_caches()
+        with torch.autocast("cuda", torch.bfloat16):
+            assert not expert._fused_tail(inputs[0])
+            assert torch.equal(expert(*inputs), stepwise(expert, *inputs))
+        assert expert._fused_tail(inputs[0])
+        if cached:  # bf16 rows from the cache: refused tensor by tensor
+            assert expert.stack.norm.projection_cache(expert.condition(torch.ones(2, device=DEVICE), 0))[0].dtype == BF16
+            assert torch.equal(expert(*inputs), stepwise(expert, *inputs))
+    undo()
+
+
+@pytest.mark.parametrize("odd", ["scale_type", "scale_batch", "gate_batch", "stream_type", "branch_width", "x_type", None])
+def test_step_tail_leaves_other_tensors_to_the_tensor_ops(odd, monkeypatch):
+    """On the CPU: what the kernel does not take is refused before the library is called; what it takes reaches the library."""
+    from rk_b200 import _lib
+
+    cfg = GemmaConfig(width=64, mlp_dim=128, depth=1, num_heads=2, num_kv_heads=1, head_dim=32, adarms_cond_dim=64)
+    expert = ActionExpert(cfg, chunk=6, action_dim=8, steps=3).init_random(1).eval()
+    t = lambda *s, dtype=BF16: torch.zeros(s, dtype=dtype)
+    scale = t(1 if odd == "scale_batch" else 2, 1, 64, dtype=BF16 if odd == "scale_type" else torch.float32)
+    monkeypatch.setattr(expert.stack.norm, "modulation", lambda cond: (scale, t(2, 1, 64, dtype=torch.float32), None))
+    stream = t(2, 6, 64, dtype=torch.float32 if odd == "stream_type" else BF16)
+    pending = (t(2, 6, 32 if odd == "branch_width" else 64), t(1 if odd == "gate_batch" else 2, 1, 64))
+    reached = []
+    monkeypatch.setattr(_lib, "load", lambda: reached.append(1) or (_ for _ in ()).throw(RuntimeError("reached")))
+    monkeypatch.setattr(torch.cuda, "device", lambda device: torch.no_grad())
+    call = lambda: expert._flow_step_tail(stream, pending, None, t(2, 6, 8, dtype=torch.float64 if odd == "x_type" else torch.float32), -0.1, False)
+    if odd is None:
+        with pytest.raises(RuntimeError, match="reached"):
+            call()
+        assert reached
+    else:
+        assert call() is None and not reached
