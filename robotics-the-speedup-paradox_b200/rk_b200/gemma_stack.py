@@ -172,12 +172,24 @@ def rope_cache_update(q, k, v, cos, sin, k_all, v_all, prefix, heads, kv_heads, 
     return q_out.transpose(1, 2) if token_major else q_out
 
 
+def modes_active():
+    """Whether a dispatch mode or a torch-function mode other than a default device sees the tensor ops: a kernel that stands in
+    for some of them would be missing from what it records or rewrites."""
+    from torch.overrides import _get_current_function_mode_stack
+    from torch.utils._device import DeviceContext
+    from torch.utils._python_dispatch import _get_current_dispatch_mode_stack
+
+    return bool(_get_current_dispatch_mode_stack()) or any(type(m) is not DeviceContext for m in _get_current_function_mode_stack())
+
+
 def kv_prefix_fill(prefix_k, prefix_v, k_all, v_all, vt_all):
     """Copies a cached prefix into the working caches and transposes its values in one kernel (`rk_kv_prefix_fill`).  Returns
     False, with nothing done, for tensors that it does not take (other types, strides or devices, an empty prefix, one that
-    the copy has to broadcast)."""
+    the copy has to broadcast) and under dispatch or function modes."""
     from . import _lib
 
+    if modes_active():
+        return False
     tensors = (prefix_k, prefix_v, k_all, v_all, vt_all)
     device = prefix_k.device
     if any(type(t) is not torch.Tensor or t.dtype != torch.bfloat16 or t.device != device or not t.is_contiguous()
@@ -522,7 +534,7 @@ class ActionExpert(nn.Module):
             return False
         if torch.is_grad_enabled() or forward_ad._current_level >= 0 or type(noise) is not torch.Tensor:
             return False
-        if torch.is_autocast_enabled("cuda"):  # the projections and the modulation are the autocast type's then
+        if torch.is_autocast_enabled("cuda") or modes_active():  # under autocast the projections and the modulation are bf16
             return False
         if noise.dtype != torch.float32 or not noise.is_cuda or not noise.is_contiguous():
             return False

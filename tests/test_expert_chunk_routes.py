@@ -121,3 +121,47 @@ def test_step_tail_leaves_other_tensors_to_the_tensor_ops(odd, monkeypatch):
         assert reached
     else:
         assert call() is None and not reached
+
+
+class CountDispatch(torch.utils._python_dispatch.TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func)
+        return func(*args, **(kwargs or {}))
+
+
+class CountFunction(torch.overrides.TorchFunctionMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func)
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("mode", [CountDispatch, CountFunction])
+def test_prefix_fill_leaves_modes_to_the_tensor_ops(mode):
+    prefix, caches = torch.zeros(2, 4, 1, 8, 256, dtype=BF16), torch.zeros(2, 2, 4, 1, 16, 256, dtype=BF16)
+    with mode():
+        assert not kv_prefix_fill(prefix, prefix, caches[0], caches[1], torch.zeros(2, 4, 1, 256, 16, dtype=BF16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [CountDispatch, CountFunction])
+def test_modes_see_every_step(mode):
+    expert, undo = fused_step_expert()
+    inputs = draws(128, 2, 2)
+    with torch.no_grad():
+        with mode() as active:
+            assert not expert._fused_tail(inputs[0])
+            out = expert(*inputs)
+        linears = [f for f in active.seen if f in (torch.ops.aten.addmm.default, torch.nn.functional.linear)]
+        assert len(linears) >= 2 * 3  # both projections of three steps
+        assert torch.equal(out, stepwise(expert, *inputs))
+        with torch.device(DEVICE):  # a default device is no reason
+            assert expert._fused_tail(inputs[0])
+    undo()
