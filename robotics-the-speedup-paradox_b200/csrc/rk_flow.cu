@@ -55,7 +55,7 @@ flow_step_tail_kernel(const FlowParams p) {
     const long long lines = static_cast<long long>(p.k) * p.d / 32;  // 128-byte lines of each weight
     for (long long i = static_cast<long long>(blockIdx.x) * kFlowThreads + threadIdx.x; i < lines; i += static_cast<long long>(gridDim.x) * kFlowThreads) {
       asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w_out + i * 32));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w_in + i * 32));
+      if (p.tokens_out != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w_in + i * 32));  // the last step may come without
     }
   }
   pdl_wait();

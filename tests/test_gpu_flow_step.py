@@ -73,6 +73,21 @@ def test_flow_step_tail_refuses_bad_arguments():
     assert call(d=68) == _lib.RK_EUNSUPPORTED
 
 
+def test_the_last_step_needs_no_input_projection():
+    """Without an output for the next step's tokens the input projection may be null; the result keeps its bits."""
+    gen = torch.Generator(device=DEVICE).manual_seed(0)
+    r = lambda *s: torch.randn(s, generator=gen, device=DEVICE)
+    x, modulation, w_out, b_out, x_t, w_in, b_in = r(50, 1024).bfloat16(), r(2, 1024), r(32, 1024), r(32), r(50, 32), r(1024, 32), r(1024)
+    P, results = _lib.ptr, []
+    for tokens, w, b in ((torch.empty_like(x), w_in, b_in), (None, None, None)):
+        x_next = torch.empty_like(x_t)
+        code = _lib.load().rk_flow_step_tail(P(x), None, None, P(modulation[0]), P(modulation[1]), 1024, 50, 50, 1024, 1e-6, P(w_out),
+                                             P(b_out), 32, P(x_t), -0.1, P(w), P(b), P(x_next), P(tokens), _lib.stream_ptr(DEVICE))
+        _lib.check(code, "rk_flow_step_tail")
+        results.append(x_next)
+    assert torch.equal(*results)
+
+
 def test_expert_loop_with_the_fused_step_tail_equals_the_stepwise_loop():
     """`ActionExpert.forward` against its own `denoise_step` loop (which a hook keeps in place), with fused norms."""
     from rk_b200.gemma_stack import ActionExpert, GemmaConfig, expert_scope, fuse_norm_quantize
