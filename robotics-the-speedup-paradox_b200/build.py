@@ -125,7 +125,12 @@ def main():
     if args.arch != "10.0a":
         parser.error("these kernels use tcgen05 / TMEM and build for 10.0a only")
     print(build(args.arch, args.build_dir, args.output, args.verbose, args.force))
-    print(build_host_calls(args.build_dir, args.force))
+    try:
+        import torch  # noqa: F401
+    except ImportError:
+        print("no torch here: the library alone; rk_b200/_host_calls.so (native eager calls of the Python package) is not built")
+    else:
+        print(build_host_calls(args.build_dir, args.force))
 
 
 if __name__ == "__main__":

@@ -186,7 +186,7 @@ def integer_gemm(a, sa, b, sb, bias, bits, tactic, residual=None, gate=None):
 
 def _native(state, x):
     global _native
-    _native = _lib.host_calls().integer_linear  # from the second call on
+    _native = _lib.native_call("integer_linear")  # from the second call on
     return _native(state, x)
 
 

@@ -53,7 +53,7 @@ def linear_w4a16(x, packed, scales, bias=None, tactic=0):
 
 def _native(state, x):
     global _native
-    _native = _lib.host_calls().w4a16_linear  # from the second call on
+    _native = _lib.native_call("w4a16_linear")  # from the second call on
     return _native(state, x)
 
 

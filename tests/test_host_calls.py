@@ -110,3 +110,38 @@ def test_replaced_methods_stay_in_charge():
 
     sub = Sub(layer.packed_weight, layer.weight_scale, layer.bias, 128, 64, 8)
     assert torch.equal(sub(x), want) and calls == [1, 2]
+
+
+WITHOUT_MODULE = """
+import sys, warnings
+sys.path.insert(0, {package!r})
+sys.modules["rk_b200._host_calls"] = None  # as if the file were missing
+import torch
+from rk_b200.integer import IntegerLinear
+from rk_b200.w4a16_linear import W4A16Linear
+x = torch.zeros(2, 128, dtype=torch.bfloat16)
+layers = [(IntegerLinear(torch.zeros(8, 128, dtype=torch.int8), torch.ones(8), None, 128, 8, 8), "Expected CUDA BF16 rows"),
+          (IntegerLinear(torch.zeros(8, 64, dtype=torch.uint8), torch.ones(8), None, 128, 8, 4), "Expected CUDA BF16 rows"),
+          (W4A16Linear(torch.zeros(8, 64, dtype=torch.uint8), torch.ones(1, 8, dtype=torch.bfloat16), None, 128, 8), "requires a contiguous CUDA")]
+with warnings.catch_warnings(record=True) as told:
+    warnings.simplefilter("always")
+    for layer, message in layers * 2:
+        try:
+            layer(x)
+        except ValueError as error:
+            assert message in str(error), error
+        else:
+            raise AssertionError("no error")
+assert [w.category for w in told] == [RuntimeWarning] * 2, told  # once for each kind of layer
+"""
+
+
+def test_without_the_native_module_the_general_path_serves_the_call():
+    """On the CPU the general path says what it needs."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    script = WITHOUT_MODULE.format(package=str(Path(_lib.__file__).resolve().parents[1]))
+    done = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
