@@ -4,7 +4,8 @@
 //
 // A call here takes the plain case only - exact CUDA tensors, contiguous rows, a workspace that exists, no dispatch mode - and
 // answers None for everything else, errors included: the caller then goes its general way in Python, which repeats the
-// checks and raises what it always raised.  Nothing is queued before all checks have passed, nothing is kept between calls.
+// checks and raises what it always raised.  Nothing is queued before all checks of arguments have passed (an error of the device
+// itself can still come between the two launches), nothing is kept between calls.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -176,7 +177,10 @@ PyObject* integer_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const void *px = x->data_ptr(), *pw = layer.weight->data_ptr();
     const float* ps = layer.scale->const_data_ptr<float>();
     const void* pb = layer.bias != nullptr ? layer.bias->data_ptr() : nullptr;
-    if (!aligned16(px) || !aligned16(pw)) Py_RETURN_NONE;
+    // what rk_gemm_int would refuse, so that no quantizer is queued for a call that the general path then repeats
+    if (!aligned16(px) || !aligned16(pw) || !aligned16(ws) || ws_bytes < RK_WORKSPACE_HEADER || layer.tactic > 7 || n % 8 != 0 ||
+        m > (1 << 24) || n > (1 << 24))
+      Py_RETURN_NONE;
     // owned until the launch: another thread may replace the module's buffers while the interpreter lock is released
     const at::Tensor weight = *layer.weight, scale = *layer.scale, bias = layer.bias != nullptr ? *layer.bias : at::Tensor();
     c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());

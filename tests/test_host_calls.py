@@ -95,6 +95,19 @@ def test_native_calls_equal_the_general_path(kind, n, k, bias):
 
 
 @pytest.mark.gpu
+def test_a_call_that_the_gemm_refuses_queues_nothing():
+    layer = make("integer", 64, 128, False)
+    x = torch.randn(4, 128, device=DEVICE).bfloat16()
+    assert layer(x) is not None
+    layer.tactic = 9
+    count = lambda: torch.cuda.memory_stats(DEVICE)["allocation.all.allocated"]  # the row codes come first
+    before = count()
+    assert _lib.host_calls().integer_linear(layer.__dict__, x) is None and count() == before
+    with pytest.raises(RuntimeError, match="tactic"):
+        layer(x)
+
+
+@pytest.mark.gpu
 def test_replaced_methods_stay_in_charge():
     layer = make("integer", 64, 128, False)
     x = torch.randn(4, 128, device=DEVICE).bfloat16()
