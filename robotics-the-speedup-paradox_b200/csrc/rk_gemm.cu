@@ -1626,7 +1626,6 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
     // CTAs of sixteen warps where a tile wants them all, where two CTAs' activations do not fit, or two fragments meet a long K
     // (8192 x 2048, 16 rows: 6.4 us against 7.0; 1024 x 1024: 3.3 against 3.0)
     const bool wide = g.share == 16 || gemv_smem(g.m, g.k, tiles8, 8) > gemv_smem_limit(8) || (tiles8 == 2 && g.k >= 2048);
-    if (!wide && g.share > 8) g.share = 8;
     if (gemv_smem(g.m, g.k, tiles8, wide ? 16 : 8) <= gemv_smem_limit(wide ? 16 : 8)) {
       cudaStream_t st = as_stream(stream);
       if (wide) return tiles8 == 1 ? launch_gemv<1, 16>(g, st) : launch_gemv<2, 16>(g, st);
