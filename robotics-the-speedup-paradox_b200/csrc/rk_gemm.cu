@@ -280,10 +280,8 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
     const int q = (block_scaled || chunks > 1) ? 32 : 16;
     int bn = static_cast<int>(round_up((m + chunks - 1) / chunks, q));
     if ((tactic & 4) && bn >= 64 && !block_scaled) bn = static_cast<int>(round_up(bn / 2, 32));
-    // A CTA's K loop runs at the pace of its issuing threads (a few hundred cycles per K block whatever
-    // the tile width), so while the machine is not full, narrower activation chunks - more CTAs, each
-    // with the same loop - beat both wide tiles and split-K (whose exchange costs more than it saves
-    // unless the tiles are very few).
+    // While the machine is not full, narrower activation chunks - more CTAs - beat both wide tiles and split-K (whose exchange
+    // costs more than it saves unless the tiles are very few).
     if (kind == KIND_I8 && !(tactic & 4) && n <= 128 * kNumSms) {
       // With two issuing warps the loop runs at the rate at which an SM takes operands from L2, (128 + bn) x 128 bytes a block:
       // as many chunks as there are SMs, of 32 rows at least (400 x 1024 x 2048 5.4 us with chunks of 64 rows, 4.9 of 32; 400 x
@@ -291,6 +289,7 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
       const int64_t fit = kNumSms / ((n + 127) / 128);
       bn = std::min(bn, static_cast<int>(round_up((m + fit - 1) / fit, 32)));
     } else if (!block_scaled && !(tactic & 4) && bn >= 64) {
+      // One issuing warp: a CTA's K loop runs at its pace, a few hundred cycles per K block whatever the tile width.
       const int64_t tiles_a = (n + 127) / 128;
       const int half = static_cast<int>(round_up(bn / 2, 32));
       if (tiles_a * ((m + half - 1) / half) <= kNumSms) {
@@ -365,8 +364,15 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
       pl.dual = 0;
     }
   }
-  // more than half of an SM's, for the reason given in few_rows_plan (chains of short loops: 816 x 2560 x 256 W8A8 6.0 -> 5.0 us)
-  pl.smem_bytes = std::max(pl.stages * stage + pl.out_bufs * kOutBufBytes + kVecBytes + 1024, 118 * 1024);
+  // More than half of an SM's, for the reason given in few_rows_plan; it adds to launches of at most two or three stages (K of
+  // 512 bytes or less).  Chains of one stream without -> with it: W8A8 640 x 4096 x 256 8.6 -> 4.9 us, FP8 64 x 2048 x 256 3.3 -> 2.9,
+  // 400 x 4096 x 128 4.9 -> 3.9, MXFP8 200 x 8192 x 256 8.3 -> 5.0 (behind its packer 9.2 -> 6.2), NVFP4 200 x 8192 x 512 8.4 -> 5.0.
+  // The price: such launches of two streams no longer share an SM.  A pair of them, of at most half the SMs each, gains all the
+  // same (FP8 64 x 2048 x 256 3.1 -> 2.9 us, MXFP8 4.1 -> 3.8); of more it loses (FP8 400 x 4096 x 128 4.9 -> 6.6 and 6.6 -> 7.1 with
+  // quantizers, MXFP8 64 x 16384 x 256 4.9 -> 7.3 and 6.3 -> 7.7, W8A8 640 x 4096 x 256 7.4 -> 8.3 and 10.6 -> 9.6), but two launches a
+  // stream apart still take less than one after the other.  Not for the rewriting kinds, where it changes nothing or loses (W4A4
+  // 64 x 2048 x 256 behind its quantizer 7.8 -> 8.0).
+  pl.smem_bytes = std::max(pl.stages * stage + pl.out_bufs * kOutBufBytes + kVecBytes + 1024, rewriting ? 0 : 118 * 1024);
   pl.grid_x = pl.splits > 1 ? static_cast<int>(tiles) : static_cast<int>(tiles < kNumSms ? tiles : kNumSms);
   return pl;
 }
