@@ -562,6 +562,21 @@ int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CU
   return RK_OK;
 }
 
+// The order of the pair tiles (see pair_tile): rows of tiles where all run at once, columns in a single group of at most eight row
+// tiles, both with a multiplication in place of the division; else equal groups of at most eight row tiles.
+void set_pair_order(Gemm2Params* p) {
+  const int groups = (p->tiles_m + 7) / 8;
+  p->group_m = (p->tiles_m + groups - 1) / groups;
+  const bool one_wave = static_cast<long long>(p->tiles_m) * p->tiles_n <= kNumSms / 2;
+  p->order = one_wave && p->tiles_n > 1 ? PAIRS_COLUMNS_FIRST : groups == 1 ? PAIRS_ROWS_FIRST : PAIRS_GROUPS;
+  if (p->order == PAIRS_GROUPS) return;
+  p->minor = p->order == PAIRS_COLUMNS_FIRST ? p->tiles_n : p->tiles_m;
+  // exact while tiles * minor < 2^32: 74 * 74 and 8 * 2^17 * 8 at most.  A single row tile has no such factor for its minor of one:
+  // the columns run alone then, and a factor of zero gives row zero.
+  if (p->minor == 1) p->order = PAIRS_COLUMNS_FIRST, p->minor = p->tiles_n;
+  p->minor_magic = p->tiles_m > 1 ? static_cast<unsigned>(((1ull << 32) + p->minor - 1) / p->minor) : 0u;
+}
+
 template <int KIND>
 int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
                const CUtensorMap& tm_sfb, const CUtensorMap& tm_tail, const Gemm2Params& p, int smem, cudaStream_t st) {
@@ -721,8 +736,7 @@ int run_tc(const TcArgs& a) {
     p2.issue_block = issue_block_mode();
     p2.tiles_m = static_cast<int>((a.m + 255) / 256);
     p2.tiles_n = static_cast<int>((a.n + p2.bn - 1) / p2.bn);
-    const int groups = (p2.tiles_m + 7) / 8;  // equal groups of at most eight row tiles
-    p2.group_m = (p2.tiles_m + groups - 1) / groups;
+    set_pair_order(&p2);
     const int stage = gemm2_stage_bytes(a.kind, p2.bn, p2.sfb_blocks);
     p2.out_bufs = 2;
     p2.stages = (kSmemBudget - kVecBytes - 2 * kOutBufBytes) / stage;

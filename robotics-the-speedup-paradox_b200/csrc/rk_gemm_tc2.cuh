@@ -74,6 +74,9 @@ struct Gemm2Params {
   int sw_mode;
   int tiles_m, tiles_n;  // pair tiles: 256 x bn
   int group_m;           // row tiles of a group, see pair_tile
+  int order;             // PairOrder
+  int minor;             // tiles of the dimension that runs first (not PAIRS_GROUPS)
+  unsigned minor_magic;  // ceil(2^32 / minor); the number of tiles times `minor` is below 2^32
   long long ldo;
   const float* scale_act;
   const float* scale_wgt;
@@ -84,13 +87,20 @@ struct Gemm2Params {
 
 // Tiles are taken group by group (p.group_m row tiles of 256 activation rows), inside a group column by column: the pairs that
 // run at once share few weight columns and the activations of one group, so that both come from L2 and the weights from HBM
-// once per group.   With all column
-// tiles of one row tile first, the weights (more than a die's L2 at these widths) came anew for every row tile: 816 x 32768 x
-// 2048 MXFP8 SwiGLU 67.6 -> 57.7 us, 3264 rows 221 -> 180, 4096 x 8192 x 8192 W8A8 200 -> 169 (4 row tiles 181, 16 165).
+// once per group.  With all column tiles of one row tile first, the weights (more than a die's L2 at these widths) came anew
+// for every row tile: 816 x 32768 x 2048 MXFP8 SwiGLU 67.6 -> 57.7 us, 3264 rows 221 -> 180, 4096 x 8192 x 8192 W8A8 200 -> 169 (4
+// row tiles 181, 16 165).  Up to 74 tiles all run at once: row tiles stay outermost.
+// Every role works its first tile out before it can start, and two divisions for it showed in short launches (W8A8 1100 x 1024 x
+// 1024 5.3 -> 5.7 us, MXFP8 816 x 2048 x 2048 8.0 -> 8.3).  One wave and a single group take a multiplication: 5.3, 8.1.
+enum PairOrder : int { PAIRS_GROUPS, PAIRS_COLUMNS_FIRST, PAIRS_ROWS_FIRST };
 struct PairTile {
   int m, n;  // row tile, column tile
 };
 __device__ __forceinline__ PairTile pair_tile(const Gemm2Params& p, int tile) {
+  if (p.order != PAIRS_GROUPS) {
+    const int major = static_cast<int>(__umulhi(static_cast<unsigned>(tile), p.minor_magic)), rest = tile - major * p.minor;
+    return p.order == PAIRS_ROWS_FIRST ? PairTile{rest, major} : PairTile{major, rest};
+  }
   const int per_group = p.group_m * p.tiles_n;
   const int first = tile / per_group * p.group_m;
   const int rows = min(p.group_m, p.tiles_m - first);

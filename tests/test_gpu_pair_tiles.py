@@ -26,6 +26,33 @@ def test_every_tile_of_every_group_is_computed_once(m, n, k):
     assert torch.equal(got, want.float().bfloat16())
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (1100, 1024, 128),   # at most 74 tiles: row tiles outermost
+    (1025, 128, 128),    # one column of five tiles
+    (2048, 9480, 128),   # eight row tiles, more tiles than pairs: columns outermost
+    (1281, 16392, 128),  # six: a factor that does not divide 2^32
+    (20000, 136, 128),   # 79 row tiles: groups
+])
+def test_every_tile_of_every_order_is_computed_once(m, n, k):
+    test_every_tile_of_every_group_is_computed_once(m, n, k)
+
+
+@pytest.mark.parametrize("m,n", [(64, 128), (200, 1024), (129, 25600), (257, 20480)])
+def test_one_and_two_row_tiles_of_the_repacking_gemm(m, n):
+    """One row tile with one, few and more column tiles than pairs; two row tiles with more than pairs."""
+    from rk_b200 import fp4_linear as P4
+
+    k, inter = 256, n // 2
+    gen = torch.Generator(device=DEVICE).manual_seed(m + n)
+    x = torch.randn(m, k, generator=gen, device=DEVICE).bfloat16()
+    qa, sfa = P4.pack_nvfp4(x)
+    qi, sfi = P4.pack_nvfp4(P4.interleave_gate_up_rows((torch.randn(n, k, generator=gen, device=DEVICE) * 0.05).bfloat16(), inter))
+    plain = P4.linear_forward_packed_gemm_bf16(qa, sfa, None, qi, sfi, None, None, k)
+    want_q, want_sf = P4.pack_swiglu_nvfp4(plain, inter, interleaved=True)
+    got_q, got_sf = P4.linear_swiglu_packed_gemm(qa, sfa, None, qi, sfi, None, k)
+    assert torch.equal(got_q, want_q) and torch.equal(got_sf, want_sf)
+
+
 @pytest.mark.parametrize("m,n", [(1300, 4992), (816, 16512), (2100, 4992)])
 def test_repacking_epilogues_in_256_column_tiles(m, n):
     """Sizes whose tiles are 256 columns wide (2048-wide rows, several rounds of the pairs), 128 of them in the last tile for NVFP4:
