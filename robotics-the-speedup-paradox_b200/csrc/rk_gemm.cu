@@ -234,9 +234,10 @@ int max_clusters(int size) {
   return entry;
 }
 
+// `residual`: the epilogue with the residual, whose kernels have one issuing warp (outside the few-row form).
 // `tactic` only nudges the shape of the decomposition (it can never change integer results and
 // only reorders fp32 partial sums): bit 0 forbids swap, bit 1 forbids split-K, bit 2 halves bn.
-Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
+Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic, bool residual = false) {
   Plan pl{};
   const bool block_scaled = kind == KIND_MXF8 || kind == KIND_NVF4;
   // Weights on the 128-lane axis whenever the activation row count fits one or a few
@@ -282,7 +283,7 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
     if ((tactic & 4) && bn >= 64 && !block_scaled) bn = static_cast<int>(round_up(bn / 2, 32));
     // While the machine is not full, narrower activation chunks - more CTAs - beat both wide tiles and split-K (whose exchange
     // costs more than it saves unless the tiles are very few).
-    if (kind == KIND_I8 && !(tactic & 4) && n <= 128 * kNumSms) {
+    if (kind == KIND_I8 && !residual && !(tactic & 4) && n <= 128 * kNumSms) {
       // With two issuing warps the loop runs at the rate at which an SM takes operands from L2, (128 + bn) x 128 bytes a block:
       // as many chunks as there are SMs, of 32 rows at least (400 x 1024 x 2048 5.4 us with chunks of 64 rows, 4.9 of 32; 400 x
       // 1024 x 4096 7.7 and 7.0; 816 x 2048 x 2048 7.5 of 128, 7.1 of 96; 600 x 2048 x 2048 7.3 of 128, 6.8 of 96).
@@ -354,7 +355,7 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
   // (Not above 128 rows: four MMAs take longer than issuing them, and the epilogue reads twice: 400 x 8192 x 1024 8.2 -> 8.4 us.)
   // The issuing warp paced the loop with five tensor-core instructions a block, 50 to 60 cycles each: 816 x 2048 x 16384 35.5 ->
   // 28.5 us, 50 x 1024 x 2048 5.5 -> 4.7, 400 x 1024 x 4096 8.7 -> 7.7; chunk of one environment 9.00 -> 8.77 ms.
-  pl.dual = kind == KIND_I8 && pl.bn <= 128 && pl.acc_bufs == 2 && (pl.splits > 1 || tiles <= kNumSms) && kb_per_cta >= 2 ? 1 : 0;
+  pl.dual = kind == KIND_I8 && !residual && pl.bn <= 128 && pl.acc_bufs == 2 && (pl.splits > 1 || tiles <= kNumSms) && kb_per_cta >= 2 ? 1 : 0;
   if (pl.dual && pl.stages < kb_per_cta && pl.stages % 2 != 0) {
     if (pl.out_bufs == 2 && pl.stages < kMaxStages && (pl.stages + 1) * stage <= budget + kOutBufBytes) {
       pl.out_bufs = 1, ++pl.stages;
@@ -394,6 +395,8 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic) {
 // 4.6, 600 x 1024 x 2048 5.6 -> 5.0, 816 x 1024 x 512 4.1 -> 3.8.  Not where a block has more operand rows than `pl`'s (816 x
 // 2048 x 2048 6.9 against 7.2) or tiles are wide (300 x 8192 x 1024 6.8 and 7.4), nor above 256 rows for a long loop (400 x 2048 x
 // 8192 12.8 and 13.5, 816 rows 16.0 and 18.0; 200 rows 11.6 -> 10.1).
+// A residual is read along the rows, 16 bytes a load (2 bytes a load cost wide tiles more than the layout gains: 1000 x 2048 x 2048
+// 11.4 -> 17.8 us; now 9.9); `pl` is then the plan without the second issuing warp.
 Plan few_rows_plan(const Plan& pl, int64_t m, int64_t n, int kblocks, int tactic) {
   if (m > 1024) return pl;  // nothing above is taken, and from 149 row tiles on no SM would be left for the columns (fit = 0)
   const int64_t tiles_a = (m + 127) / 128, rows = round_up((m + tiles_a - 1) / tiles_a, 8), fit = kNumSms / tiles_a;
@@ -799,7 +802,7 @@ int run_tc(const TcArgs& a) {
       default: return launch_tc2<KIND_NVF4>(t_act, t_wgt, t_out, t_sfa, t_sfb, t_tail, p2, smem, a.stream);
     }
   }
-  Plan pl = make_plan(a.kind, a.m, a.n, kblocks, a.tactic);
+  Plan pl = make_plan(a.kind, a.m, a.n, kblocks, a.tactic, a.residual != nullptr);
   if (a.kind == KIND_I8 && a.acc_out == nullptr && a.peer == nullptr && a.k_bytes % kStageKBytes == 0) pl = few_rows_plan(pl, a.m, a.n, kblocks, a.tactic);
 
   CUtensorMap tm_act, tm_wgt, tm_out;

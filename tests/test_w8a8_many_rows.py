@@ -66,3 +66,30 @@ def test_many_rows_give_the_exact_product(m, n, bits, form):
     want = y if residual is None else residual + y
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     assert _lib.read_status(_lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(1, 64, 256), (50, 8192, 256), (128, 2568, 128), (300, 2560, 512), (816, 2056, 384), (1000, 2048, 256),
+                                   (1024, 520, 128)])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("gated", [False, True])
+def test_residual_rows_are_read_at_any_address(m, n, k, offset, gated):
+    """Narrow, wide and ragged column tiles, one to eight row tiles; residual and gate on a 16-byte boundary or two bytes off."""
+    gen = torch.Generator(device=DEVICE).manual_seed(m + n + offset)
+    a, b = (torch.randint(-127, 128, (r, k), generator=gen, device=DEVICE, dtype=torch.int8) for r in (m, n))
+    sa, sb = (torch.rand(r, generator=gen, device=DEVICE) * 2.0 ** -5 + 2.0 ** -8 for r in (m, n))
+    at = lambda rows: torch.randn(rows * n + offset, generator=gen, device=DEVICE).bfloat16()[offset:].view(rows, n)
+    batches = next(c for c in (4, 3, 2, 1) if m % c == 0)
+    residual, gate = at(m), at(batches) if gated else None
+    out = torch.full((m + 2, n), 7.0, device=DEVICE, dtype=torch.bfloat16)
+    ws = _lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)
+    P = _lib.ptr
+    code = _lib.load().rk_gemm_int_residual(P(a), P(sa), P(b), P(sb), None, P(residual), P(gate), m // batches if gated else 1, P(out[1:]),
+                                            m, n, k, 8, 0, P(ws), ws.numel(), _lib.stream_ptr(DEVICE))
+    _lib.check(code, "rk_gemm_int_residual")
+    y = ((a.double() @ b.double().T).float() * sa[:, None] * sb).bfloat16()
+    if gated:
+        y = y * gate.repeat_interleave(m // batches, 0)
+    assert torch.equal(out[1:m + 1].view(torch.int16), (residual + y).view(torch.int16))
+    assert (out[0] == 7.0).all() and (out[m + 1] == 7.0).all()
+    assert _lib.read_status(ws) == 0
