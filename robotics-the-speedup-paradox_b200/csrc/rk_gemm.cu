@@ -399,7 +399,9 @@ Plan make_plan(int kind, int64_t m, int64_t n, int kblocks, int tactic, bool res
 // 11.4 -> 17.8 us; now 9.9); `pl` is then the plan without the second issuing warp.
 Plan few_rows_plan(const Plan& pl, int64_t m, int64_t n, int kblocks, int tactic) {
   if (m > 1024) return pl;  // nothing above is taken, and from 149 row tiles on no SM would be left for the columns (fit = 0)
-  const int64_t tiles_a = (m + 127) / 128, rows = round_up((m + tiles_a - 1) / tiles_a, 8), fit = kNumSms / tiles_a;
+  // 65 to 128 rows of a long loop: two row tiles and columns twice as wide, a block has fewer operand rows (128 x 2048 x 8192 10.1 us
+  // with one, 8.4 with two; 9.3 in the plan that splits K)
+  const int64_t tiles_a = m > 64 && m <= 128 && kblocks > 32 ? 2 : (m + 127) / 128, rows = round_up((m + tiles_a - 1) / tiles_a, 8), fit = kNumSms / tiles_a;
   const int bn = static_cast<int>(round_up((n + fit - 1) / fit, 16));
   if ((tactic & 5) || bn > std::min(128, pow2_at_least(static_cast<int>(m), 16)) || pl.splits > (kblocks <= 32 ? 6 : 1)) return pl;
   if (m > 128 && (!pl.swap || rows + bn > kTileA + pl.bn || (m > 256 && kblocks > 32))) return pl;

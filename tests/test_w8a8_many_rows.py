@@ -93,3 +93,20 @@ def test_residual_rows_are_read_at_any_address(m, n, k, offset, gated):
     assert torch.equal(out[1:m + 1].view(torch.int16), (residual + y).view(torch.int16))
     assert (out[0] == 7.0).all() and (out[m + 1] == 7.0).all()
     assert _lib.read_status(ws) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(64, 520, 4224), (65, 2048, 4224), (72, 72, 8192), (100, 1032, 4352), (128, 2048, 4224), (129, 264, 4224)])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_two_row_tiles_of_a_long_loop(m, n, k, with_residual):
+    """65 to 128 rows and more than 32 K blocks: two row tiles, even and odd; the rows on either side of the range."""
+    from rk_b200.integer import integer_gemm
+
+    gen = torch.Generator(device=DEVICE).manual_seed(m + n + k)
+    a, b = (torch.randint(-15, 16, (r, k), generator=gen, device=DEVICE, dtype=torch.int8) for r in (m, n))
+    sa, sb = (torch.rand(r, generator=gen, device=DEVICE) * 2.0 ** -5 + 2.0 ** -8 for r in (m, n))
+    residual = torch.randn(m, n, generator=gen, device=DEVICE).bfloat16() if with_residual else None
+    y = ((a.double() @ b.double().T).float() * sa[:, None] * sb).bfloat16()  # whole numbers below 2^21
+    got = integer_gemm(a, sa, b, sb, None, 8, 0, residual=residual)
+    assert torch.equal(got.view(torch.int16), (y if residual is None else residual + y).view(torch.int16))
+    assert _lib.read_status(_lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)) == 0
