@@ -586,7 +586,9 @@ template <int KIND>
 int launch_tc2(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_out, const CUtensorMap& tm_sfa,
                const CUtensorMap& tm_sfb, const CUtensorMap& tm_tail, const Gemm2Params& p, int smem, cudaStream_t st) {
   if constexpr (KIND == KIND_MXF8 || KIND == KIND_NVF4) {
-    if (p.sw_q != nullptr) return launch_tc2_kernel<KIND, true, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
+    if (p.sw_q != nullptr)
+      return p.bn == 256 ? launch_tc2_kernel<KIND, true, true>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st)
+                         : launch_tc2_kernel<KIND, true, false>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);
   }
   if constexpr (KIND == KIND_I8 || KIND == KIND_F8) {
     if (p.bn % 64 != 0) return launch_tc2_kernel<KIND, false, true>(tm_a, tm_b, tm_out, tm_sfa, tm_sfb, tm_tail, p, smem, st);

@@ -199,7 +199,7 @@ __host__ __device__ inline int gemm2_stage_bytes(int kind, int bn, int sfb_block
   return ((kTileA + bn / 2) * kStageKBytes + chunks * 512 * (1 + sfb_blocks) + 1023) / 1024 * 1024;
 }
 
-// REPACK: the epilogues that never write the bf16 tile (sw_q set), on sixteen warps.
+// REPACK: the epilogues that never write the bf16 tile (sw_q set), on sixteen warps; tiles of 128 columns, or of 256 (TAIL).
 // TAIL: tiles whose width is not a multiple of 64 (W8A8 and FP8), a form of its own because the choice in every chunk costs the
 // others up to 8 % (FP8 2304 x 8192 x 512 16.3 -> 15.2 us, W8A8 19.2 -> 18.4).
 template <int KIND, bool REPACK, bool TAIL>
@@ -497,9 +497,10 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         const int rows_sf = (p.m + 127) & ~127;  // the scale buffer covers whole 128-row blocks; padding rows get zeros
         // This thread's 16 up and 16 gate values of every 128-column group, rounded to bf16, into registers first: the
         // accumulator goes back before the arithmetic, so that a tile of 256 columns needs no second one.
-        uint32_t ups[2][8], gates[2][8];
+        constexpr int kGroups = TAIL ? 2 : 1;  // of 128 columns
+        uint32_t ups[kGroups][8], gates[kGroups][8];
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
+        for (int g = 0; g < kGroups; ++g) {
           if (g * 128 >= p.bn) continue;
           uint32_t ru[16], rg[16];
           __syncwarp();
@@ -509,15 +510,20 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
 #pragma unroll
           for (int j = 0; j < 8; ++j) ups[g][j] = scaled_pair(ru, j), gates[g][j] = scaled_pair(rg, j);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
+        auto hand_back = [&] {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(ab == 0 ? acc_empty_leader0 : acc_empty_leader1);
+        };
+        // a 128-column tile has the other accumulator beside it, and the table look-ups start sooner without the barrier
+        // (1764 x 8192 x 512 16.3 -> 15.8 us)
+        if (TAIL || KIND != KIND_NVF4 || p.sw_mode != 2) hand_back();
         if (p.sw_mode == 2) {
           // ---- the activation itself as bf16 (the arithmetic of the table mode of the row quantizers) + its maximum
           __nv_bfloat16* const prod = reinterpret_cast<__nv_bfloat16*>(p.sw_q);
           uint32_t amax = 0u;  // bits of a bf16 magnitude
 #pragma unroll
-          for (int g = 0; g < 2; ++g) {
+          for (int g = 0; g < kGroups; ++g) {
             if (g * 128 >= p.bn) continue;
             const uint32_t amax_before = amax;
             const int col0 = row_b0 + g * 128;
@@ -539,6 +545,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
               dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
             }
           }
+          if (!TAIL) hand_back();
           if (p.sw_sf != nullptr) {
             amax = __reduce_max_sync(0xffffffffu, amax);
             if (lane == 0 && ok && amax != 0u) atomicMax(&sw_amax_bits, amax << 16);
@@ -551,7 +558,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           // [2 parities][4 sets][128 rows]: magnitude bits of the larger value, bit 31 set when one is not finite
           uint32_t* const part = reinterpret_cast<uint32_t*>(smem_gen + out_stage_off);
 #pragma unroll
-          for (int g = 0; g < 2; ++g) {
+          for (int g = 0; g < kGroups; ++g) {
             if (g * 128 >= p.bn) continue;
             const int col0 = row_b0 + g * 128;
             const int ch0 = col0 >> 1;
@@ -590,7 +597,7 @@ rk_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           continue;
         }
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
+        for (int g = 0; g < kGroups; ++g) {
           if (g * 128 >= p.bn) continue;
           const int col0 = row_b0 + g * 128;  // first output column of this 128-column group
           const int ch0 = col0 >> 1;          // first activation channel of the group
