@@ -729,10 +729,19 @@ int run_tc(const TcArgs& a) {
         const int64_t stage = issue > pipe ? issue : pipe;
         const int64_t tiles = tiles_m * ((a.n + bn - 1) / bn);
         const int64_t rounds = (tiles + kNumSms / 2 - 1) / (kNumSms / 2);
-        // exposed after every tile without a second buffer, else after the last; the re-packing epilogues hand the accumulator
-        // back as soon as they hold it in registers (128 -> 256 columns: 816 x 32768 x 2048 NVFP4 43 -> 32 us, MXFP8 79 -> 67)
-        const int64_t epilogue = a.swiglu_q != nullptr && bn == 256 ? 1000 : 10 * bn;
-        const int64_t cost = rounds * (kblocks * stage + (bn == 256 ? epilogue : 0)) + (bn == 256 ? 0 : epilogue);
+        // exposed after every tile without a second buffer, else after the last
+        const int64_t epilogue = 10 * bn;
+        int64_t cost = rounds * (kblocks * stage + (bn == 256 ? epilogue : 0)) + (bn == 256 ? 0 : epilogue);
+        if (a.swiglu_q != nullptr) {
+          // The re-packing epilogues hand the accumulator back as soon as they hold it in registers, so that a round takes the
+          // longer of main loop and epilogue; cycles from 1 to 12 rounds of K = 256 to 8192.  128 -> 256 columns: 816 x 32768 x 2048
+          // NVFP4 43 -> 32 us, MXFP8 79 -> 67; with a short K the epilogue decides, and 256 columns take twice as long for it:
+          // NVFP4 128 x 4096 x 256 4.8 us against 6.5, 600 x 8192 x 1024 10.2 and 11.8, with the table 9.7 and 11.9.
+          const bool nv = a.kind == KIND_NVF4;
+          const int64_t loop = kblocks * (bn == 256 ? (nv ? 1050 : 735) : (nv ? 730 : 605));
+          const int64_t repack = bn == 256 ? (nv ? 7200 : 5400) : (nv ? 3150 + loop / 4 : 2375 + loop * 31 / 100);
+          cost = rounds * (loop > repack ? loop : repack) + (bn == 256 ? 1200 : 0);
+        }
         if (best < 0 || cost < best) best = cost, p2.bn = bn;
       }
       if (bn_env == 128 || bn_env == 192 || bn_env == 256) p2.bn = bn_env;

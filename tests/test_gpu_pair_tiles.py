@@ -1,6 +1,7 @@
 """The order in which CTA pairs take their tiles (equal groups of at most eight row tiles, column by column inside a group)
 and the 256-column tiles of the re-packing epilogues."""
 
+import numpy as np
 import pytest
 import torch
 
@@ -51,6 +52,47 @@ def test_one_and_two_row_tiles_of_the_repacking_gemm(m, n):
     want_q, want_sf = P4.pack_swiglu_nvfp4(plain, inter, interleaved=True)
     got_q, got_sf = P4.linear_swiglu_packed_gemm(qa, sfa, None, qi, sfi, None, k)
     assert torch.equal(got_q, want_q) and torch.equal(got_sf, want_sf)
+
+
+@pytest.mark.parametrize("m,n,k", [(600, 8192, 256), (600, 8192, 1024), (816, 4096, 2048), (1300, 4096, 256), (1300, 8192, 512)])
+def test_repacking_tile_widths_by_the_longer_of_loop_and_epilogue(m, n, k):
+    """Either side of the rule: short loops in tiles of 128 columns, long ones of 256, for the three epilogues."""
+    from rk_b200 import fp4_linear as P4
+    from rk_b200 import fp8_linear as P8
+    from rk_b200 import mxfp8_swiglu as MS
+    from rk_b200.cute_mxfp8_swiglu import cutlass_swiglu_mxfp8_packed
+
+    inter = n // 2
+    gen = torch.Generator(device=DEVICE).manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=gen, device=DEVICE).bfloat16()
+    w = (torch.randn(n, k, generator=gen, device=DEVICE) * 0.05).bfloat16()
+    wi = P4.interleave_gate_up_rows(w, inter)
+    qa, sfa = P4.pack_nvfp4(x)
+    qi, sfi = P4.pack_nvfp4(wi)
+    plain = P4.linear_forward_packed_gemm_bf16(qa, sfa, None, qi, sfi, None, None, k)
+    want_q, want_sf = P4.pack_swiglu_nvfp4(plain, inter, interleaved=True)
+    got_q, got_sf = P4.linear_swiglu_packed_gemm(qa, sfa, None, qi, sfi, None, k)
+    assert torch.equal(got_q, want_q) and torch.equal(got_sf, want_sf)
+    # the activation by table, and its scale
+    table = MS.make_bf16_silu_table(DEVICE)
+    blocks = plain.view(m, inter // 64, 2, 64)  # 64 up, 64 gate
+    up, gate = (blocks[:, :, i].reshape(m, inter) for i in (0, 1))
+    want = (table.view(-1)[gate.contiguous().view(torch.int16).to(torch.int32) & 0xFFFF].float() * up.float()).bfloat16()
+    out, scale = torch.empty_like(want), torch.zeros(1, device=DEVICE)
+    ws = _lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)
+    P = _lib.ptr
+    code = _lib.load().rk_gemm_nvfp4_gated_act(P(qa), P(sfa), None, P(qi), P(sfi), None, P(table), 448.0, P(out), P(scale), m, n, k, 0,
+                                               P(ws), ws.numel(), _lib.stream_ptr(DEVICE))
+    _lib.check(code, "rk_gemm_nvfp4_gated_act")
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    assert scale.item() == np.float32(want.float().abs().max().item()) / np.float32(448.0)  # the IEEE quotient
+    a, sa = P8.mxfp8_pack(x)
+    b, sb = P8.mxfp8_pack(w)
+    bi, sbi = P8.mxfp8_pack(wi)
+    want_q, want_sf = MS.silu_mul_pack_mxfp8(P8.mxfp8_linear(a, sa, b, sb), inter, table)
+    q, sf = cutlass_swiglu_mxfp8_packed(a, sa, bi, sbi, table)
+    assert torch.equal(q.view(torch.uint8), want_q.view(torch.uint8)) and torch.equal(sf, want_sf)
+    assert _lib.read_status(ws) == 0
 
 
 @pytest.mark.parametrize("m,n", [(1300, 4992), (816, 16512), (2100, 4992)])
