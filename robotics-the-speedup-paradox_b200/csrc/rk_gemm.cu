@@ -567,17 +567,20 @@ int launch_tc2_kernel(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CU
   return RK_OK;
 }
 
-// The order of the pair tiles (see pair_tile): rows of tiles where all run at once, columns in a single group of at most eight row
-// tiles, both with a multiplication in place of the division; else equal groups of at most eight row tiles.
-void set_pair_order(Gemm2Params* p) {
+// The order of the pair tiles (see pair_tile): row tiles outermost where all run at once, and for weights of at most 4 MB where there
+// is more than one group or the epilogue re-packs (6000 x 512 x 256 MXFP8 5.7 -> 5.4 us, 3264 x 2048 x 2048 14.2 -> 13.8, NVFP4 with the
+// activation table 1300 x 8192 x 512 14.7 -> 14.3); columns outermost in a single group of at most eight row tiles, both with a
+// multiplication in place of the division; else equal groups of at most eight row tiles.
+void set_pair_order(Gemm2Params* p, int64_t weight_bytes, bool repack) {
   const int groups = (p->tiles_m + 7) / 8;
   p->group_m = (p->tiles_m + groups - 1) / groups;
-  const bool one_wave = static_cast<long long>(p->tiles_m) * p->tiles_n <= kNumSms / 2;
-  p->order = one_wave && p->tiles_n > 1 ? PAIRS_COLUMNS_FIRST : groups == 1 ? PAIRS_ROWS_FIRST : PAIRS_GROUPS;
+  const int64_t tiles = static_cast<int64_t>(p->tiles_m) * p->tiles_n;
+  const bool rows_outermost = tiles <= kNumSms / 2 || ((groups > 1 || repack) && weight_bytes <= (4 << 20) && tiles * p->tiles_n < (1ll << 32));
+  p->order = rows_outermost && p->tiles_n > 1 ? PAIRS_COLUMNS_FIRST : groups == 1 ? PAIRS_ROWS_FIRST : PAIRS_GROUPS;
   if (p->order == PAIRS_GROUPS) return;
   p->minor = p->order == PAIRS_COLUMNS_FIRST ? p->tiles_n : p->tiles_m;
-  // exact while tiles * minor < 2^32: 74 * 74 and 8 * 2^17 * 8 at most.  A single row tile has no such factor for its minor of one:
-  // the columns run alone then, and a factor of zero gives row zero.
+  // exact while tiles * minor < 2^32: at most 74 * 74, as tested, or 8 * 2^17 * 8.  A single row tile has no such factor for its
+  // minor of one: the columns run alone then, and a factor of zero gives row zero.
   if (p->minor == 1) p->order = PAIRS_COLUMNS_FIRST, p->minor = p->tiles_n;
   p->minor_magic = p->tiles_m > 1 ? static_cast<unsigned>(((1ull << 32) + p->minor - 1) / p->minor) : 0u;
 }
@@ -752,7 +755,7 @@ int run_tc(const TcArgs& a) {
     p2.issue_block = issue_block_mode();
     p2.tiles_m = static_cast<int>((a.m + 255) / 256);
     p2.tiles_n = static_cast<int>((a.n + p2.bn - 1) / p2.bn);
-    set_pair_order(&p2);
+    set_pair_order(&p2, a.n * a.k_bytes, a.swiglu_q != nullptr);
     const int stage = gemm2_stage_bytes(a.kind, p2.bn, p2.sfb_blocks);
     p2.out_bufs = 2;
     p2.stages = (kSmemBudget - kVecBytes - 2 * kOutBufBytes) / stage;

@@ -32,7 +32,9 @@ def test_every_tile_of_every_group_is_computed_once(m, n, k):
     (1025, 128, 128),    # one column of five tiles
     (2048, 9480, 128),   # eight row tiles, more tiles than pairs: columns outermost
     (1281, 16392, 128),  # six: a factor that does not divide 2^32
-    (20000, 136, 128),   # 79 row tiles: groups
+    (20000, 136, 128),   # 79 row tiles, weights of a few KB: row tiles outermost
+    (2304, 8200, 640),   # nine row tiles, weights above 4 MB: groups of five and four
+    (2304, 8200, 384),   # below: row tiles outermost
 ])
 def test_every_tile_of_every_order_is_computed_once(m, n, k):
     test_every_tile_of_every_group_is_computed_once(m, n, k)
