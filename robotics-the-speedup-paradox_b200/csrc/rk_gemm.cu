@@ -1832,8 +1832,12 @@ extern "C" int rk_attention_prefix(const void* q, const void* k_cache, const voi
   // Half-filled tiles where the launch leaves most of the machine idle: 64 rows or fewer keep two of the four lane quadrants
   // out of the softmax and halve the exchanged outputs (50 tokens, 613 keys, one environment: 11.4 us with 100 rows, 9.7 with
   // 50; two: 11.6 and 10.1; at 128 CTAs, four environments, 12.1 and 12.0, with 866 keys 13.2 and 14.5).
+  // Their key slices, more than four where 1024 keys do not hold, have to run at once (two environments, 1500 keys: 16 clusters of eight
+  // take two waves, 16.7 -> 22.1 us).
+  int slices = 4;
+  while (slices < 8 && (kv_len + slices - 1) / slices > 256) slices *= 2;
   for (int g = group - 1; g >= 1 && group * tokens > 64; --g)
-    if (per_kv % g == 0 && heads / g * batch * 4 <= 96) group = g;
+    if (per_kv % g == 0 && heads / g * batch * slices <= 96 && heads / g * batch <= max_clusters(slices)) group = g;
   const int tiles = static_cast<int>(heads / group);
   // Key slices: a power of two, as many as all run at once, at most 256 keys each.  Four are enough for 768 keys: eight
   // shorten the passes over a row less than their exchange costs (50 tokens, 613 keys, one environment: 9.7 us in four, 10.2

@@ -175,6 +175,14 @@ def test_attention_at_the_edges_of_its_forms(batch, tokens, prefix, scaling):
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < TOL
 
 
+@pytest.mark.parametrize("case", [
+    (1, 50, 8, 1, 1450), (2, 50, 8, 1, 1450),  # eight slices: half-filled tiles only where their clusters run at once
+    (8, 10, 8, 1, 1490), (2, 64, 8, 1, 1984),
+])
+def test_slices_by_keys_and_clusters(case):
+    test_attention_matches_the_eager_oracle(case)
+
+
 @pytest.mark.parametrize("prefix,chunk", [(1, 50), (64, 50), (70, 3), (127, 1), (128, 8), (563, 50)])
 def test_prefix_fill_copies_and_transposes(prefix, chunk):
     """Whole and ragged tiles of 64 rows, a pitch that ends inside or beyond the last tile; nothing else is written."""
