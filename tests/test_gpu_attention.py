@@ -178,6 +178,8 @@ def test_attention_at_the_edges_of_its_forms(batch, tokens, prefix, scaling):
 @pytest.mark.parametrize("case", [
     (1, 50, 8, 1, 1450), (2, 50, 8, 1, 1450),  # eight slices: half-filled tiles only where their clusters run at once
     (8, 10, 8, 1, 1490), (2, 64, 8, 1, 1984),
+    (8, 50, 8, 1, 206), (4, 50, 8, 1, 14), (8, 64, 8, 1, 1),  # two slices in place of four short ones
+    (1, 50, 8, 1, 206), (3, 100, 8, 1, 156), (16, 10, 8, 1, 246),
 ])
 def test_slices_by_keys_and_clusters(case):
     test_attention_matches_the_eager_oracle(case)
