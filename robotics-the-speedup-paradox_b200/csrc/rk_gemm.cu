@@ -1647,7 +1647,7 @@ extern "C" int rk_gemm_w4a16_g128(const void* x, const void* q, const void* scal
   // fragment, which large weights repay only in the tensor-memory kernels.  Against those, 16384 x 2048 with 1 / 8 / 16 rows
   // 7.1 / 8.0 / 10.4 us and 9.1 / 9.1 / 9.1; 4096 x 4096 4.7 / 6.1 / 6.8 and 7.6 / 7.8 / 8.0; 1024 x 1024 2.1 / 2.4 / 3.0 and 5.4;
   // 17 to 24 rows would gain 0.9 us at 4096 x 2048 and lose 3 at 16384 x 2048.  Any tactic bit keeps the other kernels.
-  const bool few_rows = m <= 8 || (m <= 16 && n * k <= (1 << 24));
+  const bool few_rows = m <= 8 || (m <= 16 && k > 128 && n * k <= (1 << 24));  // one group: 16 x 1024 x 128 2.9 us there, 4.0 here
   if (few_rows && tactic == 0 && aligned16(x) && aligned16(q) && aligned16(out)) {
     GemvParams g{};
     g.q = static_cast<const uint8_t*>(q);
