@@ -1576,15 +1576,23 @@ int w4_scale_rows(int pairs, int splits) { return 2 * ((pairs + splits - 1) / sp
 // Activation batches above 64 rows: scale folded into the expanded weights, one accumulator for all of K.
 int run_w4_fold(const void* x, const void* q, const void* scales, W4Params p, int64_t m, int64_t n, int64_t k,
                 int tactic, cudaStream_t st, const char* who) {
-  const int bn = m > 128 ? 256 : 128;
   const int tiles_n = static_cast<int>((n + 127) / 128);
+  const int pairs = (p.groups + 1) / 2;
+  // Tiles of 128 activation rows, and of 256 above 128 rows unless the narrow ones all run at once with at most eight group pairs
+  // for a CTA: sixteen expansion warps made short loops of wide tiles slower (us with wide tiles before them, wide, narrow: 129 x
+  // 1024 x 1024 8.8, 9.2, 7.8; 256 x 2048 x 2048 10.6, 11.3, 9.5; 512 x 4096 x 512 7.5, 7.9, 6.4; 256 x 2048 x 8192 17.3, 17.5, 15.2;
+  // 200 x 4096 x 4096 13.4, 14.1, 14.1; beyond eight 257 x 2048 x 8192 19.4, 18.8, 21.0, and in two waves 512 x 8192 x 1152 11.0, 11.3,
+  // 17.3; up to 192 rows also beyond four in clusters of two, 129 x 4096 x 4096 12.3, 12.8, 13.9).  Tactic bit 3 asks for pairs of
+  // 256-row tiles.
+  const int tiles128 = tiles_n * static_cast<int>((m + 127) / 128), splits128 = w4_splits(tiles128, pairs);
+  const int most = m <= 192 && splits128 == 2 ? 4 : 8;
+  const int bn = m > 128 && ((tactic & 8) || tiles128 > kNumSms || (pairs + splits128 - 1) / splits128 > most) ? 256 : 128;
   const int tiles_m = static_cast<int>((m + bn - 1) / bn);
   // tactic bit 3: 256-row tiles on CTA pairs (each CTA stages half of the activation tile), when
   // the channel tiles pair up
   const bool pair = bn == 256 && tiles_n % 2 == 0 && (tactic & 8);
   const int x_bytes = pair ? kW4f2XBytes : bn * 128;
   const int slots = pair ? kW4f2Slots : w4f_slots(bn);
-  const int pairs = (p.groups + 1) / 2;
   p.splits = pair ? 1 : w4_splits(tiles_n * tiles_m, pairs);
   p.scale_rows = pair ? p.groups : w4_scale_rows(pairs, p.splits);
   const int copies = (pairs + p.splits - 1) / p.splits;

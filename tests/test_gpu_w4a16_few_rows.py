@@ -71,3 +71,26 @@ def test_rows_do_not_reach_each_other():
     same = [0, 1, 2, 5, 6, 7]
     assert torch.equal(got[same], clean[same]) and (got[4] == 0).all()
     assert not torch.isfinite(got[3]).any() and torch.isnan(got[8]).all()
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (129, 1000, 128),    # narrow tiles: two row tiles, the last of one row, one group
+    (256, 2048, 2048),   # narrow, eight CTAs to a tile
+    (257, 2568, 640),    # three row tiles, an odd group at the end
+    (384, 4736, 256),    # 111 narrow tiles
+    (1000, 2368, 128),   # 152: wide ones
+    (160, 4096, 4096),   # eight group pairs to a CTA, the most
+    (300, 2048, 8192),   # eleven: wide
+])
+def test_row_tiles_above_128_rows_match_the_folded_product(m, n, k):
+    """The scale folded into bf16 weights, then products and sums in 64 bits; bounds as above."""
+    gen = torch.Generator(device=DEVICE).manual_seed(n + k + m)
+    r = lambda *s: torch.randn(s, generator=gen, device=DEVICE)
+    packed, scales = pack_weight((r(n, k) * 0.02).bfloat16())
+    x, bias = r(m, k).bfloat16(), (r(n) * 0.1).bfloat16()
+    eye, _ = reference(torch.eye(k, device=DEVICE), packed, torch.ones_like(scales), None)  # [k, n] integers
+    w = (eye.bfloat16() * scales.repeat_interleave(128, 0)).double()
+    want, magnitude = x.double() @ w + bias.double(), x.double().abs() @ w.abs()
+    got = linear_w4a16(x, packed, scales, bias)
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + k * 2.0 ** -23 * magnitude).all()
+    assert _lib.read_status(_lib.workspace(DEVICE, _lib.WORKSPACE_HEADER)) == 0
