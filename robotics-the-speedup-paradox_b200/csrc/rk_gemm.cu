@@ -873,8 +873,6 @@ int run_tc(const TcArgs& a) {
   p.tmem_cols = pl.tmem_cols;
   p.acc_stride = pl.acc_stride;
   p.acc_bufs = pl.acc_bufs;
-  p.dual = pl.dual;
-  p.a_rows = static_cast<int>(box_act);
   p.out_bufs = pl.out_bufs;
   p.tiles_a = pl.tiles_a;
   p.tiles_b = pl.tiles_b;
@@ -886,12 +884,14 @@ int run_tc(const TcArgs& a) {
   p.acc_out = a.acc_out;
   p.sf_act = a.sf_act;
   p.sf_wgt = a.sf_wgt;
-  p.sf_kt = a.sf_kt;
+  if (pl.few) p.a_rows = static_cast<int>(box_act);
+  else p.sf_kt = a.sf_kt;
   p.sfb_blocks = pl.sfb_blocks;
   p.sf_rows_b = static_cast<int>(pl.swap ? a.m : a.n);
   p.wait_limit = g_debug_wait_limit > 0 ? g_debug_wait_limit : static_cast<int>(kWaitSpinMax);
   p.debug_stall = g_debug_stall;
-  p.issue_block = (issue_block_mode() && pl.sfb_blocks <= 2) ? 1 : 0;
+  if (a.kind == KIND_I8) p.dual = pl.dual;
+  else p.issue_block = (issue_block_mode() && pl.sfb_blocks <= 2) ? 1 : 0;
   const int fmt_wgt = a.wgt_u4 ? FMT_E2M1_IN_F8 : FMT_E4M3;
   p.fmt_a = pl.swap ? fmt_wgt : FMT_E4M3;
   p.fmt_b = pl.swap ? FMT_E4M3 : fmt_wgt;

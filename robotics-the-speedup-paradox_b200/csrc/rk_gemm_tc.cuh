@@ -81,12 +81,20 @@ struct GemmParams {
   int* acc_out;               // optional raw accumulators [m, n] (s32 or f32 bits), written instead of `out`
   const uint8_t* sf_act;      // block-scaled: swizzled scale-factor buffers
   const uint8_t* sf_wgt;
-  int sf_kt;                  // 512-byte scale chunks per 128-row block along K
+  union {
+    int sf_kt;                // kinds with block scales: 512-byte scale chunks per 128-row block along K
+    int a_rows;               // SCHED_FEW: activation rows of a tile (a multiple of 8; the MMA's other rows are whatever lies behind)
+  };
   int sfb_blocks;             // 128-row scale blocks fetched per B-role tile (1..3; a tile may straddle blocks)
   int sf_rows_b;              // rows of the B-role operand (its scale buffer holds ceil(rows / 128) blocks)
   int wait_limit;             // spin limit of every bounded wait (kWaitSpinMax unless a test shortens it)
   int debug_stall;            // test aid: the producer announces bytes that never arrive (first stage)
-  int issue_block;            // issue a stage's tensor-core instructions as one straight-line block
+  union {                     // fields of one kind share a place: in front they moved the others (block-scaled launches +0.13 us), at
+                              // the end they were a line of constants of their own (W8A8 launches of few rows +0.06 us)
+    int issue_block;          // block-scaled: issue a stage's tensor-core instructions as one straight-line block
+    int dual;                 // KIND_I8, one tile per CTA: two warps issue alternate K blocks, each into an accumulator buffer of its
+                              // own; `stages` is even if the ring wraps, so that a stage is always the same warp's
+  };
   int fmt_a, fmt_b;           // KIND_MXF8: element formats of the A- and B-role operands (e4m3, or e2m1 for 4-bit
                               // weights that TMA expands to the 16-byte-padded layout of kind::mxf8f6f4)
   int tx_deficit;             // bytes per stage that the copies report short of the shared-memory bytes written
@@ -112,10 +120,6 @@ struct GemmParams {
   int* peer_epoch;               // this rank's call counter (device memory): the launch that finishes call e writes e
   unsigned* peer_counter;        // device word counting the CTAs of this launch that have finished
   int* status;                // device status word
-  // last, since moving the fields above cost the block-scaled kinds 0.13 us a launch (MXFP8 64 x 2048 x 2048 6.99 -> 7.13):
-  int dual;    // KIND_I8, one tile per CTA: two warps issue alternate K blocks, each into an accumulator buffer of its own;
-               // `stages` is even if the ring wraps, so that a stage is always the same warp's
-  int a_rows;  // SCHED_FEW: activation rows of a tile (a multiple of 8; the MMA's other rows are whatever lies behind them)
 };
 
 template <int KIND>
