@@ -4,6 +4,7 @@
     python robotics-the-speedup-paradox_b200/rk_b200/microbench.py [w4a16] [w8a8] [fp8] [mxfp8] [nvfp4] [quant]
     python robotics-the-speedup-paradox_b200/rk_b200/microbench.py w8a8:400x8192x1024 quant:16384x2048   # explicit shapes
     python robotics-the-speedup-paradox_b200/rk_b200/microbench.py layer    # per-kernel device time of one expert layer
+    python robotics-the-speedup-paradox_b200/rk_b200/microbench.py chunk    # the expert's action chunk as it runs, kernel by kernel
     python robotics-the-speedup-paradox_b200/rk_b200/microbench.py prefix_layer   # the same for one NVFP4 prefix layer
 
 Each shape is timed as a CUDA graph of back-to-back launches that rotate through enough independent
@@ -265,6 +266,59 @@ def layer_breakdown(envs=8, prefix=816, repeats=5):
         GemmaAttention.fused_attention = False
 
 
+def chunk_chain(envs, prefix):
+    """What each kernel adds to the chain of one action chunk (W8A8, every option of the benchmark's loop, one CUDA graph): the
+    microseconds by which a kernel's end follows its predecessor's, by position in a layer, mean over layers and steps of one
+    replay under the torch profiler.  Launches overlap (programmatic dependents), so these are not the kernels' own times."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from rk_b200.gemma_stack import ActionExpert, GemmaAttention, expert_scope, fuse_norm_quantize
+    from rk_b200.graph import CudaGraphCall
+    from rk_b200.optimizations import quantize_linears
+
+    dev = torch.device("cuda:0")
+    expert = ActionExpert().init_random(0).to(dev).eval()
+    cfg, gen = expert.cfg, torch.Generator().manual_seed(7)
+    expert.enable_condition_caches()
+    noise = torch.randn(envs, expert.chunk, expert.action_dim, generator=gen).to(dev)
+    cache = (cfg.depth, envs, cfg.num_kv_heads, prefix, cfg.head_dim)
+    pk, pv = (torch.randn(cache, generator=gen).to(torch.bfloat16).to(dev) for _ in range(2))
+    GemmaAttention.fused_rope = GemmaAttention.fused_attention = True
+    try:
+        with torch.no_grad(), quantize_linears(expert, "int8", scopes=("expert",), selector=expert_scope, shared_quant=True,
+                                               grouped=True, group_views=True):
+            fuse_norm_quantize(expert.stack)
+            call = CudaGraphCall(lambda n, k, v: expert(n, k, v), retained_tensors=expert.retained_tensors)
+            for _ in range(5):
+                call(noise, pk, pv)
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(10):
+                call(noise, pk, pv)
+            end.record()
+            torch.cuda.synchronize()
+            chunk_ms = begin.elapsed_time(end) / 10
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                call(noise, pk, pv)
+                torch.cuda.synchronize()
+    finally:
+        GemmaAttention.fused_rope = GemmaAttention.fused_attention = False
+    events = sorted((e.time_range.end, e.name) for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA)
+    tails = [i for i, (_, name) in enumerate(events) if "flow_step_tail" in name]
+    sums, counts, names = {}, {}, {}
+    for first, last in zip(tails, tails[1:]):  # whole steps: what the step itself launches, its layers, the next tail
+        own, per_layer = (last - first - 1) % cfg.depth, (last - first - 1) // cfg.depth
+        for i in range(first + 1, last + 1):
+            n = i - first - 1
+            at = n if n < own else own + per_layer if i == last else own + (n - own) % per_layer
+            names[at] = events[i][1]
+            sums[at] = sums.get(at, 0.0) + events[i][0] - events[i - 1][0]
+            counts[at] = counts.get(at, 0) + 1
+    print(f"--- chunk of {envs} x {expert.chunk} tokens, prefix {prefix}: {chunk_ms:.2f} ms (without the profiler)")
+    for at in sorted(names):
+        print(f"{sums[at] / counts[at]:8.1f} us  x{counts[at]:4d}  {names[at][:120]}")
+
+
 def prefix_layer_breakdown(tokens=816, depth=2, repeats=5):
     """Per-kernel device time of one layer of the cfg4 prefix stack (Gemma-2B widths, every linear NVFP4
     with the fp32 per-tensor scale, shared packs): tensor-op elementwise work against the fused form
@@ -334,6 +388,10 @@ def main(argv):
     which = [a for a in which if ":" not in a]
     if "layer" in which:
         layer_breakdown()
+        return
+    if "chunk" in which:
+        for envs, prefix in ((1, 563), (8, 816)):
+            chunk_chain(envs, prefix)
         return
     if "prefix_layer" in which:
         prefix_layer_breakdown()
