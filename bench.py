@@ -64,7 +64,7 @@ def algorithmic_bytes(m):
 # DRAM bytes (read + write) of one cfg2 launch as ncu measured them (dram__bytes_read.sum +
 # dram__bytes_write.sum; the outputs stay in L2, so writes were zero).  From the capture summarised
 # in profiles/w4a16_cfg2_kernel_metrics.md; not re-measured by this program.
-NCU_DRAM_TRAFFIC = {1: 17330432, 8: 17373952, 50: 17549312, 256: 18384896}
+NCU_DRAM_TRAFFIC = {1: 17338368, 8: 17367296, 50: 17549568, 256: 18390016}
 
 
 def algorithmic_ops(m):
@@ -1261,7 +1261,7 @@ def main():
         small = [m for m in M_LIST if m <= 64]
         t_small = sum(per_m_ms[m] for m in small) * 1e-3
         roofline = {
-            "kernel": f"{'rk_gemm_w4a16_fold_kernel' if dominant > 64 else 'rk_gemm_w4a16_kernel'} (M={dominant})",
+            "kernel": f"{'rk_gemm_w4a16_fold_kernel' if dominant > 64 else 'rk_gemm_w4a16_kernel' if dominant > 8 else 'rk_gemv_w4a16_kernel'} (M={dominant})",
             "bound": "hbm" if hbm_bound else "tensor",
             "achieved": d["gbs"] if hbm_bound else d["tops"],
             "peak": peaks["hbm_gbs"] if hbm_bound else peaks["bf16_tflops"],
