@@ -29,7 +29,7 @@
 // (clock cycles of one CTA, 50 rows, 613 keys in four slices: scores complete 2900, exponentials 5500, statistics exchanged
 // 6000, output accumulated 10100, received 12200, stored 14100).  Measured before -> after: scores kept in
 // registers, two at a time through packed conversions, statistics written to every peer, outputs by bulk copies: one
-// environment, 613 keys 13.0 -> 11.4 us (9.7 with tiles of 50 rows); eight, 866 keys 17.2 -> 15.8.  Fetching the outputs 16
+// environment, 613 keys 13.0 -> 11.4 us (9.3 with tiles of 50 rows); eight, 866 keys 17.2 -> 15.8.  Fetching the outputs 16
 // bytes per thread from the peers took 5000 of 24000 cycles, the packed conversions 2400.
 //
 // Warp roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2..9 =

@@ -1838,7 +1838,7 @@ extern "C" int rk_attention_prefix(const void* q, const void* k_cache, const voi
       break;
     }
   // Half-filled tiles where the launch leaves most of the machine idle: 64 rows or fewer keep two of the four lane quadrants
-  // out of the softmax and halve the exchanged outputs (50 tokens, 613 keys, one environment: 11.4 us with 100 rows, 9.7 with
+  // out of the softmax and halve the exchanged outputs (50 tokens, 613 keys, one environment: 11.4 us with 100 rows, 9.3 with
   // 50; two: 11.6 and 10.1; at 128 CTAs, four environments, 12.1 and 12.0, with 866 keys 13.2 and 14.5).
   // Their key slices (of at most 256 keys) have to run at once (two environments, 1500 keys: 16 clusters of eight
   // take two waves, 16.7 -> 22.1 us).
@@ -1847,7 +1847,7 @@ extern "C" int rk_attention_prefix(const void* q, const void* k_cache, const voi
     if (per_kv % g == 0 && heads / g * batch * needed <= 96 && heads / g * batch <= max_clusters(needed)) group = g;
   const int tiles = static_cast<int>(heads / group);
   // Key slices: a power of two, as many as all run at once, at most 256 keys each.  Four are enough for 768 keys: eight
-  // shorten the passes over a row less than their exchange costs (50 tokens, 613 keys, one environment: 9.7 us in four, 10.2
+  // shorten the passes over a row less than their exchange costs (50 tokens, 613 keys, one environment: 9.3 us in four, 10.2
   // in eight; 866 keys: 11.6 and 10.7).  Four of fewer than 128 keys only for 64 CTAs or fewer: eight environments, 256 keys, 11.0 us in
   // two and 12.0 in four, one environment 8.9 and 7.9.
   const int most = kv_len > 768 ? 8 : 4;

@@ -1,6 +1,6 @@
 // Native form of the two linears that are called eagerly, one at a time: `W4A16Linear.forward` and `IntegerLinear.forward`
 // (W8A8).  Such a call is bound by the host: through ctypes and tensor methods, the two launches of a 64 x 2048 x 2048 W8A8
-// linear took 50 us around 9 us on the device, the one launch of a W4A16 row 26 us around 8 us.
+// linear took 50 us around 6 us on the device, the one launch of a W4A16 row 26 us around 7 us.
 //
 // A call here takes the plain case only - exact CUDA tensors, contiguous rows, a workspace that exists, no dispatch mode - and
 // answers None for everything else, errors included: the caller then goes its general way in Python, which repeats the
